@@ -25,6 +25,7 @@
 
 #include <mutex>
 
+#include "cn3d_poly.cuh"
 #include "cnn_internal.cuh"
 #include "fft.cuh"
 #include "tp_common.cuh"
@@ -1961,6 +1962,65 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
   q.ke = w.de;
   q.ks = w.ds;
   q.kn = w.dn;
+
+#ifndef TP_C128_CHECK
+  // Plain marches whose operator is a small perturbation of the identity (the
+  // paraxial sampling) solve each slice by a fixed polynomial, one kernel per
+  // step (cn3d_poly.cu); training pairs, step-by-step launches, a capturing
+  // stream, REVERSE, other kernel choices and tolerances under complex64
+  // round-off keep the Krylov march below.
+  cudaStreamCaptureStatus poly_cap = cudaStreamCaptureStatusNone;
+  TP_CHECK_CUDA(cudaStreamIsCapturing(st, &poly_cap));
+  if (a->precond == 1 && a->kernels == 0 && a->launch == 0 && a->host_check != 0 && a->train_every <= 0 &&
+      a->mode != TP_MODE_REVERSE && poly_cap == cudaStreamCaptureStatusNone && q.mu_x.x == 0.0 && q.mu_y.x == 0.0) {
+    c3_diag_kernel<<<296, 256, 0, st>>>(N, nf, q.sigma, q.conj_t, static_cast<const cx *>(op->kc),
+                                        static_cast<const cx *>(op->kw), static_cast<const cx *>(op->ke),
+                                        static_cast<const cx *>(op->ks), static_cast<const cx *>(op->kn), w.dc, w.dw,
+                                        w.de, w.ds, w.dn);
+    C3PolyJob job{};
+    job.nf = nf;
+    job.nb = nb;
+    job.nz = nz;
+    job.P = P;
+    job.mode = a->mode;
+    job.exact = q.exact;
+    job.is_delta = q.is_delta;
+    job.dtype = q.dtype;
+    job.conj_t = q.conj_t;
+    job.sigma = q.sigma;
+    job.k = q.k;
+    job.dz = q.dz;
+    job.tol = a->tol > 0 ? a->tol : 1e-6;
+    job.max_iter = a->max_iter > 0 ? a->max_iter : 20;
+    job.mu_x = q.mu_x.y;
+    job.mu_y = q.mu_y.y;
+    job.field = n_field;
+    job.kc = w.dc;
+    job.kw = w.dw;
+    job.ke = w.de;
+    job.ks = w.ds;
+    job.kn = w.dn;
+    job.vec[0] = w.u;
+    job.vec[1] = w.x;
+    job.vstride = (size_t)(reinterpret_cast<char *>(w.x) - reinterpret_cast<char *>(w.u));
+    job.scratch = reinterpret_cast<char *>(w.r);
+    job.scratch_bytes = (size_t)(reinterpret_cast<char *>(w.cdl) - reinterpret_cast<char *>(w.r));
+    job.colw = reinterpret_cast<float2 *>(w.twf);
+    job.roww = reinterpret_cast<float4 *>(w.ab);
+    job.check = reinterpret_cast<int *>(w.st);
+    job.probes = static_cast<const cx *>(a->probes);
+    job.src_exit = static_cast<const cx *>(a->src_exit);
+    job.src_shared = static_cast<const cx *>(a->src_shared);
+    job.u_fwd = static_cast<const cx *>(a->u_fwd);
+    job.u_store = static_cast<cx *>(a->u_store);
+    job.exit_out = static_cast<cx *>(a->exit_out);
+    job.grad_c = static_cast<cx *>(a->grad_c);
+    job.stats = a->stats;
+    int ran = 0;
+    const int prc = c3_poly_march(job, st, &ran);
+    if (prc != TP_OK || ran) return prc;
+  }
+#endif
 
   const FftPlan pf = make_fft_plan(nf), pb = make_fft_plan(nb);
   const int fft_on = a->precond != 0 && pf.npass > 0 && pb.npass > 0;

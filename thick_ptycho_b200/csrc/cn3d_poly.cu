@@ -1,0 +1,730 @@
+// 3D Crank-Nicolson march with each slice solved by a fixed polynomial of its
+// scaled off-diagonal part, one kernel per step.
+//
+// A step solves (I - P_s) d = b, P_s = sigma*T(K + diag c_s), b = (P_r + P_s) u
+// + src, u_new = u + d (the delta form of cn3d.cu).  With D = I - diag(P_s) and
+// J = D^{-1} offdiag(P_s) the system is (I - J) d = D^{-1} b = g.  The off-
+// diagonals of K are purely imaginary (mu = i dz / (4 k dx^2)), so the spectrum
+// of J lies close to a segment [-i tau, i tau] of the imaginary axis with
+// tau = max row sum of |J|, and the Chebyshev residual polynomial of that
+// segment gives d = p_m(J) g, p_m(z) = (1 - q_m(z)) / (1 - z), q_m(z) =
+// T_m(z / (i tau)) / T_m(1 / (i tau)): the error falls by ~(tau / 2)^m.  At the
+// paraxial sampling this path is used at (tau ~ 0.08 at wavelength 0.5 with
+// unit steps) m = 6 reaches 2e-8, against ~1.15 FFT-preconditioned BiCGStab
+// iterations per solve: 11 kernels and 34 passes over the probes' vectors per
+// step become one kernel that reads u once and writes it once.
+//
+// One CTA owns a tile of 64 x 64 pixels (8 warps of 8 rows, two adjacent columns
+// per lane) of one image for a group of probes; D^{-1} of its 16 pixels stays
+// in a thread's registers for all of them, and so do g and the Horner
+// recurrence y <- a_k g + J y, whose neighbours come from the lane's own
+// registers (the other column, the rows above and below), warp shuffles (left
+// and right) and, at the warp's first and last row, shared memory.  A tile
+// computes a core smaller than itself: the value of a pixel j rows inside the
+// core's edge depends on what is h rows outside it only through mu^h, so a halo
+// of h = 1 + log(1e-8) / log(mu) pixels (6 at mu = 0.02) gives the core to
+// below complex64 round-off, whatever m.  The tiles of u arrive by tiled tensor
+// copies (zero outside the image), double-buffered over the group's probes.
+// Each solve is judged by its true residual, as in the Krylov march.
+#include <cuda.h>
+#include <math.h>
+#include <string.h>
+
+#include <complex>
+#include <mutex>
+
+#include "cn3d_poly.cuh"
+#include "tp_errors.h"
+#include "tpcuda.h"
+
+#ifndef TP_C128_CHECK
+namespace tp {
+
+namespace {
+
+constexpr int kPW = 64, kPR = 8, kPWarps = 8, kPH = kPR * kPWarps;  // tile width, rows per warp, warps, tile height
+constexpr int kPThreads = 32 * kPWarps;
+constexpr int kPolyMaxDeg = 10, kPolyMaxHalo = 16;
+
+struct PolyCheck {
+  unsigned tau, arg;  // bits of the largest row sum of |J| and the largest |arg D| (non-negative floats)
+  int bad, pad;
+};
+
+struct PolySlices {
+  const void *field;
+  int nf, nb, N, nz, L, dtype, is_delta, exact, conj_t;
+  double sigma, k, dz;
+  const float2 *kc, *kw, *ke, *ks, *kn;
+  const float2 *colw;
+  const float4 *roww;
+  float my;  // the row coupling away from the first and last two rows
+};
+
+__device__ __forceinline__ double2 poly_coef(const PolySlices &q, size_t idx) {
+  double2 v;
+  if (q.dtype == TP_C128) {
+    v = static_cast<const double2 *>(q.field)[idx];
+  } else {
+    const float2 w = static_cast<const float2 *>(q.field)[idx];
+    v = z2(w.x, w.y);
+  }
+  const double2 d = q.is_delta ? v : z2(v.x - 1.0, v.y);
+  if (!q.exact) return z2(q.k * d.y, -q.k * d.x);
+  const double2 w = zadd(zscale(d, 2.0), zmul(d, d));
+  return z2(0.5 * q.k * w.y, -0.5 * q.k * w.x);
+}
+
+// Column weights {west, east} and row weights {south, north, x factor}: the
+// imaginary couplings of sigma*T(K) as products of one-dimensional factors.
+__global__ void c3_poly_weights_kernel(const PolySlices q, float2 *colw, float4 *roww) {
+  const int br = q.nb / 2, fr = q.nf / 2;
+  for (int f = threadIdx.x; f < q.nf; f += blockDim.x) {
+    const int i = br * q.nf + f;
+    colw[f] = make_float2(f > 0 ? q.kw[i].y : 0.f, f + 1 < q.nf ? q.ke[i].y : 0.f);
+  }
+  const float2 w0 = q.kw[br * q.nf + fr];
+  for (int b = threadIdx.x; b < q.nb; b += blockDim.x) {
+    const int i = b * q.nf + fr;
+    const float2 w = q.kw[i];
+    roww[b] = make_float4(b > 0 ? q.ks[i].y : 0.f, b + 1 < q.nb ? q.kn[i].y : 0.f,
+                          (w.x == w0.x && w.y == w0.y) ? 1.f : 0.f, 0.f);
+  }
+}
+
+// Diagonals of slices s_lo .. s_hi (slice-major, from the node-major index
+// field, through a transposing tile), and over every slice of the call's range
+// the bounds of J; rows 0 of the grid also compare K's couplings with the
+// products of the weights.  Grid (ceil(N / 32), ceil(slices / 32)), block (32, 8).
+__global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q, int s_first, int s_last, int s_lo,
+                                                             int s_hi, float2 *cd, PolyCheck *chk) {
+  __shared__ float2 tile[32][33];
+  const int i0 = blockIdx.x * 32, s0 = s_first + blockIdx.y * 32;
+  float tau = 0.f, arg = 0.f;
+  int bad = 0;
+  for (int r = threadIdx.y; r < 32; r += 8) {
+    const int i = i0 + r, s = s0 + threadIdx.x;
+    if (i >= q.N || s > s_last) continue;
+    const size_t base = (size_t)i * q.nz;
+    const double2 c = zscale(zadd(poly_coef(q, base + s - 1), poly_coef(q, base + s)), 0.25 * q.dz);
+    const double2 v = zscale(q.conj_t ? zconj(c) : c, q.sigma);
+    const float2 kc = q.kc[i];
+    const float2 d = make_float2((float)(kc.x + v.x), (float)(kc.y + v.y));
+    tile[r][threadIdx.x] = d;
+    if (chk != nullptr) {
+      const int f = i % q.nf, b = i / q.nf;
+      const float2 cw = q.colw[f];
+      const float4 rw = q.roww[b];
+      const float sum = (fabsf(cw.x) + fabsf(cw.y)) * rw.z + fabsf(rw.x) + fabsf(rw.y);
+      if (sum > 0.f) {
+        const float dr = 1.f - d.x, di = -d.y;
+        const float t = sum / sqrtf(dr * dr + di * di);
+        if (!(t < 1e6f)) bad = 1;
+        tau = fmaxf(tau, t);
+        arg = fmaxf(arg, fabsf(atan2f(di, dr)));
+      } else {
+        const float dr = 1.f - d.x, n2 = dr * dr + d.y * d.y;
+        if (!(n2 > 1e-6f && n2 < 1e12f)) bad = 1;
+      }
+      if (blockIdx.y == 0 && threadIdx.x == 0) {
+        auto differs = [](float2 v2, float im) { return v2.x != 0.f || v2.y != im; };
+        if ((f > 0 && differs(q.kw[i], cw.x * rw.z)) || (f + 1 < q.nf && differs(q.ke[i], cw.y * rw.z)) ||
+            (b > 0 && differs(q.ks[i], rw.x)) || (b + 1 < q.nb && differs(q.kn[i], rw.y)))
+          bad = 1;
+        if (b > 1 && b < q.nb - 2 && (rw.x != q.my || rw.y != q.my || rw.z != 1.f)) bad = 1;
+      }
+    }
+  }
+  __syncthreads();
+  for (int r = threadIdx.y; r < 32; r += 8) {
+    const int s = s0 + r, i = i0 + threadIdx.x;
+    if (i < q.N && s >= s_lo && s <= s_hi) cd[(size_t)(s - s_lo) * q.N + i] = tile[threadIdx.x][r];
+  }
+  if (chk == nullptr) return;
+  for (int o = 16; o > 0; o >>= 1) {
+    tau = fmaxf(tau, __shfl_down_sync(0xffffffffu, tau, o));
+    arg = fmaxf(arg, __shfl_down_sync(0xffffffffu, arg, o));
+    bad |= __shfl_down_sync(0xffffffffu, bad, o);
+  }
+  if (threadIdx.x == 0) {
+    // most blocks do not raise the maxima: read before the atomic
+    const volatile PolyCheck *c = chk;
+    if (__float_as_uint(tau) > c->tau) atomicMax(&chk->tau, __float_as_uint(tau));
+    if (__float_as_uint(arg) > c->arg) atomicMax(&chk->arg, __float_as_uint(arg));
+    if (bad) atomicOr(&chk->bad, 1);
+  }
+}
+
+struct PolyStep {
+  int nf, nb, N, P, G;
+  int tiles_x, hx, hy, cw, ch;
+  int m;
+  float a[kPolyMaxDeg];
+  float my;  // interior row coupling
+  const float2 *cdl, *cdr;
+  const float2 *colw;
+  const float4 *roww;
+  const float2 *u;
+  float2 *un;
+  int sel;    // which state vector u is (tensor map coordinate)
+  int use_u;  // 0: the first step of the exact adjoint (zero state, source only)
+  const float2 *src_exit, *src_shared;
+  float2 *store;         // the step's slice of u_store, probe stride store_stride
+  size_t store_stride;
+  float2 *exit_out;
+  double2 *norms;  // per probe: ||b||^2, ||b - (I - P) d||^2
+};
+
+struct PolySmem {
+  float4 u[2][kPH][kPW / 2];
+  float4 dsum[kPH][kPW / 2];
+  float4 edge[2][kPWarps - 1][2][kPW / 2];  // row exchange between warps w and w + 1: w's last row, (w + 1)'s first
+  float4 roww[kPH];
+  float2 red[kPWarps];
+  uint64_t bar[2];
+};
+
+// Weighted neighbour sums of both columns of one row: S = sum of real weights
+// times neighbours (the couplings are i times the weights).
+template <bool EDGE>
+__device__ __forceinline__ float4 poly_sum(float4 cur, float4 prev, float4 next, float2 cw0, float2 cw1, float my,
+                                           float4 rw) {
+  const float wx = __shfl_up_sync(0xffffffffu, cur.z, 1), wy = __shfl_up_sync(0xffffffffu, cur.w, 1);
+  const float ex = __shfl_down_sync(0xffffffffu, cur.x, 1), ey = __shfl_down_sync(0xffffffffu, cur.y, 1);
+  float4 s;
+  s.x = fmaf(cw0.x, wx, cw0.y * cur.z);
+  s.y = fmaf(cw0.x, wy, cw0.y * cur.w);
+  s.z = fmaf(cw1.x, cur.x, cw1.y * ex);
+  s.w = fmaf(cw1.x, cur.y, cw1.y * ey);
+  if (EDGE) {
+    s.x = fmaf(rw.z, s.x, fmaf(rw.x, prev.x, rw.y * next.x));
+    s.y = fmaf(rw.z, s.y, fmaf(rw.x, prev.y, rw.y * next.y));
+    s.z = fmaf(rw.z, s.z, fmaf(rw.x, prev.z, rw.y * next.z));
+    s.w = fmaf(rw.z, s.w, fmaf(rw.x, prev.w, rw.y * next.w));
+  } else {
+    s.x = fmaf(my, prev.x + next.x, s.x);
+    s.y = fmaf(my, prev.y + next.y, s.y);
+    s.z = fmaf(my, prev.z + next.z, s.z);
+    s.w = fmaf(my, prev.w + next.w, s.w);
+  }
+  return s;
+}
+
+template <bool ALIGNED>
+__global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_constant__ CUtensorMap map,
+                                                               const __grid_constant__ PolyStep q, int *err) {
+  extern __shared__ __align__(128) unsigned char raw[];
+  PolySmem &sm = *reinterpret_cast<PolySmem *>(raw);
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int tx = blockIdx.x % q.tiles_x, ty = blockIdx.x / q.tiles_x;
+  const int f0 = tx * q.cw - q.hx, b0 = ty * q.ch - q.hy;
+  const int gf = f0 + 2 * lane, gb0 = b0 + wp * kPR;
+  const int p0 = blockIdx.y * q.G, np = min(q.G, q.P - p0);
+  const bool in0 = gf >= 0 && gf < q.nf, in1 = gf + 1 >= 0 && gf + 1 < q.nf;
+  const bool staged = ALIGNED && q.use_u;
+  constexpr uint32_t kTile = kPH * kPW * sizeof(float2);
+  if (ALIGNED && threadIdx.x == 0) {
+    mbar_init(&sm.bar[0], 1);
+    mbar_init(&sm.bar[1], 1);
+    fence_mbar_init();
+  }
+  __syncthreads();
+  auto issue = [&](int j) {
+    mbar_arrive_expect_tx(&sm.bar[j & 1], kTile);
+    tma_load_4d(sm.u[j & 1], &map, f0, b0, p0 + j, q.sel, &sm.bar[j & 1]);
+  };
+  if (staged && threadIdx.x == 0) {
+    issue(0);
+    if (np > 1) issue(1);
+  }
+  // weights and diagonals of this thread's pixels; zero outside the image, so
+  // that g and y stay zero there
+  float2 cw0 = make_float2(0.f, 0.f), cw1 = cw0;
+  if (in0) cw0 = q.colw[gf];
+  if (in1) cw1 = q.colw[gf + 1];
+  if (lane == 0) cw0.x = 0.f;
+  if (lane == 31) cw1.y = 0.f;
+  for (int r = threadIdx.x; r < kPH; r += kPThreads) {
+    const int b = b0 + r;
+    sm.roww[r] = (b >= 0 && b < q.nb) ? q.roww[b] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  // a row next to the image's first or last one may have its own couplings
+  const bool edge = gb0 <= 1 || gb0 + kPR > q.nb - 2;
+  float4 Ji[kPR];  // i D^{-1} of the two columns
+#pragma unroll
+  for (int i = 0; i < kPR; ++i) {
+    const int b = gb0 + i;
+    const bool row = b >= 0 && b < q.nb;
+    const size_t at = (size_t)b * q.nf + gf;
+    float4 dl = make_float4(0.f, 0.f, 0.f, 0.f), dr = dl;
+    if (ALIGNED) {
+      if (row && in0) {
+        dl = *reinterpret_cast<const float4 *>(q.cdl + at);
+        dr = *reinterpret_cast<const float4 *>(q.cdr + at);
+      }
+    } else if (row) {
+      if (in0) {
+        const float2 l = q.cdl[at], r = q.cdr[at];
+        dl.x = l.x, dl.y = l.y, dr.x = r.x, dr.y = r.y;
+      }
+      if (in1) {
+        const float2 l = q.cdl[at + 1], r = q.cdr[at + 1];
+        dl.z = l.x, dl.w = l.y, dr.z = r.x, dr.w = r.y;
+      }
+    }
+    sm.dsum[wp * kPR + i][lane] = make_float4(dl.x + dr.x, dl.y + dr.y, dl.z + dr.z, dl.w + dr.w);
+    // i / (1 - d) = (di + i dr) / |1 - d|^2 with 1 - d = dr - i (-di)
+    const float ax = 1.f - dl.x, ay = -dl.y, az = 1.f - dl.z, aw = -dl.w;
+    const float na = 1.f / fmaf(ax, ax, ay * ay), nz = 1.f / fmaf(az, az, aw * aw);
+    Ji[i].x = (row && in0) ? ay * na : 0.f;
+    Ji[i].y = (row && in0) ? ax * na : 0.f;
+    Ji[i].z = (row && in1) ? aw * nz : 0.f;
+    Ji[i].w = (row && in1) ? az * nz : 0.f;
+  }
+  __syncthreads();
+  const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
+  const bool core0 = 2 * lane >= q.hx && 2 * lane < q.hx + q.cw && in0;
+  const bool core1 = 2 * lane + 1 >= q.hx && 2 * lane + 1 < q.hx + q.cw && in1;
+  for (int j = 0; j < np; ++j) {
+    const int p = p0 + j, buf = ALIGNED ? (j & 1) : 0;
+    if (staged) {
+      const bool got = mbar_wait_bounded(&sm.bar[buf], (uint32_t)((j >> 1) & 1), err);
+      if (__syncthreads_or(!got)) {
+        // give up: the copies in flight land before the CTA exits
+        if (threadIdx.x == 0) {
+          mbar_wait_bounded(&sm.bar[buf], (uint32_t)((j >> 1) & 1), nullptr);
+          if (j + 1 < np) mbar_wait_bounded(&sm.bar[buf ^ 1], (uint32_t)(((j + 1) >> 1) & 1), nullptr);
+        }
+        __syncthreads();
+        return;
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPR; ++i) {
+        const int b = gb0 + i;
+        float4 v = zero4;
+        if (q.use_u && b >= 0 && b < q.nb) {
+          const float2 *src = q.u + (size_t)p * q.N + (size_t)b * q.nf + gf;
+          if (in0) v.x = src[0].x, v.y = src[0].y;
+          if (in1) v.z = src[1].x, v.w = src[1].y;
+        }
+        sm.u[buf][wp * kPR + i][lane] = v;
+      }
+      __syncthreads();
+    }
+    const float4(*ut)[kPW / 2] = sm.u[buf];
+    float4 g[kPR], y[kPR];
+    // g = D^{-1} (dsum u + 2 K_off u + src), y = a_{m-1} g
+    {
+      const float am = q.a[q.m - 1];
+      float4 prev = wp > 0 ? ut[wp * kPR - 1][lane] : zero4, cur = ut[wp * kPR][lane];
+#pragma unroll
+      for (int i = 0; i < kPR; ++i) {
+        const int r = wp * kPR + i, b = gb0 + i;
+        const float4 next = r + 1 < kPH ? ut[r + 1][lane] : zero4;
+        float4 bv = zero4;
+        if (q.use_u) {
+          const float4 ds = sm.dsum[r][lane];
+          const float4 s = edge ? poly_sum<true>(cur, prev, next, cw0, cw1, q.my, sm.roww[r])
+                                : poly_sum<false>(cur, prev, next, cw0, cw1, q.my, zero4);
+          bv.x = fmaf(-2.f, s.y, fmaf(ds.x, cur.x, -ds.y * cur.y));
+          bv.y = fmaf(2.f, s.x, fmaf(ds.x, cur.y, ds.y * cur.x));
+          bv.z = fmaf(-2.f, s.w, fmaf(ds.z, cur.z, -ds.w * cur.w));
+          bv.w = fmaf(2.f, s.z, fmaf(ds.z, cur.w, ds.w * cur.z));
+        }
+        if (q.src_exit != nullptr || q.src_shared != nullptr) {
+          if (b >= 0 && b < q.nb) {
+            const size_t at = (size_t)b * q.nf + gf;
+            if (q.src_exit != nullptr) {
+              const float2 *src = q.src_exit + (size_t)p * q.N + at;
+              if (in0) bv.x += src[0].x, bv.y += src[0].y;
+              if (in1) bv.z += src[1].x, bv.w += src[1].y;
+            }
+            if (q.src_shared != nullptr) {
+              const float2 *src = q.src_shared + at;
+              if (in0) bv.x += src[0].x, bv.y += src[0].y;
+              if (in1) bv.z += src[1].x, bv.w += src[1].y;
+            }
+          }
+        }
+        // D^{-1} = -i Ji = (Ji.y, -Ji.x)
+        g[i].x = fmaf(Ji[i].y, bv.x, Ji[i].x * bv.y);
+        g[i].y = fmaf(Ji[i].y, bv.y, -Ji[i].x * bv.x);
+        g[i].z = fmaf(Ji[i].w, bv.z, Ji[i].z * bv.w);
+        g[i].w = fmaf(Ji[i].w, bv.w, -Ji[i].z * bv.z);
+        y[i] = make_float4(am * g[i].x, am * g[i].y, am * g[i].z, am * g[i].w);
+        prev = cur;
+        cur = next;
+      }
+    }
+    // the rows beside this warp's, published by its neighbours
+    auto exchange = [&](int k, float4 &above, float4 &below) {
+      if (wp > 0) sm.edge[k & 1][wp - 1][1][lane] = y[0];
+      if (wp + 1 < kPWarps) sm.edge[k & 1][wp][0][lane] = y[kPR - 1];
+      __syncthreads();
+      above = wp > 0 ? sm.edge[k & 1][wp - 1][0][lane] : zero4;
+      below = wp + 1 < kPWarps ? sm.edge[k & 1][wp][1][lane] : zero4;
+    };
+    for (int k = q.m - 2; k >= 0; --k) {  // y <- a_k g + J y
+      float4 prev, below;
+      exchange(k, prev, below);
+      const float ak = q.a[k];
+      float4 cur = y[0];
+#pragma unroll
+      for (int i = 0; i < kPR; ++i) {
+        const float4 next = i + 1 < kPR ? y[i + 1] : below;
+        const float4 s = edge ? poly_sum<true>(cur, prev, next, cw0, cw1, q.my, sm.roww[wp * kPR + i])
+                              : poly_sum<false>(cur, prev, next, cw0, cw1, q.my, zero4);
+        y[i].x = fmaf(Ji[i].x, s.x, fmaf(-Ji[i].y, s.y, ak * g[i].x));
+        y[i].y = fmaf(Ji[i].x, s.y, fmaf(Ji[i].y, s.x, ak * g[i].y));
+        y[i].z = fmaf(Ji[i].z, s.z, fmaf(-Ji[i].w, s.w, ak * g[i].z));
+        y[i].w = fmaf(Ji[i].z, s.w, fmaf(Ji[i].w, s.z, ak * g[i].w));
+        prev = cur;
+        cur = next;
+      }
+    }
+    // the true residual b - (I - P) d = D (g + J d - d), and u + d
+    float nb2 = 0.f, nr2 = 0.f;
+    {
+      float4 prev, below;
+      exchange(1, prev, below);  // the exchange before was at k = 0
+      float4 cur = y[0];
+#pragma unroll
+      for (int i = 0; i < kPR; ++i) {
+        const int r = wp * kPR + i, b = gb0 + i;
+        const float4 next = i + 1 < kPR ? y[i + 1] : below;
+        const float4 s = edge ? poly_sum<true>(cur, prev, next, cw0, cw1, q.my, sm.roww[r])
+                              : poly_sum<false>(cur, prev, next, cw0, cw1, q.my, zero4);
+        const bool row = r >= q.hy && r < q.hy + q.ch && b < q.nb;
+        if (row) {
+          const float4 uo = ut[r][lane];
+          const size_t at = (size_t)b * q.nf + gf;
+          const float4 v = make_float4(uo.x + cur.x, uo.y + cur.y, uo.z + cur.z, uo.w + cur.w);
+          auto put = [&](float2 *dst, bool stream) {
+            if (ALIGNED) {
+              if (core0) {
+                if (stream) __stcs(reinterpret_cast<float4 *>(dst), v);
+                else *reinterpret_cast<float4 *>(dst) = v;
+              }
+            } else {
+              if (core0) dst[0] = make_float2(v.x, v.y);
+              if (core1) dst[1] = make_float2(v.z, v.w);
+            }
+          };
+          put(q.un + (size_t)p * q.N + at, false);
+          if (q.store != nullptr) put(q.store + (size_t)p * q.store_stride + at, true);
+          if (q.exit_out != nullptr) put(q.exit_out + (size_t)p * q.N + at, false);
+          if (core0) {
+            const float rx = g[i].x + fmaf(Ji[i].x, s.x, fmaf(-Ji[i].y, s.y, -cur.x));
+            const float ry = g[i].y + fmaf(Ji[i].x, s.y, fmaf(Ji[i].y, s.x, -cur.y));
+            const float d2 = __fdividef(1.f, fmaf(Ji[i].x, Ji[i].x, Ji[i].y * Ji[i].y));
+            nb2 = fmaf(d2, fmaf(g[i].x, g[i].x, g[i].y * g[i].y), nb2);
+            nr2 = fmaf(d2, fmaf(rx, rx, ry * ry), nr2);
+          }
+          if (core1) {
+            const float rx = g[i].z + fmaf(Ji[i].z, s.z, fmaf(-Ji[i].w, s.w, -cur.z));
+            const float ry = g[i].w + fmaf(Ji[i].z, s.w, fmaf(Ji[i].w, s.z, -cur.w));
+            const float d2 = __fdividef(1.f, fmaf(Ji[i].z, Ji[i].z, Ji[i].w * Ji[i].w));
+            nb2 = fmaf(d2, fmaf(g[i].z, g[i].z, g[i].w * g[i].w), nb2);
+            nr2 = fmaf(d2, fmaf(rx, rx, ry * ry), nr2);
+          }
+        }
+        prev = cur;
+        cur = next;
+      }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      nb2 += __shfl_down_sync(0xffffffffu, nb2, o);
+      nr2 += __shfl_down_sync(0xffffffffu, nr2, o);
+    }
+    if (lane == 0) sm.red[wp] = make_float2(nb2, nr2);
+    __syncthreads();  // every thread is done with this probe's tile; the partial norms are in
+    if (threadIdx.x == 0) {
+      if (staged && j + 2 < np) {
+        fence_proxy_async_smem();
+        issue(j + 2);
+      }
+      double sb = 0.0, sr = 0.0;
+#pragma unroll
+      for (int w = 0; w < kPWarps; ++w) {
+        sb += (double)sm.red[w].x;
+        sr += (double)sm.red[w].y;
+      }
+      atomicAdd(&q.norms[p].x, sb);
+      atomicAdd(&q.norms[p].y, sr);
+    }
+  }
+}
+
+// Statistics of every solve of the march: m iterations each (none where the
+// right-hand side was zero), failures by the true residual.
+__global__ void c3_poly_stats_kernel(const double2 *norms, int count, int m, double tol2, int *stats) {
+  int iters = 0, failed = 0;
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < count; e += gridDim.x * blockDim.x) {
+    const double2 v = norms[e];
+    if (v.x == 0.0) continue;
+    iters += m;
+    if (!(v.y <= 100.0 * tol2 * v.x)) ++failed;  // 10x the tolerance, as the Krylov march
+  }
+  if (iters > 0) {
+    atomicAdd(&stats[0], iters);
+    atomicMax(&stats[3], m);
+  }
+  if (failed > 0) atomicAdd(&stats[2], failed);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    atomicAdd(&stats[1], count);
+    stats[4] = 2;
+  }
+}
+
+// u_store's slice of the initial state.
+__global__ void c3_poly_first_kernel(int N, int P, const float2 *__restrict__ u, float2 *store, size_t stride) {
+  const size_t total = (size_t)P * N;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x)
+    store[(e / N) * stride + e % N] = u[e];
+}
+
+// grad_c[s-1][i] += sum_p lambda_p[i] conj(u_p,s[i] + u_p,s-1[i]); one thread
+// owns element i and loops over the probes.
+__global__ void c3_poly_grad_kernel(int N, int P, int nz, int s, const float2 *__restrict__ lam,
+                                    const float2 *__restrict__ u_fwd, float2 *grad_c) {
+  constexpr int G = 8;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
+    float2 acc = make_float2(0.f, 0.f);
+    for (int p0 = 0; p0 < P; p0 += G) {
+      float2 a[G], b[G], l[G];
+#pragma unroll
+      for (int j = 0; j < G; ++j) {
+        if (p0 + j < P) {
+          const size_t pr = p0 + j;
+          a[j] = u_fwd[(pr * nz + s) * N + i];
+          b[j] = u_fwd[(pr * nz + s - 1) * N + i];
+          l[j] = lam[pr * N + i];
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < G; ++j)
+        if (p0 + j < P) acc = cadd(acc, cmulc(l[j], cadd(a[j], b[j])));
+    }
+    const float2 g = grad_c[(size_t)(s - 1) * N + i];
+    grad_c[(size_t)(s - 1) * N + i] = cadd(g, acc);
+  }
+}
+
+using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                                 const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+EncodeTiled encoder() {
+  static EncodeTiled fn = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult qr;
+    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &f, cudaEnableDefault, &qr) == cudaSuccess &&
+        qr == cudaDriverEntryPointSuccess)
+      fn = reinterpret_cast<EncodeTiled>(f);
+    (void)cudaGetLastError();
+  });
+  return fn;
+}
+
+// T_m(w) for complex w.
+std::complex<double> chebyshev(int m, std::complex<double> w) {
+  std::complex<double> t0 = 1.0, t1 = w;
+  if (m == 0) return t0;
+  for (int j = 1; j < m; ++j) {
+    const std::complex<double> t2 = 2.0 * w * t1 - t0;
+    t0 = t1;
+    t1 = t2;
+  }
+  return t1;
+}
+
+// The smallest degree whose residual polynomial stays below `target` on the
+// segment [-i tau, i tau] turned by up to `theta`; 0 if none is allowed.  a[k] are
+// the coefficients of p_m.
+int poly_degree(double tau, double theta, double target, int max_m, float *a) {
+  if (!(tau >= 0.0) || tau > 0.7) return 0;
+  if (tau < 1e-3) tau = 1e-3;
+  const std::complex<double> it(0.0, tau);
+  for (int m = 3; m <= max_m; ++m) {
+    const std::complex<double> scale = chebyshev(m, 1.0 / it);
+    const double bound = std::abs(chebyshev(m, std::polar(1.0, theta))) / std::abs(scale);
+    if (!(bound <= target)) continue;
+    // Chebyshev coefficients t_j of T_m
+    double t0[kPolyMaxDeg + 1] = {1.0}, t1[kPolyMaxDeg + 1] = {0.0, 1.0};
+    for (int n = 1; n < m; ++n) {
+      double t2[kPolyMaxDeg + 1] = {0.0};
+      for (int j = 0; j <= m; ++j) t2[j] = (j > 0 ? 2.0 * t1[j - 1] : 0.0) - t0[j];
+      for (int j = 0; j <= m; ++j) t0[j] = t1[j], t1[j] = t2[j];
+    }
+    std::complex<double> pw = 1.0, p = 1.0;  // (i tau)^{-j}
+    for (int k = 0; k < m; ++k) {
+      p -= t1[k] * pw / scale;
+      a[k] = (float)p.real();  // T_m has one parity: real
+      pw /= it;
+    }
+    return m;
+  }
+  return 0;
+}
+
+}  // namespace
+
+int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
+  *ran = 0;
+  const int nf = job.nf, nb = job.nb, N = nf * nb, nz = job.nz, L = nz - 1, P = job.P;
+  if (nf > kPolyMaxSide || nb > kPolyMaxSide || job.tol < 4e-7) return TP_OK;
+  const bool adj_exact = job.mode == TP_MODE_ADJOINT_EXACT;
+  const size_t norms_bytes = ((size_t)L * P * sizeof(double2) + 255) & ~size_t(255);
+  if (job.scratch_bytes < norms_bytes) return TP_OK;
+  size_t cap = (job.scratch_bytes - norms_bytes) / ((size_t)N * sizeof(float2));
+  if (cap > (size_t)L) cap = L;
+  if (cap < 2) return TP_OK;
+  double2 *norms = reinterpret_cast<double2 *>(job.scratch);
+  float2 *cd = reinterpret_cast<float2 *>(job.scratch + norms_bytes);
+
+  PolySlices sl{};
+  sl.field = job.field;
+  sl.nf = nf;
+  sl.nb = nb;
+  sl.N = N;
+  sl.nz = nz;
+  sl.L = L;
+  sl.dtype = job.dtype;
+  sl.is_delta = job.is_delta;
+  sl.exact = job.exact;
+  sl.conj_t = job.conj_t;
+  sl.sigma = job.sigma;
+  sl.k = job.k;
+  sl.dz = job.dz;
+  sl.kc = job.kc;
+  sl.kw = job.kw;
+  sl.ke = job.ke;
+  sl.ks = job.ks;
+  sl.kn = job.kn;
+  sl.colw = job.colw;
+  sl.roww = job.roww;
+  sl.my = (float)job.mu_y;
+  // slices [lo, hi] in cd: all of them, or as many as fit, in the march's order
+  const bool backward = job.mode != TP_MODE_FORWARD;
+  const int C = (int)cap;
+  int lo = backward ? L - C + 1 : 1, hi = backward ? L : C;
+  if (lo < 1) lo = 1;
+  if (hi > L) hi = L;
+  PolyCheck *chk = reinterpret_cast<PolyCheck *>(job.check);
+  TP_CHECK_CUDA(cudaMemsetAsync(chk, 0, sizeof(PolyCheck), st));
+  c3_poly_weights_kernel<<<1, 512, 0, st>>>(sl, job.colw, job.roww);
+  const dim3 sblock(32, 8);
+  c3_poly_slices_kernel<<<dim3((N + 31) / 32, (L + 31) / 32), sblock, 0, st>>>(sl, 1, L, lo, hi, cd, chk);
+  TP_CHECK_CUDA(cudaGetLastError());
+  PolyCheck host{};
+  TP_CHECK_CUDA(cudaMemcpyAsync(&host, chk, sizeof(PolyCheck), cudaMemcpyDeviceToHost, st));
+  TP_CHECK_CUDA(cudaStreamSynchronize(st));
+  if (host.bad) return TP_OK;
+  float tau, theta;
+  memcpy(&tau, &host.tau, 4);
+  memcpy(&theta, &host.arg, 4);
+
+  PolyStep q{};
+  const double target = 0.1 * (job.tol < 1e-6 ? job.tol : 1e-6);
+  q.m = poly_degree(tau, theta, target, kPolyMaxDeg < job.max_iter ? kPolyMaxDeg : job.max_iter, q.a);
+  if (q.m == 0) return TP_OK;
+  // halo: one pixel for the right-hand side and the reach of 1e-8 (no more than the polynomial's)
+  const double mu = fmax(1e-6, fmax(fabs(job.mu_x), fabs(job.mu_y)));
+  int h = 1 + (mu < 1.0 ? (int)ceil(log(1e-8) / log(mu)) : kPolyMaxHalo);
+  if (h > q.m + 1) h = q.m + 1;
+  if (h > kPolyMaxHalo) return TP_OK;
+
+  // 16-byte accesses and tensor copies need even rows and aligned outputs
+  auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
+  bool aligned = nf % 2 == 0 && al16(job.u_store) && al16(job.exit_out) && al16(cd) && al16(job.vec[0]);
+  CUtensorMap map{};
+  int *err = nullptr;
+  if (aligned) {
+    EncodeTiled enc = encoder();
+    err = device_error_ptr();
+    const cuuint64_t dims[4] = {(cuuint64_t)nf, (cuuint64_t)nb, (cuuint64_t)P, 2};
+    const cuuint64_t str[3] = {(cuuint64_t)nf * sizeof(float2), (cuuint64_t)N * sizeof(float2), job.vstride};
+    const cuuint32_t box[4] = {kPW, kPH, 1, 1}, es[4] = {1, 1, 1, 1};
+    aligned = enc != nullptr && err != nullptr &&
+              enc(&map, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, job.vec[0], dims, str, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  }
+  q.nf = nf;
+  q.nb = nb;
+  q.N = N;
+  q.P = P;
+  q.hx = (h + 1) & ~1;  // tensor copies start at an even column
+  q.hy = h;
+  q.tiles_x = (nf + kPW - 2 * q.hx - 1) / (kPW - 2 * q.hx);
+  const int tiles_y = (nb + kPH - 2 * q.hy - 1) / (kPH - 2 * q.hy);
+  q.cw = (((nf + q.tiles_x - 1) / q.tiles_x) + 1) & ~1;
+  q.ch = (nb + tiles_y - 1) / tiles_y;
+  const int tiles = q.tiles_x * tiles_y;
+  int dev = 0, sms = 148;
+  TP_CHECK_CUDA(cudaGetDevice(&dev));
+  TP_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  // probes per CTA: as few as give one wave of two CTAs per SM
+  const int slots = 2 * sms;
+  int groups = slots / tiles;
+  if (groups < 1) groups = 1;
+  if (groups > P) groups = P;
+  q.G = (P + groups - 1) / groups;
+  groups = (P + q.G - 1) / q.G;
+  q.colw = job.colw;
+  q.roww = job.roww;
+  q.my = sl.my;
+  const size_t smem = sizeof(PolySmem) + 128;
+  auto kern = aligned ? c3_poly_kernel<true> : c3_poly_kernel<false>;
+  TP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+
+  const size_t vec_bytes = (size_t)P * N * sizeof(float2);
+  if (job.probes != nullptr)
+    TP_CHECK_CUDA(cudaMemcpyAsync(job.vec[0], job.probes, vec_bytes, cudaMemcpyDeviceToDevice, st));
+  else
+    TP_CHECK_CUDA(cudaMemsetAsync(job.vec[0], 0, vec_bytes, st));
+  TP_CHECK_CUDA(cudaMemsetAsync(norms, 0, (size_t)L * P * sizeof(double2), st));
+  const bool flip = job.mode == TP_MODE_ADJOINT;
+  const size_t stride = (size_t)nz * N;
+  if (job.u_store)
+    c3_poly_first_kernel<<<296, 256, 0, st>>>(N, P, job.vec[0], job.u_store + (flip ? (size_t)L * N : 0), stride);
+  for (int t = 1; t <= L; ++t) {
+    const int s = backward ? L + 1 - t : t;
+    const int sr = (adj_exact && t > 1) ? s + 1 : s;
+    if (s < lo || s > hi) {  // the next run of slices (with slice s + 1 for the exact adjoint)
+      if (backward) {
+        hi = sr;
+        lo = hi - C + 1 > 1 ? hi - C + 1 : 1;
+      } else {
+        lo = s;
+        hi = lo + C - 1 < L ? lo + C - 1 : L;
+      }
+      c3_poly_slices_kernel<<<dim3((N + 31) / 32, (hi - lo) / 32 + 1), sblock, 0, st>>>(sl, lo, hi, lo, hi, cd, nullptr);
+    }
+    q.cdl = cd + (size_t)(s - lo) * N;
+    q.cdr = cd + (size_t)(sr - lo) * N;
+    q.sel = (t - 1) & 1;
+    q.u = job.vec[q.sel];
+    q.un = job.vec[q.sel ^ 1];
+    q.use_u = !(adj_exact && t == 1);
+    q.src_exit = t == 1 ? job.src_exit : nullptr;
+    q.src_shared = job.src_shared ? job.src_shared + (size_t)(t - 1) * N : nullptr;
+    q.store = job.u_store ? job.u_store + (size_t)(flip ? L - t : t) * N : nullptr;
+    q.store_stride = stride;
+    q.exit_out = t == L ? job.exit_out : nullptr;
+    q.norms = norms + (size_t)(t - 1) * P;
+    kern<<<dim3(tiles, groups), kPThreads, smem, st>>>(map, q, err);
+    if (job.grad_c)
+      c3_poly_grad_kernel<<<296, 256, 0, st>>>(N, P, nz, s, q.un, job.u_fwd, job.grad_c);
+  }
+  if (job.stats) c3_poly_stats_kernel<<<32, 256, 0, st>>>(norms, L * P, q.m, job.tol * job.tol, job.stats);
+  TP_CHECK_CUDA(cudaGetLastError());
+  *ran = 1;
+  return TP_OK;
+}
+
+}  // namespace tp
+#endif  // TP_C128_CHECK
