@@ -14,24 +14,31 @@
 // iterations per solve: 11 kernels and 34 passes over the probes' vectors per
 // step become one kernel that reads u once and writes it once.
 //
+// The 5-point stencil couples only pixels of opposite colour (checkerboard), so
+// the Horner recurrence y <- a_k g + J y needs one colour per power of J: y_k
+// lives on colour A for odd k and B for even k, ends in d on colour B, and the
+// other half of the solution is one exact substitution d^A = g^A + (J d)^A.  A
+// solve of even degree m costs m half-sweeps, and only colour B has a residual.
+//
 // One CTA owns a tile of 64 x 64 pixels (8 warps of 8 rows, two adjacent columns
-// per lane) of one image for a group of probes; D^{-1} of its 16 pixels stays
-// in a thread's registers for all of them, and so do g and the Horner
-// recurrence y <- a_k g + J y, whose neighbours come from the lane's own
-// registers (the other column, the rows above and below), warp shuffles (left
-// and right) and, at the warp's first and last row, shared memory.  A tile
-// computes a core smaller than itself: the value of a pixel j rows inside the
-// core's edge depends on what is h rows outside it only through mu^h, so a halo
-// of h = 1 + log(1e-8) / log(mu) pixels (6 at mu = 0.02) gives the core to
-// below complex64 round-off, whatever m.  The tiles of u arrive by tiled tensor
-// copies (zero outside the image), double-buffered over the group's probes.
-// Each solve is judged by its true residual, as in the Krylov march.
+// per lane: one pixel of each colour) of one image for a group of probes;
+// D^{-1} of its 16 pixels stays in a thread's registers for all of them, and so
+// do g and y, whose neighbours come from the lane's own registers (the other
+// column, the rows above and below), one warp shuffle (left or right) and, at
+// the warp's first and last row, shared memory.  A tile computes a core smaller
+// than itself: the value of a pixel at the core's edge depends on what is h rows
+// outside it only through mu^h, so a halo of h = 1 + log(1e-8) / log(mu) pixels
+// (6 at mu = 0.02) gives the core to below complex64 round-off, whatever m.  The
+// tiles of u arrive by tiled tensor copies (zero outside the image),
+// double-buffered over the group's probes.  Each solve is judged by its true
+// residual, as in the Krylov march.
 #include <cuda.h>
 #include <math.h>
 #include <string.h>
 
 #include <complex>
 #include <mutex>
+#include <type_traits>
 
 #include "cn3d_poly.cuh"
 #include "tp_errors.h"
@@ -178,43 +185,107 @@ struct PolyStep {
 struct PolySmem {
   float4 u[2][kPH][kPW / 2];
   float4 dsum[kPH][kPW / 2];
-  float4 edge[2][kPWarps - 1][2][kPW / 2];  // row exchange between warps w and w + 1: w's last row, (w + 1)'s first
+  float2 edge[2][kPWarps - 1][2][kPW / 2];  // row exchange between warps w and w + 1: w's last row, (w + 1)'s first
   float4 roww[kPH];
   float2 red[kPWarps];
   uint64_t bar[2];
 };
 
+// Two complex64 values of adjacent columns, each a packed register pair: sums and
+// real weights run as packed fp32 operations (one issue slot for both parts).
+struct cpair {
+  unsigned long long a, b;
+};
+__device__ __forceinline__ unsigned long long pk(float x, float y) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 upk(unsigned long long v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ cpair to_pair(float4 v) { return {pk(v.x, v.y), pk(v.z, v.w)}; }
+__device__ __forceinline__ float4 to_f4(cpair v) {
+  const float2 a = upk(v.a), b = upk(v.b);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// The real weights of a thread's neighbours, each in both halves of a pair:
+// left and right of its two columns, and the interior row weight.
+struct PolyWeights {
+  unsigned long long l0, r0, l1, r1, row;
+};
+
 // Weighted neighbour sums of both columns of one row: S = sum of real weights
-// times neighbours (the couplings are i times the weights).
+// times neighbours (the couplings are i times the weights).  EDGE: rw holds the
+// row's own weights {previous row, next row, columns}.
 template <bool EDGE>
-__device__ __forceinline__ float4 poly_sum(float4 cur, float4 prev, float4 next, float2 cw0, float2 cw1, float my,
-                                           float4 rw) {
-  const float wx = __shfl_up_sync(0xffffffffu, cur.z, 1), wy = __shfl_up_sync(0xffffffffu, cur.w, 1);
-  const float ex = __shfl_down_sync(0xffffffffu, cur.x, 1), ey = __shfl_down_sync(0xffffffffu, cur.y, 1);
-  float4 s;
-  s.x = fmaf(cw0.x, wx, cw0.y * cur.z);
-  s.y = fmaf(cw0.x, wy, cw0.y * cur.w);
-  s.z = fmaf(cw1.x, cur.x, cw1.y * ex);
-  s.w = fmaf(cw1.x, cur.y, cw1.y * ey);
+__device__ __forceinline__ cpair poly_sum(const cpair &cur, const cpair &prev, const cpair &next, const PolyWeights &w,
+                                          const float4 *rw) {
+  const float2 lo = upk(cur.a), hi = upk(cur.b);
+  const unsigned long long west = pk(__shfl_up_sync(0xffffffffu, hi.x, 1), __shfl_up_sync(0xffffffffu, hi.y, 1));
+  const unsigned long long east = pk(__shfl_down_sync(0xffffffffu, lo.x, 1), __shfl_down_sync(0xffffffffu, lo.y, 1));
+  cpair s;
+  s.a = fma2(w.l0, west, mul2(w.r0, cur.b));
+  s.b = fma2(w.l1, cur.a, mul2(w.r1, east));
   if (EDGE) {
-    s.x = fmaf(rw.z, s.x, fmaf(rw.x, prev.x, rw.y * next.x));
-    s.y = fmaf(rw.z, s.y, fmaf(rw.x, prev.y, rw.y * next.y));
-    s.z = fmaf(rw.z, s.z, fmaf(rw.x, prev.z, rw.y * next.z));
-    s.w = fmaf(rw.z, s.w, fmaf(rw.x, prev.w, rw.y * next.w));
+    const float4 v = *rw;
+    const unsigned long long x = pk(v.x, v.x), y = pk(v.y, v.y), z = pk(v.z, v.z);
+    s.a = fma2(z, s.a, fma2(x, prev.a, mul2(y, next.a)));
+    s.b = fma2(z, s.b, fma2(x, prev.b, mul2(y, next.b)));
   } else {
-    s.x = fmaf(my, prev.x + next.x, s.x);
-    s.y = fmaf(my, prev.y + next.y, s.y);
-    s.z = fmaf(my, prev.z + next.z, s.z);
-    s.w = fmaf(my, prev.w + next.w, s.w);
+    s.a = fma2(w.row, add2(prev.a, next.a), s.a);
+    s.b = fma2(w.row, add2(prev.b, next.b), s.b);
   }
   return s;
 }
+// The same for one pixel of colour C in row I of the thread's strip (rows start
+// even): colour A (0) is column 0 in even rows and column 1 in odd ones.  o, prev
+// and next are the other colour's pixels in this row and its neighbours.
+template <bool EDGE, int COL>
+__device__ __forceinline__ unsigned long long poly_half(unsigned long long o, unsigned long long prev,
+                                                        unsigned long long next, const PolyWeights &w,
+                                                        const float4 *rw) {
+  const float2 v = upk(o);
+  const unsigned long long side = COL == 0 ? pk(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1))
+                                           : pk(__shfl_down_sync(0xffffffffu, v.x, 1),
+                                                __shfl_down_sync(0xffffffffu, v.y, 1));
+  unsigned long long s = COL == 0 ? fma2(w.l0, side, mul2(w.r0, o)) : fma2(w.l1, o, mul2(w.r1, side));
+  if (EDGE) {
+    const float4 r = *rw;
+    s = fma2(pk(r.z, r.z), s, fma2(pk(r.x, r.x), prev, mul2(pk(r.y, r.y), next)));
+  } else {
+    s = fma2(w.row, add2(prev, next), s);
+  }
+  return s;
+}
+// c + j s (complex)
+__device__ __forceinline__ unsigned long long cmadd(float jx, float jy, unsigned long long s, unsigned long long c) {
+  const float2 sv = upk(s), cv = upk(c);
+  return pk(fmaf(jx, sv.x, fmaf(-jy, sv.y, cv.x)), fmaf(jx, sv.y, fmaf(jy, sv.x, cv.y)));
+}
 
-template <bool ALIGNED>
-__global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_constant__ CUtensorMap map,
-                                                               const __grid_constant__ PolyStep q, int *err) {
-  extern __shared__ __align__(128) unsigned char raw[];
-  PolySmem &sm = *reinterpret_cast<PolySmem *>(raw);
+// One tile and probe group.  EDGE: the tile holds one of the image's first or
+// last two rows, whose row couplings may differ from the interior's.
+template <bool ALIGNED, bool EDGE>
+__device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep &q, PolySmem &sm, int *err) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int tx = blockIdx.x % q.tiles_x, ty = blockIdx.x / q.tiles_x;
   const int f0 = tx * q.cw - q.hx, b0 = ty * q.ch - q.hy;
@@ -248,8 +319,7 @@ __global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_cons
     const int b = b0 + r;
     sm.roww[r] = (b >= 0 && b < q.nb) ? q.roww[b] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  // a row next to the image's first or last one may have its own couplings
-  const bool edge = gb0 <= 1 || gb0 + kPR > q.nb - 2;
+  const PolyWeights w = {pk(cw0.x, cw0.x), pk(cw0.y, cw0.y), pk(cw1.x, cw1.x), pk(cw1.y, cw1.y), pk(q.my, q.my)};
   float4 Ji[kPR];  // i D^{-1} of the two columns
 #pragma unroll
   for (int i = 0; i < kPR; ++i) {
@@ -313,24 +383,26 @@ __global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_cons
       __syncthreads();
     }
     const float4(*ut)[kPW / 2] = sm.u[buf];
-    float4 g[kPR], y[kPR];
-    // g = D^{-1} (dsum u + 2 K_off u + src), y = a_{m-1} g
+    const cpair zero2 = {0ull, 0ull};
+    cpair g[kPR];
+    unsigned long long y[kPR];
+    float nb2 = 0.f, nr2 = 0.f;
+    // g = D^{-1} (dsum u + 2 K_off u + src), y_{m-1} = a_{m-1} g on colour A
     {
-      const float am = q.a[q.m - 1];
-      float4 prev = wp > 0 ? ut[wp * kPR - 1][lane] : zero4, cur = ut[wp * kPR][lane];
+      const unsigned long long am = pk(q.a[q.m - 1], q.a[q.m - 1]);
+      cpair prev = wp > 0 ? to_pair(ut[wp * kPR - 1][lane]) : zero2, cur = to_pair(ut[wp * kPR][lane]);
 #pragma unroll
       for (int i = 0; i < kPR; ++i) {
         const int r = wp * kPR + i, b = gb0 + i;
-        const float4 next = r + 1 < kPH ? ut[r + 1][lane] : zero4;
+        const cpair next = r + 1 < kPH ? to_pair(ut[r + 1][lane]) : zero2;
         float4 bv = zero4;
         if (q.use_u) {
-          const float4 ds = sm.dsum[r][lane];
-          const float4 s = edge ? poly_sum<true>(cur, prev, next, cw0, cw1, q.my, sm.roww[r])
-                                : poly_sum<false>(cur, prev, next, cw0, cw1, q.my, zero4);
-          bv.x = fmaf(-2.f, s.y, fmaf(ds.x, cur.x, -ds.y * cur.y));
-          bv.y = fmaf(2.f, s.x, fmaf(ds.x, cur.y, ds.y * cur.x));
-          bv.z = fmaf(-2.f, s.w, fmaf(ds.z, cur.z, -ds.w * cur.w));
-          bv.w = fmaf(2.f, s.z, fmaf(ds.z, cur.w, ds.w * cur.z));
+          const float4 ds = sm.dsum[r][lane], uc = to_f4(cur);
+          const float4 s = to_f4(poly_sum<EDGE>(cur, prev, next, w, &sm.roww[r]));
+          bv.x = fmaf(-2.f, s.y, fmaf(ds.x, uc.x, -ds.y * uc.y));
+          bv.y = fmaf(2.f, s.x, fmaf(ds.x, uc.y, ds.y * uc.x));
+          bv.z = fmaf(-2.f, s.w, fmaf(ds.z, uc.z, -ds.w * uc.w));
+          bv.w = fmaf(2.f, s.z, fmaf(ds.z, uc.w, ds.w * uc.z));
         }
         if (q.src_exit != nullptr || q.src_shared != nullptr) {
           if (b >= 0 && b < q.nb) {
@@ -347,59 +419,85 @@ __global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_cons
             }
           }
         }
+        if (r >= q.hy && r < q.hy + q.ch && b < q.nb) {
+          if (core0) nb2 = fmaf(bv.x, bv.x, fmaf(bv.y, bv.y, nb2));
+          if (core1) nb2 = fmaf(bv.z, bv.z, fmaf(bv.w, bv.w, nb2));
+        }
         // D^{-1} = -i Ji = (Ji.y, -Ji.x)
-        g[i].x = fmaf(Ji[i].y, bv.x, Ji[i].x * bv.y);
-        g[i].y = fmaf(Ji[i].y, bv.y, -Ji[i].x * bv.x);
-        g[i].z = fmaf(Ji[i].w, bv.z, Ji[i].z * bv.w);
-        g[i].w = fmaf(Ji[i].w, bv.w, -Ji[i].z * bv.z);
-        y[i] = make_float4(am * g[i].x, am * g[i].y, am * g[i].z, am * g[i].w);
+        g[i].a = pk(fmaf(Ji[i].y, bv.x, Ji[i].x * bv.y), fmaf(Ji[i].y, bv.y, -Ji[i].x * bv.x));
+        g[i].b = pk(fmaf(Ji[i].w, bv.z, Ji[i].z * bv.w), fmaf(Ji[i].w, bv.w, -Ji[i].z * bv.z));
+        y[i] = mul2(am, (i & 1) ? g[i].b : g[i].a);
         prev = cur;
         cur = next;
       }
     }
-    // the rows beside this warp's, published by its neighbours
-    auto exchange = [&](int k, float4 &above, float4 &below) {
-      if (wp > 0) sm.edge[k & 1][wp - 1][1][lane] = y[0];
-      if (wp + 1 < kPWarps) sm.edge[k & 1][wp][0][lane] = y[kPR - 1];
+    // y_k on colour C from y_{k+1} on the other one (v, replaced row by row):
+    // a g + J v.  buf: alternates from one exchange to the next.
+    auto half_sweep = [&](auto colour, float a, unsigned long long(&v)[kPR], unsigned long long(&out)[kPR], int buf) {
+      constexpr int C = decltype(colour)::value;
+      if (wp > 0) sm.edge[buf][wp - 1][1][lane] = upk(v[0]);
+      if (wp + 1 < kPWarps) sm.edge[buf][wp][0][lane] = upk(v[kPR - 1]);
       __syncthreads();
-      above = wp > 0 ? sm.edge[k & 1][wp - 1][0][lane] : zero4;
-      below = wp + 1 < kPWarps ? sm.edge[k & 1][wp][1][lane] : zero4;
-    };
-    for (int k = q.m - 2; k >= 0; --k) {  // y <- a_k g + J y
-      float4 prev, below;
-      exchange(k, prev, below);
-      const float ak = q.a[k];
-      float4 cur = y[0];
+      unsigned long long prev = 0ull, below = 0ull;
+      if (wp > 0) {
+        const float2 e = sm.edge[buf][wp - 1][0][lane];
+        prev = pk(e.x, e.y);
+      }
+      if (wp + 1 < kPWarps) {
+        const float2 e = sm.edge[buf][wp][1][lane];
+        below = pk(e.x, e.y);
+      }
+      const unsigned long long a2 = pk(a, a);
 #pragma unroll
       for (int i = 0; i < kPR; ++i) {
-        const float4 next = i + 1 < kPR ? y[i + 1] : below;
-        const float4 s = edge ? poly_sum<true>(cur, prev, next, cw0, cw1, q.my, sm.roww[wp * kPR + i])
-                              : poly_sum<false>(cur, prev, next, cw0, cw1, q.my, zero4);
-        y[i].x = fmaf(Ji[i].x, s.x, fmaf(-Ji[i].y, s.y, ak * g[i].x));
-        y[i].y = fmaf(Ji[i].x, s.y, fmaf(Ji[i].y, s.x, ak * g[i].y));
-        y[i].z = fmaf(Ji[i].z, s.z, fmaf(-Ji[i].w, s.w, ak * g[i].z));
-        y[i].w = fmaf(Ji[i].z, s.w, fmaf(Ji[i].w, s.z, ak * g[i].w));
-        prev = cur;
-        cur = next;
+        const unsigned long long o = v[i], next = i + 1 < kPR ? v[i + 1] : below;
+        const float4 *rw = &sm.roww[wp * kPR + i];
+        if ((C + i) % 2 == 0) {
+          const unsigned long long s = poly_half<EDGE, 0>(o, prev, next, w, rw);
+          out[i] = cmadd(Ji[i].x, Ji[i].y, s, mul2(a2, g[i].a));
+        } else {
+          const unsigned long long s = poly_half<EDGE, 1>(o, prev, next, w, rw);
+          out[i] = cmadd(Ji[i].z, Ji[i].w, s, mul2(a2, g[i].b));
+        }
+        prev = o;
       }
+    };
+    using ColourA = std::integral_constant<int, 0>;
+    using ColourB = std::integral_constant<int, 1>;
+#pragma unroll 1
+    for (int k = q.m - 2; k > 0; k -= 2) {
+      half_sweep(ColourB{}, q.a[k], y, y, 0);
+      half_sweep(ColourA{}, q.a[k - 1], y, y, 1);
     }
-    // the true residual b - (I - P) d = D (g + J d - d), and u + d
-    float nb2 = 0.f, nr2 = 0.f;
+    half_sweep(ColourB{}, q.a[0], y, y, 0);  // d on colour B
+    unsigned long long da[kPR];
+    half_sweep(ColourA{}, 1.f, y, da, 1);  // d on colour A
+    // the residual of colour B, b - (I - P) d = D (g + J d - d), and u + d
     {
-      float4 prev, below;
-      exchange(1, prev, below);  // the exchange before was at k = 0
-      float4 cur = y[0];
+      if (wp > 0) sm.edge[0][wp - 1][1][lane] = upk(da[0]);
+      if (wp + 1 < kPWarps) sm.edge[0][wp][0][lane] = upk(da[kPR - 1]);
+      __syncthreads();
+      unsigned long long prev = 0ull, below = 0ull;
+      if (wp > 0) {
+        const float2 e = sm.edge[0][wp - 1][0][lane];
+        prev = pk(e.x, e.y);
+      }
+      if (wp + 1 < kPWarps) {
+        const float2 e = sm.edge[0][wp][1][lane];
+        below = pk(e.x, e.y);
+      }
 #pragma unroll
       for (int i = 0; i < kPR; ++i) {
         const int r = wp * kPR + i, b = gb0 + i;
-        const float4 next = i + 1 < kPR ? y[i + 1] : below;
-        const float4 s = edge ? poly_sum<true>(cur, prev, next, cw0, cw1, q.my, sm.roww[r])
-                              : poly_sum<false>(cur, prev, next, cw0, cw1, q.my, zero4);
-        const bool row = r >= q.hy && r < q.hy + q.ch && b < q.nb;
-        if (row) {
+        const bool odd = (i & 1) != 0;
+        const unsigned long long next = i + 1 < kPR ? da[i + 1] : below;
+        const unsigned long long s = odd ? poly_half<EDGE, 0>(da[i], prev, next, w, &sm.roww[r])
+                                         : poly_half<EDGE, 1>(da[i], prev, next, w, &sm.roww[r]);
+        if (r >= q.hy && r < q.hy + q.ch && b < q.nb) {
           const float4 uo = ut[r][lane];
+          const float2 d0 = upk(odd ? y[i] : da[i]), d1 = upk(odd ? da[i] : y[i]);
           const size_t at = (size_t)b * q.nf + gf;
-          const float4 v = make_float4(uo.x + cur.x, uo.y + cur.y, uo.z + cur.z, uo.w + cur.w);
+          const float4 v = make_float4(uo.x + d0.x, uo.y + d0.y, uo.z + d1.x, uo.w + d1.y);
           auto put = [&](float2 *dst, bool stream) {
             if (ALIGNED) {
               if (core0) {
@@ -414,23 +512,12 @@ __global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_cons
           put(q.un + (size_t)p * q.N + at, false);
           if (q.store != nullptr) put(q.store + (size_t)p * q.store_stride + at, true);
           if (q.exit_out != nullptr) put(q.exit_out + (size_t)p * q.N + at, false);
-          if (core0) {
-            const float rx = g[i].x + fmaf(Ji[i].x, s.x, fmaf(-Ji[i].y, s.y, -cur.x));
-            const float ry = g[i].y + fmaf(Ji[i].x, s.y, fmaf(Ji[i].y, s.x, -cur.y));
-            const float d2 = __fdividef(1.f, fmaf(Ji[i].x, Ji[i].x, Ji[i].y * Ji[i].y));
-            nb2 = fmaf(d2, fmaf(g[i].x, g[i].x, g[i].y * g[i].y), nb2);
-            nr2 = fmaf(d2, fmaf(rx, rx, ry * ry), nr2);
-          }
-          if (core1) {
-            const float rx = g[i].z + fmaf(Ji[i].z, s.z, fmaf(-Ji[i].w, s.w, -cur.z));
-            const float ry = g[i].w + fmaf(Ji[i].z, s.w, fmaf(Ji[i].w, s.z, -cur.w));
-            const float d2 = __fdividef(1.f, fmaf(Ji[i].z, Ji[i].z, Ji[i].w * Ji[i].w));
-            nb2 = fmaf(d2, fmaf(g[i].z, g[i].z, g[i].w * g[i].w), nb2);
-            nr2 = fmaf(d2, fmaf(rx, rx, ry * ry), nr2);
-          }
+          const float jx = odd ? Ji[i].x : Ji[i].z, jy = odd ? Ji[i].y : Ji[i].w;
+          const float2 rg = upk(cmadd(jx, jy, s, odd ? g[i].a : g[i].b)), rd = upk(y[i]);
+          const float rx = rg.x - rd.x, ry = rg.y - rd.y;
+          if (odd ? core0 : core1) nr2 = fmaf(__fdividef(1.f, fmaf(jx, jx, jy * jy)), fmaf(rx, rx, ry * ry), nr2);
         }
-        prev = cur;
-        cur = next;
+        prev = da[i];
       }
     }
 #pragma unroll
@@ -455,6 +542,16 @@ __global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_cons
       atomicAdd(&q.norms[p].y, sr);
     }
   }
+}
+
+template <bool ALIGNED>
+__global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_constant__ CUtensorMap map,
+                                                               const __grid_constant__ PolyStep q, int *err) {
+  extern __shared__ __align__(128) unsigned char raw[];
+  PolySmem &sm = *reinterpret_cast<PolySmem *>(raw);
+  const int b0 = (int)(blockIdx.x / q.tiles_x) * q.ch - q.hy;
+  if (b0 <= 1 || b0 + kPH > q.nb - 2) poly_tile<ALIGNED, true>(map, q, sm, err);
+  else poly_tile<ALIGNED, false>(map, q, sm, err);
 }
 
 // Statistics of every solve of the march: m iterations each (none where the
@@ -541,14 +638,14 @@ std::complex<double> chebyshev(int m, std::complex<double> w) {
   return t1;
 }
 
-// The smallest degree whose residual polynomial stays below `target` on the
+// The smallest even degree whose residual polynomial stays below `target` on the
 // segment [-i tau, i tau] turned by up to `theta`; 0 if none is allowed.  a[k] are
 // the coefficients of p_m.
 int poly_degree(double tau, double theta, double target, int max_m, float *a) {
   if (!(tau >= 0.0) || tau > 0.7) return 0;
   if (tau < 1e-3) tau = 1e-3;
   const std::complex<double> it(0.0, tau);
-  for (int m = 3; m <= max_m; ++m) {
+  for (int m = 4; m <= max_m; m += 2) {
     const std::complex<double> scale = chebyshev(m, 1.0 / it);
     const double bound = std::abs(chebyshev(m, std::polar(1.0, theta))) / std::abs(scale);
     if (!(bound <= target)) continue;
