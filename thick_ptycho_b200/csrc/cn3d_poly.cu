@@ -178,14 +178,13 @@ struct PolyStep {
   const float2 *src_exit, *src_shared;
   float2 *store;         // the step's slice of u_store, probe stride store_stride
   size_t store_stride;
-  float2 *exit_out;
   double2 *norms;  // per probe: ||b||^2, ||b - (I - P) d||^2
 };
 
 struct PolySmem {
   float4 u[2][kPH][kPW / 2];
   float4 dsum[kPH][kPW / 2];
-  float2 edge[2][kPWarps - 1][2][kPW / 2];  // row exchange between warps w and w + 1: w's last row, (w + 1)'s first
+  unsigned long long edge[2][kPWarps - 1][2][kPW / 2];  // row exchange between warps w and w + 1: w's last row, (w + 1)'s first
   float4 roww[kPH];
   float2 red[kPWarps];
   uint64_t bar[2];
@@ -284,7 +283,7 @@ __device__ __forceinline__ unsigned long long cmadd(float jx, float jy, unsigned
 
 // One tile and probe group.  EDGE: the tile holds one of the image's first or
 // last two rows, whose row couplings may differ from the interior's.
-template <bool ALIGNED, bool EDGE>
+template <bool ALIGNED, bool SRC, bool EDGE>
 __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep &q, PolySmem &sm, int *err) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int tx = blockIdx.x % q.tiles_x, ty = blockIdx.x / q.tiles_x;
@@ -292,7 +291,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
   const int gf = f0 + 2 * lane, gb0 = b0 + wp * kPR;
   const int p0 = blockIdx.y * q.G, np = min(q.G, q.P - p0);
   const bool in0 = gf >= 0 && gf < q.nf, in1 = gf + 1 >= 0 && gf + 1 < q.nf;
-  const bool staged = ALIGNED && q.use_u;
+  const bool staged = ALIGNED && (!SRC || q.use_u);
   constexpr uint32_t kTile = kPH * kPW * sizeof(float2);
   if (ALIGNED && threadIdx.x == 0) {
     mbar_init(&sm.bar[0], 1);
@@ -385,7 +384,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
     const float4(*ut)[kPW / 2] = sm.u[buf];
     const cpair zero2 = {0ull, 0ull};
     cpair g[kPR];
-    unsigned long long y[kPR];
+    unsigned long long ya[kPR], yb[kPR];  // the newest y of colours A and B
     float nb2 = 0.f, nr2 = 0.f;
     // g = D^{-1} (dsum u + 2 K_off u + src), y_{m-1} = a_{m-1} g on colour A
     {
@@ -396,7 +395,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
         const int r = wp * kPR + i, b = gb0 + i;
         const cpair next = r + 1 < kPH ? to_pair(ut[r + 1][lane]) : zero2;
         float4 bv = zero4;
-        if (q.use_u) {
+        if (!SRC || q.use_u) {
           const float4 ds = sm.dsum[r][lane], uc = to_f4(cur);
           const float4 s = to_f4(poly_sum<EDGE>(cur, prev, next, w, &sm.roww[r]));
           bv.x = fmaf(-2.f, s.y, fmaf(ds.x, uc.x, -ds.y * uc.y));
@@ -404,7 +403,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
           bv.z = fmaf(-2.f, s.w, fmaf(ds.z, uc.z, -ds.w * uc.w));
           bv.w = fmaf(2.f, s.z, fmaf(ds.z, uc.w, ds.w * uc.z));
         }
-        if (q.src_exit != nullptr || q.src_shared != nullptr) {
+        if (SRC) {
           if (b >= 0 && b < q.nb) {
             const size_t at = (size_t)b * q.nf + gf;
             if (q.src_exit != nullptr) {
@@ -426,76 +425,60 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
         // D^{-1} = -i Ji = (Ji.y, -Ji.x)
         g[i].a = pk(fmaf(Ji[i].y, bv.x, Ji[i].x * bv.y), fmaf(Ji[i].y, bv.y, -Ji[i].x * bv.x));
         g[i].b = pk(fmaf(Ji[i].w, bv.z, Ji[i].z * bv.w), fmaf(Ji[i].w, bv.w, -Ji[i].z * bv.z));
-        y[i] = mul2(am, (i & 1) ? g[i].b : g[i].a);
+        ya[i] = mul2(am, (i & 1) ? g[i].b : g[i].a);
         prev = cur;
         cur = next;
       }
     }
-    // y_k on colour C from y_{k+1} on the other one (v, replaced row by row):
-    // a g + J v.  buf: alternates from one exchange to the next.
-    auto half_sweep = [&](auto colour, float a, unsigned long long(&v)[kPR], unsigned long long(&out)[kPR], int buf) {
-      constexpr int C = decltype(colour)::value;
-      if (wp > 0) sm.edge[buf][wp - 1][1][lane] = upk(v[0]);
-      if (wp + 1 < kPWarps) sm.edge[buf][wp][0][lane] = upk(v[kPR - 1]);
+    // the other colour's pixels in the rows above and below the warp's strip, which
+    // the neighbouring warps publish; buf alternates from one exchange to the next
+    auto exchange = [&](const unsigned long long(&v)[kPR], int buf, unsigned long long &above, unsigned long long &below) {
+      if (wp > 0) sm.edge[buf][wp - 1][1][lane] = v[0];
+      if (wp + 1 < kPWarps) sm.edge[buf][wp][0][lane] = v[kPR - 1];
       __syncthreads();
-      unsigned long long prev = 0ull, below = 0ull;
-      if (wp > 0) {
-        const float2 e = sm.edge[buf][wp - 1][0][lane];
-        prev = pk(e.x, e.y);
-      }
-      if (wp + 1 < kPWarps) {
-        const float2 e = sm.edge[buf][wp][1][lane];
-        below = pk(e.x, e.y);
-      }
+      above = wp > 0 ? sm.edge[buf][wp - 1][0][lane] : 0ull;
+      below = wp + 1 < kPWarps ? sm.edge[buf][wp][1][lane] : 0ull;
+    };
+    // a g + J v on colour C, v on the other one
+    auto half_sweep = [&](auto colour, float a, const unsigned long long(&v)[kPR], unsigned long long(&out)[kPR]) {
+      constexpr int C = decltype(colour)::value;
+      unsigned long long prev, below;
+      exchange(v, C, prev, below);
       const unsigned long long a2 = pk(a, a);
 #pragma unroll
       for (int i = 0; i < kPR; ++i) {
-        const unsigned long long o = v[i], next = i + 1 < kPR ? v[i + 1] : below;
+        const unsigned long long next = i + 1 < kPR ? v[i + 1] : below;
         const float4 *rw = &sm.roww[wp * kPR + i];
         if ((C + i) % 2 == 0) {
-          const unsigned long long s = poly_half<EDGE, 0>(o, prev, next, w, rw);
+          const unsigned long long s = poly_half<EDGE, 0>(v[i], prev, next, w, rw);
           out[i] = cmadd(Ji[i].x, Ji[i].y, s, mul2(a2, g[i].a));
         } else {
-          const unsigned long long s = poly_half<EDGE, 1>(o, prev, next, w, rw);
+          const unsigned long long s = poly_half<EDGE, 1>(v[i], prev, next, w, rw);
           out[i] = cmadd(Ji[i].z, Ji[i].w, s, mul2(a2, g[i].b));
         }
-        prev = o;
+        prev = v[i];
       }
     };
-    using ColourA = std::integral_constant<int, 0>;
-    using ColourB = std::integral_constant<int, 1>;
 #pragma unroll 1
-    for (int k = q.m - 2; k > 0; k -= 2) {
-      half_sweep(ColourB{}, q.a[k], y, y, 0);
-      half_sweep(ColourA{}, q.a[k - 1], y, y, 1);
+    for (int k = q.m - 2; k >= 0; k -= 2) {
+      half_sweep(std::integral_constant<int, 1>{}, q.a[k], ya, yb);
+      // y_{k-1}; after y_0 = d on colour B, the substitution for colour A
+      half_sweep(std::integral_constant<int, 0>{}, k > 0 ? q.a[k - 1] : 1.f, yb, ya);
     }
-    half_sweep(ColourB{}, q.a[0], y, y, 0);  // d on colour B
-    unsigned long long da[kPR];
-    half_sweep(ColourA{}, 1.f, y, da, 1);  // d on colour A
     // the residual of colour B, b - (I - P) d = D (g + J d - d), and u + d
     {
-      if (wp > 0) sm.edge[0][wp - 1][1][lane] = upk(da[0]);
-      if (wp + 1 < kPWarps) sm.edge[0][wp][0][lane] = upk(da[kPR - 1]);
-      __syncthreads();
-      unsigned long long prev = 0ull, below = 0ull;
-      if (wp > 0) {
-        const float2 e = sm.edge[0][wp - 1][0][lane];
-        prev = pk(e.x, e.y);
-      }
-      if (wp + 1 < kPWarps) {
-        const float2 e = sm.edge[0][wp][1][lane];
-        below = pk(e.x, e.y);
-      }
+      unsigned long long prev, below;
+      exchange(ya, 1, prev, below);
 #pragma unroll
       for (int i = 0; i < kPR; ++i) {
         const int r = wp * kPR + i, b = gb0 + i;
         const bool odd = (i & 1) != 0;
-        const unsigned long long next = i + 1 < kPR ? da[i + 1] : below;
-        const unsigned long long s = odd ? poly_half<EDGE, 0>(da[i], prev, next, w, &sm.roww[r])
-                                         : poly_half<EDGE, 1>(da[i], prev, next, w, &sm.roww[r]);
+        const unsigned long long next = i + 1 < kPR ? ya[i + 1] : below;
+        const unsigned long long s = odd ? poly_half<EDGE, 0>(ya[i], prev, next, w, &sm.roww[r])
+                                         : poly_half<EDGE, 1>(ya[i], prev, next, w, &sm.roww[r]);
         if (r >= q.hy && r < q.hy + q.ch && b < q.nb) {
           const float4 uo = ut[r][lane];
-          const float2 d0 = upk(odd ? y[i] : da[i]), d1 = upk(odd ? da[i] : y[i]);
+          const float2 d0 = upk(odd ? yb[i] : ya[i]), d1 = upk(odd ? ya[i] : yb[i]);
           const size_t at = (size_t)b * q.nf + gf;
           const float4 v = make_float4(uo.x + d0.x, uo.y + d0.y, uo.z + d1.x, uo.w + d1.y);
           auto put = [&](float2 *dst, bool stream) {
@@ -511,13 +494,12 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
           };
           put(q.un + (size_t)p * q.N + at, false);
           if (q.store != nullptr) put(q.store + (size_t)p * q.store_stride + at, true);
-          if (q.exit_out != nullptr) put(q.exit_out + (size_t)p * q.N + at, false);
           const float jx = odd ? Ji[i].x : Ji[i].z, jy = odd ? Ji[i].y : Ji[i].w;
-          const float2 rg = upk(cmadd(jx, jy, s, odd ? g[i].a : g[i].b)), rd = upk(y[i]);
+          const float2 rg = upk(cmadd(jx, jy, s, odd ? g[i].a : g[i].b)), rd = upk(yb[i]);
           const float rx = rg.x - rd.x, ry = rg.y - rd.y;
           if (odd ? core0 : core1) nr2 = fmaf(__fdividef(1.f, fmaf(jx, jx, jy * jy)), fmaf(rx, rx, ry * ry), nr2);
         }
-        prev = da[i];
+        prev = ya[i];
       }
     }
 #pragma unroll
@@ -544,14 +526,15 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
   }
 }
 
-template <bool ALIGNED>
+// SRC: the step has a source, or (use_u = 0) nothing but a source.
+template <bool ALIGNED, bool SRC>
 __global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_constant__ CUtensorMap map,
                                                                const __grid_constant__ PolyStep q, int *err) {
   extern __shared__ __align__(128) unsigned char raw[];
   PolySmem &sm = *reinterpret_cast<PolySmem *>(raw);
   const int b0 = (int)(blockIdx.x / q.tiles_x) * q.ch - q.hy;
-  if (b0 <= 1 || b0 + kPH > q.nb - 2) poly_tile<ALIGNED, true>(map, q, sm, err);
-  else poly_tile<ALIGNED, false>(map, q, sm, err);
+  if (b0 <= 1 || b0 + kPH > q.nb - 2) poly_tile<ALIGNED, SRC, true>(map, q, sm, err);
+  else poly_tile<ALIGNED, SRC, false>(map, q, sm, err);
 }
 
 // Statistics of every solve of the march: m iterations each (none where the
@@ -775,8 +758,11 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
   q.roww = job.roww;
   q.my = sl.my;
   const size_t smem = sizeof(PolySmem) + 128;
-  auto kern = aligned ? c3_poly_kernel<true> : c3_poly_kernel<false>;
-  TP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  using PolyKernel = void (*)(const CUtensorMap, const PolyStep, int *);
+  const PolyKernel kerns[2] = {aligned ? c3_poly_kernel<true, false> : c3_poly_kernel<false, false>,
+                               aligned ? c3_poly_kernel<true, true> : c3_poly_kernel<false, true>};
+  for (PolyKernel k : kerns)
+    TP_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 
   const size_t vec_bytes = (size_t)P * N * sizeof(float2);
   if (job.probes != nullptr)
@@ -805,15 +791,15 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
     q.cdr = cd + (size_t)(sr - lo) * N;
     q.sel = (t - 1) & 1;
     q.u = job.vec[q.sel];
-    q.un = job.vec[q.sel ^ 1];
+    q.un = (t == L && job.exit_out) ? job.exit_out : job.vec[q.sel ^ 1];
     q.use_u = !(adj_exact && t == 1);
     q.src_exit = t == 1 ? job.src_exit : nullptr;
     q.src_shared = job.src_shared ? job.src_shared + (size_t)(t - 1) * N : nullptr;
     q.store = job.u_store ? job.u_store + (size_t)(flip ? L - t : t) * N : nullptr;
     q.store_stride = stride;
-    q.exit_out = t == L ? job.exit_out : nullptr;
     q.norms = norms + (size_t)(t - 1) * P;
-    kern<<<dim3(tiles, groups), kPThreads, smem, st>>>(map, q, err);
+    const bool src = q.src_exit != nullptr || q.src_shared != nullptr || !q.use_u;
+    kerns[src]<<<dim3(tiles, groups), kPThreads, smem, st>>>(map, q, err);
     if (job.grad_c)
       c3_poly_grad_kernel<<<296, 256, 0, st>>>(N, P, nz, s, q.un, job.u_fwd, job.grad_c);
   }
