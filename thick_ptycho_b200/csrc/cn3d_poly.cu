@@ -179,6 +179,10 @@ struct PolyStep {
   float2 *store;         // the step's slice of u_store, probe stride store_stride
   size_t store_stride;
   double2 *norms;  // per probe: ||b||^2, ||b - (I - P) d||^2
+  // gradient (exact adjoint): the slice's accumulator += sum_p u_new conj(f1 + f0),
+  // f1 and f0 the forward field at the slice's two nodes (probe stride store_stride)
+  const float2 *f0, *f1;
+  float2 *grad;
 };
 
 struct PolySmem {
@@ -283,7 +287,7 @@ __device__ __forceinline__ unsigned long long cmadd(float jx, float jy, unsigned
 
 // One tile and probe group.  EDGE: the tile holds one of the image's first or
 // last two rows, whose row couplings may differ from the interior's.
-template <bool ALIGNED, bool SRC, bool EDGE>
+template <bool ALIGNED, bool SRC, bool GRAD, bool EDGE>
 __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep &q, PolySmem &sm, int *err) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int tx = blockIdx.x % q.tiles_x, ty = blockIdx.x / q.tiles_x;
@@ -303,10 +307,9 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
     mbar_arrive_expect_tx(&sm.bar[j & 1], kTile);
     tma_load_4d(sm.u[j & 1], &map, f0, b0, p0 + j, q.sel, &sm.bar[j & 1]);
   };
-  if (staged && threadIdx.x == 0) {
-    issue(0);
-    if (np > 1) issue(1);
-  }
+  // The next step's CTAs may start as this one's leave: what they do before
+  // their own wait reads only the slices' diagonals and the weights.
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   // weights and diagonals of this thread's pixels; zero outside the image, so
   // that g and y stay zero there
   float2 cw0 = make_float2(0.f, 0.f), cw1 = cw0;
@@ -350,7 +353,12 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
     Ji[i].z = (row && in1) ? aw * nz : 0.f;
     Ji[i].w = (row && in1) ? az * nz : 0.f;
   }
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the step before is complete
   __syncthreads();
+  if (staged && threadIdx.x == 0) {
+    issue(0);
+    if (np > 1) issue(1);
+  }
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   const bool core0 = 2 * lane >= q.hx && 2 * lane < q.hx + q.cw && in0;
   const bool core1 = 2 * lane + 1 >= q.hx && 2 * lane + 1 < q.hx + q.cw && in1;
@@ -380,6 +388,15 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
         sm.u[buf][wp * kPR + i][lane] = v;
       }
       __syncthreads();
+    }
+    if (GRAD && ALIGNED) {
+      // the forward field's rows on their way into L2 while the slice is solved
+      const int i = lane >> 1, b = gb0 + i, r = wp * kPR + i;
+      if (lane < 2 * kPR && r >= q.hy && r < q.hy + q.ch && b < q.nb) {
+        const int c0 = f0 + q.hx, cols = min(q.cw, q.nf - c0);
+        const float2 *src = ((lane & 1) ? q.f1 : q.f0) + (size_t)p * q.store_stride + (size_t)b * q.nf + c0;
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(cols * (int)sizeof(float2)) : "memory");
+      }
     }
     const float4(*ut)[kPW / 2] = sm.u[buf];
     const cpair zero2 = {0ull, 0ull};
@@ -494,6 +511,21 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
           };
           put(q.un + (size_t)p * q.N + at, false);
           if (q.store != nullptr) put(q.store + (size_t)p * q.store_stride + at, true);
+          if (GRAD) {
+            const size_t fo = (size_t)p * q.store_stride + at;
+            if (ALIGNED) {
+              if (core0) {
+                const float4 a = *reinterpret_cast<const float4 *>(q.f0 + fo);
+                const float4 c = *reinterpret_cast<const float4 *>(q.f1 + fo);
+                const float2 g0 = cmulc(make_float2(v.x, v.y), make_float2(a.x + c.x, a.y + c.y));
+                const float2 g1 = cmulc(make_float2(v.z, v.w), make_float2(a.z + c.z, a.w + c.w));
+                red_add_cx2(reinterpret_cast<float4 *>(q.grad + at), make_float4(g0.x, g0.y, g1.x, g1.y));
+              }
+            } else {
+              if (core0) red_add_cx(q.grad + at, cmulc(make_float2(v.x, v.y), cadd(q.f0[fo], q.f1[fo])));
+              if (core1) red_add_cx(q.grad + at + 1, cmulc(make_float2(v.z, v.w), cadd(q.f0[fo + 1], q.f1[fo + 1])));
+            }
+          }
           const float jx = odd ? Ji[i].x : Ji[i].z, jy = odd ? Ji[i].y : Ji[i].w;
           const float2 rg = upk(cmadd(jx, jy, s, odd ? g[i].a : g[i].b)), rd = upk(yb[i]);
           const float rx = rg.x - rd.x, ry = rg.y - rd.y;
@@ -526,15 +558,16 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
   }
 }
 
-// SRC: the step has a source, or (use_u = 0) nothing but a source.
-template <bool ALIGNED, bool SRC>
+// SRC: the step has a source, or (use_u = 0) nothing but a source.  GRAD: the step
+// adds its gradient contributions.
+template <bool ALIGNED, bool SRC, bool GRAD>
 __global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_constant__ CUtensorMap map,
                                                                const __grid_constant__ PolyStep q, int *err) {
   extern __shared__ __align__(128) unsigned char raw[];
   PolySmem &sm = *reinterpret_cast<PolySmem *>(raw);
   const int b0 = (int)(blockIdx.x / q.tiles_x) * q.ch - q.hy;
-  if (b0 <= 1 || b0 + kPH > q.nb - 2) poly_tile<ALIGNED, SRC, true>(map, q, sm, err);
-  else poly_tile<ALIGNED, SRC, false>(map, q, sm, err);
+  if (b0 <= 1 || b0 + kPH > q.nb - 2) poly_tile<ALIGNED, SRC, GRAD, true>(map, q, sm, err);
+  else poly_tile<ALIGNED, SRC, GRAD, false>(map, q, sm, err);
 }
 
 // Statistics of every solve of the march: m iterations each (none where the
@@ -563,33 +596,6 @@ __global__ void c3_poly_first_kernel(int N, int P, const float2 *__restrict__ u,
   const size_t total = (size_t)P * N;
   for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x)
     store[(e / N) * stride + e % N] = u[e];
-}
-
-// grad_c[s-1][i] += sum_p lambda_p[i] conj(u_p,s[i] + u_p,s-1[i]); one thread
-// owns element i and loops over the probes.
-__global__ void c3_poly_grad_kernel(int N, int P, int nz, int s, const float2 *__restrict__ lam,
-                                    const float2 *__restrict__ u_fwd, float2 *grad_c) {
-  constexpr int G = 8;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < N; i += gridDim.x * blockDim.x) {
-    float2 acc = make_float2(0.f, 0.f);
-    for (int p0 = 0; p0 < P; p0 += G) {
-      float2 a[G], b[G], l[G];
-#pragma unroll
-      for (int j = 0; j < G; ++j) {
-        if (p0 + j < P) {
-          const size_t pr = p0 + j;
-          a[j] = u_fwd[(pr * nz + s) * N + i];
-          b[j] = u_fwd[(pr * nz + s - 1) * N + i];
-          l[j] = lam[pr * N + i];
-        }
-      }
-#pragma unroll
-      for (int j = 0; j < G; ++j)
-        if (p0 + j < P) acc = cadd(acc, cmulc(l[j], cadd(a[j], b[j])));
-    }
-    const float2 g = grad_c[(size_t)(s - 1) * N + i];
-    grad_c[(size_t)(s - 1) * N + i] = cadd(g, acc);
-  }
 }
 
 using EncodeTiled = CUresult (*)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
@@ -719,7 +725,7 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
 
   // 16-byte accesses and tensor copies need even rows and aligned outputs
   auto al16 = [](const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
-  bool aligned = nf % 2 == 0 && al16(job.u_store) && al16(job.exit_out) && al16(cd) && al16(job.vec[0]);
+  bool aligned = nf % 2 == 0 && al16(job.u_store) && al16(job.exit_out) && al16(job.u_fwd) && al16(job.grad_c) && al16(cd) && al16(job.vec[0]);
   CUtensorMap map{};
   int *err = nullptr;
   if (aligned) {
@@ -759,8 +765,12 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
   q.my = sl.my;
   const size_t smem = sizeof(PolySmem) + 128;
   using PolyKernel = void (*)(const CUtensorMap, const PolyStep, int *);
-  const PolyKernel kerns[2] = {aligned ? c3_poly_kernel<true, false> : c3_poly_kernel<false, false>,
-                               aligned ? c3_poly_kernel<true, true> : c3_poly_kernel<false, true>};
+  // [source][gradient]
+  const PolyKernel kerns[4] = {
+      aligned ? c3_poly_kernel<true, false, false> : c3_poly_kernel<false, false, false>,
+      aligned ? c3_poly_kernel<true, false, true> : c3_poly_kernel<false, false, true>,
+      aligned ? c3_poly_kernel<true, true, false> : c3_poly_kernel<false, true, false>,
+      aligned ? c3_poly_kernel<true, true, true> : c3_poly_kernel<false, true, true>};
   for (PolyKernel k : kerns)
     TP_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 
@@ -774,6 +784,7 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
   const size_t stride = (size_t)nz * N;
   if (job.u_store)
     c3_poly_first_kernel<<<296, 256, 0, st>>>(N, P, job.vec[0], job.u_store + (flip ? (size_t)L * N : 0), stride);
+  bool fresh = true;
   for (int t = 1; t <= L; ++t) {
     const int s = backward ? L + 1 - t : t;
     const int sr = (adj_exact && t > 1) ? s + 1 : s;
@@ -786,6 +797,7 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
         hi = lo + C - 1 < L ? lo + C - 1 : L;
       }
       c3_poly_slices_kernel<<<dim3((N + 31) / 32, (hi - lo) / 32 + 1), sblock, 0, st>>>(sl, lo, hi, lo, hi, cd, nullptr);
+      fresh = true;
     }
     q.cdl = cd + (size_t)(s - lo) * N;
     q.cdr = cd + (size_t)(sr - lo) * N;
@@ -799,9 +811,23 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
     q.store_stride = stride;
     q.norms = norms + (size_t)(t - 1) * P;
     const bool src = q.src_exit != nullptr || q.src_shared != nullptr || !q.use_u;
-    kerns[src]<<<dim3(tiles, groups), kPThreads, smem, st>>>(map, q, err);
-    if (job.grad_c)
-      c3_poly_grad_kernel<<<296, 256, 0, st>>>(N, P, nz, s, q.un, job.u_fwd, job.grad_c);
+    if (job.grad_c) {
+      q.f0 = job.u_fwd + (size_t)(s - 1) * N;
+      q.f1 = job.u_fwd + (size_t)s * N;
+      q.grad = job.grad_c + (size_t)(s - 1) * N;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(tiles, groups);
+    cfg.blockDim = dim3(kPThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = fresh ? 0 : 1;  // behind another kernel than a step's: after all of it
+    TP_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kerns[(src ? 2 : 0) + (job.grad_c ? 1 : 0)], map, q, err));
+    fresh = false;
   }
   if (job.stats) c3_poly_stats_kernel<<<32, 256, 0, st>>>(norms, L * P, q.m, job.tol * job.tol, job.stats);
   TP_CHECK_CUDA(cudaGetLastError());
