@@ -412,7 +412,8 @@ typedef struct tp_cn3d_march_args {
   int32_t *stats;            /* device int32[5]: total iterations, solves, solves
                                 whose true residual exceeded 10 tol, largest
                                 iteration count (accumulated), and [4] = 1 when
-                                the march ran as one graph (0 step by step);
+                                the march ran as one graph (0 step by step, 2 as
+                                polynomial steps);
                                 or NULL.  A caller of the learned form re-runs
                                 the march with precond = 1 when stats[2] grew
                                 (fallback) */
@@ -447,8 +448,24 @@ typedef struct tp_cn3d_march_args {
                                 is even; complex64 build).  Bit 2: the learned
                                 filter by register shuffles (automatic: rows
                                 staged by bulk copies where nf is 64, 128, 192
-                                or 256).                                        */
+                                or 256).  Bit 3: the Krylov march always
+                                (automatic, precond = 1: where the slices'
+                                scaled off-diagonal part J is small enough, the
+                                tolerance at least 4e-7 and max_iter allows its
+                                degree m, each slice is solved by a fixed
+                                polynomial of J of that degree, one kernel per
+                                step after one host wait for the bounds of J;
+                                stats then count m iterations per solve and
+                                stats[4] = 2; not for REVERSE, training pairs,
+                                launch = 1, host_check = 0 or a capturing
+                                stream).  Bit 8: pair sums, see
+                                TP_CN3D_PAIR_SUMS.                              */
 } tp_cn3d_march_args;
+
+/* tp_cn3d_march_args.kernels: a FORWARD march stores u_s + u_{s-1} at slice s of
+ * u_store (slice 0: the initial field), an ADJOINT_EXACT march reads u_fwd as
+ * those: what the gradient contracts with, one slice per step instead of two. */
+#define TP_CN3D_PAIR_SUMS 0x100
 
 TP_API size_t tp_cn3d_workspace_bytes(int32_t n_total, int32_t num_probes);
 /* Learned-form workspace: the CNN activations of 64 slices, the filters of

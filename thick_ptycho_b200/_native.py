@@ -28,6 +28,7 @@ MODES = {"forward": MODE_FORWARD, "adjoint": MODE_ADJOINT, "reverse": MODE_REVER
 
 C128 = 0
 C64 = 1
+CN3D_PAIR_SUMS = 0x100  # tp_cn3d_march_args.kernels
 
 
 class NativeLibraryError(RuntimeError):

@@ -63,7 +63,8 @@ class CN3D:
         # kernel choice (tp_cn3d_march_args.kernels; the same arithmetic):
         # 0 = automatic; bit 0 = Stockham transforms always, bit 1 = the
         # stencil kernels with per-thread loads instead of tensor-memory copies,
-        # bit 2 = the learned filter by register shuffles instead of bulk-staged rows
+        # bit 2 = the learned filter by register shuffles instead of bulk-staged rows,
+        # bit 3 = the Krylov march also where a fixed polynomial solves each slice
         self.kernels = 0
 
     def op(self, is_delta=False) -> _native.TpCn3dOp:
@@ -95,7 +96,7 @@ class CN3D:
     def march(self, field: torch.Tensor, num_probes: int, mode="forward", probes=None, src_shared=None, src_exit=None,
               u_store=None, exit_out=None, u_fwd=None, grad_c=None, tol=1e-6, max_iter=20, precond=True,
               host_check=True, is_delta=False, model=None, train=None, train_every=0, fallback=True,
-              reuse_filters=False):
+              reuse_filters=False, store_sums=False):
         """One batched march; tensors complex64 (complex128 in the check build;
         field complex128/complex64 (N, nz)).
 
@@ -106,21 +107,25 @@ class CN3D:
         (judged by the true residual) is re-run with the plain FFT
         preconditioner; ``self.fallbacks`` counts such re-runs.  ``train`` is a
         :class:`learned.TrainingPairs` whose buffers receive the pair of every
-        ``train_every``-th step (see :func:`generate_pairs`)."""
+        ``train_every``-th step (see :func:`generate_pairs`).
+        ``store_sums``: a forward march stores the pair sums u_s + u_{s−1} at
+        slice s of ``u_store`` (slice 0: the initial field), an exact-adjoint
+        march reads ``u_fwd`` as those."""
         if precond == "learned":
             if model is None:
                 raise ValueError('precond="learned" needs a model')
             if fallback:
                 before = int(self.stats[2].item())
                 self._march(field, num_probes, mode, probes, src_shared, src_exit, u_store, exit_out, u_fwd, grad_c, tol,
-                            max_iter, 2, host_check, is_delta, model, train, train_every, reuse_filters)
+                            max_iter, 2, host_check, is_delta, model, train, train_every, reuse_filters, store_sums)
                 if int(self.stats[2].item()) > before:
                     self.fallbacks += 1
                     if grad_c is not None:
                         raise RuntimeError("learned adjoint solve missed its tolerance; re-run with precond=True "
                                            "(the gradient accumulator already holds a partial sum)")
                     self._march(field, num_probes, mode, probes, src_shared, src_exit, u_store, exit_out, u_fwd,
-                                grad_c, tol, max_iter, 1, host_check, is_delta, None, train, train_every)
+                                grad_c, tol, max_iter, 1, host_check, is_delta, None, train, train_every,
+                                store_sums=store_sums)
                 return
             code = 2
         elif precond in (True, "fft", 1):
@@ -130,10 +135,11 @@ class CN3D:
         else:
             raise ValueError(f"unknown preconditioner {precond!r}")
         self._march(field, num_probes, mode, probes, src_shared, src_exit, u_store, exit_out, u_fwd, grad_c, tol,
-                    max_iter, code, host_check, is_delta, model, train, train_every, reuse_filters)
+                    max_iter, code, host_check, is_delta, model, train, train_every, reuse_filters, store_sums)
 
     def _march(self, field, num_probes, mode, probes, src_shared, src_exit, u_store, exit_out, u_fwd, grad_c, tol,
-               max_iter, precond, host_check, is_delta, model, train, train_every, reuse_filters=False):
+               max_iter, precond, host_check, is_delta, model, train, train_every, reuse_filters=False,
+               store_sums=False):
         P = int(num_probes)
         field = field.reshape(self.N, self.nz).contiguous()
         mode_i = _native.MODES[mode] if isinstance(mode, str) else int(mode)
@@ -146,7 +152,7 @@ class CN3D:
         a.num_probes, a.mode, a.max_iter, a.precond, a.host_check = P, mode_i, int(max_iter), int(precond), int(host_check)
         a.tol = float(tol)
         a.launch = int(self.launch)
-        a.kernels = int(self.kernels)
+        a.kernels = int(self.kernels) | (_native.CN3D_PAIR_SUMS if store_sums else 0)
         a.probes, a.src_shared, a.src_exit = _ptr(probes), _ptr(src_shared), _ptr(src_exit)
         a.u_store, a.exit_out, a.u_fwd, a.grad_c = _ptr(u_store), _ptr(exit_out), _ptr(u_fwd), _ptr(grad_c)
         a.stats = ctypes.c_void_p(self.stats.data_ptr())
@@ -225,7 +231,7 @@ class PWEGradient3D:
             self._store = e.new_store(P)
         ex = torch.empty((P, e.N), dtype=torch.complex64, device=self.device)
         e.march(field, P, "forward", probes=probes.reshape(P, e.N).contiguous(), u_store=self._store, exit_out=ex,
-                **self.kw)
+                store_sums=True, **self.kw)
         self._filters_of = field  # the learned filters now in the engine's workspace
         return ex
 
@@ -234,7 +240,7 @@ class PWEGradient3D:
         P = exit_grad.shape[0]
         gc = torch.zeros((e.L, e.N), dtype=torch.complex64, device=self.device)
         e.march(field, P, "adjoint_exact", src_exit=exit_grad.reshape(P, e.N).contiguous(), u_fwd=self._store,
-                grad_c=gc, reuse_filters=getattr(self, "_filters_of", None) is field, **self.kw)
+                grad_c=gc, reuse_filters=getattr(self, "_filters_of", None) is field, store_sums=True, **self.kw)
         self.grad_c = gc
         return e.grad_to_n(gc, field)
 

@@ -814,11 +814,12 @@ __global__ void __launch_bounds__(k3Threads) c3_update_kernel(const C3Params q, 
 
 // True residual of each solve: res2 = ||rhs - (I - P) d||^2 (rhs = r0, d = x),
 // then u += d, stored into node `to` of u_store (to = t, or L - t for the
-// flipped reference adjoint) and, at the last step, into exit_out.
+// flipped reference adjoint; with `sums` the pair sum u_new + u instead) and,
+// at the last step, into exit_out.
 __global__ void __launch_bounds__(k3Threads, 4) c3_finish_kernel(const C3Params q, const C3State *st,
                                                               const cx *__restrict__ cd,
                                                               const cx *__restrict__ x, const cx *__restrict__ r0,
-                                                              cx *u, Krylov *K, cx *u_store, int flip,
+                                                              cx *u, Krylov *K, cx *u_store, int flip, int sums,
                                                               cx *exit_out) {
   __shared__ double red[kStencilProbes * (k3Threads / 32)];
   const int p0 = blockIdx.y * kStencilProbes;
@@ -839,7 +840,7 @@ __global__ void __launch_bounds__(k3Threads, 4) c3_finish_kernel(const C3Params 
       k = stencil_at(q, i);
       dc = cd[i];
     }
-    cx unv[kStencilProbes];
+    cx unv[kStencilProbes], stv[kStencilProbes];
 #pragma unroll
     for (int j = 0; j < kStencilProbes; ++j) {
       if (j >= np) break;
@@ -849,7 +850,9 @@ __global__ void __launch_bounds__(k3Threads, 4) c3_finish_kernel(const C3Params 
       const cx mx = it ? csub(xi, stencil_off(q, k, x + off, i, cmul(dc, xi))) : xi;
       const cx d = csub(r0[off + i], mx);
       acc[j] += (double)d.x * d.x + (double)d.y * d.y;
-      unv[j] = cadd(u[off + i], xi);
+      const cx uo = u[off + i];
+      unv[j] = cadd(uo, xi);
+      stv[j] = sums ? cadd(uo, unv[j]) : unv[j];
     }
 #pragma unroll
     for (int j = 0; j < kStencilProbes; ++j) {
@@ -857,7 +860,7 @@ __global__ void __launch_bounds__(k3Threads, 4) c3_finish_kernel(const C3Params 
       const int pr = p0 + j;
       const size_t off = (size_t)pr * q.N;
       u[off + i] = unv[j];
-      if (u_store) u_store[((size_t)pr * q.nz + node) * q.N + i] = unv[j];
+      if (u_store) u_store[((size_t)pr * q.nz + node) * q.N + i] = stv[j];
       if (exit_out && t == q.L) exit_out[off + i] = unv[j];
     }
   }
@@ -896,7 +899,7 @@ struct TmaArgs {
   cx *out;       // init: r0; matvec: v or t; finish: u
   const cx *src_exit, *src_shared;
   cx *u_store, *exit_out;
-  int adj_exact, flip;
+  int adj_exact, flip, sums;
 };
 
 // vectors staged without halo: 0 (init), 1 (matvec), 2 (finish)
@@ -1060,7 +1063,7 @@ __global__ void __launch_bounds__(k3Threads, 1) c3_tma_kernel(const __grid_const
           }
         }
       } else {  // finish
-        cx unv[SP];
+        cx unv[SP], stv[SP];
 #pragma unroll
         for (int j = 0; j < SP; ++j) {
           if (!((act >> j) & 1u)) continue;
@@ -1070,7 +1073,9 @@ __global__ void __launch_bounds__(k3Threads, 1) c3_tma_kernel(const __grid_const
           const cx mx = itd ? csub(xi, off(xt, cmul(dc, xi))) : xi;
           const cx d = csub(v0[j * TE + e], mx);
           acc[j] += (double)d.x * d.x + (double)d.y * d.y;
-          unv[j] = cadd(v1[j * TE + e], xi);
+          const cx uo = v1[j * TE + e];
+          unv[j] = cadd(uo, xi);
+          stv[j] = a.sums ? cadd(uo, unv[j]) : unv[j];
         }
 #pragma unroll
         for (int j = 0; j < SP; ++j) {
@@ -1078,7 +1083,7 @@ __global__ void __launch_bounds__(k3Threads, 1) c3_tma_kernel(const __grid_const
           const int pr = p0 + j;
           const size_t offp = (size_t)pr * q.N;
           a.out[offp + i] = unv[j];
-          if (a.u_store) a.u_store[((size_t)pr * q.nz + node) * q.N + i] = unv[j];
+          if (a.u_store) a.u_store[((size_t)pr * q.nz + node) * q.N + i] = stv[j];
           if (a.exit_out && t == q.L) a.exit_out[offp + i] = unv[j];
         }
       }
@@ -1139,8 +1144,8 @@ __global__ void c3_store_kernel(int N, int P, int nz, int t, const cx *__restric
 
 // grad_c[s-1][i] += sum_p lambda_p[i] conj(u_p,s[i] + u_p,s-1[i]) for the
 // current step's slice s (no atomics: one thread owns element i and loops
-// over the probes).
-__global__ void c3_grad_kernel(int N, int P, int nz, const C3State *st, const cx *__restrict__ lam,
+// over the probes).  sums: u_fwd holds the pair sums u_s + u_{s-1} at s.
+__global__ void c3_grad_kernel(int N, int P, int nz, int sums, const C3State *st, const cx *__restrict__ lam,
                                const cx *__restrict__ u_fwd, cx *grad_c) {
   constexpr int G = 8;  // probes whose loads are issued together
   const int s = st->s;
@@ -1153,7 +1158,7 @@ __global__ void c3_grad_kernel(int N, int P, int nz, const C3State *st, const cx
         if (p0 + j < P) {
           const size_t pr = p0 + j;
           a[j] = u_fwd[(pr * nz + s) * N + i];
-          b[j] = u_fwd[(pr * nz + s - 1) * N + i];
+          b[j] = sums ? czero() : u_fwd[(pr * nz + s - 1) * N + i];
           l[j] = lam[pr * N + i];
         }
       }
@@ -1934,6 +1939,10 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
     return set_error(TP_ERR_INVALID, "the gradient needs TP_MODE_ADJOINT_EXACT with u_fwd and grad_c");
   if (a->mode == TP_MODE_ADJOINT_EXACT && a->probes != nullptr)
     return set_error(TP_ERR_INVALID, "TP_MODE_ADJOINT_EXACT starts from lambda = 0 (probes must be NULL)");
+  const int sums = (a->kernels & TP_CN3D_PAIR_SUMS) != 0 ? 1 : 0;
+  if (sums && ((a->u_store != nullptr && a->mode != TP_MODE_FORWARD) ||
+               (a->mode != TP_MODE_FORWARD && a->mode != TP_MODE_ADJOINT_EXACT)))
+    return set_error(TP_ERR_INVALID, "pair sums: a FORWARD march stores them, an ADJOINT_EXACT one reads them");
   if ((reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return set_error(TP_ERR_INVALID, "workspace must be 256-byte aligned");
   C3Work w = c3_layout(static_cast<char *>(workspace), N, P);
   if (workspace_bytes < w.bytes) return set_error(TP_ERR_WORKSPACE, "3D workspace %zu B < %zu B", workspace_bytes, w.bytes);
@@ -1971,7 +1980,7 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
   // round-off keep the Krylov march below.
   cudaStreamCaptureStatus poly_cap = cudaStreamCaptureStatusNone;
   TP_CHECK_CUDA(cudaStreamIsCapturing(st, &poly_cap));
-  if (a->precond == 1 && a->kernels == 0 && a->launch == 0 && a->host_check != 0 && a->train_every <= 0 &&
+  if (a->precond == 1 && (a->kernels & 0xff) == 0 && a->launch == 0 && a->host_check != 0 && a->train_every <= 0 &&
       a->mode != TP_MODE_REVERSE && poly_cap == cudaStreamCaptureStatusNone && q.mu_x.x == 0.0 && q.mu_y.x == 0.0) {
     c3_diag_kernel<<<296, 256, 0, st>>>(N, nf, q.sigma, q.conj_t, static_cast<const cx *>(op->kc),
                                         static_cast<const cx *>(op->kw), static_cast<const cx *>(op->ke),
@@ -2016,6 +2025,7 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
     job.exit_out = static_cast<cx *>(a->exit_out);
     job.grad_c = static_cast<cx *>(a->grad_c);
     job.stats = a->stats;
+    job.sums = sums;
     int ran = 0;
     const int prc = c3_poly_march(job, st, &ran);
     if (prc != TP_OK || ran) return prc;
@@ -2220,11 +2230,12 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
       ta.u_store = ust;
       ta.exit_out = exit_out;
       ta.flip = flip ? 1 : 0;
+      ta.sums = sums;
       t_fin.kern<<<t_fin.grid, k3Threads, t_fin.smem, s>>>(tmaps.mh, tmaps.mv, tmaps.md, tmaps.md4, q, w.st, ta, w.K, derr);
       return;
     }
 #endif
-    c3_finish_kernel<<<sg_fin, k3Threads, 0, s>>>(q, w.st, w.cdl, w.x, w.r0, w.u, w.K, ust, flip ? 1 : 0, exit_out);
+    c3_finish_kernel<<<sg_fin, k3Threads, 0, s>>>(q, w.st, w.cdl, w.x, w.r0, w.u, w.K, ust, flip ? 1 : 0, sums, exit_out);
   };
   // step head: slice state, operators, right-hand side, Krylov start
   auto step_head = [&](cudaStream_t s, int use_cond, cudaGraphConditionalHandle outer, cudaGraphConditionalHandle inner) {
@@ -2269,7 +2280,7 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
     finish(s);
     c3_stats_kernel<<<1, one_cta, 0, s>>>(w.K, P, tol2, stats, w.st);
     if (a->grad_c)
-      c3_grad_kernel<<<eb, 256, 0, s>>>(N, P, nz, w.st, w.u, static_cast<const cx *>(a->u_fwd),
+      c3_grad_kernel<<<eb, 256, 0, s>>>(N, P, nz, sums, w.st, w.u, static_cast<const cx *>(a->u_fwd),
                                         static_cast<cx *>(a->grad_c));
   };
 
@@ -2407,7 +2418,7 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
     }
     c3_stats_kernel<<<1, one_cta, 0, st>>>(w.K, P, tol2, stats, w.st);
     if (a->grad_c)
-      c3_grad_kernel<<<eb, 256, 0, st>>>(N, P, nz, w.st, w.u, static_cast<const cx *>(a->u_fwd),
+      c3_grad_kernel<<<eb, 256, 0, st>>>(N, P, nz, sums, w.st, w.u, static_cast<const cx *>(a->u_fwd),
                                          static_cast<cx *>(a->grad_c));
   }
   if (stats) c3_flag_kernel<<<1, 1, 0, st>>>(stats, 0);

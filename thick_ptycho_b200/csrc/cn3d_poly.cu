@@ -177,10 +177,12 @@ struct PolyStep {
   int use_u;  // 0: the first step of the exact adjoint (zero state, source only)
   const float2 *src_exit, *src_shared;
   float2 *store;         // the step's slice of u_store, probe stride store_stride
+  float keep;            // what is stored: u_new + keep u (keep = 1: pair sums)
   size_t store_stride;
   double2 *norms;  // per probe: ||b||^2, ||b - (I - P) d||^2
   // gradient (exact adjoint): the slice's accumulator += sum_p u_new conj(f1 + f0),
-  // f1 and f0 the forward field at the slice's two nodes (probe stride store_stride)
+  // f1 and f0 the forward field at the slice's two nodes (probe stride
+  // store_stride; f0 NULL: f1 is their sum)
   const float2 *f0, *f1;
   float2 *grad;
 };
@@ -392,7 +394,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
     if (GRAD && ALIGNED) {
       // the forward field's rows on their way into L2 while the slice is solved
       const int i = lane >> 1, b = gb0 + i, r = wp * kPR + i;
-      if (lane < 2 * kPR && r >= q.hy && r < q.hy + q.ch && b < q.nb) {
+      if (lane < 2 * kPR && ((lane & 1) || q.f0 != nullptr) && r >= q.hy && r < q.hy + q.ch && b < q.nb) {
         const int c0 = f0 + q.hx, cols = min(q.cw, q.nf - c0);
         const float2 *src = ((lane & 1) ? q.f1 : q.f0) + (size_t)p * q.store_stride + (size_t)b * q.nf + c0;
         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(cols * (int)sizeof(float2)) : "memory");
@@ -498,7 +500,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
           const float2 d0 = upk(odd ? yb[i] : ya[i]), d1 = upk(odd ? ya[i] : yb[i]);
           const size_t at = (size_t)b * q.nf + gf;
           const float4 v = make_float4(uo.x + d0.x, uo.y + d0.y, uo.z + d1.x, uo.w + d1.y);
-          auto put = [&](float2 *dst, bool stream) {
+          auto put = [&](float2 *dst, float4 v, bool stream) {
             if (ALIGNED) {
               if (core0) {
                 if (stream) __stcs(reinterpret_cast<float4 *>(dst), v);
@@ -509,29 +511,61 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
               if (core1) dst[1] = make_float2(v.z, v.w);
             }
           };
-          put(q.un + (size_t)p * q.N + at, false);
-          if (q.store != nullptr) put(q.store + (size_t)p * q.store_stride + at, true);
-          if (GRAD) {
-            const size_t fo = (size_t)p * q.store_stride + at;
-            if (ALIGNED) {
-              if (core0) {
-                const float4 a = *reinterpret_cast<const float4 *>(q.f0 + fo);
-                const float4 c = *reinterpret_cast<const float4 *>(q.f1 + fo);
-                const float2 g0 = cmulc(make_float2(v.x, v.y), make_float2(a.x + c.x, a.y + c.y));
-                const float2 g1 = cmulc(make_float2(v.z, v.w), make_float2(a.z + c.z, a.w + c.w));
-                red_add_cx2(reinterpret_cast<float4 *>(q.grad + at), make_float4(g0.x, g0.y, g1.x, g1.y));
-              }
-            } else {
-              if (core0) red_add_cx(q.grad + at, cmulc(make_float2(v.x, v.y), cadd(q.f0[fo], q.f1[fo])));
-              if (core1) red_add_cx(q.grad + at + 1, cmulc(make_float2(v.z, v.w), cadd(q.f0[fo + 1], q.f1[fo + 1])));
-            }
-          }
+          put(q.un + (size_t)p * q.N + at, v, false);
+          if (q.store != nullptr)
+            put(q.store + (size_t)p * q.store_stride + at,
+                make_float4(fmaf(q.keep, uo.x, v.x), fmaf(q.keep, uo.y, v.y), fmaf(q.keep, uo.z, v.z),
+                            fmaf(q.keep, uo.w, v.w)),
+                true);
           const float jx = odd ? Ji[i].x : Ji[i].z, jy = odd ? Ji[i].y : Ji[i].w;
           const float2 rg = upk(cmadd(jx, jy, s, odd ? g[i].a : g[i].b)), rd = upk(yb[i]);
           const float rx = rg.x - rd.x, ry = rg.y - rd.y;
           if (odd ? core0 : core1) nr2 = fmaf(__fdividef(1.f, fmaf(jx, jx, jy * jy)), fmaf(rx, rx, ry * ry), nr2);
         }
         prev = ya[i];
+      }
+    }
+    if (GRAD) {
+      // every row's forward field before the first reduction (Ji and g are done with)
+      float4 fs[kPR];
+#pragma unroll
+      for (int i = 0; i < kPR; ++i) {
+        const int r = wp * kPR + i, b = gb0 + i;
+        const size_t fo = (size_t)p * q.store_stride + (size_t)b * q.nf + gf;
+        fs[i] = zero4;
+        if (r < q.hy || r >= q.hy + q.ch || b >= q.nb) continue;
+        if (ALIGNED) {
+          if (core0) {
+            fs[i] = __ldcs(reinterpret_cast<const float4 *>(q.f1 + fo));
+            if (q.f0 != nullptr) {
+              const float4 c0 = *reinterpret_cast<const float4 *>(q.f0 + fo);
+              fs[i] = make_float4(c0.x + fs[i].x, c0.y + fs[i].y, c0.z + fs[i].z, c0.w + fs[i].w);
+            }
+          }
+        } else {
+          if (core0) fs[i].x = q.f1[fo].x, fs[i].y = q.f1[fo].y;
+          if (core1) fs[i].z = q.f1[fo + 1].x, fs[i].w = q.f1[fo + 1].y;
+          if (q.f0 != nullptr) {
+            if (core0) fs[i].x += q.f0[fo].x, fs[i].y += q.f0[fo].y;
+            if (core1) fs[i].z += q.f0[fo + 1].x, fs[i].w += q.f0[fo + 1].y;
+          }
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < kPR; ++i) {
+        const int r = wp * kPR + i, b = gb0 + i;
+        if (r < q.hy || r >= q.hy + q.ch || b >= q.nb) continue;
+        const float4 uo = ut[r][lane];
+        const float2 d0 = upk((i & 1) ? yb[i] : ya[i]), d1 = upk((i & 1) ? ya[i] : yb[i]);
+        const float2 g0 = cmulc(make_float2(uo.x + d0.x, uo.y + d0.y), make_float2(fs[i].x, fs[i].y));
+        const float2 g1 = cmulc(make_float2(uo.z + d1.x, uo.w + d1.y), make_float2(fs[i].z, fs[i].w));
+        float2 *dst = q.grad + (size_t)b * q.nf + gf;
+        if (ALIGNED) {
+          if (core0) red_add_cx2(reinterpret_cast<float4 *>(dst), make_float4(g0.x, g0.y, g1.x, g1.y));
+        } else {
+          if (core0) red_add_cx(dst, g0);
+          if (core1) red_add_cx(dst + 1, g1);
+        }
       }
     }
 #pragma unroll
@@ -808,11 +842,12 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
     q.src_exit = t == 1 ? job.src_exit : nullptr;
     q.src_shared = job.src_shared ? job.src_shared + (size_t)(t - 1) * N : nullptr;
     q.store = job.u_store ? job.u_store + (size_t)(flip ? L - t : t) * N : nullptr;
+    q.keep = job.sums ? 1.f : 0.f;
     q.store_stride = stride;
     q.norms = norms + (size_t)(t - 1) * P;
     const bool src = q.src_exit != nullptr || q.src_shared != nullptr || !q.use_u;
     if (job.grad_c) {
-      q.f0 = job.u_fwd + (size_t)(s - 1) * N;
+      q.f0 = job.sums ? nullptr : job.u_fwd + (size_t)(s - 1) * N;
       q.f1 = job.u_fwd + (size_t)s * N;
       q.grad = job.grad_c + (size_t)(s - 1) * N;
     }

@@ -29,6 +29,7 @@ struct C3PolyJob {
   const float2 *probes, *src_exit, *src_shared, *u_fwd;
   float2 *u_store, *exit_out, *grad_c;
   int *stats;
+  int sums;  // u_store and u_fwd hold pair sums u_s + u_{s-1} at s
 };
 
 // Widths up to this many rows or columns fit the small arrays.
