@@ -184,6 +184,7 @@ struct PolyStep {
   // f1 and f0 the forward field at the slice's two nodes (probe stride
   // store_stride; f0 NULL: f1 is their sum)
   const float2 *f0, *f1;
+  int f_node;  // the pair sums' slice (tensor map coordinate)
   float2 *grad;
 };
 
@@ -289,8 +290,8 @@ __device__ __forceinline__ unsigned long long cmadd(float jx, float jy, unsigned
 
 // One tile and probe group.  EDGE: the tile holds one of the image's first or
 // last two rows, whose row couplings may differ from the interior's.
-template <bool ALIGNED, bool SRC, bool GRAD, bool EDGE>
-__device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep &q, PolySmem &sm, int *err) {
+template <bool ALIGNED, bool SRC, int GRAD, bool EDGE>
+__device__ __forceinline__ void poly_tile(const CUtensorMap &map, const CUtensorMap &fmap, const PolyStep &q, PolySmem &sm, int *err) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int tx = blockIdx.x % q.tiles_x, ty = blockIdx.x / q.tiles_x;
   const int f0 = tx * q.cw - q.hx, b0 = ty * q.ch - q.hy;
@@ -305,9 +306,14 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
     fence_mbar_init();
   }
   __syncthreads();
-  auto issue = [&](int j) {
-    mbar_arrive_expect_tx(&sm.bar[j & 1], kTile);
-    tma_load_4d(sm.u[j & 1], &map, f0, b0, p0 + j, q.sel, &sm.bar[j & 1]);
+  auto issue = [&](int j) {  // thread 0: probe j's tile of u
+    const int buf = GRAD == 2 ? 0 : j & 1;
+    mbar_arrive_expect_tx(&sm.bar[buf], kTile);
+    tma_load_4d(sm.u[buf], &map, f0, b0, p0 + j, q.sel, &sm.bar[buf]);
+  };
+  auto issue_f = [&](int j) {  // thread 0: probe j's tile of the forward pair sums
+    mbar_arrive_expect_tx(&sm.bar[1], kTile);
+    tma_load_4d(sm.u[1], &fmap, f0, b0, q.f_node, p0 + j, &sm.bar[1]);
   };
   // The next step's CTAs may start as this one's leave: what they do before
   // their own wait reads only the slices' diagonals and the weights.
@@ -359,22 +365,39 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
   __syncthreads();
   if (staged && threadIdx.x == 0) {
     issue(0);
-    if (np > 1) issue(1);
+    if (GRAD != 2 && np > 1) issue(1);
   }
+  if (GRAD == 2 && threadIdx.x == 0) issue_f(0);
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   const bool core0 = 2 * lane >= q.hx && 2 * lane < q.hx + q.cw && in0;
+  // this warp's rows in the core (a bit each), and the thread's first pixel
+  unsigned rows = 0;
+#pragma unroll
+  for (int i = 0; i < kPR; ++i) {
+    const int r = wp * kPR + i;
+    if (r >= q.hy && r < q.hy + q.ch && b0 + r < q.nb) rows |= 1u << i;
+  }
+  const int at0 = gb0 * q.nf + gf;
   const bool core1 = 2 * lane + 1 >= q.hx && 2 * lane + 1 < q.hx + q.cw && in1;
   for (int j = 0; j < np; ++j) {
-    const int p = p0 + j, buf = ALIGNED ? (j & 1) : 0;
-    if (staged) {
-      const bool got = mbar_wait_bounded(&sm.bar[buf], (uint32_t)((j >> 1) & 1), err);
-      if (__syncthreads_or(!got)) {
-        // give up: the copies in flight land before the CTA exits
-        if (threadIdx.x == 0) {
+    const int p = p0 + j, buf = (ALIGNED && GRAD != 2) ? (j & 1) : 0;
+    // a wait gave up: the copies in flight land before the CTA exits
+    auto give_up = [&]() {
+      if (threadIdx.x == 0) {
+        if (GRAD == 2) {
+          if (staged) mbar_wait_bounded(&sm.bar[0], (uint32_t)(j & 1), nullptr);
+          mbar_wait_bounded(&sm.bar[1], (uint32_t)(j & 1), nullptr);
+        } else {
           mbar_wait_bounded(&sm.bar[buf], (uint32_t)((j >> 1) & 1), nullptr);
           if (j + 1 < np) mbar_wait_bounded(&sm.bar[buf ^ 1], (uint32_t)(((j + 1) >> 1) & 1), nullptr);
         }
-        __syncthreads();
+      }
+      __syncthreads();
+    };
+    if (staged) {
+      const bool got = mbar_wait_bounded(&sm.bar[buf], (uint32_t)((GRAD == 2 ? j : j >> 1) & 1), err);
+      if (__syncthreads_or(!got)) {
+        give_up();
         return;
       }
     } else {
@@ -391,7 +414,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
       }
       __syncthreads();
     }
-    if (GRAD && ALIGNED) {
+    if (GRAD == 1 && ALIGNED) {
       // the forward field's rows on their way into L2 while the slice is solved
       const int i = lane >> 1, b = gb0 + i, r = wp * kPR + i;
       if (lane < 2 * kPR && ((lane & 1) || q.f0 != nullptr) && r >= q.hy && r < q.hy + q.ch && b < q.nb) {
@@ -437,7 +460,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
             }
           }
         }
-        if (r >= q.hy && r < q.hy + q.ch && b < q.nb) {
+        if ((rows >> i) & 1u) {
           if (core0) nb2 = fmaf(bv.x, bv.x, fmaf(bv.y, bv.y, nb2));
           if (core1) nb2 = fmaf(bv.z, bv.z, fmaf(bv.w, bv.w, nb2));
         }
@@ -488,17 +511,19 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
     {
       unsigned long long prev, below;
       exchange(ya, 1, prev, below);
+      float2 *un = q.un + ((ptrdiff_t)p * q.N + at0);
+      float2 *store = q.store + ((ptrdiff_t)p * (ptrdiff_t)q.store_stride + at0);
 #pragma unroll
       for (int i = 0; i < kPR; ++i) {
-        const int r = wp * kPR + i, b = gb0 + i;
+        const int r = wp * kPR + i;
         const bool odd = (i & 1) != 0;
         const unsigned long long next = i + 1 < kPR ? ya[i + 1] : below;
         const unsigned long long s = odd ? poly_half<EDGE, 0>(ya[i], prev, next, w, &sm.roww[r])
                                          : poly_half<EDGE, 1>(ya[i], prev, next, w, &sm.roww[r]);
-        if (r >= q.hy && r < q.hy + q.ch && b < q.nb) {
+        if ((rows >> i) & 1u) {
           const float4 uo = ut[r][lane];
           const float2 d0 = upk(odd ? yb[i] : ya[i]), d1 = upk(odd ? ya[i] : yb[i]);
-          const size_t at = (size_t)b * q.nf + gf;
+          const int row = i * q.nf;
           const float4 v = make_float4(uo.x + d0.x, uo.y + d0.y, uo.z + d1.x, uo.w + d1.y);
           auto put = [&](float2 *dst, float4 v, bool stream) {
             if (ALIGNED) {
@@ -511,9 +536,9 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
               if (core1) dst[1] = make_float2(v.z, v.w);
             }
           };
-          put(q.un + (size_t)p * q.N + at, v, false);
+          put(un + row, v, false);
           if (q.store != nullptr)
-            put(q.store + (size_t)p * q.store_stride + at,
+            put(store + row,
                 make_float4(fmaf(q.keep, uo.x, v.x), fmaf(q.keep, uo.y, v.y), fmaf(q.keep, uo.z, v.z),
                             fmaf(q.keep, uo.w, v.w)),
                 true);
@@ -525,16 +550,25 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
         prev = ya[i];
       }
     }
-    if (GRAD) {
+    if (GRAD == 2) {
+      const bool got = mbar_wait_bounded(&sm.bar[1], (uint32_t)(j & 1), err);
+      if (__syncthreads_or(!got)) {
+        give_up();
+        return;
+      }
+    }
+    if (GRAD != 0) {
       // every row's forward field before the first reduction (Ji and g are done with)
       float4 fs[kPR];
+      const ptrdiff_t fo0 = (ptrdiff_t)p * (ptrdiff_t)q.store_stride + at0;
 #pragma unroll
       for (int i = 0; i < kPR; ++i) {
-        const int r = wp * kPR + i, b = gb0 + i;
-        const size_t fo = (size_t)p * q.store_stride + (size_t)b * q.nf + gf;
         fs[i] = zero4;
-        if (r < q.hy || r >= q.hy + q.ch || b >= q.nb) continue;
-        if (ALIGNED) {
+        if (!((rows >> i) & 1u)) continue;
+        const ptrdiff_t fo = fo0 + i * q.nf;
+        if (GRAD == 2) {
+          fs[i] = sm.u[1][wp * kPR + i][lane];
+        } else if (ALIGNED) {
           if (core0) {
             fs[i] = __ldcs(reinterpret_cast<const float4 *>(q.f1 + fo));
             if (q.f0 != nullptr) {
@@ -551,15 +585,15 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
           }
         }
       }
+      float2 *grad = q.grad + at0;
 #pragma unroll
       for (int i = 0; i < kPR; ++i) {
-        const int r = wp * kPR + i, b = gb0 + i;
-        if (r < q.hy || r >= q.hy + q.ch || b >= q.nb) continue;
-        const float4 uo = ut[r][lane];
+        if (!((rows >> i) & 1u)) continue;
+        const float4 uo = ut[wp * kPR + i][lane];
         const float2 d0 = upk((i & 1) ? yb[i] : ya[i]), d1 = upk((i & 1) ? ya[i] : yb[i]);
         const float2 g0 = cmulc(make_float2(uo.x + d0.x, uo.y + d0.y), make_float2(fs[i].x, fs[i].y));
         const float2 g1 = cmulc(make_float2(uo.z + d1.x, uo.w + d1.y), make_float2(fs[i].z, fs[i].w));
-        float2 *dst = q.grad + (size_t)b * q.nf + gf;
+        float2 *dst = grad + i * q.nf;
         if (ALIGNED) {
           if (core0) red_add_cx2(reinterpret_cast<float4 *>(dst), make_float4(g0.x, g0.y, g1.x, g1.y));
         } else {
@@ -576,7 +610,13 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
     if (lane == 0) sm.red[wp] = make_float2(nb2, nr2);
     __syncthreads();  // every thread is done with this probe's tile; the partial norms are in
     if (threadIdx.x == 0) {
-      if (staged && j + 2 < np) {
+      if (GRAD == 2) {
+        if (j + 1 < np) {
+          fence_proxy_async_smem();
+          if (staged) issue(j + 1);
+          issue_f(j + 1);
+        }
+      } else if (staged && j + 2 < np) {
         fence_proxy_async_smem();
         issue(j + 2);
       }
@@ -593,15 +633,17 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
 }
 
 // SRC: the step has a source, or (use_u = 0) nothing but a source.  GRAD: the step
-// adds its gradient contributions.
-template <bool ALIGNED, bool SRC, bool GRAD>
+// adds its gradient contributions (2: from pair sums that arrive as a tile of
+// their own, in the place of the next probe's u).
+template <bool ALIGNED, bool SRC, int GRAD>
 __global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_constant__ CUtensorMap map,
+                                                               const __grid_constant__ CUtensorMap fmap,
                                                                const __grid_constant__ PolyStep q, int *err) {
   extern __shared__ __align__(128) unsigned char raw[];
   PolySmem &sm = *reinterpret_cast<PolySmem *>(raw);
   const int b0 = (int)(blockIdx.x / q.tiles_x) * q.ch - q.hy;
-  if (b0 <= 1 || b0 + kPH > q.nb - 2) poly_tile<ALIGNED, SRC, GRAD, true>(map, q, sm, err);
-  else poly_tile<ALIGNED, SRC, GRAD, false>(map, q, sm, err);
+  if (b0 <= 1 || b0 + kPH > q.nb - 2) poly_tile<ALIGNED, SRC, GRAD, true>(map, fmap, q, sm, err);
+  else poly_tile<ALIGNED, SRC, GRAD, false>(map, fmap, q, sm, err);
 }
 
 // Statistics of every solve of the march: m iterations each (none where the
@@ -798,13 +840,26 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
   q.roww = job.roww;
   q.my = sl.my;
   const size_t smem = sizeof(PolySmem) + 128;
-  using PolyKernel = void (*)(const CUtensorMap, const PolyStep, int *);
-  // [source][gradient]
-  const PolyKernel kerns[4] = {
-      aligned ? c3_poly_kernel<true, false, false> : c3_poly_kernel<false, false, false>,
-      aligned ? c3_poly_kernel<true, false, true> : c3_poly_kernel<false, false, true>,
-      aligned ? c3_poly_kernel<true, true, false> : c3_poly_kernel<false, true, false>,
-      aligned ? c3_poly_kernel<true, true, true> : c3_poly_kernel<false, true, true>};
+  // the gradient from pair sums stages them by tensor copies as well
+  CUtensorMap fmap{};
+  int grad = job.grad_c ? 1 : 0;
+  if (aligned && job.grad_c && job.sums) {
+    const cuuint64_t dims[4] = {(cuuint64_t)nf, (cuuint64_t)nb, (cuuint64_t)nz, (cuuint64_t)P};
+    const cuuint64_t str[3] = {(cuuint64_t)nf * sizeof(float2), (cuuint64_t)N * sizeof(float2),
+                               (cuuint64_t)N * nz * sizeof(float2)};
+    const cuuint32_t box[4] = {kPW, kPH, 1, 1}, es[4] = {1, 1, 1, 1};
+    if (encoder()(&fmap, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<float2 *>(job.u_fwd), dims, str, box, es,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
+      grad = 2;
+  }
+  using PolyKernel = void (*)(const CUtensorMap, const CUtensorMap, const PolyStep, int *);
+  PolyKernel kerns[2];  // without and with a source
+  if (aligned && grad == 2) kerns[0] = c3_poly_kernel<true, false, 2>, kerns[1] = c3_poly_kernel<true, true, 2>;
+  else if (aligned && grad) kerns[0] = c3_poly_kernel<true, false, 1>, kerns[1] = c3_poly_kernel<true, true, 1>;
+  else if (aligned) kerns[0] = c3_poly_kernel<true, false, 0>, kerns[1] = c3_poly_kernel<true, true, 0>;
+  else if (grad) kerns[0] = c3_poly_kernel<false, false, 1>, kerns[1] = c3_poly_kernel<false, true, 1>;
+  else kerns[0] = c3_poly_kernel<false, false, 0>, kerns[1] = c3_poly_kernel<false, true, 0>;
   for (PolyKernel k : kerns)
     TP_CHECK_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
 
@@ -849,6 +904,7 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
     if (job.grad_c) {
       q.f0 = job.sums ? nullptr : job.u_fwd + (size_t)(s - 1) * N;
       q.f1 = job.u_fwd + (size_t)s * N;
+      q.f_node = s;
       q.grad = job.grad_c + (size_t)(s - 1) * N;
     }
     cudaLaunchConfig_t cfg = {};
@@ -861,7 +917,7 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = fresh ? 0 : 1;  // behind another kernel than a step's: after all of it
-    TP_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kerns[(src ? 2 : 0) + (job.grad_c ? 1 : 0)], map, q, err));
+    TP_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kerns[src ? 1 : 0], map, fmap, q, err));
     fresh = false;
   }
   if (job.stats) c3_poly_stats_kernel<<<32, 256, 0, st>>>(norms, L * P, q.m, job.tol * job.tol, job.stats);
