@@ -184,7 +184,6 @@ struct PolyStep {
   // f1 and f0 the forward field at the slice's two nodes (probe stride
   // store_stride; f0 NULL: f1 is their sum)
   const float2 *f0, *f1;
-  int f_node;  // the pair sums' slice (tensor map coordinate)
   float2 *grad;
 };
 
@@ -291,7 +290,7 @@ __device__ __forceinline__ unsigned long long cmadd(float jx, float jy, unsigned
 // One tile and probe group.  EDGE: the tile holds one of the image's first or
 // last two rows, whose row couplings may differ from the interior's.
 template <bool ALIGNED, bool SRC, int GRAD, bool EDGE>
-__device__ __forceinline__ void poly_tile(const CUtensorMap &map, const CUtensorMap &fmap, const PolyStep &q, PolySmem &sm, int *err) {
+__device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep &q, PolySmem &sm, int *err) {
   const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
   const int tx = blockIdx.x % q.tiles_x, ty = blockIdx.x / q.tiles_x;
   const int f0 = tx * q.cw - q.hx, b0 = ty * q.ch - q.hy;
@@ -310,10 +309,6 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const CUtensor
     const int buf = GRAD == 2 ? 0 : j & 1;
     mbar_arrive_expect_tx(&sm.bar[buf], kTile);
     tma_load_4d(sm.u[buf], &map, f0, b0, p0 + j, q.sel, &sm.bar[buf]);
-  };
-  auto issue_f = [&](int j) {  // thread 0: probe j's tile of the forward pair sums
-    mbar_arrive_expect_tx(&sm.bar[1], kTile);
-    tma_load_4d(sm.u[1], &fmap, f0, b0, q.f_node, p0 + j, &sm.bar[1]);
   };
   // The next step's CTAs may start as this one's leave: what they do before
   // their own wait reads only the slices' diagonals and the weights.
@@ -367,7 +362,6 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const CUtensor
     issue(0);
     if (GRAD != 2 && np > 1) issue(1);
   }
-  if (GRAD == 2 && threadIdx.x == 0) issue_f(0);
   const float4 zero4 = make_float4(0.f, 0.f, 0.f, 0.f);
   const bool core0 = 2 * lane >= q.hx && 2 * lane < q.hx + q.cw && in0;
   // this warp's rows in the core (a bit each), and the thread's first pixel
@@ -381,23 +375,25 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const CUtensor
   const bool core1 = 2 * lane + 1 >= q.hx && 2 * lane + 1 < q.hx + q.cw && in1;
   for (int j = 0; j < np; ++j) {
     const int p = p0 + j, buf = (ALIGNED && GRAD != 2) ? (j & 1) : 0;
-    // a wait gave up: the copies in flight land before the CTA exits
-    auto give_up = [&]() {
-      if (threadIdx.x == 0) {
-        if (GRAD == 2) {
-          if (staged) mbar_wait_bounded(&sm.bar[0], (uint32_t)(j & 1), nullptr);
-          mbar_wait_bounded(&sm.bar[1], (uint32_t)(j & 1), nullptr);
-        } else {
-          mbar_wait_bounded(&sm.bar[buf], (uint32_t)((j >> 1) & 1), nullptr);
-          if (j + 1 < np) mbar_wait_bounded(&sm.bar[buf ^ 1], (uint32_t)(((j + 1) >> 1) & 1), nullptr);
-        }
-      }
-      __syncthreads();
-    };
+    const ptrdiff_t fo0 = (ptrdiff_t)p * (ptrdiff_t)q.store_stride + at0;
+    if (GRAD == 2) {
+      // the forward pair sums of this thread's own pixels, on their way while the
+      // slice is solved (no tensor copy: those of u would queue behind its misses)
+#pragma unroll
+      for (int i = 0; i < kPR; ++i)
+        if (core0 && ((rows >> i) & 1u)) cp_async16(&sm.u[1][wp * kPR + i][lane], q.f1 + fo0 + i * q.nf);
+    }
     if (staged) {
-      const bool got = mbar_wait_bounded(&sm.bar[buf], (uint32_t)((GRAD == 2 ? j : j >> 1) & 1), err);
+      const uint32_t phase = (uint32_t)((GRAD == 2 ? j : j >> 1) & 1);
+      const bool got = mbar_wait_bounded(&sm.bar[buf], phase, err);
       if (__syncthreads_or(!got)) {
-        give_up();
+        // give up: the copies in flight land before the CTA exits
+        cp_async_wait_all();
+        if (threadIdx.x == 0) {
+          mbar_wait_bounded(&sm.bar[buf], phase, nullptr);
+          if (GRAD != 2 && j + 1 < np) mbar_wait_bounded(&sm.bar[buf ^ 1], (uint32_t)(((j + 1) >> 1) & 1), nullptr);
+        }
+        __syncthreads();
         return;
       }
     } else {
@@ -550,17 +546,10 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const CUtensor
         prev = ya[i];
       }
     }
-    if (GRAD == 2) {
-      const bool got = mbar_wait_bounded(&sm.bar[1], (uint32_t)(j & 1), err);
-      if (__syncthreads_or(!got)) {
-        give_up();
-        return;
-      }
-    }
     if (GRAD != 0) {
       // every row's forward field before the first reduction (Ji and g are done with)
       float4 fs[kPR];
-      const ptrdiff_t fo0 = (ptrdiff_t)p * (ptrdiff_t)q.store_stride + at0;
+      if (GRAD == 2) cp_async_wait_all();
 #pragma unroll
       for (int i = 0; i < kPR; ++i) {
         fs[i] = zero4;
@@ -611,10 +600,9 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const CUtensor
     __syncthreads();  // every thread is done with this probe's tile; the partial norms are in
     if (threadIdx.x == 0) {
       if (GRAD == 2) {
-        if (j + 1 < np) {
+        if (staged && j + 1 < np) {
           fence_proxy_async_smem();
-          if (staged) issue(j + 1);
-          issue_f(j + 1);
+          issue(j + 1);
         }
       } else if (staged && j + 2 < np) {
         fence_proxy_async_smem();
@@ -633,17 +621,16 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const CUtensor
 }
 
 // SRC: the step has a source, or (use_u = 0) nothing but a source.  GRAD: the step
-// adds its gradient contributions (2: from pair sums that arrive as a tile of
-// their own, in the place of the next probe's u).
+// adds its gradient contributions (2: from pair sums copied into the place of
+// the next probe's u).
 template <bool ALIGNED, bool SRC, int GRAD>
 __global__ void __launch_bounds__(kPThreads, 2) c3_poly_kernel(const __grid_constant__ CUtensorMap map,
-                                                               const __grid_constant__ CUtensorMap fmap,
                                                                const __grid_constant__ PolyStep q, int *err) {
   extern __shared__ __align__(128) unsigned char raw[];
   PolySmem &sm = *reinterpret_cast<PolySmem *>(raw);
   const int b0 = (int)(blockIdx.x / q.tiles_x) * q.ch - q.hy;
-  if (b0 <= 1 || b0 + kPH > q.nb - 2) poly_tile<ALIGNED, SRC, GRAD, true>(map, fmap, q, sm, err);
-  else poly_tile<ALIGNED, SRC, GRAD, false>(map, fmap, q, sm, err);
+  if (b0 <= 1 || b0 + kPH > q.nb - 2) poly_tile<ALIGNED, SRC, GRAD, true>(map, q, sm, err);
+  else poly_tile<ALIGNED, SRC, GRAD, false>(map, q, sm, err);
 }
 
 // Statistics of every solve of the march: m iterations each (none where the
@@ -840,20 +827,8 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
   q.roww = job.roww;
   q.my = sl.my;
   const size_t smem = sizeof(PolySmem) + 128;
-  // the gradient from pair sums stages them by tensor copies as well
-  CUtensorMap fmap{};
-  int grad = job.grad_c ? 1 : 0;
-  if (aligned && job.grad_c && job.sums) {
-    const cuuint64_t dims[4] = {(cuuint64_t)nf, (cuuint64_t)nb, (cuuint64_t)nz, (cuuint64_t)P};
-    const cuuint64_t str[3] = {(cuuint64_t)nf * sizeof(float2), (cuuint64_t)N * sizeof(float2),
-                               (cuuint64_t)N * nz * sizeof(float2)};
-    const cuuint32_t box[4] = {kPW, kPH, 1, 1}, es[4] = {1, 1, 1, 1};
-    if (encoder()(&fmap, CU_TENSOR_MAP_DATA_TYPE_UINT64, 4, const_cast<float2 *>(job.u_fwd), dims, str, box, es,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS)
-      grad = 2;
-  }
-  using PolyKernel = void (*)(const CUtensorMap, const CUtensorMap, const PolyStep, int *);
+  const int grad = job.grad_c ? (aligned && job.sums ? 2 : 1) : 0;
+  using PolyKernel = void (*)(const CUtensorMap, const PolyStep, int *);
   PolyKernel kerns[2];  // without and with a source
   if (aligned && grad == 2) kerns[0] = c3_poly_kernel<true, false, 2>, kerns[1] = c3_poly_kernel<true, true, 2>;
   else if (aligned && grad) kerns[0] = c3_poly_kernel<true, false, 1>, kerns[1] = c3_poly_kernel<true, true, 1>;
@@ -904,7 +879,6 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
     if (job.grad_c) {
       q.f0 = job.sums ? nullptr : job.u_fwd + (size_t)(s - 1) * N;
       q.f1 = job.u_fwd + (size_t)s * N;
-      q.f_node = s;
       q.grad = job.grad_c + (size_t)(s - 1) * N;
     }
     cudaLaunchConfig_t cfg = {};
@@ -917,7 +891,7 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
     at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at;
     cfg.numAttrs = fresh ? 0 : 1;  // behind another kernel than a step's: after all of it
-    TP_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kerns[src ? 1 : 0], map, fmap, q, err));
+    TP_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kerns[src ? 1 : 0], map, q, err));
     fresh = false;
   }
   if (job.stats) c3_poly_stats_kernel<<<32, 256, 0, st>>>(norms, L * P, q.m, job.tol * job.tol, job.stats);
