@@ -325,28 +325,29 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
     sm.roww[r] = (b >= 0 && b < q.nb) ? q.roww[b] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
   const PolyWeights w = {pk(cw0.x, cw0.x), pk(cw0.y, cw0.y), pk(cw1.x, cw1.x), pk(cw1.y, cw1.y), pk(q.my, q.my)};
-  float4 Ji[kPR];  // i D^{-1} of the two columns
+  // every load before the first use, outside pixels from a clamped address
+  float4 Ji[kPR], Dr[kPR];  // i D^{-1} of the two columns
+#pragma unroll
+  for (int i = 0; i < kPR; ++i) {
+    const int row = min(max(gb0 + i, 0), q.nb - 1) * q.nf;
+    if (ALIGNED) {
+      const int at = row + min(max(gf, 0), q.nf - 2);
+      Ji[i] = *reinterpret_cast<const float4 *>(q.cdl + at);
+      Dr[i] = *reinterpret_cast<const float4 *>(q.cdr + at);
+    } else {
+      const int c0 = row + min(max(gf, 0), q.nf - 1), c1 = row + min(max(gf + 1, 0), q.nf - 1);
+      const float2 l0 = q.cdl[c0], l1 = q.cdl[c1], r0 = q.cdr[c0], r1 = q.cdr[c1];
+      Ji[i] = make_float4(l0.x, l0.y, l1.x, l1.y);
+      Dr[i] = make_float4(r0.x, r0.y, r1.x, r1.y);
+    }
+  }
 #pragma unroll
   for (int i = 0; i < kPR; ++i) {
     const int b = gb0 + i;
     const bool row = b >= 0 && b < q.nb;
-    const size_t at = (size_t)b * q.nf + gf;
-    float4 dl = make_float4(0.f, 0.f, 0.f, 0.f), dr = dl;
-    if (ALIGNED) {
-      if (row && in0) {
-        dl = *reinterpret_cast<const float4 *>(q.cdl + at);
-        dr = *reinterpret_cast<const float4 *>(q.cdr + at);
-      }
-    } else if (row) {
-      if (in0) {
-        const float2 l = q.cdl[at], r = q.cdr[at];
-        dl.x = l.x, dl.y = l.y, dr.x = r.x, dr.y = r.y;
-      }
-      if (in1) {
-        const float2 l = q.cdl[at + 1], r = q.cdr[at + 1];
-        dl.z = l.x, dl.w = l.y, dr.z = r.x, dr.w = r.y;
-      }
-    }
+    float4 dl = Ji[i], dr = Dr[i];
+    if (!row || !in0) dl.x = dl.y = dr.x = dr.y = 0.f;
+    if (!row || !in1) dl.z = dl.w = dr.z = dr.w = 0.f;
     sm.dsum[wp * kPR + i][lane] = make_float4(dl.x + dr.x, dl.y + dr.y, dl.z + dr.z, dl.w + dr.w);
     // i / (1 - d) = (di + i dr) / |1 - d|^2 with 1 - d = dr - i (-di)
     const float ax = 1.f - dl.x, ay = -dl.y, az = 1.f - dl.z, aw = -dl.w;
