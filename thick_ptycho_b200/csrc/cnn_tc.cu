@@ -280,79 +280,136 @@ __global__ void __launch_bounds__(128) conv3x3_tc_kernel(const ConvArgs a) {
 }
 
 // ------------------------------------------------------------ weight gradient
-// dW[tap][c][o] = sum_q x[q + off_tap][c] dy[q][o] and db[o] = sum_q dy[q][o]
-// over the computed pixels (dy is zero off the interior).  Thread (tap, c) of
-// 10*CIN threads keeps its 32 sums in registers (tap 9 is the bias, c = 0
-// only); a persistent CTA loops over tiles staged by bulk copies and adds its
-// sums to dW/db once at the end (fp32 CUDA cores: this runs only in training).
-template <int CIN>
-__global__ void __launch_bounds__(10 * CIN) conv3x3_wgrad_kernel(const ConvGeom g, const bf16 *x, const bf16 *dy,
-                                                                 float *dw, float *db, int ntiles, int *err) {
-  constexpr int COUT = kConvCout;
-  extern __shared__ __align__(128) uint8_t smem[];
-  const uint32_t R = conv_slab_pixels(g.Wp);
-  bf16 *sx = reinterpret_cast<bf16 *>(smem);
-  bf16 *sdy = reinterpret_cast<bf16 *>(smem + (size_t)(CIN / 8) * R * 16);
-  uint64_t *bar = reinterpret_cast<uint64_t *>(smem + (size_t)(CIN / 8) * R * 16 + (size_t)(COUT / 8) * kConvTile * 16);
-  const int tid = threadIdx.x;
-  const int tap = tid / CIN, c = tid % CIN;
-  const int ty = tap / 3, tx = tap % 3;
-  const bool active = tap < 9 || c == 0;
-  float acc[COUT];
-#pragma unroll
-  for (int o = 0; o < COUT; ++o) acc[o] = 0.f;
-  if (tid == 0) {
-    mbar_init(bar, 1);
-    fence_mbar_init();
-  }
-  __syncthreads();
-  uint32_t phase = 0;
-  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const long long l0 = g.l_begin + (long long)tile * kConvTile;
-    if (tid == 0) {
-      fence_proxy_async_smem();
-      mbar_arrive_expect_tx(bar, (CIN / 8) * R * 16 + (COUT / 8) * kConvTile * 16);
-      for (int j = 0; j < CIN / 8; ++j)
-        bulk_g2s(sx + (size_t)j * R * 8, x + ((size_t)j * g.CS + (l0 - g.Wp - 1)) * 8, R * 16, bar);
-      for (int j = 0; j < COUT / 8; ++j)
-        bulk_g2s(sdy + (size_t)j * kConvTile * 8, dy + ((size_t)j * g.CS + l0) * 8, kConvTile * 16, bar);
-    }
-    const bool ok = mbar_wait_bounded(bar, phase, err);
-    phase ^= 1u;
-    if (__syncthreads_or(!ok)) {
-      if (tid == 0) mbar_wait_bounded(bar, phase ^ 1u, nullptr);
-      __syncthreads();
-      return;
-    }
-    if (active) {
-      const bf16 *xs = sx + (size_t)(c / 8) * R * 8 + (c % 8);
-      const int off = ty * g.Wp + tx;
-#pragma unroll 2
-      for (int q = 0; q < kConvTile; ++q) {
-        const float xv = (tap < 9) ? __bfloat162float(xs[(size_t)(q + off) * 8]) : 1.f;
-#pragma unroll
-        for (int j = 0; j < COUT / 8; ++j) {
-          float d[8];
-          unpack_bf8(*reinterpret_cast<const uint4 *>(sdy + ((size_t)j * kConvTile + q) * 8), d);
-#pragma unroll
-          for (int k = 0; k < 8; ++k) acc[8 * j + k] = fmaf(xv, d[k], acc[8 * j + k]);
-        }
-      }
-    }
-    __syncthreads();
-  }
-  if (!active) return;
-  if (tap < 9) {
-#pragma unroll
-    for (int o = 0; o < COUT; ++o) atomicAdd(&dw[((size_t)tap * CIN + c) * COUT + o], acc[o]);
-  } else if (db != nullptr) {
-#pragma unroll
-    for (int o = 0; o < COUT; ++o) atomicAdd(&db[o], acc[o]);
-  }
+// dW[ty][tx][c][o] = sum_q x[q + (ty-1) Wp + (tx-1)][c] dy[q][o] and db[o] =
+// sum_q dy[q][o] over the computed pixels (dy is zero off the interior), on the
+// tensor cores with the pixels as the contraction: with k = q + tx - 1,
+//   D_ty[(tx, o)][c] += sum_k dy[k - (tx-1)][o] x[k + (ty-1) Wp][c].
+// A (128 x 16 per instruction) is dy in three shifted copies, 4 channel chunks
+// each (rows 96..127 read the next planes and are dropped), B (16 x CIN) the x row
+// of one ty; both are MN-major (8 channels of a pixel contiguous), so a pixel's 16
+// bytes are a row of a core matrix, 8 pixels 128 bytes apart along K (LBO) and the
+// channel chunks one plane apart along M / N (SBO).  A CTA of 4 warps loops over
+// tiles of kWgTile pixels (bulk copies, mbarrier), its three accumulators stay in
+// TMEM for all of them and are added to dW once at the end.  Both operands leave
+// and reach memory once per tile and the 3 x 16 instructions of a tile take under
+// a microsecond, so two CTAs per SM alternate between copies and products.
+// 256 x 256, 4 images, 32 channels: 28 us against 326 us on the fp32 cores.
+constexpr int kWgTile = 256;
+
+__host__ __device__ constexpr uint32_t wgrad_planes(int cin) { return 12u + 3u * (uint32_t)(cin / 8); }
+__host__ __device__ constexpr size_t wgrad_smem_bytes(int cin) {
+  return (size_t)(wgrad_planes(cin) < 16 ? 16 : wgrad_planes(cin)) * kWgTile * 16 + 64;
 }
 
-__host__ __device__ inline size_t wgrad_smem_bytes(int cin, int Wp) {
-  return (size_t)(cin / 8) * conv_slab_pixels(Wp) * 16 + (size_t)(kConvCout / 8) * kConvTile * 16 + 16;
+template <int CIN>
+__global__ void __launch_bounds__(128, 2) conv3x3_wgrad_kernel(const ConvGeom g, const bf16 *x, const bf16 *dy,
+                                                               float *dw, float *db, int ntiles, int *err) {
+  constexpr int COUT = kConvCout, XC = CIN / 8, DC = COUT / 8;
+  constexpr uint32_t PLANE = kWgTile * 16;
+  constexpr uint32_t NCOL = CIN == 32 ? 128 : 64;  // three accumulators of CIN columns
+  // bf16 A and B, both MN-major, fp32 accumulator
+  constexpr uint32_t idesc = umma_idesc_bf16(128, CIN) | (1u << 15) | (1u << 16);
+  extern __shared__ __align__(128) uint8_t smem[];
+  __shared__ float sdb[COUT];
+  uint8_t *sa = smem, *sx = smem + 12 * PLANE;
+  uint64_t *bars = reinterpret_cast<uint64_t *>(smem + wgrad_smem_bytes(CIN) - 64);
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 2);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    fence_mbar_init();
+  }
+  if (tid < COUT) sdb[tid] = 0.f;
+  if (warp == 0) tmem_alloc(tslot, NCOL);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t taddr = *tslot;
+  float bsum[8] = {};  // this thread's share of db: chunk tid % DC, every (128 / DC)-th pixel
+  uint32_t phase = 0;
+  bool bad = false;
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+    const long long l0 = g.l_begin + (long long)tile * kWgTile;
+    if (tid == 0) {
+      fence_proxy_async_smem();
+      mbar_arrive_expect_tx(&bars[0], wgrad_planes(CIN) * PLANE);
+#pragma unroll
+      for (int tx = 0; tx < 3; ++tx)
+#pragma unroll
+        for (int j = 0; j < DC; ++j)
+          bulk_g2s(sa + (tx * DC + j) * PLANE, dy + ((size_t)j * g.CS + (l0 - (tx - 1))) * 8, PLANE, &bars[0]);
+#pragma unroll
+      for (int ty = 0; ty < 3; ++ty)
+#pragma unroll
+        for (int j = 0; j < XC; ++j)
+          bulk_g2s(sx + (ty * XC + j) * PLANE, x + ((size_t)j * g.CS + (l0 + (long long)(ty - 1) * g.Wp)) * 8, PLANE,
+                   &bars[0]);
+    }
+    bool ok = mbar_wait_bounded(&bars[0], phase, err);
+    if (__syncthreads_or(!ok)) {
+      if (tid == 0) mbar_wait_bounded(&bars[0], phase, nullptr);
+      bad = true;
+      break;
+    }
+    if (tid == 0) {
+      tc_fence_after();
+      const uint32_t sA = smem_addr(sa), sX = smem_addr(sx);
+#pragma unroll 1
+      for (int k = 0; k < kWgTile / 16; ++k) {
+        const uint64_t ad = umma_desc(sA + (uint32_t)k * 256, 128, PLANE);
+#pragma unroll
+        for (int ty = 0; ty < 3; ++ty)
+          umma_bf16(taddr + (uint32_t)(ty * CIN), ad, umma_desc(sX + (uint32_t)(ty * XC) * PLANE + (uint32_t)k * 256, 128, PLANE),
+                    idesc, (tile != (int)blockIdx.x) || k != 0);
+      }
+      umma_commit(&bars[1]);
+    }
+    if (db != nullptr) {  // beside the products: the unshifted copy of dy
+      const uint8_t *p = sa + (DC + tid % DC) * PLANE;
+#pragma unroll 4
+      for (int q = tid / DC; q < kWgTile; q += 128 / DC) {
+        float d[8];
+        unpack_bf8(*reinterpret_cast<const uint4 *>(p + q * 16), d);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) bsum[c] += d[c];
+      }
+    }
+    ok = mbar_wait_bounded(&bars[1], phase, err);
+    phase ^= 1u;
+    if (__syncthreads_or(!ok)) {
+      if (tid == 0) mbar_wait_bounded(&bars[1], phase ^ 1u, nullptr);
+      bad = true;
+      break;
+    }
+  }
+  tc_fence_after();
+  if (!bad) {
+    if (db != nullptr) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) atomicAdd(&sdb[(tid % DC) * 8 + c], bsum[c]);
+    }
+    // lane m = (tx, o) of D_ty holds dW[ty][tx][.][o]; warp 3's rows are the dropped ones
+#pragma unroll 1
+    for (int ty = 0; ty < 3; ++ty) {
+      float v[32];
+      if (warp < 3) {
+        // 32 columns also for CIN = 16 (the last columns of the allocation stay unused)
+        tmem_ld32(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(ty * CIN), v);
+        float *dst = dw + ((size_t)(ty * 3 + warp) * CIN) * COUT + lane;
+#pragma unroll
+        for (int c = 0; c < CIN; ++c) atomicAdd(dst + (size_t)c * COUT, v[c]);
+      }
+      __syncwarp();
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (!bad && db != nullptr && tid < COUT) atomicAdd(&db[tid], sdb[tid]);
+  if (warp == 0) {
+    tc_fence_after();
+    tmem_dealloc(taddr, NCOL);
+  }
 }
 
 // ------------------------------------------------------------ elementwise parts
@@ -563,21 +620,13 @@ extern "C" int tp_conv3x3_wgrad(int32_t nf, int32_t nb, int32_t batch, int32_t c
   int dev = 0, sms = 148;
   TP_CHECK_CUDA(cudaGetDevice(&dev));
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int ntiles = conv_tiles(g);
+  if (cin != 16 && cin != 32) return set_error(TP_ERR_UNSUPPORTED, "tp_conv3x3_wgrad: cin must be 16 or 32");
+  const int ntiles = (int)((g.l_end - g.l_begin + kWgTile - 1) / kWgTile);
   const int grid = ntiles < 2 * sms ? ntiles : 2 * sms;
-  const size_t smem = wgrad_smem_bytes(cin, g.Wp);
-  if (smem > (size_t)max_smem_optin()) return set_error(TP_ERR_UNSUPPORTED, "wgrad needs %zu B of shared memory", smem);
-  if (cin == 16) {
-    TP_CHECK_CUDA(cudaFuncSetAttribute(conv3x3_wgrad_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    conv3x3_wgrad_kernel<16><<<grid, 160, smem, st>>>(g, static_cast<const bf16 *>(x), static_cast<const bf16 *>(dy),
-                                                       dw, db, ntiles, err);
-  } else if (cin == 32) {
-    TP_CHECK_CUDA(cudaFuncSetAttribute(conv3x3_wgrad_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    conv3x3_wgrad_kernel<32><<<grid, 320, smem, st>>>(g, static_cast<const bf16 *>(x), static_cast<const bf16 *>(dy),
-                                                       dw, db, ntiles, err);
-  } else {
-    return set_error(TP_ERR_UNSUPPORTED, "tp_conv3x3_wgrad: cin must be 16 or 32");
-  }
+  const size_t smem = wgrad_smem_bytes(cin);
+  auto kern = cin == 32 ? conv3x3_wgrad_kernel<32> : conv3x3_wgrad_kernel<16>;
+  TP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<grid, 128, smem, st>>>(g, static_cast<const bf16 *>(x), static_cast<const bf16 *>(dy), dw, db, ntiles, err);
   return check_cuda(cudaGetLastError(), "conv3x3_wgrad_kernel launch");
 }
 
