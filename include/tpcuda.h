@@ -520,6 +520,12 @@ TP_API int tp_conv3x3_wgrad(int32_t nf, int32_t nb, int32_t batch, int32_t cin, 
  * conj != 0 applies conj(F) (the adjoint modes). */
 TP_API int tp_cnn_filter_apply(int32_t nf, int32_t nb, int32_t nvec, int32_t per_image, int32_t conj,
                                const void *filt, const void *z, void *y, tp_stream_t stream);
+/* The residuals of the same product and their loss in one pass:
+ * e_v = scale_v (y_v - target_v), *loss += sum_v scale_v |y_v - target_v|^2
+ * (target, e (nvec, nf*nb) float2; scale (nvec) float; loss device double). */
+TP_API int tp_cnn_filter_residual(int32_t nf, int32_t nb, int32_t nvec, int32_t per_image, const void *filt,
+                                  const void *z, const void *target, const float *scale, void *e, double *loss,
+                                  tp_stream_t stream);
 /* Last-layer gradient (bf16, 32 channels, padded-linear) of
  * sum_v |y_v - t_v|^2 s_v given e_v = s_v (y_v - t_v):
  * 2 out_scale conj(z_v(x+o_t)) e_v(x) summed over the per_image vectors of

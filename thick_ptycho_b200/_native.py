@@ -225,6 +225,7 @@ SIGNATURES = [
     ("tp_conv3x3_bf16", ctypes.c_int, [ctypes.c_int32] * 5 + [ctypes.c_void_p] * 5 + [ctypes.c_float, ctypes.c_void_p]),
     ("tp_conv3x3_wgrad", ctypes.c_int, [ctypes.c_int32] * 4 + [ctypes.c_void_p] * 5),
     ("tp_cnn_filter_apply", ctypes.c_int, [ctypes.c_int32] * 5 + [ctypes.c_void_p] * 4),
+    ("tp_cnn_filter_residual", ctypes.c_int, [ctypes.c_int32] * 4 + [ctypes.c_void_p] * 7),
     ("tp_cnn_filter_grad", ctypes.c_int, [ctypes.c_int32] * 4 + [ctypes.c_void_p] * 2 + [ctypes.c_float] +
      [ctypes.c_void_p] * 2),
     ("tp_cnn_forward_ws_bytes", ctypes.c_size_t, [ctypes.c_int32] * 3),

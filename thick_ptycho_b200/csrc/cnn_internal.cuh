@@ -64,23 +64,4 @@ size_t cnn_forward_ws_bytes(const ConvGeom &g);
 int cnn_forward(const ConvGeom &g, const tp_cnn_model &m, const float2 *diag, long long diag_stride, const float2 *kc,
                 void *ws, float2 *filt, cudaStream_t st);
 
-// y = z + sum_t F_t(x) z(x + o_t) (F conjugated when conj != 0) for `nvec`
-// vectors of H*W; vector v uses filter image v / per_image (per_image = 0: image 0).
-__device__ __forceinline__ float2 filter_apply_px(const float2 *__restrict__ F, size_t fimg, size_t np,
-                                                   const float2 *__restrict__ z, int H, int W, int b, int f, int conj) {
-  const size_t i = (size_t)b * W + f;
-  float2 acc = z[i];
-#pragma unroll
-  for (int t = 0; t < kFilterTaps; ++t) {
-    const int bb = b + filter_tap_dy(t), ff = f + filter_tap_dx(t);
-    if (bb < 0 || bb >= H || ff < 0 || ff >= W) continue;
-    float2 w = F[(size_t)t * np + fimg + i];
-    if (conj) w.y = -w.y;
-    const float2 v = z[(size_t)bb * W + ff];
-    acc.x = fmaf(w.x, v.x, fmaf(-w.y, v.y, acc.x));
-    acc.y = fmaf(w.x, v.y, fmaf(w.y, v.x, acc.y));
-  }
-  return acc;
-}
-
 }  // namespace tp

@@ -181,6 +181,23 @@ __global__ void __launch_bounds__(128) conv3x3_tc_kernel(const ConvArgs a) {
 #pragma unroll
     for (int j = 0; j < CIN / 8; ++j) bulk_g2s(sa + (size_t)j * R * 16, a.in + ((size_t)j * g.CS + src0) * 8, R * 16, &bars[0]);
   }
+  // the ReLU mask of this thread's pixels (a bit per channel), read while the
+  // operands are copied and multiplied
+  uint32_t mask[B];
+  if constexpr (EPI == kEpiMask) {
+#pragma unroll
+    for (int b = 0; b < B; ++b) {
+      const long long l = l0 + b * 128 + warp * 32 + lane;
+      mask[b] = 0u;
+#pragma unroll
+      for (int j = 0; j < COUT / 8; ++j) {
+        float m[8];
+        unpack_bf8(*reinterpret_cast<const uint4 *>(a.aux + ((size_t)j * g.CS + l) * 8), m);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) mask[b] |= (m[c] > 0.f ? 1u : 0u) << (8 * j + c);
+      }
+    }
+  }
   bool ok = mbar_wait_bounded(&bars[0], 0, a.err);
   if (__syncthreads_or(!ok)) {
     if (tid == 0) mbar_wait_bounded(&bars[0], 0, nullptr);
@@ -231,9 +248,10 @@ __global__ void __launch_bounds__(128) conv3x3_tc_kernel(const ConvArgs a) {
 #pragma unroll
   for (int c = 0; c < COUT; ++c) bias[c] = (a.bias != nullptr) ? a.bias[c] : 0.f;
 
-#pragma unroll 1
+#pragma unroll
   for (int b = 0; b < B; ++b) {
     float v[32];
+    __syncwarp();
     tmem_ld32(taddr + ((uint32_t)(warp * 32) << 16) + (uint32_t)(b * COUT), v);
     __syncwarp();
     const long long l = l0 + b * 128 + warp * 32 + lane;
@@ -256,10 +274,8 @@ __global__ void __launch_bounds__(128) conv3x3_tc_kernel(const ConvArgs a) {
 #pragma unroll
           for (int c = 0; c < 8; ++c) t[c] = fmaxf(t[c], 0.f);
         } else {
-          float m[8];
-          unpack_bf8(*reinterpret_cast<const uint4 *>(a.aux + ((size_t)j * g.CS + l) * 8), m);
 #pragma unroll
-          for (int c = 0; c < 8; ++c) t[c] = (m[c] > 0.f) ? t[c] : 0.f;
+          for (int c = 0; c < 8; ++c) t[c] = ((mask[b] >> (8 * j + c)) & 1u) ? t[c] : 0.f;
         }
         uint4 o;
         o.x = pack_bf2(t[0], t[1]);
@@ -436,16 +452,158 @@ __global__ void cnn_features_kernel(const ConvGeom g, const float2 *__restrict__
   }
 }
 
-// y[v] = z[v] + sum_t F_t z[v](x + o_t), vector v using filter image v / per_image.
-__global__ void cnn_filter_apply_kernel(int H, int W, int nvec, int per_image, int nimg, int conj,
-                                        const float2 *__restrict__ F, const float2 *__restrict__ z, float2 *y) {
-  const size_t hw = (size_t)H * W, np = hw * nimg;
-  const int v = blockIdx.y;
-  const size_t fimg = (per_image > 0) ? (size_t)(v / per_image) * hw : 0;
-  const float2 *zv = z + (size_t)v * hw;
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < hw; i += (size_t)gridDim.x * blockDim.x) {
-    const int b = (int)(i / W), f = (int)(i - (size_t)b * W);
-    y[(size_t)v * hw + i] = filter_apply_px(F, fimg, np, zv, H, W, b, f, conj);
+// The filter passes over vectors (apply, residual, filter gradient) share one
+// tiling: a CTA owns kFtW x kFtH pixels of one filter image, a thread two vertically
+// adjacent ones, and loops over the image's vectors, whose tiles with a 2-pixel
+// border (zero outside the image) arrive by asynchronous copies two vectors ahead.
+// The pair's 26 taps read 18 distinct neighbours from shared memory and the taps (or
+// the tap gradients) stay in registers for all vectors.  One thread per pixel that
+// reads every neighbour from global memory is bound by load latency: 256 x 256, 4
+// images of 16 vectors, gradient 88 -> 39 us, apply with the residual and its loss
+// 83 us plus five elementwise passes of ~12 us -> 51 us.
+constexpr int kFtW = 64, kFtH = 8, kFtThreads = kFtW * kFtH / 2, kFtStages = 3;
+constexpr int kFtSW = kFtW + 4, kFtSH = kFtH + 4;
+
+// The 18 neighbours of the pixel pair (rows y, y + 1) at column x of a staged tile.
+struct FilterWindow {
+  float2 m2, m1l, m1c, m1r, al2, al1, ac, ar1, ar2, bl2, bl1, bc, br1, br2, p2l, p2c, p2r, p3;
+  __device__ __forceinline__ explicit FilterWindow(const float2 *c) {  // c: the upper pixel
+    constexpr int W = kFtSW;
+    m2 = c[-2 * W];
+    m1l = c[-W - 1], m1c = c[-W], m1r = c[-W + 1];
+    al2 = c[-2], al1 = c[-1], ac = c[0], ar1 = c[1], ar2 = c[2];
+    bl2 = c[W - 2], bl1 = c[W - 1], bc = c[W], br1 = c[W + 1], br2 = c[W + 2];
+    p2l = c[2 * W - 1], p2c = c[2 * W], p2r = c[2 * W + 1];
+    p3 = c[3 * W];
+  }
+  // taps (dy, dx): (0,0) (0,-1) (0,1) (-1,0) (1,0) (-1,-1) (-1,1) (1,-1) (1,1) (0,-2) (0,2) (-2,0) (2,0)
+  __device__ __forceinline__ void upper(float2 (&v)[kFilterTaps]) const {
+    const float2 t[kFilterTaps] = {ac, al1, ar1, m1c, bc, m1l, m1r, bl1, br1, al2, ar2, m2, p2c};
+#pragma unroll
+    for (int i = 0; i < kFilterTaps; ++i) v[i] = t[i];
+  }
+  __device__ __forceinline__ void lower(float2 (&v)[kFilterTaps]) const {
+    const float2 t[kFilterTaps] = {bc, bl1, br1, ac, p2c, al1, ar1, p2l, p2r, bl2, br2, m1c, p3};
+#pragma unroll
+    for (int i = 0; i < kFilterTaps; ++i) v[i] = t[i];
+  }
+};
+
+// Vector zv's tile at columns c0 - 2 .., rows r0 - 2 .. into `dst`.
+__device__ __forceinline__ void filter_stage(float2 *dst, const float2 *__restrict__ zv, int H, int W, int r0, int c0) {
+  for (int e = threadIdx.x; e < kFtSW * kFtSH; e += kFtThreads) {
+    const int y = e / kFtSW, x = e - y * kFtSW;
+    const int r = r0 - 2 + y, c = c0 - 2 + x;
+    if (r >= 0 && r < H && c >= 0 && c < W) cp_async8(&dst[e], &zv[(size_t)r * W + c]);
+    else dst[e] = make_float2(0.f, 0.f);
+  }
+}
+
+// Calls body(v, window) for vectors v0 .. v1 - 1, copies running two ahead.
+template <class Body>
+__device__ __forceinline__ void filter_vectors(float2 (*sm)[kFtSW * kFtSH], const float2 *__restrict__ z, size_t hw, int H,
+                                               int W, int r0, int c0, int v0, int v1, Body body) {
+#pragma unroll
+  for (int s = 0; s < kFtStages - 1; ++s) {
+    if (v0 + s < v1) filter_stage(sm[s], z + (size_t)(v0 + s) * hw, H, W, r0, c0);
+    cp_async_commit();
+  }
+  const int px = (2 + 2 * (threadIdx.x / kFtW)) * kFtSW + 2 + threadIdx.x % kFtW;
+  for (int v = v0; v < v1; ++v) {
+    const int k = (v - v0) % kFtStages, n = v + kFtStages - 1;
+    cp_async_wait<kFtStages - 2>();
+    __syncthreads();  // vector v is staged for all, and vector v - 1's tile is free
+    if (n < v1) filter_stage(sm[(n - v0) % kFtStages], z + (size_t)n * hw, H, W, r0, c0);
+    cp_async_commit();
+    body(v, FilterWindow(&sm[k][px]));
+  }
+}
+
+struct FilterArgs {
+  int H, W, nvec, per, nsplit, conj;  // per: vectors of an image
+  size_t np_img;                      // pixels of all filter images
+  const float2 *F, *z;
+  float2 *y;                // apply: the result
+  const float2 *target;     // residual: e = scale (y - target), loss += scale |y - target|^2
+  const float *scale;
+  float2 *e;
+  double *loss;
+};
+
+// y_v = z_v + sum_t F_t z_v(x + o_t).  Grid (tiles of columns, of rows, images * nsplit).
+template <bool RESIDUAL>
+__global__ void __launch_bounds__(kFtThreads, 2) cnn_filter_kernel(const FilterArgs a) {
+  __shared__ __align__(16) float2 sm[kFtStages][kFtSW * kFtSH];
+  __shared__ double red[kFtThreads / 32];
+  const int img = blockIdx.z / a.nsplit, part = blockIdx.z % a.nsplit;
+  const int chunk = (a.per + a.nsplit - 1) / a.nsplit;
+  const int v0 = img * a.per + part * chunk;
+  const int v1 = min(min(v0 + chunk, (img + 1) * a.per), a.nvec);
+  const int c0 = blockIdx.x * kFtW, r0 = blockIdx.y * kFtH;
+  const int c = c0 + threadIdx.x % kFtW, r = r0 + 2 * (threadIdx.x / kFtW);
+  const bool ina = c < a.W && r < a.H, inb = c < a.W && r + 1 < a.H;
+  const size_t hw = (size_t)a.H * a.W, at = (size_t)r * a.W + c;
+  const float2 *F = a.F + (size_t)img * hw + at;
+  const float cs = a.conj ? -1.f : 1.f;
+  float2 wa[kFilterTaps], wb[kFilterTaps];
+#pragma unroll
+  for (int t = 0; t < kFilterTaps; ++t) {
+    const float2 fa = ina ? F[(size_t)t * a.np_img] : make_float2(0.f, 0.f);
+    const float2 fb = inb ? F[(size_t)t * a.np_img + a.W] : make_float2(0.f, 0.f);
+    wa[t] = make_float2(fa.x, cs * fa.y);
+    wb[t] = make_float2(fb.x, cs * fb.y);
+  }
+  double loss = 0.0;
+  const float2 zero = make_float2(0.f, 0.f);
+  float2 ta = zero, tb = zero;
+  if (RESIDUAL && v0 < v1) {
+    if (ina) ta = a.target[(size_t)v0 * hw + at];
+    if (inb) tb = a.target[(size_t)v0 * hw + at + a.W];
+  }
+  filter_vectors(sm, a.z, hw, a.H, a.W, r0, c0, v0, v1, [&](int v, const FilterWindow &w) {
+    float2 na[kFilterTaps], nb[kFilterTaps];
+    w.upper(na);
+    w.lower(nb);
+    float2 ya = w.ac, yb = w.bc;
+#pragma unroll
+    for (int t = 0; t < kFilterTaps; ++t) {
+      ya = cfma(wa[t], na[t], ya);
+      yb = cfma(wb[t], nb[t], yb);
+    }
+    const size_t o = (size_t)v * hw + at;
+    if (RESIDUAL) {
+      const float s = a.scale[v];
+      const float2 xa = ta, xb = tb;
+      if (v + 1 < v1) {  // the next vector's target while this one is used
+        if (ina) ta = a.target[o + hw];
+        if (inb) tb = a.target[o + hw + a.W];
+      }
+      float l = 0.f;
+      if (ina) {
+        const float2 d = csub(ya, xa);
+        a.e[o] = make_float2(d.x * s, d.y * s);
+        l = fmaf(d.x, d.x, d.y * d.y);
+      }
+      if (inb) {
+        const float2 d = csub(yb, xb);
+        a.e[o + a.W] = make_float2(d.x * s, d.y * s);
+        l += fmaf(d.x, d.x, d.y * d.y);
+      }
+      loss += (double)s * (double)l;
+    } else {
+      if (ina) a.y[o] = ya;
+      if (inb) a.y[o + a.W] = yb;
+    }
+  });
+  if (RESIDUAL) {
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = loss;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      double s = 0.0;
+      for (int w = 0; w < kFtThreads / 32; ++w) s += red[w];
+      atomicAdd(a.loss, s);
+    }
   }
 }
 
@@ -453,32 +611,41 @@ __global__ void cnn_filter_apply_kernel(int H, int W, int nvec, int per_image, i
 // e_v = scale_v (y_v - target_v):  dF_t(x) = 2 sum_v conj(z_v(x + o_t)) e_v(x)
 // (d/dRe + i d/dIm), times out_scale (F = out_scale * last layer), written as
 // the 32-channel bf16 gradient of the last layer (channels 2t, 2t+1;
-// channels 26..31 zero).  One thread per pixel of
-// each filter image sums over the image's `per_image` vectors.
-__global__ void cnn_filter_grad_kernel(const ConvGeom g, int per_image, const float2 *__restrict__ z,
-                                       const float2 *__restrict__ e, float out_scale, bf16 *dy) {
-  const long long hw = (long long)g.H * g.W, np = hw * g.batch;
-  for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < np;
-       idx += (long long)gridDim.x * blockDim.x) {
-    const long long img = idx / hw, i = idx - img * hw;
-    const int b = (int)(i / g.W), f = (int)(i - (long long)b * g.W);
-    float2 acc[kFilterTaps];
+// channels 26..31 zero).  Grid (tiles of columns, of rows, images).
+__global__ void __launch_bounds__(kFtThreads, 2) cnn_filter_grad_kernel(const ConvGeom g, int per_image,
+                                                                        const float2 *__restrict__ z,
+                                                                        const float2 *__restrict__ e, float out_scale,
+                                                                        bf16 *dy) {
+  __shared__ __align__(16) float2 sm[kFtStages][kFtSW * kFtSH];
+  const int img = blockIdx.z, c0 = blockIdx.x * kFtW, r0 = blockIdx.y * kFtH;
+  const int c = c0 + threadIdx.x % kFtW, r = r0 + 2 * (threadIdx.x / kFtW);
+  const bool ina = c < g.W && r < g.H, inb = c < g.W && r + 1 < g.H;
+  const size_t hw = (size_t)g.H * g.W, at = (size_t)r * g.W + c;
+  float2 ga[kFilterTaps], gb[kFilterTaps];
 #pragma unroll
-    for (int t = 0; t < kFilterTaps; ++t) acc[t] = make_float2(0.f, 0.f);
-    for (int s = 0; s < per_image; ++s) {
-      const size_t v = (size_t)img * per_image + s;
-      const float2 ev = e[v * hw + i];
-#pragma unroll
-      for (int t = 0; t < kFilterTaps; ++t) {
-        const int bb = b + filter_tap_dy(t), ff = f + filter_tap_dx(t);
-        if (bb < 0 || bb >= g.H || ff < 0 || ff >= g.W) continue;
-        const float2 zv = z[v * hw + (size_t)bb * g.W + ff];
-        // conj(z) * e
-        acc[t].x = fmaf(zv.x, ev.x, fmaf(zv.y, ev.y, acc[t].x));
-        acc[t].y = fmaf(zv.x, ev.y, fmaf(-zv.y, ev.x, acc[t].y));
-      }
+  for (int t = 0; t < kFilterTaps; ++t) ga[t] = gb[t] = make_float2(0.f, 0.f);
+  const int v0 = img * per_image;
+  const float2 zero = make_float2(0.f, 0.f);
+  float2 ea = ina ? e[(size_t)v0 * hw + at] : zero, eb = inb ? e[(size_t)v0 * hw + at + g.W] : zero;
+  filter_vectors(sm, z, hw, g.H, g.W, r0, c0, v0, v0 + per_image, [&](int v, const FilterWindow &w) {
+    const float2 xa = ea, xb = eb;
+    if (v + 1 < v0 + per_image) {  // the next vector's residuals while this one is used
+      ea = ina ? e[(size_t)(v + 1) * hw + at] : zero;
+      eb = inb ? e[(size_t)(v + 1) * hw + at + g.W] : zero;
     }
-    const long long l = g.G0 + img * g.S + (long long)(b + 1) * g.Wp + (f + 1);
+    float2 na[kFilterTaps], nb[kFilterTaps];
+    w.upper(na);
+    w.lower(nb);
+#pragma unroll
+    for (int t = 0; t < kFilterTaps; ++t) {  // conj(z) e
+      ga[t].x = fmaf(na[t].x, xa.x, fmaf(na[t].y, xa.y, ga[t].x));
+      ga[t].y = fmaf(na[t].x, xa.y, fmaf(-na[t].y, xa.x, ga[t].y));
+      gb[t].x = fmaf(nb[t].x, xb.x, fmaf(nb[t].y, xb.y, gb[t].x));
+      gb[t].y = fmaf(nb[t].x, xb.y, fmaf(-nb[t].y, xb.x, gb[t].y));
+    }
+  });
+  auto put = [&](const float2(&acc)[kFilterTaps], int row) {
+    const long long l = g.G0 + img * g.S + (long long)(row + 1) * g.Wp + (c + 1);
     float ch[32];
 #pragma unroll
     for (int t = 0; t < kFilterTaps; ++t) {
@@ -486,7 +653,7 @@ __global__ void cnn_filter_grad_kernel(const ConvGeom g, int per_image, const fl
       ch[2 * t + 1] = 2.f * out_scale * acc[t].y;
     }
 #pragma unroll
-    for (int c = 2 * kFilterTaps; c < 32; ++c) ch[c] = 0.f;
+    for (int k = 2 * kFilterTaps; k < 32; ++k) ch[k] = 0.f;
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       uint4 o;
@@ -496,7 +663,9 @@ __global__ void cnn_filter_grad_kernel(const ConvGeom g, int per_image, const fl
       o.w = pack_bf2(ch[8 * j + 6], ch[8 * j + 7]);
       *reinterpret_cast<uint4 *>(dy + ((size_t)j * g.CS + l) * 8) = o;
     }
-  }
+  };
+  if (ina) put(ga, r);
+  if (inb) put(gb, r + 1);
 }
 
 // ------------------------------------------------------------ host
@@ -504,6 +673,24 @@ static int max_smem_optin() {
   int dev = 0, v = 232448;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&v, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   return v;
+}
+
+// Vectors of an image are split over CTAs until the grid holds about two waves.
+template <bool RESIDUAL>
+static int launch_filter(FilterArgs a, int nf, int nb, int nvec, int per_image, cudaStream_t st) {
+  const int nimg = per_image > 0 ? (nvec + per_image - 1) / per_image : 1;
+  a.H = nb;
+  a.W = nf;
+  a.nvec = nvec;
+  a.per = per_image > 0 ? per_image : nvec;
+  a.np_img = (size_t)nf * nb * nimg;
+  const int gx = (nf + kFtW - 1) / kFtW, gy = (nb + kFtH - 1) / kFtH;
+  int split = 888 / (gx * gy * nimg);
+  if (split > (a.per + 3) / 4) split = (a.per + 3) / 4;
+  a.nsplit = split < 1 ? 1 : split;
+  if ((long long)nimg * a.nsplit > 65535 || gy > 65535) return set_error(TP_ERR_UNSUPPORTED, "filter: grid too large");
+  cnn_filter_kernel<RESIDUAL><<<dim3(gx, gy, nimg * a.nsplit), kFtThreads, 0, st>>>(a);
+  return check_cuda(cudaGetLastError(), "cnn_filter_kernel launch");
 }
 
 static int check_geom(const ConvGeom &g) {
@@ -634,13 +821,27 @@ extern "C" int tp_cnn_filter_apply(int32_t nf, int32_t nb, int32_t nvec, int32_t
                                    const void *filt, const void *z, void *y, tp_stream_t stream) {
   if (filt == nullptr || z == nullptr || y == nullptr || nvec < 1 || nf < 1 || nb < 1 || per_image < 0)
     return set_error(TP_ERR_INVALID, "tp_cnn_filter_apply: bad argument");
-  const int nimg = per_image > 0 ? (nvec + per_image - 1) / per_image : 1;
-  const size_t hw = (size_t)nf * nb;
-  const int gx = (int)((hw + 255) / 256 < 4096 ? (hw + 255) / 256 : 4096);
-  cnn_filter_apply_kernel<<<dim3(gx, nvec), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      nb, nf, nvec, per_image, nimg, conj, static_cast<const float2 *>(filt), static_cast<const float2 *>(z),
-      static_cast<float2 *>(y));
-  return check_cuda(cudaGetLastError(), "cnn_filter_apply_kernel launch");
+  FilterArgs a{};
+  a.conj = conj;
+  a.F = static_cast<const float2 *>(filt);
+  a.z = static_cast<const float2 *>(z);
+  a.y = static_cast<float2 *>(y);
+  return launch_filter<false>(a, nf, nb, nvec, per_image, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int tp_cnn_filter_residual(int32_t nf, int32_t nb, int32_t nvec, int32_t per_image, const void *filt,
+                                      const void *z, const void *target, const float *scale, void *e, double *loss,
+                                      tp_stream_t stream) {
+  if (!filt || !z || !target || !scale || !e || !loss || nvec < 1 || nf < 1 || nb < 1 || per_image < 0)
+    return set_error(TP_ERR_INVALID, "tp_cnn_filter_residual: bad argument");
+  FilterArgs a{};
+  a.F = static_cast<const float2 *>(filt);
+  a.z = static_cast<const float2 *>(z);
+  a.target = static_cast<const float2 *>(target);
+  a.scale = scale;
+  a.e = static_cast<float2 *>(e);
+  a.loss = loss;
+  return launch_filter<true>(a, nf, nb, nvec, per_image, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tp_cnn_filter_grad(int32_t nf, int32_t nb, int32_t nimg, int32_t per_image, const void *z, const void *e,
@@ -650,7 +851,9 @@ extern "C" int tp_cnn_filter_grad(int32_t nf, int32_t nb, int32_t nimg, int32_t 
   const ConvGeom g = conv_geom(nb, nf, nimg);
   int rc = check_geom(g);
   if (rc != TP_OK) return rc;
-  cnn_filter_grad_kernel<<<592, 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+  if (nimg > 65535 || (nb + kFtH - 1) / kFtH > 65535) return set_error(TP_ERR_UNSUPPORTED, "tp_cnn_filter_grad: grid too large");
+  cnn_filter_grad_kernel<<<dim3((nf + kFtW - 1) / kFtW, (nb + kFtH - 1) / kFtH, nimg), kFtThreads, 0,
+                           reinterpret_cast<cudaStream_t>(stream)>>>(
       g, per_image, static_cast<const float2 *>(z), static_cast<const float2 *>(e), out_scale, static_cast<bf16 *>(dy));
   return check_cuda(cudaGetLastError(), "cnn_filter_grad_kernel launch");
 }

@@ -234,29 +234,38 @@ class LearnedPreconditioner:
         L = self.lib
         st = _stream(self.device)
         F = self.filter(diag)
-        y = self.apply(F, z, per_image)
-        r = y - target
-        e = (r * scale[:, None]).contiguous()
-        loss = torch.sum(scale[:, None] * (r.real ** 2 + r.imag ** 2))
+        z = z.contiguous()
+        target = torch.broadcast_to(target, z.shape).contiguous()
+        scale = torch.broadcast_to(scale, (V,)).contiguous()
+        if z.dtype != torch.complex64 or target.dtype != torch.complex64 or scale.dtype != torch.float32:
+            raise TypeError("z and target must be complex64, scale float32")
+        e = torch.empty_like(z)
+        # the sums that the kernels add to, in one cleared buffer: the loss (fp64),
+        # then the weight gradients (9, cin, 32) and the bias gradients of the layers
+        n0, n1 = 9 * CHANNELS_IN * WIDTH, 9 * WIDTH * WIDTH
+        acc = torch.zeros(2 + n0 + 3 * n1 + 4 * WIDTH, dtype=torch.float32, device=self.device)
+        loss64 = acc[:2].view(torch.float64)[0]
+        dws = [acc[2:2 + n0]] + [acc[2 + n0 + i * n1:2 + n0 + (i + 1) * n1] for i in range(3)]
+        gb = [acc[2 + n0 + 3 * n1 + i * WIDTH:2 + n0 + 3 * n1 + (i + 1) * WIDTH] for i in range(4)]
+        _native.check(L.tp_cnn_filter_residual(self.nf, self.nb, V, int(per_image), _ptr(F), _ptr(z), _ptr(target),
+                                               _ptr(scale), _ptr(e), _ptr(loss64), st), "tp_cnn_filter_residual")
         buf = self._buffers(B)
-        _native.check(L.tp_cnn_filter_grad(self.nf, self.nb, B, int(per_image), _ptr(z.contiguous()), _ptr(e),
+        _native.check(L.tp_cnn_filter_grad(self.nf, self.nb, B, int(per_image), _ptr(z), _ptr(e),
                                            self.out_scale, _ptr(buf.g[0]), st), "tp_cnn_filter_grad")
-        gw, gb = [None] * 4, [None] * 4
         acts = [buf.feat, buf.a[0], buf.a[1], buf.a[2]]
         dys = [buf.g[3], buf.g[2], buf.g[1], buf.g[0]]  # gradient at each layer's output
         for i in (3, 2, 1, 0):
             cin = CHANNELS_IN if i == 0 else WIDTH
-            dw = torch.zeros((9, cin, WIDTH), dtype=torch.float32, device=self.device)
-            db = torch.zeros(WIDTH, dtype=torch.float32, device=self.device)
-            _native.check(L.tp_conv3x3_wgrad(self.nf, self.nb, B, cin, _ptr(acts[i]), _ptr(dys[i]), _ptr(dw), _ptr(db),
-                                             st), "tp_conv3x3_wgrad")
-            gw[i] = wgrad_to_torch(dw, cin)
-            gb[i] = db
+            _native.check(L.tp_conv3x3_wgrad(self.nf, self.nb, B, cin, _ptr(acts[i]), _ptr(dys[i]), _ptr(dws[i]),
+                                             _ptr(gb[i]), st), "tp_conv3x3_wgrad")
             if i > 0:
                 # gradient at layer i's input = conv(dy_i, W_i^T) masked by ReLU'(a_{i})
                 _native.check(L.tp_conv3x3_bf16(self.nf, self.nb, B, WIDTH, _native.CONV_MASK, _ptr(dys[i]),
                                                 _ptr(self.wt[i]), None, _ptr(acts[i]), _ptr(dys[i - 1]), 1.0, st),
                               "tp_conv3x3_bf16")
+        wide = acc[2 + n0:2 + n0 + 3 * n1].view(3, 3, 3, WIDTH, WIDTH).permute(0, 4, 3, 1, 2).contiguous()
+        gw = [wgrad_to_torch(dws[0], CHANNELS_IN), wide[0], wide[1], wide[2]]
+        loss = loss64.to(torch.float32)
         return loss, gw, gb
 
     # ----------------------------------------------------------- training
