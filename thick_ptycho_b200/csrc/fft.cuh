@@ -21,7 +21,14 @@ struct FftPlan {
   int n;
   int npass;
   int radix[kFftMaxPasses];
+  // reciprocals of the passes' n / R and Ns (fast_div)
+  uint32_t mt[kFftMaxPasses], ms[kFftMaxPasses];
 };
+
+// w / d for w d < 2^32 with m = fast_recip(d): the error of m, below one, adds
+// less than w / 2^32 to the quotient, which is a multiple of 1 / d.
+inline uint32_t fast_recip(uint32_t d) { return d == 1 ? 0u : (uint32_t)(((1ull << 32) + d - 1) / d); }
+__device__ __forceinline__ int fast_div(int w, uint32_t m) { return m ? (int)__umulhi((uint32_t)w, m) : w; }
 
 // Host: radices of n (8s first, then 4, 2, 3, 5); npass = 0 if unsupported.
 inline FftPlan make_fft_plan(int n) {
@@ -35,6 +42,12 @@ inline FftPlan make_fft_plan(int n) {
   while (m % 3 == 0 && k < kFftMaxPasses) { p.radix[k++] = 3; m /= 3; }
   while (m % 5 == 0 && k < kFftMaxPasses) { p.radix[k++] = 5; m /= 5; }
   p.npass = (m == 1) ? k : 0;
+  int ns = 1;
+  for (int i = 0; i < p.npass; ++i) {
+    p.mt[i] = fast_recip((uint32_t)(n / p.radix[i]));
+    p.ms[i] = fast_recip((uint32_t)ns);
+    ns *= p.radix[i];
+  }
   return p;
 }
 
@@ -165,26 +178,30 @@ __device__ __forceinline__ void dft_small<5>(cx (&v)[8], rx sign) {
   v[3] = csub(m2, n2);
 }
 
+// One pass; the twiddle exponent r k n / (Ns R) stays below n (k < Ns, r < R).
 template <int R>
-__device__ __forceinline__ void fft_pass(const cx *a, cx *b, int n, int Ns, const cx *tw, rx sign,
-                                         int nb, int tid, int nth) {
+__device__ __forceinline__ void fft_pass(const cx *a, cx *b, int n, int Ns, uint32_t mt, uint32_t ms, const cx *tw,
+                                         rx sign, int nb, int tid, int nth) {
   const int T = n / R;
-  const int step = n / (Ns * R);
+  const int step = T / Ns;
   for (int w = tid; w < nb * T; w += nth) {
-    const int bi = w / T, j = w - bi * T;
+    const int bi = fast_div(w, mt), j = w - bi * T;
     const cx *src = a + bi * n;
     cx *dst = b + bi * n;
-    const int k = j % Ns;
+    const int jn = fast_div(j, ms), k = j - jn * Ns;
     cx v[8];
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = src[j + r * T];
+    if (Ns > 1) {
+      const int ks = k * step;
 #pragma unroll
-    for (int r = 1; r < R; ++r) {
-      const cx t = tw[(r * k * step) % n];
-      v[r] = cmul(v[r], mkcx(t.x, sign < 0 ? t.y : -t.y));
+      for (int r = 1; r < R; ++r) {
+        const cx t = tw[r * ks];
+        v[r] = cmul(v[r], mkcx(t.x, sign < 0 ? t.y : -t.y));
+      }
     }
     dft_small<R>(v, sign);
-    const int idx = (j / Ns) * Ns * R + k;
+    const int idx = jn * Ns * R + k;
 #pragma unroll
     for (int r = 0; r < R; ++r) dst[idx + r * Ns] = v[r];
   }
@@ -326,11 +343,11 @@ __device__ __forceinline__ cx *fft_block(cx *a, cx *b, const FftPlan &pl, const 
   for (int ps = 0; ps < pl.npass; ++ps) {
     const int R = pl.radix[ps];
     switch (R) {
-      case 8: fft_pass<8>(a, b, pl.n, Ns, tw, sign, nb, tid, nth); break;
-      case 4: fft_pass<4>(a, b, pl.n, Ns, tw, sign, nb, tid, nth); break;
-      case 2: fft_pass<2>(a, b, pl.n, Ns, tw, sign, nb, tid, nth); break;
-      case 3: fft_pass<3>(a, b, pl.n, Ns, tw, sign, nb, tid, nth); break;
-      default: fft_pass<5>(a, b, pl.n, Ns, tw, sign, nb, tid, nth); break;
+      case 8: fft_pass<8>(a, b, pl.n, Ns, pl.mt[ps], pl.ms[ps], tw, sign, nb, tid, nth); break;
+      case 4: fft_pass<4>(a, b, pl.n, Ns, pl.mt[ps], pl.ms[ps], tw, sign, nb, tid, nth); break;
+      case 2: fft_pass<2>(a, b, pl.n, Ns, pl.mt[ps], pl.ms[ps], tw, sign, nb, tid, nth); break;
+      case 3: fft_pass<3>(a, b, pl.n, Ns, pl.mt[ps], pl.ms[ps], tw, sign, nb, tid, nth); break;
+      default: fft_pass<5>(a, b, pl.n, Ns, pl.mt[ps], pl.ms[ps], tw, sign, nb, tid, nth); break;
     }
     __syncthreads();
     cx *t = a;
