@@ -38,7 +38,7 @@ int ms_transmission_launch(int n_total, int nz, double k, double dz, double nmr,
 struct Ms3Params {
   int n1, n2, N, nz, L, P;
   const float2 *trans;  // (L, N): T_z - 1
-  const float2 *hm1t;   // (n2, n1): (H - 1) / N, transposed
+  const float2 *hm1t;   // (H - 1) / N, (n2, n1), or (n1, n2) for the four-step column kernel
   const float2 *tw1, *tw2;
   float2 *psi;          // (P, N): field (forward) or lambda (adjoint), in place
   float2 *W;            // (P, N): spectrum work buffer, in place
@@ -58,12 +58,13 @@ __global__ void ms3_twiddle_kernel(int n, float2 *tw) {
   }
 }
 
-// (H - 1) / N at hm1t[b * n1 + a]; H - 1 = exp(i th) - 1 = -2 sin^2(th/2) + i sin th.
-__global__ void ms3_kernel_h_kernel(int n1, int n2, double k, double d1, double d2, double dz, float2 *hm1t) {
+// (H - 1) / N at hm1t[b * n1 + a] (by_row: at a * n2 + b); H - 1 = exp(i th) - 1 = -2 sin^2(th/2) + i sin th.
+__global__ void ms3_kernel_h_kernel(int n1, int n2, double k, double d1, double d2, double dz, int by_row,
+                                    float2 *hm1t) {
   const int N = n1 * n2;
   const double inv = 1.0 / (double)N;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N; e += gridDim.x * blockDim.x) {
-    const int b = e / n1, a = e - b * n1;
+    const int a = by_row ? e / n2 : e % n1, b = by_row ? e % n2 : e / n1;
     const int fa = (a < (n1 + 1) / 2) ? a : a - n1;
     const int fb = (b < (n2 + 1) / 2) ? b : b - n2;
     const double k1 = 2.0 * 3.14159265358979323846 * (double)fa / ((double)n1 * d1);
@@ -245,6 +246,191 @@ __global__ void __launch_bounds__(kMs3Threads) ms3_cols_kernel(const FftPlan pl,
   }
 }
 
+// ------------------------------------------------ register four-step kernels
+// The same two passes for row and column lengths 64, 128, 192 and 256 (R1 R2) with
+// the transforms in registers (fft.cuh): 256 threads, 256 / R1 rows or columns per
+// CTA.  The row kernel's inverse transform ends with the field's elements in the
+// registers where the next forward transform starts, so the multiplication by T and
+// everything else between the two happens there, and an element crosses shared memory
+// once per transform.  The psi buffer holds X_z = psi_z T_z here (psi_{z+1} = X_z +
+// update needs no T_z).  The shared-memory passes above were bound by shared memory
+// (73-83 % of its throughput); a slice of 64 probes of 256 x 256 took 95 us with them
+// (adjoint 99) and takes %F% us (%B%) with these.
+template <int R1, int R2, int PHASE>
+__global__ void __launch_bounds__(256, 2) ms3_rows4_kernel(const Ms3Params q, const float2 *__restrict__ twg, int z) {
+  constexpr int N = R1 * R2, RPC = 256 / R1, S = R1 * (R2 + 1);
+  __shared__ float2 buf[RPC * S];
+  __shared__ float2 tw[R1 * (R2 + 1)];
+  const int pr = blockIdx.y, tid = threadIdx.x;
+  const size_t pbase = (size_t)pr * q.N;
+  const int g0 = blockIdx.x * RPC * N;
+  for (int e = tid; e < R1 * (R2 + 1); e += 256) tw[e] = twg[e];
+  const int ra = tid / R2, n2 = tid % R2;  // stage A: (row, n2), element R2 n1 + n2
+  const int rc = tid / R1, k1 = tid % R1;  // stage C: (row, k1), frequency k1 + R1 k2
+  const bool inA = tid < RPC * R2;
+  const int ga = g0 + ra * N + n2;
+  float2 *wrow = q.W + pbase + g0 + rc * N + k1;
+  const bool last = PHASE == kMs3FwdStep && z + 1 == q.L;
+  float2 x[16], pz[R1], tz[R1], uz[R1];
+  if (PHASE == kMs3FwdStart || PHASE == kMs3BwdStart) {
+    __syncthreads();
+    if (inA) {
+#pragma unroll
+      for (int j = 0; j < R1; ++j) {
+        const int g = ga + R2 * j;
+        float2 v = (PHASE == kMs3FwdStart ? q.probes : q.src_exit)[pbase + g];
+        if (PHASE == kMs3FwdStart) {
+          if (q.u_store) q.u_store[(size_t)pr * q.nz * q.N + g] = v;
+          v = cfma(q.trans[g], v, v);
+        }
+        q.psi[pbase + g] = v;
+        x[j] = v;
+      }
+    }
+  } else {
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) x[k2] = wrow[R1 * k2];
+    if (inA) {  // under the inverse transform
+      const float2 *T = q.trans + (size_t)(PHASE == kMs3FwdStep ? (last ? z : z + 1) : z) * q.N;
+      const float2 *u = PHASE == kMs3BwdStep ? q.u_fwd + ((size_t)pr * q.nz + z) * q.N : nullptr;
+#pragma unroll
+      for (int j = 0; j < R1; ++j) {
+        pz[j] = q.psi[pbase + ga + R2 * j];
+        tz[j] = T[ga + R2 * j];
+        if (PHASE == kMs3BwdStep) uz[j] = __ldcs(&u[ga + R2 * j]);
+      }
+    }
+    dft_reg<R2>(x, 1.f);
+    __syncthreads();  // the twiddles are in place
+#pragma unroll
+    for (int m = 0; m < R2; ++m)
+      buf[rc * S + k1 * (R2 + 1) + m] = m ? cmulc(x[m], tw[k1 * (R2 + 1) + m]) : x[0];
+    __syncthreads();
+    if (inA) {
+#pragma unroll
+      for (int k = 0; k < R1; ++k) x[k] = buf[ra * S + k * (R2 + 1) + n2];
+      dft_reg<R1>(x, 1.f);
+      if (PHASE == kMs3FwdStep) {
+        // psi_{z+1} = X_z + IFFT2((H-1) FFT2 X_z), X_{z+1} = psi_{z+1} T_{z+1}
+        float2 *us = q.u_store ? q.u_store + ((size_t)pr * q.nz + z + 1) * q.N + ga : nullptr;
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+          const float2 v = cadd(pz[j], x[j]);
+          if (us) __stcs(&us[R2 * j], v);
+          if (last) {
+            if (q.exit_out) q.exit_out[pbase + ga + R2 * j] = v;
+          } else {
+            x[j] = cfma(tz[j], v, v);
+            q.psi[pbase + ga + R2 * j] = x[j];
+          }
+        }
+      } else {
+        // g_z = lambda_{z+1} + IFFT2(conj(H-1) FFT2 lambda_{z+1});
+        // grad_t[z] += g_z conj(T_z u_z);  lambda_z = conj(T_z) g_z
+        float2 *gt = q.grad_t + (size_t)z * q.N + ga;
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+          const float2 gv = cadd(pz[j], x[j]);
+          red_add_cx(gt + R2 * j, cmulc(gv, cfma(tz[j], uz[j], uz[j])));
+          x[j] = cadd(gv, cmulc(gv, tz[j]));
+          if (z > 0) q.psi[pbase + ga + R2 * j] = x[j];
+        }
+      }
+    }
+    if (last || (PHASE == kMs3BwdStep && z == 0)) return;
+  }
+  if (inA) {  // (in a step, into the slots that this thread has just read)
+    dft_reg<R1>(x, -1.f);
+#pragma unroll
+    for (int k = 0; k < R1; ++k)
+      buf[ra * S + k * (R2 + 1) + n2] = k ? cmul(x[k], tw[k * (R2 + 1) + n2]) : x[0];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < R2; ++m) x[m] = buf[rc * S + k1 * (R2 + 1) + m];
+  dft_reg<R2>(x, -1.f);
+#pragma unroll
+  for (int k2 = 0; k2 < R2; ++k2) wrow[R1 * k2] = x[k2];
+}
+
+// Column pass (hm1t by rows).  Grid (n2 / CPC, P).
+template <int R1, int R2, bool CONJ>
+__global__ void __launch_bounds__(256, 3) ms3_cols4_kernel(const Ms3Params q, const float2 *__restrict__ twg) {
+  constexpr int N = R1 * R2, CPC = 256 / R1;
+  __shared__ float2 buf[N * CPC];  // [k1][n2][c]
+  __shared__ float2 tw[R1 * (R2 + 1)];
+  const int tid = threadIdx.x, w = q.n2;
+  for (int e = tid; e < R1 * (R2 + 1); e += 256) tw[e] = twg[e];
+  const int c = tid % CPC, n2 = tid / CPC;  // stage A: (c, n2); stage C: (c, k1)
+  const int k1 = n2;
+  const bool inA = n2 < R2;
+  float2 *base = q.W + (size_t)blockIdx.y * q.N + blockIdx.x * CPC + c;
+  const float2 *h = q.hm1t + blockIdx.x * CPC + c + (size_t)k1 * w;
+  float2 x[16];
+  if (inA) {
+#pragma unroll
+    for (int j = 0; j < R1; ++j) x[j] = base[(size_t)(R2 * j + n2) * w];
+    dft_reg<R1>(x, -1.f);
+  }
+  __syncthreads();
+  if (inA) {
+#pragma unroll
+    for (int k = 0; k < R1; ++k) buf[(k * R2 + n2) * CPC + c] = k ? cmul(x[k], tw[k * (R2 + 1) + n2]) : x[0];
+  }
+  float2 hv[R2];
+#pragma unroll
+  for (int k2 = 0; k2 < R2; ++k2) hv[k2] = h[(size_t)R1 * k2 * w];
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < R2; ++m) x[m] = buf[(k1 * R2 + m) * CPC + c];
+  dft_reg<R2>(x, -1.f);
+#pragma unroll
+  for (int k2 = 0; k2 < R2; ++k2) x[k2] = CONJ ? cmulc(x[k2], hv[k2]) : cmul(x[k2], hv[k2]);
+  dft_reg<R2>(x, 1.f);
+  // this thread's own slots: no other thread reads (k1, ., c) before the barrier
+#pragma unroll
+  for (int m = 0; m < R2; ++m) buf[(k1 * R2 + m) * CPC + c] = m ? cmulc(x[m], tw[k1 * (R2 + 1) + m]) : x[0];
+  __syncthreads();
+  if (inA) {
+#pragma unroll
+    for (int k = 0; k < R1; ++k) x[k] = buf[(k * R2 + n2) * CPC + c];
+    dft_reg<R1>(x, 1.f);
+#pragma unroll
+    for (int j = 0; j < R1; ++j) base[(size_t)(R2 * j + n2) * w] = x[j];
+  }
+}
+
+// The padded twiddle table W_N^{n2 k1} at k1 (R2 + 1) + n2.
+__global__ void ms3_twiddle4_kernel(int r1, int r2, float2 *tw) {
+  for (int e = threadIdx.x; e < r1 * (r2 + 1); e += blockDim.x) {
+    const int k1 = e / (r2 + 1), n2 = e % (r2 + 1);
+    double sv, cv;
+    sincospi(-2.0 * (double)(k1 * n2) / (double)(r1 * r2), &sv, &cv);
+    tw[e] = make_float2((float)cv, (float)sv);
+  }
+}
+
+using Ms3Rows4 = void (*)(const Ms3Params, const float2 *, int);
+using Ms3Cols4 = void (*)(const Ms3Params, const float2 *);
+template <int PHASE>
+static Ms3Rows4 pick_rows4(int n) {
+  switch (n) {
+    case 64: return ms3_rows4_kernel<8, 8, PHASE>;
+    case 128: return ms3_rows4_kernel<16, 8, PHASE>;
+    case 192: return ms3_rows4_kernel<16, 12, PHASE>;
+    default: return ms3_rows4_kernel<16, 16, PHASE>;
+  }
+}
+template <bool CONJ>
+static Ms3Cols4 pick_cols4(int n) {
+  switch (n) {
+    case 64: return ms3_cols4_kernel<8, 8, CONJ>;
+    case 128: return ms3_cols4_kernel<16, 8, CONJ>;
+    case 192: return ms3_cols4_kernel<16, 12, CONJ>;
+    default: return ms3_cols4_kernel<16, 16, CONJ>;
+  }
+}
+
 using Ms3Rows = void (*)(const FftPlan, const Ms3Params, int, int, int);
 using Ms3Cols = void (*)(const FftPlan, const Ms3Params, int, int);
 
@@ -305,8 +491,9 @@ static Ms3Work ms3_layout(char *base, int n1, int n2, int P) {
   w.psi = take((size_t)P * N * sizeof(float2));
   w.W = take((size_t)P * N * sizeof(float2));
   w.hm1t = take(N * sizeof(float2));
-  w.tw1 = take((size_t)n1 * sizeof(float2));
-  w.tw2 = take((size_t)n2 * sizeof(float2));
+  // room for the four-step kernels' padded tables as well
+  w.tw1 = take((size_t)(n1 + 16) * sizeof(float2));
+  w.tw2 = take((size_t)(n2 + 16) * sizeof(float2));
   w.bytes = off;
   return w;
 }
@@ -336,10 +523,16 @@ static int ms3_run(const tp_ms3d_op *op, Ms3Params q, bool backward, void *works
   q.hm1t = w.hm1t;
   q.tw1 = w.tw1;
   q.tw2 = w.tw2;
-  ms3_twiddle_kernel<<<(n1 + 255) / 256, 256, 0, st>>>(n1, w.tw1);
-  ms3_twiddle_kernel<<<(n2 + 255) / 256, 256, 0, st>>>(n2, w.tw2);
-  ms3_kernel_h_kernel<<<(q.N + 255) / 256 < 1184 ? (q.N + 255) / 256 : 1184, 256, 0, st>>>(n1, n2, op->k, op->d1,
-                                                                                           op->d2, op->dz, w.hm1t);
+  // register four-step kernels where the length has a plan and the other axis
+  // splits into whole CTAs
+  const bool four_r = four_step_size(n2) && n1 % (256 / four_r1(n2)) == 0;
+  const bool four_c = four_step_size(n1) && n2 % (256 / four_r1(n1)) == 0;
+  if (four_c) ms3_twiddle4_kernel<<<1, 256, 0, st>>>(four_r1(n1), four_r2(n1), w.tw1);
+  else ms3_twiddle_kernel<<<(n1 + 255) / 256, 256, 0, st>>>(n1, w.tw1);
+  if (four_r) ms3_twiddle4_kernel<<<1, 256, 0, st>>>(four_r1(n2), four_r2(n2), w.tw2);
+  else ms3_twiddle_kernel<<<(n2 + 255) / 256, 256, 0, st>>>(n2, w.tw2);
+  ms3_kernel_h_kernel<<<(q.N + 255) / 256 < 1184 ? (q.N + 255) / 256 : 1184, 256, 0, st>>>(
+      n1, n2, op->k, op->d1, op->d2, op->dz, four_c ? 1 : 0, w.hm1t);
   TP_CHECK_CUDA(cudaGetLastError());
   const FftPlan p1 = make_fft_plan(n1), p2 = make_fft_plan(n2);
   // compile-time plans (padded layout, fixed transforms per CTA) where the
@@ -356,18 +549,21 @@ static int ms3_run(const tp_ms3d_op *op, Ms3Params q, bool backward, void *works
   TP_CHECK_CUDA(cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r));
   TP_CHECK_CUDA(cudaFuncSetAttribute(cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c));
   const dim3 gr(n1 / rpc, q.P), gc(n2 / cpc, q.P);
-  if (!backward) {
-    rows<<<gr, kMs3Threads, smem_r, st>>>(p2, q, kMs3FwdStart, 0, rpc);
-    for (int z = 0; z < q.L; ++z) {
-      cols<<<gc, kMs3Threads, smem_c, st>>>(p1, q, 0, cpc);
-      rows<<<gr, kMs3Threads, smem_r, st>>>(p2, q, kMs3FwdStep, z, rpc);
-    }
-  } else {
-    rows<<<gr, kMs3Threads, smem_r, st>>>(p2, q, kMs3BwdStart, q.L, rpc);
-    for (int z = q.L - 1; z >= 0; --z) {
-      cols<<<gc, kMs3Threads, smem_c, st>>>(p1, q, 1, cpc);
-      rows<<<gr, kMs3Threads, smem_r, st>>>(p2, q, kMs3BwdStep, z, rpc);
-    }
+  const dim3 gr4(four_r ? n1 / (256 / four_r1(n2)) : 1, q.P), gc4(four_c ? n2 / (256 / four_r1(n1)) : 1, q.P);
+  const Ms3Rows4 start4 = backward ? pick_rows4<kMs3BwdStart>(n2) : pick_rows4<kMs3FwdStart>(n2);
+  const Ms3Rows4 step4 = backward ? pick_rows4<kMs3BwdStep>(n2) : pick_rows4<kMs3FwdStep>(n2);
+  const Ms3Cols4 cols4 = backward ? pick_cols4<true>(n1) : pick_cols4<false>(n1);
+  auto row_pass = [&](bool start, int z) {
+    if (four_r) (start ? start4 : step4)<<<gr4, 256, 0, st>>>(q, w.tw2, z);
+    else
+      rows<<<gr, kMs3Threads, smem_r, st>>>(p2, q, backward ? (start ? kMs3BwdStart : kMs3BwdStep)
+                                                            : (start ? kMs3FwdStart : kMs3FwdStep), z, rpc);
+  };
+  row_pass(true, backward ? q.L : 0);
+  for (int t = 0; t < q.L; ++t) {
+    if (four_c) cols4<<<gc4, 256, 0, st>>>(q, w.tw1);
+    else cols<<<gc, kMs3Threads, smem_c, st>>>(p1, q, backward ? 1 : 0, cpc);
+    row_pass(false, backward ? q.L - 1 - t : t);
   }
   return check_cuda(cudaGetLastError(), "ms3d march launch");
 }
