@@ -312,7 +312,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
   };
   // The next step's CTAs may start as this one's leave: what they do before
   // their own wait reads only the slices' diagonals and the weights.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_trigger();
   // weights and diagonals of this thread's pixels; zero outside the image, so
   // that g and y stay zero there
   float2 cw0 = make_float2(0.f, 0.f), cw1 = cw0;
@@ -357,7 +357,7 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
     Ji[i].z = (row && in1) ? aw * nz : 0.f;
     Ji[i].w = (row && in1) ? az * nz : 0.f;
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // the step before is complete
+  pdl_wait();  // the step before is complete
   __syncthreads();
   if (staged && threadIdx.x == 0) {
     issue(0);
@@ -882,17 +882,8 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
       q.f1 = job.u_fwd + (size_t)s * N;
       q.grad = job.grad_c + (size_t)(s - 1) * N;
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(tiles, groups);
-    cfg.blockDim = dim3(kPThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = fresh ? 0 : 1;  // behind another kernel than a step's: after all of it
-    TP_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kerns[src ? 1 : 0], map, q, err));
+    // behind another kernel than a step's: after all of it
+    TP_CHECK_CUDA(launch_dependent(kerns[src ? 1 : 0], dim3(tiles, groups), dim3(kPThreads), smem, st, !fresh, map, q, err));
     fresh = false;
   }
   if (job.stats) c3_poly_stats_kernel<<<32, 256, 0, st>>>(norms, L * P, q.m, job.tol * job.tol, job.stats);

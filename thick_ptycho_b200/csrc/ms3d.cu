@@ -264,6 +264,7 @@ __global__ void __launch_bounds__(256, 2) ms3_rows4_kernel(const Ms3Params q, co
   const int pr = blockIdx.y, tid = threadIdx.x;
   const size_t pbase = (size_t)pr * q.N;
   const int g0 = blockIdx.x * RPC * N;
+  pdl_trigger();
   for (int e = tid; e < R1 * (R2 + 1); e += 256) tw[e] = twg[e];
   const int ra = tid / R2, n2 = tid % R2;  // stage A: (row, n2), element R2 n1 + n2
   const int rc = tid / R1, k1 = tid % R1;  // stage C: (row, k1), frequency k1 + R1 k2
@@ -288,17 +289,21 @@ __global__ void __launch_bounds__(256, 2) ms3_rows4_kernel(const Ms3Params q, co
       }
     }
   } else {
-#pragma unroll
-    for (int k2 = 0; k2 < R2; ++k2) x[k2] = wrow[R1 * k2];
-    if (inA) {  // under the inverse transform
+    if (inA) {  // what no kernel of the march writes, before the column pass is complete
       const float2 *T = q.trans + (size_t)(PHASE == kMs3FwdStep ? (last ? z : z + 1) : z) * q.N;
       const float2 *u = PHASE == kMs3BwdStep ? q.u_fwd + ((size_t)pr * q.nz + z) * q.N : nullptr;
 #pragma unroll
       for (int j = 0; j < R1; ++j) {
-        pz[j] = q.psi[pbase + ga + R2 * j];
         tz[j] = T[ga + R2 * j];
         if (PHASE == kMs3BwdStep) uz[j] = __ldcs(&u[ga + R2 * j]);
       }
+    }
+    pdl_wait();
+#pragma unroll
+    for (int k2 = 0; k2 < R2; ++k2) x[k2] = wrow[R1 * k2];
+    if (inA) {
+#pragma unroll
+      for (int j = 0; j < R1; ++j) pz[j] = q.psi[pbase + ga + R2 * j];
     }
     dft_reg<R2>(x, 1.f);
     __syncthreads();  // the twiddles are in place
@@ -360,13 +365,17 @@ __global__ void __launch_bounds__(256, 3) ms3_cols4_kernel(const Ms3Params q, co
   __shared__ float2 buf[N * CPC];  // [k1][n2][c]
   __shared__ float2 tw[R1 * (R2 + 1)];
   const int tid = threadIdx.x, w = q.n2;
+  pdl_trigger();
   for (int e = tid; e < R1 * (R2 + 1); e += 256) tw[e] = twg[e];
   const int c = tid % CPC, n2 = tid / CPC;  // stage A: (c, n2); stage C: (c, k1)
   const int k1 = n2;
   const bool inA = n2 < R2;
   float2 *base = q.W + (size_t)blockIdx.y * q.N + blockIdx.x * CPC + c;
   const float2 *h = q.hm1t + blockIdx.x * CPC + c + (size_t)k1 * w;
-  float2 x[16];
+  float2 x[16], hv[R2];
+#pragma unroll
+  for (int k2 = 0; k2 < R2; ++k2) hv[k2] = h[(size_t)R1 * k2 * w];
+  pdl_wait();
   if (inA) {
 #pragma unroll
     for (int j = 0; j < R1; ++j) x[j] = base[(size_t)(R2 * j + n2) * w];
@@ -377,9 +386,6 @@ __global__ void __launch_bounds__(256, 3) ms3_cols4_kernel(const Ms3Params q, co
 #pragma unroll
     for (int k = 0; k < R1; ++k) buf[(k * R2 + n2) * CPC + c] = k ? cmul(x[k], tw[k * (R2 + 1) + n2]) : x[0];
   }
-  float2 hv[R2];
-#pragma unroll
-  for (int k2 = 0; k2 < R2; ++k2) hv[k2] = h[(size_t)R1 * k2 * w];
   __syncthreads();
 #pragma unroll
   for (int m = 0; m < R2; ++m) x[m] = buf[(k1 * R2 + m) * CPC + c];
@@ -553,17 +559,19 @@ static int ms3_run(const tp_ms3d_op *op, Ms3Params q, bool backward, void *works
   const Ms3Rows4 start4 = backward ? pick_rows4<kMs3BwdStart>(n2) : pick_rows4<kMs3FwdStart>(n2);
   const Ms3Rows4 step4 = backward ? pick_rows4<kMs3BwdStep>(n2) : pick_rows4<kMs3FwdStep>(n2);
   const Ms3Cols4 cols4 = backward ? pick_cols4<true>(n1) : pick_cols4<false>(n1);
-  auto row_pass = [&](bool start, int z) {
-    if (four_r) (start ? start4 : step4)<<<gr4, 256, 0, st>>>(q, w.tw2, z);
-    else
-      rows<<<gr, kMs3Threads, smem_r, st>>>(p2, q, backward ? (start ? kMs3BwdStart : kMs3BwdStep)
-                                                            : (start ? kMs3FwdStart : kMs3FwdStep), z, rpc);
+  // the passes of a march with both four-step kernels start early (pdl_wait)
+  const bool early = four_r && four_c;
+  auto row_pass = [&](bool start, int z) -> cudaError_t {
+    if (four_r) return launch_dependent(start ? start4 : step4, gr4, dim3(256), 0, st, early && !start, q, w.tw2, z);
+    rows<<<gr, kMs3Threads, smem_r, st>>>(p2, q, backward ? (start ? kMs3BwdStart : kMs3BwdStep)
+                                                          : (start ? kMs3FwdStart : kMs3FwdStep), z, rpc);
+    return cudaSuccess;
   };
-  row_pass(true, backward ? q.L : 0);
+  TP_CHECK_CUDA(row_pass(true, backward ? q.L : 0));
   for (int t = 0; t < q.L; ++t) {
-    if (four_c) cols4<<<gc4, 256, 0, st>>>(q, w.tw1);
+    if (four_c) TP_CHECK_CUDA(launch_dependent(cols4, gc4, dim3(256), 0, st, early, q, w.tw1));
     else cols<<<gc, kMs3Threads, smem_c, st>>>(p1, q, backward ? 1 : 0, cpc);
-    row_pass(false, backward ? q.L - 1 - t : t);
+    TP_CHECK_CUDA(row_pass(false, backward ? q.L - 1 - t : t));
   }
   return check_cuda(cudaGetLastError(), "ms3d march launch");
 }

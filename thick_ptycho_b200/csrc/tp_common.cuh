@@ -271,4 +271,26 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar, uint32_t parity
   return false;
 }
 
+// Programmatic dependent launch: a kernel launched with launch_dependent may start
+// while the kernel before it on the stream finishes (once all of that one's CTAs have
+// called pdl_trigger or left); what it does before pdl_wait must not touch what that
+// kernel, or one before it, writes.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <class... P, class... A>
+inline cudaError_t launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, bool early,
+                                    A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;  // early = false: an ordinary launch
+  return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
+}
+
 }  // namespace tp
