@@ -152,6 +152,11 @@ __host__ __device__ __forceinline__ double2 zdiv(double2 a, double2 b) {
   double r = b.x / b.y, d = b.x * r + b.y;
   return z2((a.x * r + a.y) / d, (a.y * r - a.x) / d);
 }
+// 1 / a with one real division (|a|^2 within the range of fp64)
+__device__ __forceinline__ double2 zinv(double2 a) {
+  const double n = 1.0 / fma(a.x, a.x, a.y * a.y);
+  return z2(a.x * n, -a.y * n);
+}
 __device__ __forceinline__ float2 to_f2(double2 a) { return make_float2((float)a.x, (float)a.y); }
 // fp64 value to the march's complex type (rounded to complex64 in the normal build)
 __host__ __device__ __forceinline__ cx to_cx(double2 a) { return mkcx((rx)a.x, (rx)a.y); }
