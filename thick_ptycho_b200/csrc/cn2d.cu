@@ -155,10 +155,21 @@ __global__ void __launch_bounds__(256) cn2d_diag_kernel(const FactorParams f, in
   __shared__ double2 tile[32][33];
   const int e0 = blockIdx.x * 32, i = e0 / f.C, c0 = e0 % f.C;
   const int s0 = blockIdx.y * 32;
+  bool bad = false;
   for (int r = threadIdx.y; r < 32; r += 8) {
-    const int s = s0 + threadIdx.x;
-    if (s < count) tile[r][threadIdx.x] = p_diag(f, (c0 + r) * f.M + i, f.sl0 + s);
+    const int s = s0 + threadIdx.x, g = (c0 + r) * f.M + i;
+    if (s >= count) continue;
+    const double2 pd = p_diag(f, g, f.sl0 + s);
+    tile[r][threadIdx.x] = pd;
+    if (f.poly_bad != nullptr && g < f.N) {  // the polynomial march's bounds on this row
+      // (K's own row also for the transposed modes: the spectra are conjugate)
+      const float sum = (float)((g > 0 ? fabs(k_sub(f, g).y) : 0.0) + (g < f.N - 1 ? fabs(k_sup(f, g).y) : 0.0));
+      const float dr = (float)(1.0 - pd.x), di = (float)-pd.y, d2 = dr * dr + di * di;
+      if (!(d2 > 1e-4f && d2 < 1e8f)) bad = true;
+      if (sum > 0.f && !(sum * sum <= f.tau_max * f.tau_max * d2 && fabsf(atan2f(di, dr)) <= f.arg_max)) bad = true;
+    }
   }
+  if (bad) atomicOr(f.poly_bad, 1u);
   __syncthreads();
   for (int r = threadIdx.y; r < 32; r += 8) {
     const int s = s0 + r;
@@ -406,6 +417,7 @@ __device__ __forceinline__ void add_natural(cx (&U)[M], const cx *__restrict__ s
 
 template <int M, bool ALIGNED, bool LAGGED>
 __global__ void __launch_bounds__(kMarchWarps * 32, 1) cn2d_march_kernel(const MarchParams p) {
+  if (p.poly_bad != nullptr && *p.poly_bad == 0u) return;  // the polynomial kernel ran this march
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int probe = blockIdx.x * kMarchWarps + warp;
@@ -776,14 +788,24 @@ static int factor_slices(const tp_cn2d_op *op, const void *n_field, int32_t n_dt
   f.factors = static_cast<char *>(factors);
   f.slice_bytes = slice_bytes(pt);
   f.coupling = reinterpret_cast<unsigned *>(f.factors + (size_t)f.L * f.slice_bytes);
+#ifndef TP_C128_CHECK
+  if (!pt.team) {
+    const Poly2DPlan plan = poly2d_plan(op);
+    if (plan.m > 0) {
+      f.poly_bad = f.coupling + 1;
+      f.tau_max = plan.tau_max;
+      f.arg_max = plan.arg_max;
+    }
+  }
+#endif
   f.err = err;
   if (s_begin < 1 || s_end > f.L || s_begin > s_end)
     return set_error(TP_ERR_INVALID, "slice range [%d, %d] outside [1, %d]", s_begin, s_end, f.L);
   f.sl0 = s_begin - 1;
-  // the PCR coupling bound is a running maximum over the slices factorised
+  // the PCR coupling bound (and the word after it) is a running maximum over the slices factorised
   // since the last reset, which the range starting at slice 1 performs
   if (s_begin == 1)
-    TP_CHECK_CUDA(cudaMemsetAsync(f.coupling, 0, sizeof(unsigned), reinterpret_cast<cudaStream_t>(stream)));
+    TP_CHECK_CUDA(cudaMemsetAsync(f.coupling, 0, 2 * sizeof(unsigned), reinterpret_cast<cudaStream_t>(stream)));
   const size_t smem = 5 * (size_t)pt.C * sizeof(double2);
   const int count = s_end - s_begin + 1;
   cn2d_diag_kernel<<<dim3(pt.C * pt.M / 32, (count + 31) / 32), dim3(32, 8), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
@@ -894,6 +916,14 @@ extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp
         return set_error(TP_ERR_INVALID, "the team path needs 16-byte aligned u_store, u_fwd, grad_c, state_in, state_out");
     return launch_team_march(pt, mp, lagged, reinterpret_cast<cudaStream_t>(stream));
   }
+#ifndef TP_C128_CHECK
+  const Poly2DPlan plan = poly2d_plan(op);
+  if (plan.m > 0) {
+    mp.poly_bad = mp.coupling + 1;
+    rc = launch_poly_march(pt, mp, plan, mp.poly_bad, lagged, reinterpret_cast<cudaStream_t>(stream));
+    if (rc) return rc;
+  }
+#endif
   return launch_march(pt.M, mp, op->n == pt.C * pt.M, lagged, reinterpret_cast<cudaStream_t>(stream));
 }
 

@@ -33,7 +33,8 @@ __host__ __device__ inline int rec_rde(int levels) { return 2 + 2 * levels; }
 // Global factor set of one slice: QD, LF, EP, V, W ([M][C] complex values
 // each) then the records ([nrec][C]), padded to 256 bytes.  The workspace of a
 // factorisation holds L slices and then kFactorTailBytes: the largest PCR
-// coefficient of all slices (float bits), which the team march reads.
+// coefficient of all slices (float bits), which the team march reads, and a word
+// that is non-zero when a row is outside the polynomial march's bounds.
 __host__ __device__ inline size_t slice_bytes(const Partition &pt) {
   size_t b = (size_t)(5 * pt.M + pt.nrec) * pt.C * sizeof(cx);
   return (b + 255) & ~size_t(255);
@@ -71,6 +72,8 @@ struct FactorParams {
   char *factors;
   size_t slice_bytes;
   unsigned *coupling;  // max |alpha|, |gamma| of the PCR records (float bits), atomically maxed
+  unsigned *poly_bad;  // set where a row exceeds the bounds below (the word after `coupling`)
+  float tau_max, arg_max;
   int *err;
 };
 
@@ -94,6 +97,7 @@ struct MarchParams {
   const cx *u_fwd;
   cx *grad_c;
   const unsigned *coupling;     // the factor set's PCR coupling bound (float bits), or NULL
+  const unsigned *poly_bad;     // direct kernel of the 32-chunk layout: 0 = the polynomial kernel runs instead
   int *err;
   int t0, t1;                   // step range
   const cx *state_in;           // chunked (P, Npad) or null
@@ -121,6 +125,19 @@ __host__ __device__ inline int store_index(const MarchParams &p, int t) {
 // diagonal magnitude of the free-space matrix; keep rows until rho^T is
 // below kSpikeDrop (plus one).  The factor kernel verifies the choice on the actual matrices.
 int team_spike_rows(const tp_cn2d_op *op, int M);
+
+// Polynomial march of the 32-chunk layout (cn2d_poly.cu): its degree and
+// coefficients for an operator (m = 0: none), and the bounds every row of a
+// factor set has to keep (row sum of |J|, |arg D|).
+constexpr int kPoly2DMaxDeg = 10;
+struct Poly2DPlan {
+  int m;
+  float a[kPoly2DMaxDeg];
+  float tau_max, arg_max;
+};
+Poly2DPlan poly2d_plan(const tp_cn2d_op *op);
+int launch_poly_march(const Partition &pt, const MarchParams &mp, const Poly2DPlan &plan, const unsigned *bad,
+                      bool lagged, cudaStream_t st);
 
 // Team-path launcher (cn2d_team.cu).
 int launch_team_march(const Partition &pt, MarchParams &mp, bool lagged, cudaStream_t st);

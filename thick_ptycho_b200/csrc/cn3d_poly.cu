@@ -54,8 +54,9 @@ constexpr int kPThreads = 32 * kPWarps;
 constexpr int kPolyMaxDeg = 10, kPolyMaxHalo = 16;
 
 struct PolyCheck {
-  unsigned tau, arg;  // bits of the largest row sum of |J| and the largest |arg D| (non-negative floats)
-  int bad, pad;
+  // bits of the largest row and column sums of |J| and the largest |arg D| (non-negative floats)
+  unsigned tau, tau_col, arg;
+  int bad;
 };
 
 struct PolySlices {
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q,
                                                              int s_hi, float2 *cd, PolyCheck *chk) {
   __shared__ float2 tile[32][33];
   const int i0 = blockIdx.x * 32, s0 = s_first + blockIdx.y * 32;
-  float tau = 0.f, arg = 0.f;
+  float tau = 0.f, tcol = 0.f, arg = 0.f;
   int bad = 0;
   for (int r = threadIdx.y; r < 32; r += 8) {
     const int i = i0 + r, s = s0 + threadIdx.x;
@@ -128,6 +129,10 @@ __global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q,
         const float t = sum / sqrtf(dr * dr + di * di);
         if (!(t < 1e6f)) bad = 1;
         tau = fmaxf(tau, t);
+        // what row i's element reaches: its neighbours' couplings back to it
+        const float col = ((f + 1 < q.nf ? fabsf(q.colw[f + 1].x) : 0.f) + (f > 0 ? fabsf(q.colw[f - 1].y) : 0.f)) * rw.z +
+                          (b + 1 < q.nb ? fabsf(q.roww[b + 1].x) : 0.f) + (b > 0 ? fabsf(q.roww[b - 1].y) : 0.f);
+        tcol = fmaxf(tcol, col / sqrtf(dr * dr + di * di));
         arg = fmaxf(arg, fabsf(atan2f(di, dr)));
       } else {
         const float dr = 1.f - d.x, n2 = dr * dr + d.y * d.y;
@@ -150,6 +155,7 @@ __global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q,
   if (chk == nullptr) return;
   for (int o = 16; o > 0; o >>= 1) {
     tau = fmaxf(tau, __shfl_down_sync(0xffffffffu, tau, o));
+    tcol = fmaxf(tcol, __shfl_down_sync(0xffffffffu, tcol, o));
     arg = fmaxf(arg, __shfl_down_sync(0xffffffffu, arg, o));
     bad |= __shfl_down_sync(0xffffffffu, bad, o);
   }
@@ -157,6 +163,7 @@ __global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q,
     // most blocks do not raise the maxima: read before the atomic
     const volatile PolyCheck *c = chk;
     if (__float_as_uint(tau) > c->tau) atomicMax(&chk->tau, __float_as_uint(tau));
+    if (__float_as_uint(tcol) > c->tau_col) atomicMax(&chk->tau_col, __float_as_uint(tcol));
     if (__float_as_uint(arg) > c->arg) atomicMax(&chk->arg, __float_as_uint(arg));
     if (bad) atomicOr(&chk->bad, 1);
   }
@@ -773,8 +780,12 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
   TP_CHECK_CUDA(cudaMemcpyAsync(&host, chk, sizeof(PolyCheck), cudaMemcpyDeviceToHost, st));
   TP_CHECK_CUDA(cudaStreamSynchronize(st));
   if (host.bad) return TP_OK;
-  float tau, theta;
+  // either norm bounds the spectral radius (a transposed operator's rows are the
+  // original's columns: the doubled Neumann couplings add up in one of the two)
+  float tau, tcol, theta;
   memcpy(&tau, &host.tau, 4);
+  memcpy(&tcol, &host.tau_col, 4);
+  if (tcol < tau) tau = tcol;
   memcpy(&theta, &host.arg, 4);
 
   PolyStep q{};
