@@ -261,14 +261,14 @@ __global__ void pit_factor_kernel(const PitKd K, int L, double alpha_root, float
   const double2 omw = z2(1.0 - w.x, -w.y), opw = z2(1.0 + w.x, w.y);
   auto dval = [&](int i) { return zsub(omw, zmul(opw, K.dia(i))); };
   double2 d = dval(0);
-  double2 dinv = zdiv(z2(1.0, 0.0), d);
+  double2 dinv = zinv(d);
   F[k] = make_float4(0.f, 0.f, (float)dinv.x, (float)dinv.y);
   for (int i = 1; i < K.N; ++i) {
     const double2 a = zneg(zmul(opw, K.sub(i)));          // row i, column i-1
     const double2 cprev = zneg(zmul(opw, K.sup(i - 1)));  // row i-1, column i
     const double2 m = zmul(a, dinv);
     d = zsub(dval(i), zmul(m, cprev));
-    dinv = zdiv(z2(1.0, 0.0), d);
+    dinv = zinv(d);
     F[(size_t)i * L + k] = make_float4((float)m.x, (float)m.y, (float)dinv.x, (float)dinv.y);
   }
 }
@@ -340,6 +340,25 @@ __global__ void pit_block_solve_kernel(const PitK K, int L, int P, double alpha_
 }
 
 // ------------------------------------------------------------------ Krylov
+// dst[r] += the CTA's sums of the first cnt complex accumulators.
+__device__ __forceinline__ void pit_reduce_dots(const double (&acc)[2 * kPitDotGroup], int cnt,
+                                                double (*red)[2 * kPitDotGroup], double2 *dst) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
+  for (int r = 0; r < 2 * kPitDotGroup; ++r) {
+    if (r >= 2 * cnt) break;
+    double v = acc[r];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if (lane == 0) red[wid][r] = v;
+  }
+  __syncthreads();
+  if (threadIdx.x < 2 * cnt) {
+    double s = 0.0;
+    for (int q = 0; q < kPitThreads / 32; ++q) s += red[q][threadIdx.x];
+    atomicAdd(reinterpret_cast<double *>(&dst[threadIdx.x >> 1]) + (threadIdx.x & 1), s);
+  }
+}
+
 // h[p][r0 + r] += <V_{r0+r}[p], w[p]> (fp64) for r < min(kPitDotGroup, nv - r0).
 __global__ void __launch_bounds__(kPitThreads) pit_dots_kernel(size_t n, int P, const float2 *__restrict__ V,
                                                                size_t vstride, int r0, int nv,
@@ -364,30 +383,20 @@ __global__ void __launch_bounds__(kPitThreads) pit_dots_kernel(size_t n, int P, 
       }
     }
   }
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int r = 0; r < 2 * kPitDotGroup; ++r) {
-    double v = acc[r];
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) red[wid][r] = v;
-  }
-  __syncthreads();
-  if (threadIdx.x < 2 * cnt) {
-    double s = 0.0;
-    for (int q = 0; q < kPitThreads / 32; ++q) s += red[q][threadIdx.x];
-    double *dst = reinterpret_cast<double *>(&h[(size_t)p * hld + r0 + (threadIdx.x >> 1)]) + (threadIdx.x & 1);
-    atomicAdd(dst, s);
-  }
+  pit_reduce_dots(acc, cnt, red, &h[(size_t)p * hld + r0]);
 }
 
-// w[p] += sign * sum_{r < nv} coef[p][r] V_r[p]  (coef fp64, per probe)
+// w[p] += sign * sum_{r < nv} coef[p][r] V_r[p]  (coef fp64, per probe); nrm (or
+// NULL): nrm[p] += ||w[p]||^2 of the result.
 __global__ void __launch_bounds__(kPitThreads) pit_combine_kernel(size_t n, int P, const float2 *__restrict__ V,
                                                                   size_t vstride, int nv,
                                                                   const double2 *__restrict__ coef, int cld,
-                                                                  float sign, float2 *__restrict__ w,
+                                                                  float sign, float2 *__restrict__ w, double *nrm,
                                                                   const int *active) {
   const int p = blockIdx.y;
   if (active != nullptr && !active[p]) return;
+  __shared__ double red[kPitThreads / 32];
+  double sum = 0.0;
   __shared__ float2 cf[kPitMaxRestart + 1];
   for (int r = threadIdx.x; r < nv; r += blockDim.x) {
     const double2 c = coef[(size_t)p * cld + r];
@@ -399,7 +408,56 @@ __global__ void __launch_bounds__(kPitThreads) pit_combine_kernel(size_t n, int 
     float2 acc = wp[e];
     for (int r = 0; r < nv; ++r) acc = cfma(cf[r], V[(size_t)r * vstride + (size_t)p * n + e], acc);
     wp[e] = acc;
+    if (nrm != nullptr) sum += (double)acc.x * acc.x + (double)acc.y * acc.y;
   }
+  if (nrm == nullptr) return;
+  for (int o = 16; o > 0; o >>= 1) sum += __shfl_down_sync(0xffffffffu, sum, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double s = 0.0;
+    for (int q = 0; q < kPitThreads / 32; ++q) s += red[q];
+    atomicAdd(&nrm[p], s);
+  }
+}
+
+// The second Gram-Schmidt pass' first half in one reading of the basis (nv <=
+// kPitDotGroup): w[p] -= sum_r coef[p][r] V_r[p], then h[p][r] += <V_r[p], w[p]>.
+__global__ void __launch_bounds__(kPitThreads) pit_combine_dots_kernel(size_t n, const float2 *__restrict__ V,
+                                                                       size_t vstride, int nv,
+                                                                       const double2 *__restrict__ coef, int cld,
+                                                                       float2 *__restrict__ w, double2 *h,
+                                                                       const int *active) {
+  const int p = blockIdx.y;
+  if (active != nullptr && !active[p]) return;
+  __shared__ double red[kPitThreads / 32][2 * kPitDotGroup];
+  float2 cf[kPitDotGroup];
+  double acc[2 * kPitDotGroup];
+#pragma unroll
+  for (int r = 0; r < kPitDotGroup; ++r) {
+    acc[2 * r] = acc[2 * r + 1] = 0.0;
+    const double2 c = r < nv ? coef[(size_t)p * cld + r] : z2(0.0, 0.0);
+    cf[r] = make_float2((float)-c.x, (float)-c.y);
+  }
+  float2 *wp = w + (size_t)p * n;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+    float2 v[kPitDotGroup], x = wp[e];
+#pragma unroll
+    for (int r = 0; r < kPitDotGroup; ++r)
+      if (r < nv) v[r] = V[(size_t)r * vstride + (size_t)p * n + e];
+#pragma unroll
+    for (int r = 0; r < kPitDotGroup; ++r)
+      if (r < nv) x = cfma(cf[r], v[r], x);
+    wp[e] = x;
+#pragma unroll
+    for (int r = 0; r < kPitDotGroup; ++r) {
+      if (r < nv) {
+        acc[2 * r] += (double)v[r].x * x.x + (double)v[r].y * x.y;
+        acc[2 * r + 1] += (double)v[r].x * x.y - (double)v[r].y * x.x;
+      }
+    }
+  }
+  pit_reduce_dots(acc, nv, red, &h[(size_t)p * cld]);
 }
 
 // nrm[p] += ||x[p]||^2 (fp64)
@@ -445,7 +503,8 @@ struct PitWork {
   float2 *V, *Z, *w, *xh, *b, *C, *chirp, *bker, *bhat, *tw;
   float4 *F;
   float *gamma;
-  double2 *h;
+  // the two passes' inner products (P x hld each) and the norms, back to back
+  double2 *h, *h2;
   double *nrm, *s;
   int *active;
   size_t bytes;
@@ -481,8 +540,10 @@ static PitWork pit_layout(char *base, int N, int L, int P, int m) {
   w.bker = reinterpret_cast<float2 *>(take((size_t)M * sizeof(float2)));
   w.bhat = reinterpret_cast<float2 *>(take((size_t)M * sizeof(float2)));
   w.tw = reinterpret_cast<float2 *>(take((size_t)M * sizeof(float2)));
-  w.h = reinterpret_cast<double2 *>(take((size_t)P * (kPitMaxRestart + 1) * sizeof(double2)));
-  w.nrm = reinterpret_cast<double *>(take((size_t)P * sizeof(double)));
+  const size_t hlen = (size_t)P * (kPitMaxRestart + 1);
+  w.h = reinterpret_cast<double2 *>(take(2 * hlen * sizeof(double2) + (size_t)P * sizeof(double)));
+  w.h2 = w.h + hlen;
+  w.nrm = reinterpret_cast<double *>(w.h + 2 * hlen);
   w.s = reinterpret_cast<double *>(take((size_t)P * sizeof(double)));
   w.active = reinterpret_cast<int *>(take((size_t)P * sizeof(int)));
   w.bytes = off;
@@ -586,23 +647,47 @@ class PitSolver {
     TP_CHECK_CUDA(cudaStreamSynchronize(st_));
     return TP_OK;
   }
-  // h[p][0..nv) = V_{0..nv}^H w (device)
-  int dots(int nv, const float2 *w) {
-    TP_CHECK_CUDA(cudaMemsetAsync(w_.h, 0, (size_t)P_ * (kPitMaxRestart + 1) * sizeof(double2), st_));
-    for (int r0 = 0; r0 < nv; r0 += kPitDotGroup)
-      pit_dots_kernel<<<dim3(red_blocks(), P_), kPitThreads, 0, st_>>>(n_, P_, w_.V, n_ * P_, r0, nv, w, w_.h,
-                                                                      kPitMaxRestart + 1, w_.active);
-    return check_cuda(cudaGetLastError(), "pit dots launch");
+  // w orthogonalised against V_0..V_{nv-1} by classical Gram-Schmidt, twice: the two
+  // passes' products in w_.h and w_.h2 and the remaining norms in w_.nrm, read back
+  // together (one host wait per Arnoldi step).
+  int orthogonalise(int nv, float2 *w, std::vector<double> &out) {
+    const size_t hlen = (size_t)P_ * (kPitMaxRestart + 1), bytes = 2 * hlen * sizeof(double2) + P_ * sizeof(double);
+    TP_CHECK_CUDA(cudaMemsetAsync(w_.h, 0, bytes, st_));
+    const dim3 grid(red_blocks(), P_);
+    auto dots = [&](double2 *h) {
+      for (int r0 = 0; r0 < nv; r0 += kPitDotGroup)
+        pit_dots_kernel<<<grid, kPitThreads, 0, st_>>>(n_, P_, w_.V, n_ * P_, r0, nv, w, h, kPitMaxRestart + 1, w_.active);
+    };
+    dots(w_.h);
+    if (nv <= kPitDotGroup) {
+      pit_combine_dots_kernel<<<grid, kPitThreads, 0, st_>>>(n_, w_.V, n_ * P_, nv, w_.h, kPitMaxRestart + 1, w, w_.h2,
+                                                             w_.active);
+    } else {
+      pit_combine_kernel<<<grid, kPitThreads, 0, st_>>>(n_, P_, w_.V, n_ * P_, nv, w_.h, kPitMaxRestart + 1, -1.f, w,
+                                                        nullptr, w_.active);
+      dots(w_.h2);
+    }
+    pit_combine_kernel<<<grid, kPitThreads, 0, st_>>>(n_, P_, w_.V, n_ * P_, nv, w_.h2, kPitMaxRestart + 1, -1.f, w,
+                                                      w_.nrm, w_.active);
+    TP_CHECK_CUDA(cudaGetLastError());
+    out.resize(bytes / sizeof(double));
+    TP_CHECK_CUDA(cudaMemcpyAsync(out.data(), w_.h, bytes, cudaMemcpyDeviceToHost, st_));
+    TP_CHECK_CUDA(cudaStreamSynchronize(st_));
+    return TP_OK;
   }
   // target += sign * sum_r h[p][r] basis_r[p]
   int combine(const float2 *basis, int nv, float sign, float2 *target) {
     pit_combine_kernel<<<dim3(red_blocks(), P_), kPitThreads, 0, st_>>>(n_, P_, basis, n_ * P_, nv, w_.h,
-                                                                       kPitMaxRestart + 1, sign, target, w_.active);
+                                                                       kPitMaxRestart + 1, sign, target, nullptr,
+                                                                       w_.active);
     return check_cuda(cudaGetLastError(), "pit combine launch");
   }
   int red_blocks() const {
+    // enough CTAs for every SM over all probes; more would spend their time on the
+    // sums at their ends (dots of 32 probes, 32512 elements: 22 us with 64 per probe)
     const size_t g = (n_ + kPitThreads - 1) / kPitThreads;
-    return (int)(g < 64 ? g : 64);
+    const size_t want = (size_t)std::max(1, std::min(64, (4 * 148 + P_ - 1) / P_));
+    return (int)(g < want ? g : want);
   }
 
   PitK K_;   // the operator's K: right-hand side, preconditioner blocks
@@ -675,6 +760,7 @@ extern "C" int tp_pit_solve(const tp_cn2d_op *op, const void *n_field, int32_t n
   using cd = std::complex<double>;
   std::vector<cd> H((size_t)P * (m + 1) * m), cs((size_t)P * m), sn((size_t)P * m), g((size_t)P * (m + 1));
   std::vector<double2> hh((size_t)P * (kPitMaxRestart + 1));
+  std::vector<double> back;
   std::vector<int> inner(P), kdim(P);
   auto Hat = [&](int p, int r, int c) -> cd & { return H[((size_t)p * (m + 1) + r) * m + c]; };
 
@@ -712,29 +798,20 @@ extern "C" int tp_pit_solve(const tp_cn2d_op *op, const void *n_field, int32_t n
       if (rc) return rc;
       rc = S.matvec(Zj, w.w);
       if (rc) return rc;
-      // classical Gram-Schmidt, twice
-      std::vector<cd> hsum((size_t)P * (j + 1), cd(0.0));
-      for (int pass = 0; pass < 2; ++pass) {
-        rc = S.dots(j + 1, w.w);
-        if (rc) return rc;
-        rc = S.combine(w.V, j + 1, -1.f, w.w);
-        if (rc) return rc;
-        TP_CHECK_CUDA(cudaMemcpyAsync(hh.data(), w.h, hh.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
-        TP_CHECK_CUDA(cudaStreamSynchronize(st));
-        for (int p = 0; p < P; ++p)
-          for (int r = 0; r <= j; ++r) {
-            const double2 v = hh[(size_t)p * (kPitMaxRestart + 1) + r];
-            hsum[(size_t)p * (j + 1) + r] += cd(v.x, v.y);
-          }
-      }
-      rc = S.norms(w.w, rn);
+      rc = S.orthogonalise(j + 1, w.w, back);
       if (rc) return rc;
+      const size_t hlen = (size_t)P * (kPitMaxRestart + 1);
+      const cd *h1 = reinterpret_cast<const cd *>(back.data()), *h2 = h1 + hlen;
+      const double *nrm = back.data() + 4 * hlen;
       bool cont = false;
       for (int p = 0; p < P; ++p) {
         sc[p] = 0.0;
         if (!inner[p]) continue;
-        for (int r = 0; r <= j; ++r) Hat(p, r, j) = hsum[(size_t)p * (j + 1) + r];
-        const double eta = std::sqrt(rn[p]);
+        for (int r = 0; r <= j; ++r) {
+          const size_t at = (size_t)p * (kPitMaxRestart + 1) + r;
+          Hat(p, r, j) = h1[at] + h2[at];
+        }
+        const double eta = std::sqrt(nrm[p]);
         Hat(p, j + 1, j) = eta;
         cd *csp = &cs[(size_t)p * m], *snp = &sn[(size_t)p * m], *gp = &g[(size_t)p * (m + 1)];
         for (int r = 0; r < j; ++r) {  // previous rotations
