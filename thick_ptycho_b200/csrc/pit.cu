@@ -185,15 +185,15 @@ __global__ void pit_tables_kernel(int L, int M, double alpha, float *gamma, floa
   }
 }
 
-// Unitary DFT along z by Bluestein's chirp-z, cpc columns per CTA.
-//   INV (into the block domain): x_j = gamma_j v[p][j][i] (slice-major in),
-//     out Xh[p][i][k] = (1/sqrt L) sum_j x_j e^{+2 pi i jk/L}   (i-major out)
-//   !INV (back):  x_k = Xh[p][i][k],
+// Unitary DFT along z by Bluestein's chirp-z, cpc columns per CTA; both domains are
+// slice-major (P, L, N).
+//   INV (into the block domain): x_j = gamma_j v[p][j][i],
+//     out Xh[p][k][i] = (1/sqrt L) sum_j x_j e^{+2 pi i jk/L}
+//   !INV (back):  x_k = Xh[p][k][i],
 //     out[p][j][i] = (1/sqrt L) sum_k x_k e^{-2 pi i jk/L} / gamma_j
-// The inverse direction is conj(DFT(conj x)).  Grid (ceil(N/cpc), P).  MF:
-// the transform length when it has a compile-time plan (128, 256, 512,
-// 2048; radix-16 passes for 256 and 2048), else 0 and the runtime plan `pl`.
-template <bool INV, int MF>
+// The inverse direction is conj(DFT(conj x)).  Grid (ceil(N/cpc), P).  Transform
+// lengths below 128 on the shared-memory passes.
+template <bool INV>
 __global__ void __launch_bounds__(kPitThreads) pit_zdft_kernel(const FftPlan pl, int N, int L, int cpc,
                                                                const float2 *__restrict__ in, float2 *__restrict__ out,
                                                                const float *__restrict__ gamma,
@@ -205,53 +205,163 @@ __global__ void __launch_bounds__(kPitThreads) pit_zdft_kernel(const FftPlan pl,
   if (active != nullptr && !active[p]) return;
   float2 *tw = zsm, *a = tw + M, *b = a + cpc * M;
   load_twiddles(tw, twg, M);
-  const size_t per = (size_t)L * N;
+  const size_t base = (size_t)p * L * N + i0;
   for (int e = threadIdx.x; e < cpc * M; e += blockDim.x) a[e] = make_float2(0.f, 0.f);
   __syncthreads();
-  if (INV) {
-    for (int e = threadIdx.x; e < cpc * L; e += blockDim.x) {
-      const int q = e % cpc, j = e / cpc;  // coalesced over q
-      if (i0 + q >= N) continue;
-      const float2 v = in[(size_t)p * per + (size_t)j * N + i0 + q];
-      const float g = gamma[j];
-      a[q * M + j] = cmul(make_float2(g * v.x, -g * v.y), chirp[j]);  // conj(x) c_j
-    }
-  } else {
-    for (int e = threadIdx.x; e < cpc * L; e += blockDim.x) {
-      const int q = e / L, k = e % L;  // coalesced over k
-      if (i0 + q >= N) continue;
-      a[q * M + k] = cmul(in[(size_t)p * per + (size_t)(i0 + q) * L + k], chirp[k]);
-    }
+  for (int e = threadIdx.x; e < cpc * L; e += blockDim.x) {
+    const int q = e % cpc, j = e / cpc;  // coalesced over q
+    if (i0 + q >= N) continue;
+    float2 v = in[base + (size_t)j * N + q];
+    if (INV) v = make_float2(gamma[j] * v.x, -gamma[j] * v.y);
+    a[q * M + j] = cmul(v, chirp[j]);
   }
   __syncthreads();
-  float2 *F = MF > 0 ? fft_block_fixed<MF>(a, b, tw, false, cpc, threadIdx.x, blockDim.x)
-                     : fft_block(a, b, pl, tw, false, cpc, threadIdx.x, blockDim.x);
+  float2 *F = fft_block(a, b, pl, tw, false, cpc, threadIdx.x, blockDim.x);
   float2 *o = (F == a) ? b : a;
   for (int e = threadIdx.x; e < cpc * M; e += blockDim.x) F[e] = cmul(F[e], bhat[e % M]);
   __syncthreads();
-  const float2 *R = MF > 0 ? fft_block_fixed<MF>(F, o, tw, true, cpc, threadIdx.x, blockDim.x)
-                           : fft_block(F, o, pl, tw, true, cpc, threadIdx.x, blockDim.x);
+  const float2 *R = fft_block(F, o, pl, tw, true, cpc, threadIdx.x, blockDim.x);
   const float sc = 1.f / ((float)M * sqrtf((float)L));
-  if (INV) {
-    for (int e = threadIdx.x; e < cpc * L; e += blockDim.x) {
-      const int q = e / L, k = e % L;
-      if (i0 + q >= N) continue;
-      const float2 X = cmul(R[q * M + k], chirp[k]);
-      out[(size_t)p * per + (size_t)(i0 + q) * L + k] = make_float2(sc * X.x, -sc * X.y);  // conj
+  for (int e = threadIdx.x; e < cpc * L; e += blockDim.x) {
+    const int q = e % cpc, j = e / cpc;
+    if (i0 + q >= N) continue;
+    const float2 X = cmul(R[q * M + j], chirp[j]);
+    const float t = INV ? sc : sc / gamma[j];
+    out[base + (size_t)j * N + q] = make_float2(t * X.x, INV ? -t * X.y : t * X.y);
+  }
+}
+
+// The same for M = 16 R2 R3 in 128 .. 4096 with the transforms in registers: M / 16
+// threads per column keep 16 values each; the forward transform leaves the spectrum in
+// the order of its last step, where it meets bhat and the inverse starts (the steps of
+// the 2D multislice's register transforms, ms2d.cu; R3 = 1: two steps).  Threads run
+// over the CTA's columns first, so the loads, the stores and the shared-memory exchanges
+// move runs of neighbouring columns.  M = 256, 32 x 256 columns: 40 -> 13 us.
+template <int R2, int R3>
+struct PitFft {
+  static constexpr int M = 16 * R2 * R3, T = M / 16, CPC = kPitThreads / T, M2 = 16 / R2, M3 = 16 / R3;
+  static constexpr int S1 = T + R3, S2 = ((R2 * (R3 + 1) + 15) / 16) * 16 + R3;
+  static constexpr int BUF = 16 * (S1 > S2 ? S1 : S2);
+};
+template <int R>
+__device__ __forceinline__ void pit_dft(float2 *x, float sign) {
+  if constexpr (R > 1) {
+    float2 w[16];
+#pragma unroll
+    for (int i = 0; i < R; ++i) w[i] = x[i];
+    if constexpr (R == 2) {
+      const float2 t = w[0];
+      w[0] = cadd(t, w[1]);
+      w[1] = csub(t, w[1]);
+    } else {
+      dft_reg<R>(w, sign);
     }
-  } else {
-    for (int e = threadIdx.x; e < cpc * L; e += blockDim.x) {
-      const int q = e % cpc, j = e / cpc;
-      if (i0 + q >= N) continue;
-      const float2 X = cmul(R[q * M + j], chirp[j]);
-      const float s = sc / gamma[j];
-      out[(size_t)p * per + (size_t)j * N + i0 + q] = make_float2(s * X.x, s * X.y);
+#pragma unroll
+    for (int i = 0; i < R; ++i) x[i] = w[i];
+  }
+}
+
+template <bool INV, int R2, int R3>
+__global__ void __launch_bounds__(kPitThreads, 2) pit_zdft_reg_kernel(int N, int L, const float2 *__restrict__ in,
+                                                                      float2 *__restrict__ out,
+                                                                      const float *__restrict__ gamma,
+                                                                      const float2 *__restrict__ chirp,
+                                                                      const float2 *__restrict__ bhat,
+                                                                      const float2 *__restrict__ tw, const int *active) {
+  using F = PitFft<R2, R3>;
+  constexpr int M = F::M, T = F::T, CPC = F::CPC, S1 = F::S1, S2 = F::S2;
+  extern __shared__ __align__(16) float2 zsm[];
+  const int p = blockIdx.y, i0 = blockIdx.x * CPC;
+  if (active != nullptr && !active[p]) return;
+  const int q = threadIdx.x % CPC, v = threadIdx.x / CPC;
+  float2 *b0 = zsm + q, *b1 = b0 + F::BUF * CPC;  // slot s of this column: s * CPC
+  const size_t base = (size_t)p * L * N + i0 + q;
+  const bool col = i0 + q < N;
+  float2 x[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const int z = v + T * j;
+    x[j] = make_float2(0.f, 0.f);
+    if (col && z < L) {
+      float2 w = in[base + (size_t)z * N];
+      if (INV) {
+        const float g = gamma[z];
+        w = make_float2(g * w.x, -g * w.y);  // conj(x) c_j
+      }
+      x[j] = cmul(w, chirp[z]);
     }
+  }
+  pit_dft<16>(x, -1.f);
+#pragma unroll
+  for (int k = 0; k < 16; ++k) b0[(k * S1 + v) * CPC] = k ? cmul(x[k], tw[v * k]) : x[0];
+  __syncthreads();
+#pragma unroll
+  for (int m = 0; m < F::M2; ++m) {
+    const int u = v + T * m, k1 = u / R3, a = u % R3;
+#pragma unroll
+    for (int b = 0; b < R2; ++b) x[m * R2 + b] = b0[(k1 * S1 + a + R3 * b) * CPC];
+    pit_dft<R2>(x + m * R2, -1.f);
+    if constexpr (R3 == 1) {
+#pragma unroll
+      for (int k = 0; k < R2; ++k) x[m * R2 + k] = cmul(x[m * R2 + k], bhat[k1 + 16 * k]);
+      pit_dft<R2>(x + m * R2, 1.f);
+    } else {
+#pragma unroll
+      for (int k = 0; k < R2; ++k)
+        b1[(k1 * S2 + k * (R3 + 1) + a) * CPC] = k ? cmul(x[m * R2 + k], tw[16 * a * k]) : x[m * R2];
+    }
+  }
+  if constexpr (R3 > 1) {
+    __syncthreads();
+#pragma unroll
+    for (int m = 0; m < F::M3; ++m) {
+      const int u = v + T * m, k1 = u / R2, k2 = u % R2;
+      float2 *c = b1 + (k1 * S2 + k2 * (R3 + 1)) * CPC;  // this unit's own slots in both directions
+#pragma unroll
+      for (int a = 0; a < R3; ++a) x[m * R3 + a] = c[a * CPC];
+      pit_dft<R3>(x + m * R3, -1.f);
+#pragma unroll
+      for (int k = 0; k < R3; ++k) x[m * R3 + k] = cmul(x[m * R3 + k], bhat[k1 + 16 * k2 + 16 * R2 * k]);
+      pit_dft<R3>(x + m * R3, 1.f);
+#pragma unroll
+      for (int a = 0; a < R3; ++a) c[a * CPC] = x[m * R3 + a];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int m = 0; m < F::M2; ++m) {
+    const int u = v + T * m, k1 = u / R3, a = u % R3;
+    if constexpr (R3 > 1) {
+#pragma unroll
+      for (int k = 0; k < R2; ++k) {
+        const float2 w = b1[(k1 * S2 + k * (R3 + 1) + a) * CPC];
+        x[m * R2 + k] = k ? cmulc(w, tw[16 * a * k]) : w;
+      }
+      pit_dft<R2>(x + m * R2, 1.f);
+    }
+#pragma unroll
+    for (int b = 0; b < R2; ++b) b0[(k1 * S1 + a + R3 * b) * CPC] = x[m * R2 + b];  // slots this thread read
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    const float2 w = b0[(k * S1 + v) * CPC];
+    x[k] = k ? cmulc(w, tw[v * k]) : w;
+  }
+  pit_dft<16>(x, 1.f);
+  const float sc = 1.f / ((float)M * sqrtf((float)L));
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const int z = v + T * j;
+    if (!col || z >= L) continue;
+    const float2 X = cmul(x[j], chirp[z]);
+    const float t = INV ? sc : sc / gamma[z];
+    out[base + (size_t)z * N] = make_float2(t * X.x, INV ? -t * X.y : t * X.y);
   }
 }
 
 // LU factors of the L blocks (A - w_k B) = (1 - w_k) I - (1 + w_k) K, fp64
-// Thomas elimination, stored as float4 (m_i, 1/d_i) at [i][k].
+// Thomas elimination, stored as float4 (m_i, 1/d_i) at [k][i].
 __global__ void pit_factor_kernel(const PitKd K, int L, double alpha_root, float4 *__restrict__ F) {
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   if (k >= L) return;
@@ -262,80 +372,114 @@ __global__ void pit_factor_kernel(const PitKd K, int L, double alpha_root, float
   auto dval = [&](int i) { return zsub(omw, zmul(opw, K.dia(i))); };
   double2 d = dval(0);
   double2 dinv = zinv(d);
-  F[k] = make_float4(0.f, 0.f, (float)dinv.x, (float)dinv.y);
+  F += (size_t)k * K.N;
+  F[0] = make_float4(0.f, 0.f, (float)dinv.x, (float)dinv.y);
   for (int i = 1; i < K.N; ++i) {
     const double2 a = zneg(zmul(opw, K.sub(i)));          // row i, column i-1
     const double2 cprev = zneg(zmul(opw, K.sup(i - 1)));  // row i-1, column i
     const double2 m = zmul(a, dinv);
     d = zsub(dval(i), zmul(m, cprev));
     dinv = zinv(d);
-    F[(size_t)i * L + k] = make_float4((float)m.x, (float)m.y, (float)dinv.x, (float)dinv.y);
+    F[i] = make_float4((float)m.x, (float)m.y, (float)dinv.x, (float)dinv.y);
   }
 }
 
-// Block solves in place on Xh (P, N, L): thread (p, k) solves along i.
-constexpr int kPitRows = 16;  // rows loaded together per pass of the recurrences
-__global__ void pit_block_solve_kernel(const PitK K, int L, int P, double alpha_root, const float4 *__restrict__ F,
-                                       float2 *__restrict__ Xh, const int *active) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+// Block solves in place on Xh (P, L, N): warp (p, k) solves along i, kPitRows rows per
+// lane at a time.  Both sweeps are first-order recurrences y_i = x_i + c_i y_{i-1} (c =
+// -m forward; c_i = -sup_i / d_i on y / d backward): a lane runs its rows from zero and
+// the products of their c, the lanes' (product, last y) pairs are combined by a warp
+// scan, and each row adds its product times what enters its lane.  One thread per block
+// instead runs N dependent rows twice: N = 256, 4064 blocks: 42 -> 14 us.
+constexpr int kPitRows = 8;
+struct PitAffine {
+  float2 a, b;  // y -> a y + b
+};
+// What enters this lane: the composition of all earlier lanes' maps applied to `carry`
+// (DOWN: of all later lanes'); carry becomes the value behind the last one.
+template <bool DOWN>
+__device__ __forceinline__ float2 pit_enter(PitAffine f, float2 &carry) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int s = 1; s < 32; s <<= 1) {
+    const float2 a = DOWN ? shfl_down2(f.a, s) : shfl_up2(f.a, s), b = DOWN ? shfl_down2(f.b, s) : shfl_up2(f.b, s);
+    if (DOWN ? lane + s < 32 : lane >= s) {
+      f.b = cfma(f.a, b, f.b);
+      f.a = cmul(f.a, a);
+    }
+  }
+  const float2 y = cfma(f.a, carry, f.b);
+  const float2 prev = DOWN ? shfl_down2(y, 1) : shfl_up2(y, 1);
+  const float2 in = (DOWN ? lane == 31 : lane == 0) ? carry : prev;
+  const int last = DOWN ? 0 : 31;
+  carry = make_float2(__shfl_sync(0xffffffffu, y.x, last), __shfl_sync(0xffffffffu, y.y, last));
+  return in;
+}
+__global__ void __launch_bounds__(256) pit_block_solve_kernel(const PitK K, int L, int P, double alpha_root,
+                                                              const float4 *__restrict__ F, float2 *__restrict__ Xh,
+                                                              const int *active) {
+  const int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (t >= L * P) return;
   const int p = t / L, k = t % L;
   if (active != nullptr && !active[p]) return;
   const int N = K.N;
   double s, c;
   sincospi(2.0 * (double)k / (double)L, &s, &c);
-  const float2 opw = make_float2((float)(1.0 + alpha_root * c), (float)(alpha_root * s));
-  float2 *x = Xh + (size_t)p * N * L + k;
-  // The recurrences are serial along i, but their inputs are not: each pass
-  // loads kPitRows rows of x and of the factors at once (independent loads in
-  // flight together) before running the recurrence over them.
-  float2 y = x[0];
-  for (int i0 = 1; i0 < N; i0 += kPitRows) {
-    float2 xv[kPitRows], mv[kPitRows];
+  const float2 mopw = make_float2((float)-(1.0 + alpha_root * c), (float)-(alpha_root * s));
+  float2 *x = Xh + (size_t)t * N;
+  const float4 *f = F + (size_t)k * N;
+  constexpr int R = kPitRows, TILE = 32 * R;
+  const float2 zero = make_float2(0.f, 0.f);
+  const int tiles = (N + TILE - 1) / TILE;
+  float2 y[R], a[R], di[R], carry = zero;
+  for (int n = 0; n < tiles; ++n) {
+    const int i0 = n * TILE + lane * R;
 #pragma unroll
-    for (int j = 0; j < kPitRows; ++j) {
-      const int i = i0 + j;
-      if (i < N) {
-        const float4 f = F[(size_t)i * L + k];
-        xv[j] = x[(size_t)i * L];
-        mv[j] = make_float2(f.x, f.y);
-      }
+    for (int j = 0; j < R; ++j) {
+      const bool in = i0 + j < N;
+      const float4 v = in ? f[i0 + j] : make_float4(0.f, 0.f, 0.f, 0.f);
+      y[j] = in ? x[i0 + j] : zero;
+      a[j] = make_float2(-v.x, -v.y);
+      di[j] = make_float2(v.z, v.w);
     }
 #pragma unroll
-    for (int j = 0; j < kPitRows; ++j) {
-      const int i = i0 + j;
-      if (i < N) {
-        y = cfnma(mv[j], y, xv[j]);
-        x[(size_t)i * L] = y;
-      }
+    for (int j = 1; j < R; ++j) {
+      y[j] = cfma(a[j], y[j - 1], y[j]);
+      a[j] = cmul(a[j], a[j - 1]);
+    }
+    const float2 in = pit_enter<false>({a[R - 1], y[R - 1]}, carry);
+#pragma unroll
+    for (int j = 0; j < R; ++j) y[j] = cfma(a[j], in, y[j]);
+    if (n + 1 < tiles) {  // the last tile stays in registers
+#pragma unroll
+      for (int j = 0; j < R; ++j) x[i0 + j] = y[j];
     }
   }
-  {
-    const float4 f = F[(size_t)(N - 1) * L + k];
-    y = cmul(y, make_float2(f.z, f.w));
-    x[(size_t)(N - 1) * L] = y;
-  }
-  const float2 mopw = make_float2(-opw.x, -opw.y);
-  for (int i1 = N - 2; i1 >= 0; i1 -= kPitRows) {
-    float2 xv[kPitRows], dv[kPitRows];
+  carry = zero;
+  for (int n = tiles - 1; n >= 0; --n) {
+    const int i0 = n * TILE + lane * R;
+    if (n < tiles - 1) {
 #pragma unroll
-    for (int j = 0; j < kPitRows; ++j) {
-      const int i = i1 - j;
-      if (i >= 0) {
-        const float4 f = F[(size_t)i * L + k];
-        xv[j] = x[(size_t)i * L];
-        dv[j] = make_float2(f.z, f.w);
+      for (int j = 0; j < R; ++j) {
+        const float4 v = f[i0 + j];
+        y[j] = x[i0 + j];
+        di[j] = make_float2(v.z, v.w);
       }
     }
 #pragma unroll
-    for (int j = 0; j < kPitRows; ++j) {
-      const int i = i1 - j;
-      if (i >= 0) {
-        const float2 ci = cmul(mopw, K.sup(i));  // row i, column i+1
-        y = cmul(cfnma(ci, y, xv[j]), dv[j]);
-        x[(size_t)i * L] = y;
-      }
+    for (int j = 0; j < R; ++j) {  // y_i / d_i - (c_i / d_i) y_{i+1}, c_i row i's coupling to column i + 1
+      const int i = i0 + j;
+      a[j] = i < N - 1 ? cmul(cmul(mopw, K.sup(i)), make_float2(-di[j].x, -di[j].y)) : zero;
+      y[j] = cmul(y[j], di[j]);
     }
+#pragma unroll
+    for (int j = R - 2; j >= 0; --j) {
+      y[j] = cfma(a[j], y[j + 1], y[j]);
+      a[j] = cmul(a[j], a[j + 1]);
+    }
+    const float2 in = pit_enter<true>({a[0], y[0]}, carry);
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+      if (i0 + j < N) x[i0 + j] = cfma(a[j], in, y[j]);
   }
 }
 
@@ -589,47 +733,45 @@ class PitSolver {
     if (rc) return rc;
     pit_factor_kernel<<<(L_ + 127) / 128, 128, 0, st_>>>(kd_, L_, alpha_root_, w_.F);
     TP_CHECK_CUDA(cudaGetLastError());
-    switch (M_) {
-      case 128: return zdft_attributes<128>();
-      case 256: return zdft_attributes<256>();
-      case 512: return zdft_attributes<512>();
-      case 2048: return zdft_attributes<2048>();
-      default: return zdft_attributes<0>();
-    }
-  }
-  template <int MF>
-  int zdft_attributes() {
-    TP_CHECK_CUDA(cudaFuncSetAttribute(pit_zdft_kernel<true, MF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)zsmem_));
-    TP_CHECK_CUDA(cudaFuncSetAttribute(pit_zdft_kernel<false, MF>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       (int)zsmem_));
+    TP_CHECK_CUDA(cudaFuncSetAttribute(pit_zdft_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem_));
+    TP_CHECK_CUDA(cudaFuncSetAttribute(pit_zdft_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zsmem_));
     return TP_OK;
   }
-  template <int MF>
-  void zdft(bool inv, const float2 *in, float2 *out) {
-    const dim3 gz((N_ + cpc_ - 1) / cpc_, P_);
-    if (inv)
-      pit_zdft_kernel<true, MF><<<gz, kPitThreads, zsmem_, st_>>>(pl_, N_, L_, cpc_, in, out, w_.gamma, w_.chirp,
-                                                                  w_.bhat, w_.tw, w_.active);
-    else
-      pit_zdft_kernel<false, MF><<<gz, kPitThreads, zsmem_, st_>>>(pl_, N_, L_, cpc_, in, out, w_.gamma, w_.chirp,
-                                                                   w_.bhat, w_.tw, w_.active);
+  template <bool INV, int R2, int R3>
+  int zdft_reg(const float2 *in, float2 *out) {
+    using F = PitFft<R2, R3>;
+    constexpr size_t smem = (size_t)(R3 > 1 ? 2 : 1) * F::BUF * F::CPC * sizeof(float2);
+    auto kern = pit_zdft_reg_kernel<INV, R2, R3>;
+    TP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<dim3((N_ + F::CPC - 1) / F::CPC, P_), kPitThreads, smem, st_>>>(N_, L_, in, out, w_.gamma, w_.chirp, w_.bhat,
+                                                                          w_.tw, w_.active);
+    return check_cuda(cudaGetLastError(), "pit_zdft_reg_kernel launch");
   }
-  void zdft_any(bool inv, const float2 *in, float2 *out) {
+  template <bool INV>
+  int zdft(const float2 *in, float2 *out) {
     switch (M_) {
-      case 128: return zdft<128>(inv, in, out);
-      case 256: return zdft<256>(inv, in, out);
-      case 512: return zdft<512>(inv, in, out);
-      case 2048: return zdft<2048>(inv, in, out);
-      default: return zdft<0>(inv, in, out);
+      case 128: return zdft_reg<INV, 8, 1>(in, out);
+      case 256: return zdft_reg<INV, 16, 1>(in, out);
+      case 512: return zdft_reg<INV, 8, 4>(in, out);
+      case 1024: return zdft_reg<INV, 8, 8>(in, out);
+      case 2048: return zdft_reg<INV, 16, 8>(in, out);
+      case 4096: return zdft_reg<INV, 16, 16>(in, out);
+      default: break;
     }
+    pit_zdft_kernel<INV><<<dim3((N_ + cpc_ - 1) / cpc_, P_), kPitThreads, zsmem_, st_>>>(
+        pl_, N_, L_, cpc_, in, out, w_.gamma, w_.chirp, w_.bhat, w_.tw, w_.active);
+    return check_cuda(cudaGetLastError(), "pit_zdft_kernel launch");
   }
 
   // out = R in (the preconditioner), active probes only.
   int precond(const float2 *in, float2 *out) {
-    zdft_any(true, in, w_.xh);
-    pit_block_solve_kernel<<<(L_ * P_ + 127) / 128, 128, 0, st_>>>(K_, L_, P_, alpha_root_, w_.F, w_.xh, w_.active);
-    zdft_any(false, w_.xh, out);
+    int rc = zdft<true>(in, w_.xh);
+    if (rc) return rc;
+    const size_t threads = (size_t)L_ * P_ * 32;
+    pit_block_solve_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st_>>>(K_, L_, P_, alpha_root_, w_.F, w_.xh,
+                                                                              w_.active);
+    rc = zdft<false>(w_.xh, out);
+    if (rc) return rc;
     return check_cuda(cudaGetLastError(), "pit preconditioner launch");
   }
   // out = M in (M of the forward or the reference's adjoint system)
