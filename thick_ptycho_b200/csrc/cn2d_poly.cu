@@ -59,7 +59,9 @@ __device__ __forceinline__ float2 jmul(float2 ji, float wl, float2 l, float wr, 
   return make_float2(fmaf(ji.x, sx, fmaf(-ji.y, sy, c.x)), fmaf(ji.x, sy, fmaf(ji.y, sx, c.y)));
 }
 
-template <int R, bool LAGGED, int MAXT, int MINB>
+// DEG: the degree when it is compiled in (its coefficients are then operands of the
+// unrolled half-sweeps), else 0.
+template <int R, int DEG, bool LAGGED, int MAXT, int MINB>
 __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_constant__ Poly2DParams q) {
   static_assert(R % 2 == 0 && kHaloRows % R == 0, "whole lanes of halo");
   constexpr int HL = kHaloRows / R, USE = (32 - 2 * HL) * R;  // halo lanes, rows a warp owns
@@ -160,12 +162,11 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
     // y_k on even rows (odd k) and odd rows (even k) in e[]
     float2 e[R];
     {
-      const float am = q.a[q.m - 1];
+      const float am = q.a[(DEG > 0 ? DEG : q.m) - 1];
 #pragma unroll
       for (int i = 0; i < R; i += 2) e[i] = make_float2(am * g[i].x, am * g[i].y);
     }
-#pragma unroll 1
-    for (int k = q.m - 2; k >= 0; k -= 2) {
+    auto pair = [&](int k) {
       {
         const float a = q.a[k];
         const float2 right = shfl_down2(e[0], 1);
@@ -184,6 +185,13 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
           e[i] = jmul(ji[i], wl[i], l, wr[i], e[i + 1], make_float2(a * g[i].x, a * g[i].y));
         }
       }
+    };
+    if constexpr (DEG > 0) {
+#pragma unroll
+      for (int k = DEG - 2; k >= 0; k -= 2) pair(k);
+    } else {
+#pragma unroll 1
+      for (int k = q.m - 2; k >= 0; k -= 2) pair(k);
     }
     float2 *dst = nullptr;
     if (p.u_store != nullptr && store_index(p, t) >= 0)
@@ -246,11 +254,11 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
   if (p.state_out != nullptr) store(p.state_out + probe * p.Npad, u);
 }
 
-template <int R, int MAXT, int MINB>
-int launch(const Poly2DParams &q, bool lagged, cudaStream_t st) {
+template <int R, bool LAGGED, int MAXT, int MINB>
+int launch(const Poly2DParams &q, cudaStream_t st) {
   constexpr int HL = kHaloRows / R;
   const size_t smem = (size_t)4 * q.nwarps * HL * R * sizeof(float2);
-  auto kern = lagged ? cn2d_poly_kernel<R, true, MAXT, MINB> : cn2d_poly_kernel<R, false, MAXT, MINB>;
+  auto kern = q.m == 6 ? cn2d_poly_kernel<R, 6, LAGGED, MAXT, MINB> : cn2d_poly_kernel<R, 0, LAGGED, MAXT, MINB>;
   kern<<<q.p.P, 32 * q.nwarps, smem, st>>>(q);
   return check_cuda(cudaGetLastError(), "cn2d_poly_kernel launch");
 }
@@ -320,18 +328,18 @@ int launch_poly_march(const Partition &pt, const MarchParams &mp, const Poly2DPl
   // SM at 128 registers (1500, 300 probes: 3.25 -> 2.96; the exact adjoint would spill).
   if (warps(2) <= 10) {
     q.nwarps = warps(2);
-    return launch<2, 320, 3>(q, lagged, st);
+    return lagged ? launch<2, true, 320, 3>(q, st) : launch<2, false, 320, 3>(q, st);
   }
   if (warps(4) <= 10) {
     q.nwarps = warps(4);
-    return launch<4, 320, 2>(q, lagged, st);
+    return lagged ? launch<4, true, 320, 2>(q, st) : launch<4, false, 320, 2>(q, st);
   }
   q.nwarps = warps(8);
   int dev = 0, sms = 148;
   TP_CHECK_CUDA(cudaGetDevice(&dev));
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (q.nwarps <= 7 && !lagged && mp.P > sms) return launch<8, 224, 2>(q, lagged, st);
-  return launch<8, 288, 1>(q, lagged, st);
+  if (q.nwarps <= 7 && !lagged && mp.P > sms) return launch<8, false, 224, 2>(q, st);
+  return lagged ? launch<8, true, 288, 1>(q, st) : launch<8, false, 288, 1>(q, st);
 }
 
 }  // namespace tp
