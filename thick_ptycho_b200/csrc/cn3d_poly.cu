@@ -41,6 +41,7 @@
 #include <type_traits>
 
 #include "cn3d_poly.cuh"
+#include "cn3d_poly_dev.cuh"
 #include "tp_errors.h"
 #include "tpcuda.h"
 
@@ -48,10 +49,6 @@
 namespace tp {
 
 namespace {
-
-constexpr int kPW = 64, kPR = 8, kPWarps = 8, kPH = kPR * kPWarps;  // tile width, rows per warp, warps, tile height
-constexpr int kPThreads = 32 * kPWarps;
-constexpr int kPolyMaxDeg = 10, kPolyMaxHalo = 16;
 
 struct PolyCheck {
   // bits of the largest row and column sums of |J| and the largest |arg D| (non-negative floats)
@@ -203,97 +200,6 @@ struct PolySmem {
   uint64_t bar[2];
 };
 
-// Two complex64 values of adjacent columns, each a packed register pair: sums and
-// real weights run as packed fp32 operations (one issue slot for both parts).
-struct cpair {
-  unsigned long long a, b;
-};
-__device__ __forceinline__ unsigned long long pk(float x, float y) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
-__device__ __forceinline__ float2 upk(unsigned long long v) {
-  float2 r;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-  unsigned long long r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-__device__ __forceinline__ cpair to_pair(float4 v) { return {pk(v.x, v.y), pk(v.z, v.w)}; }
-__device__ __forceinline__ float4 to_f4(cpair v) {
-  const float2 a = upk(v.a), b = upk(v.b);
-  return make_float4(a.x, a.y, b.x, b.y);
-}
-
-// The real weights of a thread's neighbours, each in both halves of a pair:
-// left and right of its two columns, and the interior row weight.
-struct PolyWeights {
-  unsigned long long l0, r0, l1, r1, row;
-};
-
-// Weighted neighbour sums of both columns of one row: S = sum of real weights
-// times neighbours (the couplings are i times the weights).  EDGE: rw holds the
-// row's own weights {previous row, next row, columns}.
-template <bool EDGE>
-__device__ __forceinline__ cpair poly_sum(const cpair &cur, const cpair &prev, const cpair &next, const PolyWeights &w,
-                                          const float4 *rw) {
-  const float2 lo = upk(cur.a), hi = upk(cur.b);
-  const unsigned long long west = pk(__shfl_up_sync(0xffffffffu, hi.x, 1), __shfl_up_sync(0xffffffffu, hi.y, 1));
-  const unsigned long long east = pk(__shfl_down_sync(0xffffffffu, lo.x, 1), __shfl_down_sync(0xffffffffu, lo.y, 1));
-  cpair s;
-  s.a = fma2(w.l0, west, mul2(w.r0, cur.b));
-  s.b = fma2(w.l1, cur.a, mul2(w.r1, east));
-  if (EDGE) {
-    const float4 v = *rw;
-    const unsigned long long x = pk(v.x, v.x), y = pk(v.y, v.y), z = pk(v.z, v.z);
-    s.a = fma2(z, s.a, fma2(x, prev.a, mul2(y, next.a)));
-    s.b = fma2(z, s.b, fma2(x, prev.b, mul2(y, next.b)));
-  } else {
-    s.a = fma2(w.row, add2(prev.a, next.a), s.a);
-    s.b = fma2(w.row, add2(prev.b, next.b), s.b);
-  }
-  return s;
-}
-// The same for one pixel of colour C in row I of the thread's strip (rows start
-// even): colour A (0) is column 0 in even rows and column 1 in odd ones.  o, prev
-// and next are the other colour's pixels in this row and its neighbours.
-template <bool EDGE, int COL>
-__device__ __forceinline__ unsigned long long poly_half(unsigned long long o, unsigned long long prev,
-                                                        unsigned long long next, const PolyWeights &w,
-                                                        const float4 *rw) {
-  const float2 v = upk(o);
-  const unsigned long long side = COL == 0 ? pk(__shfl_up_sync(0xffffffffu, v.x, 1), __shfl_up_sync(0xffffffffu, v.y, 1))
-                                           : pk(__shfl_down_sync(0xffffffffu, v.x, 1),
-                                                __shfl_down_sync(0xffffffffu, v.y, 1));
-  unsigned long long s = COL == 0 ? fma2(w.l0, side, mul2(w.r0, o)) : fma2(w.l1, o, mul2(w.r1, side));
-  if (EDGE) {
-    const float4 r = *rw;
-    s = fma2(pk(r.z, r.z), s, fma2(pk(r.x, r.x), prev, mul2(pk(r.y, r.y), next)));
-  } else {
-    s = fma2(w.row, add2(prev, next), s);
-  }
-  return s;
-}
-// c + j s (complex)
-__device__ __forceinline__ unsigned long long cmadd(float jx, float jy, unsigned long long s, unsigned long long c) {
-  const float2 sv = upk(s), cv = upk(c);
-  return pk(fmaf(jx, sv.x, fmaf(-jy, sv.y, cv.x)), fmaf(jx, sv.y, fmaf(jy, sv.x, cv.y)));
-}
-
 // One tile and probe group.  EDGE: the tile holds one of the image's first or
 // last two rows, whose row couplings may differ from the interior's.
 template <bool ALIGNED, bool SRC, int GRAD, bool EDGE>
@@ -444,10 +350,10 @@ __device__ __forceinline__ void poly_tile(const CUtensorMap &map, const PolyStep
         if (!SRC || q.use_u) {
           const float4 ds = sm.dsum[r][lane], uc = to_f4(cur);
           const float4 s = to_f4(poly_sum<EDGE>(cur, prev, next, w, &sm.roww[r]));
-          bv.x = fmaf(-2.f, s.y, fmaf(ds.x, uc.x, -ds.y * uc.y));
-          bv.y = fmaf(2.f, s.x, fmaf(ds.x, uc.y, ds.y * uc.x));
-          bv.z = fmaf(-2.f, s.w, fmaf(ds.z, uc.z, -ds.w * uc.w));
-          bv.w = fmaf(2.f, s.z, fmaf(ds.z, uc.w, ds.w * uc.z));
+          bv.x = fmaf(ds.x, uc.x, fmaf(-ds.y, uc.y, -2.f * s.y));
+          bv.y = fmaf(ds.x, uc.y, fmaf(ds.y, uc.x, 2.f * s.x));
+          bv.z = fmaf(ds.z, uc.z, fmaf(-ds.w, uc.w, -2.f * s.w));
+          bv.w = fmaf(ds.z, uc.w, fmaf(ds.w, uc.z, 2.f * s.z));
         }
         if (SRC) {
           if (b >= 0 && b < q.nb) {
@@ -698,6 +604,8 @@ std::complex<double> chebyshev(int m, std::complex<double> w) {
   return t1;
 }
 
+}  // namespace
+
 // The smallest even degree whose residual polynomial stays below `target` on the
 // segment [-i tau, i tau] turned by up to `theta`; 0 if none is allowed.  a[k] are
 // the coefficients of p_m.
@@ -726,8 +634,6 @@ int poly_degree(double tau, double theta, double target, int max_m, float *a) {
   }
   return 0;
 }
-
-}  // namespace
 
 int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
   *ran = 0;

@@ -35,6 +35,11 @@ struct C3PolyJob {
 // Widths up to this many rows or columns fit the small arrays.
 constexpr int kPolyMaxSide = 2048;
 
+// The smallest even degree m <= max_m whose residual polynomial stays below `target`
+// on the segment [-i tau, i tau] turned by up to `theta` (0: none); a[k], k < m, are the
+// coefficients of p_m.
+int poly_degree(double tau, double theta, double target, int max_m, float *a);
+
 // Runs the march if its operator allows the polynomial form (*ran = 1);
 // otherwise leaves it to the Krylov march (*ran = 0, nothing written that the
 // Krylov march reads).  Waits once for `stream`, before the first step.
