@@ -437,9 +437,11 @@ typedef struct tp_cn3d_march_args {
                                 forward before the adjoint): the network is not
                                 run again                                       */
   int32_t kernels;           /* kernel choice, the same arithmetic either way
-                                (0 = automatic).  Bit 0: the preconditioner's
-                                transforms always by the shared-memory Stockham
-                                kernels (automatic: register four-step kernels
+                                (0 = automatic).  Bit 0: the preconditioner
+                                always by the shared-memory Stockham transforms
+                                (automatic: on tiles by a polynomial that equals
+                                it to 1e-7 where nf is even and the couplings
+                                are small, else register four-step kernels
                                 where nf = nb is 64, 128, 192 or 256).  Bit 1:
                                 the stencil kernels (right-hand side, matvecs,
                                 finish) always with per-thread loads

@@ -61,7 +61,7 @@ class CN3D:
         # iteration loops; 1: step by step (host loop)
         self.launch = 0
         # kernel choice (tp_cn3d_march_args.kernels; the same arithmetic):
-        # 0 = automatic; bit 0 = Stockham transforms always, bit 1 = the
+        # 0 = automatic; bit 0 = the preconditioner by Stockham transforms always, bit 1 = the
         # stencil kernels with per-thread loads instead of tensor-memory copies,
         # bit 2 = the learned filter by register shuffles instead of bulk-staged rows,
         # bit 3 = the Krylov march also where a fixed polynomial solves each slice

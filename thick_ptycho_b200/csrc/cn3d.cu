@@ -16,16 +16,19 @@
 // judged by its true residual ||rhs - (I - P_s) d||.  Preconditioner: the
 // periodic 5-point operator diagonalised by a 2D FFT, applied as
 // IFFT2(FFT2(v) / (1 - sigma*T K_per(kf, kb))),
-// K_per = mu_x (2 cos kf - 2) + mu_y (2 cos kb - 2), with register four-step
+// K_per = mu_x (2 cos kf - 2) + mu_y (2 cos kb - 2): on tiles by the polynomial
+// that equals it to 1e-7 where the couplings are small, else with register four-step
 // transforms for square 64..256 grids and the shared-memory Stockham FFT of
-// fft.cuh otherwise; optionally followed by the learned per-pixel correction.
+// fft.cuh; optionally followed by the learned per-pixel correction.
 #include <cuda.h>
 #include <cuda_runtime.h>
 #include <math.h>
 
 #include <mutex>
+#include <type_traits>
 
 #include "cn3d_poly.cuh"
+#include "cn3d_poly_dev.cuh"
 #include "cnn_internal.cuh"
 #include "fft.cuh"
 #include "tp_common.cuh"
@@ -572,6 +575,161 @@ __device__ __forceinline__ PrecInput prec_input(int mode, const cx *r, cx *p, co
   }
   return in;
 }
+
+#ifndef TP_C128_CHECK
+// M0^{-1} without transforms: the periodic 5-point operator (I - sigma*T K_per) has the
+// constant diagonal D0 and couplings i mu, so its inverse is the polynomial p_m(J0)
+// D0^{-1} of cn3d_poly.cu to 1e-7 (m = 6 at the paraxial sampling), evaluated on tiles
+// whose halo wraps around the grid: one kernel that reads the input's vectors and
+// writes z, in the place of the row, column and inverse row transforms and two passes
+// over the spectrum between them.  A CTA owns one 64 x 64 tile of one probe (8 warps of
+// 8 rows, two columns per lane, checkerboard half-sweeps).  The halo reads neighbours'
+// p, so a new p goes to the other of two vectors (pa at odd iterations, pb at even ones).
+// 192 x 192, 64 probes: 26 us per application against 18 + 13 + 10 of the four-step
+// kernels; bound by latency and the arithmetic of the half-sweeps together (48 KB of
+// a tile's vectors in flight per CTA, three CTAs per SM).  Grid (tiles, P).
+struct PrecTile {
+  int tiles_x, hx, hy, cw, ch, m;
+  float a[kPolyMaxDeg];
+  float mx, my;        // couplings (imaginary parts)
+  float dix, diy;      // D0^{-1}
+};
+__global__ void __launch_bounds__(kPThreads, 3) c3_prec_tile_kernel(const __grid_constant__ PrecTile q, int nf, int nb,
+                                                                    int mode, const float2 *r, float2 *pa, float2 *pb,
+                                                                    const float2 *v, float2 *s, float2 *out,
+                                                                    const Krylov *K, const float2 *r0, float2 *out_first,
+                                                                    const C3State *st) {
+  __shared__ unsigned long long edge[2][kPWarps - 1][2][kPW / 2];
+  const int pr = blockIdx.y;
+  if (K != nullptr && K[pr].done) return;
+  const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+  const int f0 = (int)(blockIdx.x % q.tiles_x) * q.cw - q.hx, b0 = (int)(blockIdx.x / q.tiles_x) * q.ch - q.hy;
+  const int it = mode == 2 ? 0 : st->it;
+  float2 *pw = (it & 1) ? pa : pb;
+  PrecInput in = prec_input(mode, r, pw, v, s, r0, K, pr, st);
+  if (mode == 0 && it > 1) in.pin = (it & 1) ? pb : pa;
+  const size_t base = (size_t)pr * nf * nb;
+  // wrapped places of this thread's pixels
+  const int gf = f0 + 2 * lane, gb0 = b0 + wp * kPR;
+  const int cf = ((gf % nf) + nf) % nf;
+  const bool core = 2 * lane >= q.hx && 2 * lane < q.hx + q.cw && gf < nf;
+  unsigned long long g[kPR][2];
+  {
+    float4 raw[kPR];
+    int row[kPR];
+    const bool first = in.first != 0;
+    const bool direct = mode == 2 || (mode == 0 && first);
+    const float2 *x0 = mode == 2 ? r : (mode == 0 ? (first ? r0 : r) : (first ? r0 : r));
+#pragma unroll
+    for (int i = 0; i < kPR; ++i) {
+      int b = (gb0 + i) % nb;
+      if (b < 0) b += nb;
+      row[i] = b * nf + cf;
+      raw[i] = *reinterpret_cast<const float4 *>(x0 + base + row[i]);
+    }
+    if (!direct) {
+#pragma unroll
+      for (int i = 0; i < kPR; ++i) {
+        const float4 vv = *reinterpret_cast<const float4 *>(v + base + row[i]);
+        if (mode == 1) {  // r - alpha v
+          const float2 a = cfnma(in.al, make_float2(vv.x, vv.y), make_float2(raw[i].x, raw[i].y));
+          const float2 b = cfnma(in.al, make_float2(vv.z, vv.w), make_float2(raw[i].z, raw[i].w));
+          raw[i] = make_float4(a.x, a.y, b.x, b.y);
+        } else {  // r + beta (p - omega v)
+          const float4 pp = *reinterpret_cast<const float4 *>(in.pin + base + row[i]);
+          const float2 a = cfma(in.bt, cfnma(in.om, make_float2(vv.x, vv.y), make_float2(pp.x, pp.y)),
+                                make_float2(raw[i].x, raw[i].y));
+          const float2 b = cfma(in.bt, cfnma(in.om, make_float2(vv.z, vv.w), make_float2(pp.z, pp.w)),
+                                make_float2(raw[i].z, raw[i].w));
+          raw[i] = make_float4(a.x, a.y, b.x, b.y);
+        }
+      }
+    }
+    float2 *dst = in.dest();
+#pragma unroll
+    for (int i = 0; i < kPR; ++i) {
+      const int rr = wp * kPR + i;
+      if (dst != nullptr && core && rr >= q.hy && rr < q.hy + q.ch && b0 + rr < nb)
+        *reinterpret_cast<float4 *>(dst + base + row[i]) = raw[i];
+      const float2 ga = cmul(make_float2(q.dix, q.diy), make_float2(raw[i].x, raw[i].y));
+      const float2 gb = cmul(make_float2(q.dix, q.diy), make_float2(raw[i].z, raw[i].w));
+      g[i][0] = pk(ga.x, ga.y);
+      g[i][1] = pk(gb.x, gb.y);
+    }
+  }
+  const float l0 = lane == 0 ? 0.f : q.mx, r1 = lane == 31 ? 0.f : q.mx;
+  const PolyWeights w = {pk(l0, l0), pk(q.mx, q.mx), pk(q.mx, q.mx), pk(r1, r1), pk(q.my, q.my)};
+  const float jx = -q.diy, jy = q.dix;  // i D0^{-1}
+  unsigned long long ya[kPR], yb[kPR];  // the newest y of colours A (row + column even) and B
+  {
+    const unsigned long long am = pk(q.a[q.m - 1], q.a[q.m - 1]);
+#pragma unroll
+    for (int i = 0; i < kPR; ++i) ya[i] = mul2(am, g[i][i & 1]);
+  }
+  auto half_sweep = [&](auto colour, float a, const unsigned long long(&x)[kPR], unsigned long long(&y)[kPR]) {
+    constexpr int C = decltype(colour)::value;
+    if (wp > 0) edge[C][wp - 1][1][lane] = x[0];
+    if (wp + 1 < kPWarps) edge[C][wp][0][lane] = x[kPR - 1];
+    __syncthreads();
+    unsigned long long prev = wp > 0 ? edge[C][wp - 1][0][lane] : 0ull;
+    const unsigned long long below = wp + 1 < kPWarps ? edge[C][wp][1][lane] : 0ull;
+    const unsigned long long a2 = pk(a, a);
+#pragma unroll
+    for (int i = 0; i < kPR; ++i) {
+      const unsigned long long next = i + 1 < kPR ? x[i + 1] : below;
+      if ((C + i) % 2 == 0) y[i] = cmadd(jx, jy, poly_half<false, 0>(x[i], prev, next, w, nullptr), mul2(a2, g[i][0]));
+      else y[i] = cmadd(jx, jy, poly_half<false, 1>(x[i], prev, next, w, nullptr), mul2(a2, g[i][1]));
+      prev = x[i];
+    }
+  };
+#pragma unroll 1
+  for (int k = q.m - 2; k >= 0; k -= 2) {
+    half_sweep(std::integral_constant<int, 1>{}, q.a[k], ya, yb);
+    half_sweep(std::integral_constant<int, 0>{}, k > 0 ? q.a[k - 1] : 1.f, yb, ya);
+  }
+  float2 *z = (out_first != nullptr && st->it == 0 && st->cheap) ? out_first : out;
+  if (!core) return;
+#pragma unroll
+  for (int i = 0; i < kPR; ++i) {
+    const int rr = wp * kPR + i;
+    if (rr < q.hy || rr >= q.hy + q.ch || b0 + rr >= nb) continue;
+    const float2 d0 = upk((i & 1) ? yb[i] : ya[i]), d1 = upk((i & 1) ? ya[i] : yb[i]);
+    *reinterpret_cast<float4 *>(z + base + (size_t)(b0 + rr) * nf + gf) = make_float4(d0.x, d0.y, d1.x, d1.y);
+  }
+}
+
+// The tile kernel's plan for the symbol coefficients of q (m = 0: not applicable).
+// four: the transform has register four-step kernels.  Those are the faster ones
+// once the halo grows past 6 pixels (mu > 0.046): a preconditioned march of 256 x
+// 256, 64 probes takes 453 us per step on tiles and 510 by transforms at mu = 0.02
+// (m = 6, halo 5), 477 and 522 at 0.044 (m = 8, halo 6), 562 and 541 at 0.061 (m = 8,
+// halo 7).  The shared-memory transforms are slower at every mu in reach (150 x 150:
+// 225 and 385 us at 0.02, 255 and 393 at 0.051).
+static PrecTile prec_tile_plan(const C3Params &q, bool four) {
+  PrecTile t{};
+  if (q.nf % 2 != 0 || q.nf < 2 || q.mu_x.x != 0.0 || q.mu_y.x != 0.0) return t;
+  const double mx = q.mu_x.y, my = q.mu_y.y, dim = 2.0 * (mx + my);  // D0 = 1 + i dim
+  const double d = hypot(1.0, dim), mu = fmax(1e-6, fmax(fabs(mx), fabs(my)));
+  t.m = poly_degree(2.0 * (fabs(mx) + fabs(my)) / d, fabs(atan2(dim, 1.0)), 1e-7, kPolyMaxDeg, t.a);
+  int h = mu < 1.0 ? (int)ceil(log(1e-8) / log(mu)) : kPolyMaxHalo + 1;
+  if (h > t.m) h = t.m;
+  if (t.m == 0 || h > (four ? 6 : kPolyMaxHalo)) {
+    t.m = 0;
+    return t;
+  }
+  t.hy = h;
+  t.hx = (h + 1) & ~1;
+  t.tiles_x = (q.nf + kPW - 2 * t.hx - 1) / (kPW - 2 * t.hx);
+  const int tiles_y = (q.nb + kPH - 2 * t.hy - 1) / (kPH - 2 * t.hy);
+  t.cw = (((q.nf + t.tiles_x - 1) / t.tiles_x) + 1) & ~1;
+  t.ch = (q.nb + tiles_y - 1) / tiles_y;
+  t.mx = (float)mx;
+  t.my = (float)my;
+  t.dix = (float)(1.0 / (d * d));
+  t.diy = (float)(-dim / (d * d));
+  return t;
+}
+#endif  // TP_C128_CHECK
 
 // Four-step preconditioner kernels for nf = nb = R1 R2 (R1 >= R2): 256
 // threads, 256 / R1 rows (or columns) per CTA, one short DFT per thread and
@@ -1439,12 +1597,14 @@ __global__ void __launch_bounds__(NF, 2) c3_filter_shfl_kernel(const C3Params q,
 // order of c3_filter_shfl_kernel, so both kernels give the same bits.  Waits
 // are bounded (kDevMbarTimeout); a thread that gives up waits for the CTA's
 // other copies before it returns.  nf = NF in {64, 128, 192, 256}, z 16-byte
-// aligned; a CTA of NF threads, one row pair, kFilterProbes probes.
+// aligned; a CTA of NF threads, one row pair, kFilterProbes probes.  The register
+// limit of three CTAs per SM (two at NF = 256) keeps more copies in flight: 192 x 192,
+// 64 probes 27.2 -> 23.7 us.
 // Grid (ceil(nb / 2), ceil(P / kFilterProbes)).
 constexpr int kFilterRows = 6;
 
 template <int NF>
-__global__ void __launch_bounds__(NF, 2) c3_filter_bulk_kernel(const C3Params q, const C3State *st, int chunk,
+__global__ void __launch_bounds__(NF, NF <= 192 ? 3 : 2) c3_filter_bulk_kernel(const C3Params q, const C3State *st, int chunk,
                                                                const cx *__restrict__ Fall,
                                                                const cx *__restrict__ z, cx *__restrict__ out,
                                                                const Krylov *K, int second, int *err) {
@@ -2144,10 +2304,25 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
   const ConvGeom gch = learned ? conv_geom(nb, nf, lw.chunk) : ConvGeom{};
 #endif
 
+#ifndef TP_C128_CHECK
+  // the periodic inverse on tiles (bit 0 of kernels: by transforms always; training
+  // pairs are defined by the transform)
+  PrecTile ptile{};
+  if (fft_on && (a->kernels & 1) == 0) ptile = prec_tile_plan(q, four);
+#endif
+
   // ---- launch sequences (recorded into a graph, or issued step by step)
   // M0^{-1} in -> out (mode 0/1/2 input of the row kernel; Kp NULL = all probes)
   auto precondition = [&](cudaStream_t s, int mode, const cx *rin, cx *out, const Krylov *Kp,
                           cx *out_first = nullptr) {
+#ifndef TP_C128_CHECK
+    if (ptile.m > 0 && mode != 2) {
+      const int tiles = ptile.tiles_x * ((nb + ptile.ch - 1) / ptile.ch);
+      c3_prec_tile_kernel<<<dim3(tiles, P), kPThreads, 0, s>>>(ptile, nf, nb, mode, rin, w.p, w.hat, w.v, w.s, out, Kp,
+                                                               w.r0, out_first, w.st);
+      return;
+    }
+#endif
     if (four) {
       p4.rows<<<dim3(nb / rpc4, P), 256, 0, s>>>(q, mode, rin, w.p, w.v, w.s, w.hat, Kp, w.tw4, w.r0, w.st);
       p4.cols<<<dim3(nf / rpc4, P), 256, 0, s>>>(q, w.hat, Kp, w.tw4, w.ab);
