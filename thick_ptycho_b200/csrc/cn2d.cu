@@ -917,7 +917,17 @@ extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp
     return launch_team_march(pt, mp, lagged, reinterpret_cast<cudaStream_t>(stream));
   }
 #ifndef TP_C128_CHECK
-  const Poly2DPlan plan = poly2d_plan(op);
+  // The polynomial kernel holds a CTA per probe, the direct one a warp: with more than
+  // two probes per SM the direct one's throughput wins where its chain is short (us per
+  // step to the exit, polynomial and direct: N = 1023, 296 probes 1.68 and 2.20, 512
+  // 3.15 and 2.27; 257: 0.95 and 1.20, 1.51 and 1.21; 1201: 1.96 and 3.98, 3.65 and
+  // 4.32) or, for the adjoint, at any N (1201: 3.43 and 4.54, 6.57 and 4.94).  The
+  // direct kernel's gradient is the slower one always (1023, 512: 5.9 and 20.8).
+  int dev = 0, sms = 148;
+  TP_CHECK_CUDA(cudaGetDevice(&dev));
+  TP_CHECK_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const bool direct = mp.P > 2 * sms && mp.grad_c == nullptr && (pt.M <= 32 || lagged);
+  const Poly2DPlan plan = direct ? Poly2DPlan{} : poly2d_plan(op);
   if (plan.m > 0) {
     mp.poly_bad = mp.coupling + 1;
     rc = launch_poly_march(pt, mp, plan, mp.poly_bad, lagged, reinterpret_cast<cudaStream_t>(stream));

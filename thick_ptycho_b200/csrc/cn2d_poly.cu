@@ -284,11 +284,16 @@ Poly2DPlan poly2d_plan(const tp_cn2d_op *op) {
   const double dr = 1.0 - op->k_diag[0], di = op->k_diag[1], d = hypot(dr, di);
   if (!(d > 0.5)) return pl;
   // margins over the free-space slice for the object and the boundary rows
-  const double tau = 1.15 * 2.0 * mu / d + 0.002, arg = fabs(atan2(di, dr)) + 0.1;
+  const double tau = 1.15 * 2.0 * mu / d + 0.002;
+  double arg = fabs(atan2(di, dr)) + 0.1;
   const std::complex<double> it(0.0, tau);
   for (int m = 4; m <= kPoly2DMaxDeg; m += 2) {
     const std::complex<double> scale = chebyshev(m, 1.0 / it);
-    if (!(std::abs(chebyshev(m, std::polar(1.0, arg))) <= 3e-8 * std::abs(scale))) continue;
+    auto holds = [&](double x) { return std::abs(chebyshev(m, std::polar(1.0, x))) <= 3e-8 * std::abs(scale); };
+    if (!holds(arg)) continue;
+    // the widest object the degree covers: |n - 1| up to 0.08 at wavelength 0.5 with unit
+    // steps (m = 6), against 0.016 at the first margin
+    while (arg < 1.2 && holds(arg + 0.05)) arg += 0.05;
     double t0[kPoly2DMaxDeg + 1] = {1.0}, t1[kPoly2DMaxDeg + 1] = {0.0, 1.0};
     for (int n = 1; n < m; ++n) {
       double t2[kPoly2DMaxDeg + 1] = {0.0};
