@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(kMs3Threads) ms3_cols_kernel(const FftPlan pl,
 // once per transform.  The psi buffer holds X_z = psi_z T_z here (psi_{z+1} = X_z +
 // update needs no T_z).  The shared-memory passes above were bound by shared memory
 // (73-83 % of its throughput); a slice of 64 probes of 256 x 256 took 95 us with them
-// (adjoint 99) and takes 46 us (60) with these.
+// (adjoint 99) and takes 42 us (51) with these.
 template <int R1, int R2, int PHASE>
 __global__ void __launch_bounds__(256, 2) ms3_rows4_kernel(const Ms3Params q, const float2 *__restrict__ twg, int z) {
   constexpr int N = R1 * R2, RPC = 256 / R1, S = R1 * (R2 + 1);
