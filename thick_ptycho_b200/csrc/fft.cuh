@@ -10,6 +10,8 @@
 // numpy.fft.ifft); callers fold the 1/n into an adjacent multiply.
 #pragma once
 
+#include <type_traits>
+
 #include "tp_common.cuh"
 
 namespace tp {
@@ -418,6 +420,211 @@ __device__ __forceinline__ void dft_reg(cx (&v)[16], rx sign) {
     for (int j = 0; j < 8; ++j) v[j] = w[j];
   } else {
     dft4_inplace(v[0], v[1], v[2], v[3], sign);
+  }
+}
+
+// ------------------------------------------------ in-place transforms, any 2^a 3^b 5^c
+// For callers that multiply a spectrum and go back: the forward transform runs
+// decimation-in-frequency stages in place (stage s splits blocks of len_s = n /
+// (R_0 .. R_{s-1}) into R_s parts, str_s = len_s / R_s apart) and leaves the spectrum
+// at p = k_0 str_0 + k_1 str_1 + ..., frequency k_0 + R_0 k_1 + R_0 R_1 k_2 + ...; the
+// inverse undoes the stages in the opposite order.  A unit's R_s values keep their
+// places, so a stage is one read and one write between two barriers and no pass
+// reorders.
+constexpr int kMixStages = 6;
+struct MixPlan {
+  int n, stages, threads, tw_total;
+  int radix[kMixStages], len[kMixStages], str[kMixStages], tw[kMixStages];
+  uint32_t ms[kMixStages];  // fast_div reciprocals of str
+};
+
+// The fewest stages with radices up to 16 and of those the most even split, the
+// largest first; stages = 0 where there are none (or only one).
+inline MixPlan make_mix_plan(int n) {
+  MixPlan p{};
+  p.n = n;
+  if (n < 2 || n > kFftMaxN) return p;
+  constexpr int radices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
+  int cur[kMixStages] = {}, best_len = kMixStages + 1, best_sum = 0;
+  // non-increasing sequences of radices with product n (a few hundred nodes at most)
+  auto search = [&](auto &self, int m, int k, int first, int sum) -> void {
+    if (m == 1) {
+      if (k < best_len || (k == best_len && sum < best_sum)) {
+        best_len = k;
+        best_sum = sum;
+        for (int i = 0; i < k; ++i) p.radix[i] = cur[i];
+      }
+      return;
+    }
+    if (k >= kMixStages || k + 1 > best_len) return;
+    for (int i = first; i < (int)(sizeof(radices) / sizeof(radices[0])); ++i)
+      if (m % radices[i] == 0) {
+        cur[k] = radices[i];
+        self(self, m / radices[i], k + 1, i, sum + radices[i]);
+      }
+  };
+  search(search, n, 0, 0, 0);
+  if (best_len > kMixStages || best_len < 2) return p;
+  p.stages = best_len;
+  int len = n, units = 0;
+  for (int i = 0; i < p.stages; ++i) {
+    p.len[i] = len;
+    p.str[i] = len / p.radix[i];
+    p.tw[i] = p.tw_total;
+    p.ms[i] = fast_recip((uint32_t)p.str[i]);
+    p.tw_total += i + 1 < p.stages ? len : 0;
+    if (n / p.radix[i] > units) units = n / p.radix[i];
+    len = p.str[i];
+  }
+  p.threads = (units + 31) / 32 * 32;
+  return p;
+}
+
+// Slot of place i in shared memory: one spare per 16, so that the strides of the
+// last stages (multiples of the radix) spread over the banks.
+__host__ __device__ __forceinline__ int mix_pad(int i) { return i + (i >> 4); }
+// Frequency at place p.
+__device__ __forceinline__ int mix_frequency(const MixPlan &pl, int p) {
+  int f = 0, mult = 1;
+  for (int s = 0; s < pl.stages; ++s) {
+    const int k = p / pl.str[s];
+    p -= k * pl.str[s];
+    f += mult * k;
+    mult *= pl.radix[s];
+  }
+  return f;
+}
+// The stages' twiddles exp(-2 pi i k t / len_s) at tw[s] + k str_s + t (none for the last).
+__device__ __forceinline__ void mix_twiddles(const MixPlan &pl, cx *tw, int tid, int nth) {
+  for (int s = 0; s + 1 < pl.stages; ++s)
+    for (int e = tid; e < pl.len[s]; e += nth) {
+      const int k = e / pl.str[s], t = e - k * pl.str[s];
+      double sv, cv;
+      sincospi(-2.0 * (double)(k * t) / (double)pl.len[s], &sv, &cv);
+      tw[pl.tw[s] + e] = mkcx((rx)cv, (rx)sv);
+    }
+}
+
+// exp(2 pi i m / R), m < R, at compile time (Taylor series about 0 of an angle of at
+// most pi / 4, quadrants by symmetry).
+template <int R>
+struct UnitRoots {
+  rx c[R] = {}, s[R] = {};
+  constexpr UnitRoots() {
+    for (int m = 0; m < R; ++m) {
+      int q = (8 * m + R) / (2 * R);  // nearest quarter turn
+      const double x = 6.283185307179586476925 * ((double)(4 * m - q * R) / (4.0 * R));
+      double cs = 1.0, sn = x, tc = 1.0, ts = x;
+      for (int k = 1; k < 12; ++k) {
+        tc *= -x * x / ((2 * k - 1) * (2 * k));
+        ts *= -x * x / ((2 * k) * (2 * k + 1));
+        cs += tc;
+        sn += ts;
+      }
+      q &= 3;
+      c[m] = (rx)(q == 0 ? cs : q == 1 ? -sn : q == 2 ? -cs : sn);
+      s[m] = (rx)(q == 0 ? sn : q == 1 ? cs : q == 2 ? -sn : -cs);
+    }
+  }
+};
+
+// R = A B points: n = B n1 + n2, k = k1 + A k2; A-point DFTs over n1, the roots
+// exp(sign 2 pi i n2 k1 / R), B-point DFTs over n2.
+template <int A, int B>
+__device__ __forceinline__ void dft_two(cx (&v)[16], rx sign) {
+  constexpr UnitRoots<A * B> w{};
+  cx o[A * B];
+#pragma unroll
+  for (int n2 = 0; n2 < B; ++n2) {
+    cx t[8];
+#pragma unroll
+    for (int n1 = 0; n1 < A; ++n1) t[n1] = v[B * n1 + n2];
+    dft_small<A>(t, sign);
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1)
+      o[B * k1 + n2] = n2 * k1 ? cmul(t[k1], mkcx(w.c[n2 * k1], sign * w.s[n2 * k1])) : t[k1];
+  }
+#pragma unroll
+  for (int k1 = 0; k1 < A; ++k1) {
+    cx t[8];
+#pragma unroll
+    for (int n2 = 0; n2 < B; ++n2) t[n2] = o[B * k1 + n2];
+    dft_small<B>(t, sign);
+#pragma unroll
+    for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = t[k2];
+  }
+}
+
+// R-point DFT of v[0..R), R in {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16}.
+template <int R>
+__device__ __forceinline__ void mix_dft(cx (&v)[16], rx sign) {
+  if constexpr (R == 16) dft16(v, sign);
+  else if constexpr (R == 15) dft_two<3, 5>(v, sign);
+  else if constexpr (R == 12) dft12(v, sign);
+  else if constexpr (R == 10) dft_two<2, 5>(v, sign);
+  else if constexpr (R == 9) dft_two<3, 3>(v, sign);
+  else if constexpr (R == 6) dft_two<2, 3>(v, sign);
+  else {
+    cx w[8];
+#pragma unroll
+    for (int j = 0; j < R; ++j) w[j] = v[j];
+    dft_small<R>(w, sign);
+#pragma unroll
+    for (int j = 0; j < R; ++j) v[j] = w[j];
+  }
+}
+
+// KIND 0: forward stage s; 1: its inverse; 2: the last stage, the product with h (by
+// place) and its inverse.
+template <int R, int KIND>
+__device__ __forceinline__ void mix_stage(const MixPlan &pl, int s, cx *buf, const cx *tw, const cx *h, int tid,
+                                          int nth) {
+  const int str = KIND == 2 ? 1 : pl.str[s];
+  for (int u = tid; u < pl.n / R; u += nth) {
+    int t = 0, base = u * R;
+    if (KIND != 2) {
+      const int b = fast_div(u, pl.ms[s]);
+      t = u - b * str;
+      base = b * (R * str) + t;
+    }
+    const cx *w = tw + pl.tw[s] + t;
+    cx v[16];
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      v[r] = buf[mix_pad(base + r * str)];
+      if (KIND == 1 && r > 0) v[r] = cmulc(v[r], w[r * str]);
+    }
+    mix_dft<R>(v, KIND == 1 ? TP_R(1.0) : -TP_R(1.0));
+    if (KIND == 2) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = cmul(v[r], h[base + r]);
+      mix_dft<R>(v, TP_R(1.0));
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) buf[mix_pad(base + r * str)] = KIND == 0 && r > 0 ? cmul(v[r], w[r * str]) : v[r];
+  }
+}
+// The stage's radix is at most RMAX (the first one).
+template <int RMAX, int KIND>
+__device__ __forceinline__ void mix_run(const MixPlan &pl, int s, cx *buf, const cx *tw, const cx *h, int tid,
+                                        int nth) {
+  auto at = [&](auto r) {
+    constexpr int R = decltype(r)::value;
+    if constexpr (R <= RMAX) mix_stage<R, KIND>(pl, s, buf, tw, h, tid, nth);
+  };
+  using std::integral_constant;
+  switch (pl.radix[s]) {
+    case 16: at(integral_constant<int, 16>{}); break;
+    case 15: at(integral_constant<int, 15>{}); break;
+    case 12: at(integral_constant<int, 12>{}); break;
+    case 10: at(integral_constant<int, 10>{}); break;
+    case 9: at(integral_constant<int, 9>{}); break;
+    case 8: at(integral_constant<int, 8>{}); break;
+    case 6: at(integral_constant<int, 6>{}); break;
+    case 5: at(integral_constant<int, 5>{}); break;
+    case 4: at(integral_constant<int, 4>{}); break;
+    case 3: at(integral_constant<int, 3>{}); break;
+    default: at(integral_constant<int, 2>{}); break;
   }
 }
 

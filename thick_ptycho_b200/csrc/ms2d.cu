@@ -159,64 +159,48 @@ __device__ __forceinline__ void ms_kernel_H(float2 *H, const MsParams &q, int ti
   for (int j = tid; j < q.n; j += nth) H[j] = ms_h_minus_1(q, j);
 }
 
-// One CTA marches `rows` probes through all slices (the field stays in
-// shared memory).  Each slice is evaluated in delta form,
+// The march at the lengths of a single radix (n <= 16): one CTA marches `rows` probes
+// through all slices (the field stays in shared memory).  Each slice is evaluated in
+// delta form,
 //   X = psi + (T_z - 1) psi,   psi' = X + IFFT((H - 1) . FFT(X)),
 // so the FFT round-off scales with the small update instead of the field
-// (the same reason the CN march keeps "1 + eps" coefficients).  X stays in
-// registers: a thread owns elements tid + j*nth, j < E (E = 8, 16 or 32:
-// rows * n <= E * kFftThreads).
-constexpr int kMsElems = 32;  // the largest E
+// (the same reason the CN march keeps "1 + eps" coefficients).  X stays in a
+// register: a thread owns one element (rows * n <= 64).
+constexpr int kMsRows = 4;
 
-template <int E>
 __global__ void __launch_bounds__(kFftThreads) ms_march_kernel(const FftPlan pl, const MsParams q, int rows) {
   extern __shared__ __align__(16) float2 fsm[];
   const int n = q.n, tid = threadIdx.x, nth = blockDim.x;
   float2 *tw = fsm, *H = tw + n, *a = H + n, *b = a + rows * n;
-  auto col = [n](int e) {  // e % n, at most four probes
-    while (e >= n) e -= n;
-    return e;
-  };
   const int p0 = blockIdx.x * rows;
   const int nb = min(rows, q.P - p0);
   const int tot = nb * n;
   fft_twiddles(tw, n, tid, nth);
   ms_kernel_H(H, q, tid, nth);
-  float2 X[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) {
-    const int e = tid + j * nth;
-    if (e < tot) {
-      X[j] = q.probes[(size_t)p0 * n + e];
-      if (q.u_store) q.u_store[((size_t)(p0 + e / n) * q.nz) * n + e % n] = X[j];
-    }
+  float2 X = {};
+  const int e = tid;
+  if (e < tot) {
+    X = q.probes[(size_t)p0 * n + e];
+    if (q.u_store) q.u_store[((size_t)(p0 + e / n) * q.nz) * n + e % n] = X;
   }
   __syncthreads();
   const float s = 1.f / (float)n;
   for (int z = 0; z < q.L; ++z) {
     const float2 *Tz = q.trans + (size_t)z * n;
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int e = tid + j * nth;
-      if (e < tot) {
-        X[j] = cfma(Tz[col(e)], X[j], X[j]);
-        a[e] = X[j];
-      }
+    if (e < tot) {
+      X = cfma(Tz[e % n], X, X);
+      a[e] = X;
     }
     __syncthreads();
     float2 *F = fft_block(a, b, pl, tw, false, nb, tid, nth);
     float2 *o = (F == a) ? b : a;
-    for (int e = tid; e < tot; e += nth) F[e] = cmul(F[e], H[col(e)]);
+    if (e < tot) F[e] = cmul(F[e], H[e % n]);
     __syncthreads();
     float2 *R = fft_block(F, o, pl, tw, true, nb, tid, nth);
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int e = tid + j * nth;
-      if (e < tot) {
-        X[j] = make_float2(fmaf(R[e].x, s, X[j].x), fmaf(R[e].y, s, X[j].y));
-        if (q.u_store) q.u_store[((size_t)(p0 + e / n) * q.nz + z + 1) * n + e % n] = X[j];
-        if (z == q.L - 1 && q.exit_out) q.exit_out[(size_t)p0 * n + e] = X[j];
-      }
+    if (e < tot) {
+      X = make_float2(fmaf(R[e].x, s, X.x), fmaf(R[e].y, s, X.y));
+      if (q.u_store) q.u_store[((size_t)(p0 + e / n) * q.nz + z + 1) * n + e % n] = X;
+      if (z == q.L - 1 && q.exit_out) q.exit_out[(size_t)p0 * n + e] = X;
     }
     __syncthreads();
   }
@@ -225,53 +209,41 @@ __global__ void __launch_bounds__(kFftThreads) ms_march_kernel(const FftPlan pl,
 // Adjoint march (delta form as the forward): g = lambda + IFFT(conj(H - 1) .
 // FFT(lambda)); grad_t[z] += sum_p g conj(T_z u_z); lambda <- conj(T_z) g,
 // from lambda = src_exit at the exit plane.
-template <int E>
 __global__ void __launch_bounds__(kFftThreads) ms_backward_kernel(const FftPlan pl, const MsParams q, int rows) {
   extern __shared__ __align__(16) float2 fsm[];
   const int n = q.n, tid = threadIdx.x, nth = blockDim.x;
   float2 *tw = fsm, *H = tw + n, *a = H + n, *b = a + rows * n;
-  auto col = [n](int e) {  // e % n, at most four probes
-    while (e >= n) e -= n;
-    return e;
-  };
   const int p0 = blockIdx.x * rows;
   const int nb = min(rows, q.P - p0);
   const int tot = nb * n;
   fft_twiddles(tw, n, tid, nth);
   ms_kernel_H(H, q, tid, nth);
-  float2 X[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) {
-    const int e = tid + j * nth;
-    if (e < tot) {
-      X[j] = q.src_exit[(size_t)p0 * n + e];
-      a[e] = X[j];
-    }
+  float2 X = {};
+  const int e = tid;
+  if (e < tot) {
+    X = q.src_exit[(size_t)p0 * n + e];
+    a[e] = X;
   }
   __syncthreads();
   const float s = 1.f / (float)n;
   for (int z = q.L - 1; z >= 0; --z) {
     float2 *F = fft_block(a, b, pl, tw, false, nb, tid, nth);
     float2 *o = (F == a) ? b : a;
-    for (int e = tid; e < tot; e += nth) F[e] = cmulc(F[e], H[col(e)]);
+    if (e < tot) F[e] = cmulc(F[e], H[e % n]);
     __syncthreads();
     float2 *G = fft_block(F, o, pl, tw, true, nb, tid, nth);
     const float2 *Tz = q.trans + (size_t)z * n;
     // g = X + s*G ; contribution g conj(T u); X <- conj(T) g = g + conj(T-1) g
-#pragma unroll
-    for (int j = 0; j < E; ++j) {
-      const int e = tid + j * nth;
-      if (e < tot) {
-        const float2 g = make_float2(fmaf(G[e].x, s, X[j].x), fmaf(G[e].y, s, X[j].y));
-        const float2 tm1 = Tz[col(e)];
-        const float2 u = q.u_fwd[((size_t)(p0 + e / n) * q.nz + z) * n + e % n];
-        const float2 tu = cfma(tm1, u, u);
-        const float2 c = cmulc(g, tu);
-        float2 *dst = q.grad_t + (size_t)z * n + e % n;
-        asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(c.x), "f"(c.y) : "memory");
-        X[j] = cadd(g, cmulc(g, tm1));
-        a[e] = X[j];
-      }
+    if (e < tot) {
+      const float2 g = make_float2(fmaf(G[e].x, s, X.x), fmaf(G[e].y, s, X.y));
+      const float2 tm1 = Tz[e % n];
+      const float2 u = q.u_fwd[((size_t)(p0 + e / n) * q.nz + z) * n + e % n];
+      const float2 tu = cfma(tm1, u, u);
+      const float2 c = cmulc(g, tu);
+      float2 *dst = q.grad_t + (size_t)z * n + e % n;
+      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(c.x), "f"(c.y) : "memory");
+      X = cadd(g, cmulc(g, tm1));
+      a[e] = X;
     }
     __syncthreads();
   }
@@ -508,6 +480,146 @@ static int ms_reg_launch(const MsParams &q, cudaStream_t st, int *ran) {
   return TP_OK;
 }
 
+// ------------------------------------------- in-place transforms, other lengths
+// The marches at every other n = 2^a 3^b 5^c with at least two stages (fft.cuh's
+// in-place plan), one probe per CTA: a thread keeps the values of its unit of the
+// first stage in registers across slices, so that the inverse's last stage, the slice's
+// own arithmetic and the next forward transform's first stage need no exchange between
+// them; the last forward stage, the product with H - 1 and the first inverse one are a
+// single pass.  A slice is 2 (stages - 1) barriers, against two per pass and four more of
+// the shared-memory passes above: 64 probes, n = 1500 (10 10 15): 9.1 -> 3.3 us per slice
+// with the field kept, the adjoint 9.7 -> 3.8 (1000: 6.0 -> 2.3; 243, 32 probes: 4.1 -> 1.8).
+template <int R0>
+constexpr int kMixThreads = R0 == 5 ? 640 : 512;  // n / R0 at most (625 = 3125 / 5)
+template <int R0, bool BACKWARD>
+__global__ void __launch_bounds__(kMixThreads<R0>) ms_mix_kernel(const MsParams q, const __grid_constant__ MixPlan pl) {
+  extern __shared__ __align__(16) float2 fsm[];
+  const int n = q.n, tid = threadIdx.x, nth = blockDim.x, str = pl.str[0];
+  float2 *ts = fsm, *us = ts + n, *H = us + (BACKWARD ? n : 0), *tw = H + n, *buf = tw + pl.tw_total;
+  const size_t p = blockIdx.x;
+  const bool act = tid < str;
+  // T - 1 (and u) of a slice into this thread's own slots, issued as soon as those of the
+  // slice before are used
+  auto stage = [&](int z) {
+    if (!act) return;
+#pragma unroll
+    for (int j = 0; j < R0; ++j) {
+      cp_async8(&ts[tid + str * j], &q.trans[(size_t)z * n + tid + str * j]);
+      if (BACKWARD) cp_async8(&us[tid + str * j], &q.u_fwd[(p * q.nz + z) * n + tid + str * j]);
+    }
+    cp_async_commit();
+  };
+  stage(BACKWARD ? q.L - 1 : 0);
+  mix_twiddles(pl, tw, tid, nth);
+  const float s = 1.f / (float)n;
+  for (int e = tid; e < n; e += nth) {
+    const float2 w = ms_h_minus_1(q, mix_frequency(pl, e));
+    H[e] = make_float2(s * w.x, BACKWARD ? -s * w.y : s * w.y);
+  }
+  float2 X[16], y[16];
+  float2 *store = !BACKWARD && q.u_store ? q.u_store + p * q.nz * n + tid : nullptr;
+  if (act) {
+#pragma unroll
+    for (int j = 0; j < R0; ++j) {
+      X[j] = (BACKWARD ? q.src_exit : q.probes)[p * n + tid + str * j];
+      if (store) store[str * j] = X[j];
+    }
+  }
+  __syncthreads();  // twiddles and H are in place
+  for (int i = 0; i < q.L; ++i) {
+    const int z = BACKWARD ? q.L - 1 - i : i;
+    if (act) {
+      if (!BACKWARD) {
+        cp_async_wait<0>();
+#pragma unroll
+        for (int j = 0; j < R0; ++j) {
+          const float2 t = ts[tid + str * j];
+          X[j] = cfma(t, X[j], X[j]);
+        }
+        if (z + 1 < q.L) stage(z + 1);
+      }
+#pragma unroll
+      for (int j = 0; j < R0; ++j) y[j] = X[j];
+      mix_dft<R0>(y, -1.f);
+#pragma unroll
+      for (int k = 0; k < R0; ++k) buf[mix_pad(tid + str * k)] = k ? cmul(y[k], tw[tid + str * k]) : y[0];
+    }
+    __syncthreads();
+    for (int g = 1; g + 1 < pl.stages; ++g) {
+      mix_run<R0, 0>(pl, g, buf, tw, H, tid, nth);
+      __syncthreads();
+    }
+    mix_run<R0, 2>(pl, pl.stages - 1, buf, tw, H, tid, nth);
+    __syncthreads();
+    for (int g = pl.stages - 2; g > 0; --g) {
+      mix_run<R0, 1>(pl, g, buf, tw, H, tid, nth);
+      __syncthreads();
+    }
+    if (!act) continue;
+#pragma unroll
+    for (int k = 0; k < R0; ++k) {
+      const float2 w = buf[mix_pad(tid + str * k)];
+      y[k] = k ? cmulc(w, tw[tid + str * k]) : w;
+    }
+    mix_dft<R0>(y, 1.f);
+    if (!BACKWARD) {
+      if (store) store += n;
+#pragma unroll
+      for (int j = 0; j < R0; ++j) {
+        X[j] = cadd(X[j], y[j]);
+        if (store) __stcs(&store[str * j], X[j]);
+      }
+    } else {
+      cp_async_wait<0>();
+      float2 *grad = q.grad_t + (size_t)z * n + tid;
+#pragma unroll
+      for (int j = 0; j < R0; ++j) {
+        const float2 g = cadd(X[j], y[j]);
+        const float2 tm1 = ts[tid + str * j], u = us[tid + str * j];
+        red_add_cx(grad + str * j, cmulc(g, cfma(tm1, u, u)));
+        X[j] = cadd(g, cmulc(g, tm1));
+      }
+      if (z > 0) stage(z - 1);
+    }
+  }
+  if (!BACKWARD && act && q.exit_out) {
+#pragma unroll
+    for (int j = 0; j < R0; ++j) q.exit_out[p * n + tid + str * j] = X[j];
+  }
+}
+
+// Launches the in-place kernel, if n has a plan (*ran = 1).
+template <bool BACKWARD>
+static int ms_mix_launch(const MsParams &q, cudaStream_t st, int *ran) {
+  const MixPlan pl = make_mix_plan(q.n);
+  *ran = 1;
+  auto go = [&](auto r0) -> int {
+    constexpr int R0 = decltype(r0)::value;
+    auto kern = ms_mix_kernel<R0, BACKWARD>;
+    const int threads = pl.threads < kMixThreads<R0> ? pl.threads : kMixThreads<R0>;
+    const size_t smem = (size_t)((BACKWARD ? 3 : 2) * q.n + pl.tw_total + mix_pad(q.n) + 1) * sizeof(float2);
+    TP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    kern<<<q.P, threads, smem, st>>>(q, pl);
+    return check_cuda(cudaGetLastError(), "multislice in-place kernel launch");
+  };
+  using std::integral_constant;
+  if (pl.stages >= 2) {
+    switch (pl.radix[0]) {
+      case 16: return go(integral_constant<int, 16>{});
+      case 15: return go(integral_constant<int, 15>{});
+      case 12: return go(integral_constant<int, 12>{});
+      case 10: return go(integral_constant<int, 10>{});
+      case 9: return go(integral_constant<int, 9>{});
+      case 8: return go(integral_constant<int, 8>{});
+      case 6: return go(integral_constant<int, 6>{});
+      case 5: return go(integral_constant<int, 5>{});
+      default: break;
+    }
+  }
+  *ran = 0;
+  return TP_OK;
+}
+
 static size_t fft_smem(int n, int rows, int extra) { return (size_t)(extra * n + 2 * rows * n) * sizeof(float2); }
 
 int ms_transmission_launch(int n_total, int nz, double k, double dz, double nmr, double nmi, const void *field,
@@ -612,25 +724,13 @@ extern "C" int tp_ms2d_transmission(const tp_ms2d_op *op, const void *n_field, i
                                 reinterpret_cast<cudaStream_t>(stream));
 }
 
-// Probes per CTA: at most what kMsElems field values per thread hold and
-// what fits in 200 KB of shared memory (two FFT buffers per probe, H and the
-// twiddles), at most 4, and no more than needed to give every SM a CTA.
-static int ms_rows(int n, int num_probes) {
-  int r = (kMsElems * kFftThreads) / n;
-  const int rs = (200 * 1024 / (int)sizeof(float2) - 2 * n) / (2 * n);
-  if (rs < r) r = rs;
-  if (r > 4) r = 4;
+// Probes per CTA of the single-radix lengths: at most kMsRows, and no more than needed
+// to give every SM a CTA.
+static int ms_rows(int num_probes) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int fill = (num_probes + sms - 1) / sms;
-  if (r > fill) r = fill < 1 ? 1 : fill;
-  return r;
-}
-
-// Field values per thread for `rows` probes of length n (a compiled E).
-static int ms_elems(int n, int rows) {
-  const int e = (rows * n + kFftThreads - 1) / kFftThreads;
-  return e <= 8 ? 8 : (e <= 16 ? 16 : 32);
+  return fill < kMsRows ? fill : kMsRows;
 }
 
 extern "C" int tp_ms2d_march(const tp_ms2d_op *op, const void *trans, const void *probes, int32_t num_probes,
@@ -650,14 +750,11 @@ extern "C" int tp_ms2d_march(const tp_ms2d_op *op, const void *trans, const void
   int ran = 0;
   rc = ms_reg_launch<false>(q, reinterpret_cast<cudaStream_t>(stream), &ran);
   if (rc != TP_OK || ran) return rc;
-  const int rows = ms_rows(op->n, num_probes);
-  if (rows < 1) return set_error(TP_ERR_UNSUPPORTED, "N=%d too large for the multislice kernel", op->n);
+  rc = ms_mix_launch<false>(q, reinterpret_cast<cudaStream_t>(stream), &ran);
+  if (rc != TP_OK || ran) return rc;
+  const int rows = ms_rows(num_probes);
   const size_t smem = fft_smem(op->n, rows, 2);
-  const int E = ms_elems(op->n, rows);
-  auto kern = E == 8 ? ms_march_kernel<8> : (E == 16 ? ms_march_kernel<16> : ms_march_kernel<32>);
-  rc = fft_launch_setup((const void *)kern, smem);
-  if (rc) return rc;
-  kern<<<(num_probes + rows - 1) / rows, kFftThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(pl, q, rows);
+  ms_march_kernel<<<(num_probes + rows - 1) / rows, kFftThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(pl, q, rows);
   return check_cuda(cudaGetLastError(), "ms_march_kernel launch");
 }
 
@@ -678,13 +775,10 @@ extern "C" int tp_ms2d_backward(const tp_ms2d_op *op, const void *trans, const v
   int ran = 0;
   rc = ms_reg_launch<true>(q, reinterpret_cast<cudaStream_t>(stream), &ran);
   if (rc != TP_OK || ran) return rc;
-  const int rows = ms_rows(op->n, num_probes);
-  if (rows < 1) return set_error(TP_ERR_UNSUPPORTED, "N=%d too large for the multislice kernel", op->n);
+  rc = ms_mix_launch<true>(q, reinterpret_cast<cudaStream_t>(stream), &ran);
+  if (rc != TP_OK || ran) return rc;
+  const int rows = ms_rows(num_probes);
   const size_t smem = fft_smem(op->n, rows, 2);
-  const int E = ms_elems(op->n, rows);
-  auto kern = E == 8 ? ms_backward_kernel<8> : (E == 16 ? ms_backward_kernel<16> : ms_backward_kernel<32>);
-  rc = fft_launch_setup((const void *)kern, smem);
-  if (rc) return rc;
-  kern<<<(num_probes + rows - 1) / rows, kFftThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(pl, q, rows);
+  ms_backward_kernel<<<(num_probes + rows - 1) / rows, kFftThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(pl, q, rows);
   return check_cuda(cudaGetLastError(), "ms_backward_kernel launch");
 }
