@@ -285,12 +285,7 @@ __device__ __forceinline__ cx *fft_run_padded(cx *a, cx *b, const cx *tw, rx sig
   }
 }
 
-// Lengths with a compile-time plan (radix 16 for 128 and 256, else 8s first,
-// then 4, 2, 3).
-__host__ __device__ constexpr bool fft_fixed_size(int n) {
-  return n == 32 || n == 64 || n == 128 || n == 192 || n == 256 || n == 512;
-}
-
+// Radix 16 for 128 and 256, else 8s first, then 4, 2, 3.
 // The fixed-size transforms in the padded layout (FftPad).
 template <int N>
 __device__ __forceinline__ cx *fft_block_padded(cx *a, cx *b, const cx *tw, bool inverse, int nb,
@@ -439,11 +434,12 @@ struct MixPlan {
 };
 
 // The fewest stages with radices up to 16 and of those the most even split, the
-// largest first; stages = 0 where there are none (or only one).
+// largest first, and at least two (n <= 16: a last one of radix 1); stages = 0 where
+// there are none.
 inline MixPlan make_mix_plan(int n) {
   MixPlan p{};
   p.n = n;
-  if (n < 2 || n > kFftMaxN) return p;
+  if (n < 1 || n > kFftMaxN) return p;
   constexpr int radices[] = {16, 15, 12, 10, 9, 8, 6, 5, 4, 3, 2};
   int cur[kMixStages] = {}, best_len = kMixStages + 1, best_sum = 0;
   // non-increasing sequences of radices with product n (a few hundred nodes at most)
@@ -464,7 +460,9 @@ inline MixPlan make_mix_plan(int n) {
       }
   };
   search(search, n, 0, 0, 0);
-  if (best_len > kMixStages || best_len < 2) return p;
+  if (n == 1) p.radix[best_len++] = 1;
+  if (best_len > kMixStages) return p;
+  if (best_len < 2) p.radix[best_len++] = 1;
   p.stages = best_len;
   int len = n, units = 0;
   for (int i = 0; i < p.stages; ++i) {
@@ -555,7 +553,7 @@ __device__ __forceinline__ void dft_two(cx (&v)[16], rx sign) {
   }
 }
 
-// R-point DFT of v[0..R), R in {2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16}.
+// R-point DFT of v[0..R), R in {1, 2, 3, 4, 5, 6, 8, 9, 10, 12, 15, 16}.
 template <int R>
 __device__ __forceinline__ void mix_dft(cx (&v)[16], rx sign) {
   if constexpr (R == 16) dft16(v, sign);
@@ -564,7 +562,7 @@ __device__ __forceinline__ void mix_dft(cx (&v)[16], rx sign) {
   else if constexpr (R == 10) dft_two<2, 5>(v, sign);
   else if constexpr (R == 9) dft_two<3, 3>(v, sign);
   else if constexpr (R == 6) dft_two<2, 3>(v, sign);
-  else {
+  else if constexpr (R > 1) {
     cx w[8];
 #pragma unroll
     for (int j = 0; j < R; ++j) w[j] = v[j];
@@ -574,46 +572,14 @@ __device__ __forceinline__ void mix_dft(cx (&v)[16], rx sign) {
   }
 }
 
-// KIND 0: forward stage s; 1: its inverse; 2: the last stage, the product with h (by
-// place) and its inverse.
-template <int R, int KIND>
-__device__ __forceinline__ void mix_stage(const MixPlan &pl, int s, cx *buf, const cx *tw, const cx *h, int tid,
-                                          int nth) {
-  const int str = KIND == 2 ? 1 : pl.str[s];
-  for (int u = tid; u < pl.n / R; u += nth) {
-    int t = 0, base = u * R;
-    if (KIND != 2) {
-      const int b = fast_div(u, pl.ms[s]);
-      t = u - b * str;
-      base = b * (R * str) + t;
-    }
-    const cx *w = tw + pl.tw[s] + t;
-    cx v[16];
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      v[r] = buf[mix_pad(base + r * str)];
-      if (KIND == 1 && r > 0) v[r] = cmulc(v[r], w[r * str]);
-    }
-    mix_dft<R>(v, KIND == 1 ? TP_R(1.0) : -TP_R(1.0));
-    if (KIND == 2) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) v[r] = cmul(v[r], h[base + r]);
-      mix_dft<R>(v, TP_R(1.0));
-    }
-#pragma unroll
-    for (int r = 0; r < R; ++r) buf[mix_pad(base + r * str)] = KIND == 0 && r > 0 ? cmul(v[r], w[r * str]) : v[r];
-  }
-}
-// The stage's radix is at most RMAX (the first one).
-template <int RMAX, int KIND>
-__device__ __forceinline__ void mix_run(const MixPlan &pl, int s, cx *buf, const cx *tw, const cx *h, int tid,
-                                        int nth) {
+// Calls f with the radix (at most RMAX) as a constant.
+template <int RMAX, class F>
+__device__ __forceinline__ void mix_radix(int radix, F f) {
   auto at = [&](auto r) {
-    constexpr int R = decltype(r)::value;
-    if constexpr (R <= RMAX) mix_stage<R, KIND>(pl, s, buf, tw, h, tid, nth);
+    if constexpr (decltype(r)::value <= RMAX) f(r);
   };
   using std::integral_constant;
-  switch (pl.radix[s]) {
+  switch (radix) {
     case 16: at(integral_constant<int, 16>{}); break;
     case 15: at(integral_constant<int, 15>{}); break;
     case 12: at(integral_constant<int, 12>{}); break;
@@ -624,8 +590,45 @@ __device__ __forceinline__ void mix_run(const MixPlan &pl, int s, cx *buf, const
     case 5: at(integral_constant<int, 5>{}); break;
     case 4: at(integral_constant<int, 4>{}); break;
     case 3: at(integral_constant<int, 3>{}); break;
-    default: at(integral_constant<int, 2>{}); break;
+    case 2: at(integral_constant<int, 2>{}); break;
+    default: at(integral_constant<int, 1>{}); break;
   }
+}
+
+// Stage s of `count` elements (whole transforms, back to back, at mix_pad) in shared
+// memory.  KIND 0: forward; 1: inverse; 2: the last stage, the product with h (by place)
+// and its inverse; 3, 4: the last stage alone, forward and inverse (no twiddles).
+template <int RMAX, int KIND>
+__device__ __forceinline__ void mix_run(const MixPlan &pl, int s, int count, cx *buf, const cx *tw, const cx *h,
+                                        int tid, int nth) {
+  mix_radix<RMAX>(pl.radix[s], [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+    constexpr bool LAST = KIND >= 2, INV = KIND == 1 || KIND == 4;
+    const int str = LAST ? 1 : pl.str[s];
+    for (int u = tid; u < count / R; u += nth) {
+      int t = 0, base = u * R;
+      if (!LAST) {
+        const int b = fast_div(u, pl.ms[s]);
+        t = u - b * str;
+        base = b * (R * str) + t;
+      }
+      const cx *w = tw + pl.tw[s] + t;
+      cx v[16];
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        v[r] = buf[mix_pad(base + r * str)];
+        if (KIND == 1 && r > 0) v[r] = cmulc(v[r], w[r * str]);
+      }
+      mix_dft<R>(v, INV ? TP_R(1.0) : -TP_R(1.0));
+      if (KIND == 2) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[r] = cmul(v[r], h[base + r]);
+        mix_dft<R>(v, TP_R(1.0));
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) buf[mix_pad(base + r * str)] = KIND == 0 && r > 0 ? cmul(v[r], w[r * str]) : v[r];
+    }
+  });
 }
 
 // Factors of the lengths with a four-step plan (R1 >= R2, both <= 16).

@@ -155,99 +155,12 @@ __device__ __forceinline__ float2 ms_h_minus_1(const MsParams &q, int j) {
   sincos(0.5 * th, &sh, &ch);
   return make_float2((float)(-2.0 * sh * sh), (float)s);
 }
-__device__ __forceinline__ void ms_kernel_H(float2 *H, const MsParams &q, int tid, int nth) {
-  for (int j = tid; j < q.n; j += nth) H[j] = ms_h_minus_1(q, j);
-}
-
-// The march at the lengths of a single radix (n <= 16): one CTA marches `rows` probes
-// through all slices (the field stays in shared memory).  Each slice is evaluated in
-// delta form,
+// Each slice is evaluated in delta form,
 //   X = psi + (T_z - 1) psi,   psi' = X + IFFT((H - 1) . FFT(X)),
-// so the FFT round-off scales with the small update instead of the field
-// (the same reason the CN march keeps "1 + eps" coefficients).  X stays in a
-// register: a thread owns one element (rows * n <= 64).
-constexpr int kMsRows = 4;
-
-__global__ void __launch_bounds__(kFftThreads) ms_march_kernel(const FftPlan pl, const MsParams q, int rows) {
-  extern __shared__ __align__(16) float2 fsm[];
-  const int n = q.n, tid = threadIdx.x, nth = blockDim.x;
-  float2 *tw = fsm, *H = tw + n, *a = H + n, *b = a + rows * n;
-  const int p0 = blockIdx.x * rows;
-  const int nb = min(rows, q.P - p0);
-  const int tot = nb * n;
-  fft_twiddles(tw, n, tid, nth);
-  ms_kernel_H(H, q, tid, nth);
-  float2 X = {};
-  const int e = tid;
-  if (e < tot) {
-    X = q.probes[(size_t)p0 * n + e];
-    if (q.u_store) q.u_store[((size_t)(p0 + e / n) * q.nz) * n + e % n] = X;
-  }
-  __syncthreads();
-  const float s = 1.f / (float)n;
-  for (int z = 0; z < q.L; ++z) {
-    const float2 *Tz = q.trans + (size_t)z * n;
-    if (e < tot) {
-      X = cfma(Tz[e % n], X, X);
-      a[e] = X;
-    }
-    __syncthreads();
-    float2 *F = fft_block(a, b, pl, tw, false, nb, tid, nth);
-    float2 *o = (F == a) ? b : a;
-    if (e < tot) F[e] = cmul(F[e], H[e % n]);
-    __syncthreads();
-    float2 *R = fft_block(F, o, pl, tw, true, nb, tid, nth);
-    if (e < tot) {
-      X = make_float2(fmaf(R[e].x, s, X.x), fmaf(R[e].y, s, X.y));
-      if (q.u_store) q.u_store[((size_t)(p0 + e / n) * q.nz + z + 1) * n + e % n] = X;
-      if (z == q.L - 1 && q.exit_out) q.exit_out[(size_t)p0 * n + e] = X;
-    }
-    __syncthreads();
-  }
-}
-
-// Adjoint march (delta form as the forward): g = lambda + IFFT(conj(H - 1) .
-// FFT(lambda)); grad_t[z] += sum_p g conj(T_z u_z); lambda <- conj(T_z) g,
-// from lambda = src_exit at the exit plane.
-__global__ void __launch_bounds__(kFftThreads) ms_backward_kernel(const FftPlan pl, const MsParams q, int rows) {
-  extern __shared__ __align__(16) float2 fsm[];
-  const int n = q.n, tid = threadIdx.x, nth = blockDim.x;
-  float2 *tw = fsm, *H = tw + n, *a = H + n, *b = a + rows * n;
-  const int p0 = blockIdx.x * rows;
-  const int nb = min(rows, q.P - p0);
-  const int tot = nb * n;
-  fft_twiddles(tw, n, tid, nth);
-  ms_kernel_H(H, q, tid, nth);
-  float2 X = {};
-  const int e = tid;
-  if (e < tot) {
-    X = q.src_exit[(size_t)p0 * n + e];
-    a[e] = X;
-  }
-  __syncthreads();
-  const float s = 1.f / (float)n;
-  for (int z = q.L - 1; z >= 0; --z) {
-    float2 *F = fft_block(a, b, pl, tw, false, nb, tid, nth);
-    float2 *o = (F == a) ? b : a;
-    if (e < tot) F[e] = cmulc(F[e], H[e % n]);
-    __syncthreads();
-    float2 *G = fft_block(F, o, pl, tw, true, nb, tid, nth);
-    const float2 *Tz = q.trans + (size_t)z * n;
-    // g = X + s*G ; contribution g conj(T u); X <- conj(T) g = g + conj(T-1) g
-    if (e < tot) {
-      const float2 g = make_float2(fmaf(G[e].x, s, X.x), fmaf(G[e].y, s, X.y));
-      const float2 tm1 = Tz[e % n];
-      const float2 u = q.u_fwd[((size_t)(p0 + e / n) * q.nz + z) * n + e % n];
-      const float2 tu = cfma(tm1, u, u);
-      const float2 c = cmulc(g, tu);
-      float2 *dst = q.grad_t + (size_t)z * n + e % n;
-      asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(dst), "f"(c.x), "f"(c.y) : "memory");
-      X = cadd(g, cmulc(g, tm1));
-      a[e] = X;
-    }
-    __syncthreads();
-  }
-}
+// so the FFT round-off scales with the small update instead of the field (the same
+// reason the CN march keeps "1 + eps" coefficients); the adjoint: g = lambda +
+// IFFT(conj(H - 1) . FFT(lambda)), grad_t[z] += sum_p g conj(T_z u_z), lambda <-
+// conj(T_z) g, from lambda = src_exit at the exit plane.
 
 // ------------------------------------------- register transforms, n = 16 R2 R3
 // The march at n = 512, 1024, 2048 and 4096 with one probe per CTA of n / 16
@@ -266,7 +179,7 @@ __global__ void __launch_bounds__(kFftThreads) ms_backward_kernel(const FftPlan 
 // (one barrier each).  T - 1 (and the adjoint's u) of the next slice arrive by
 // asynchronous copies into the thread's own slots.  What remains is the latency of
 // a slice's dependent steps: n = 2048, 64 probes, 1023 slices: forward with the field
-// kept 13.7 -> 1.65 ms, adjoint 13.5 -> 2.30 ms against the shared-memory passes above.
+// kept 13.7 -> 1.65 ms, adjoint 13.5 -> 2.30 ms against Stockham passes in shared memory.
 template <int R2, int R3>
 struct RegFft {
   static constexpr int N = 16 * R2 * R3, T = N / 16, M2 = 16 / R2, M3 = 16 / R3;
@@ -481,14 +394,13 @@ static int ms_reg_launch(const MsParams &q, cudaStream_t st, int *ran) {
 }
 
 // ------------------------------------------- in-place transforms, other lengths
-// The marches at every other n = 2^a 3^b 5^c with at least two stages (fft.cuh's
-// in-place plan), one probe per CTA: a thread keeps the values of its unit of the
+// The marches at every other n = 2^a 3^b 5^c (fft.cuh's in-place plan), one probe per CTA: a thread keeps the values of its unit of the
 // first stage in registers across slices, so that the inverse's last stage, the slice's
 // own arithmetic and the next forward transform's first stage need no exchange between
 // them; the last forward stage, the product with H - 1 and the first inverse one are a
 // single pass.  A slice is 2 (stages - 1) barriers, against two per pass and four more of
-// the shared-memory passes above: 64 probes, n = 1500 (10 10 15): 9.1 -> 3.3 us per slice
-// with the field kept, the adjoint 9.7 -> 3.8 (1000: 6.0 -> 2.3; 243, 32 probes: 4.1 -> 1.8).
+// Stockham passes in shared memory: 64 probes, n = 1500 (10 10 15): 9.1 -> 3.1 us per slice
+// with the field kept, the adjoint 9.7 -> 3.4 (1000: 6.0 -> 2.4; 243, 32 probes: 4.1 -> 1.9).
 template <int R0>
 constexpr int kMixThreads = R0 == 5 ? 640 : 512;  // n / R0 at most (625 = 3125 / 5)
 template <int R0, bool BACKWARD>
@@ -546,13 +458,13 @@ __global__ void __launch_bounds__(kMixThreads<R0>) ms_mix_kernel(const MsParams 
     }
     __syncthreads();
     for (int g = 1; g + 1 < pl.stages; ++g) {
-      mix_run<R0, 0>(pl, g, buf, tw, H, tid, nth);
+      mix_run<R0, 0>(pl, g, n, buf, tw, H, tid, nth);
       __syncthreads();
     }
-    mix_run<R0, 2>(pl, pl.stages - 1, buf, tw, H, tid, nth);
+    mix_run<R0, 2>(pl, pl.stages - 1, n, buf, tw, H, tid, nth);
     __syncthreads();
     for (int g = pl.stages - 2; g > 0; --g) {
-      mix_run<R0, 1>(pl, g, buf, tw, H, tid, nth);
+      mix_run<R0, 1>(pl, g, n, buf, tw, H, tid, nth);
       __syncthreads();
     }
     if (!act) continue;
@@ -588,11 +500,13 @@ __global__ void __launch_bounds__(kMixThreads<R0>) ms_mix_kernel(const MsParams 
   }
 }
 
-// Launches the in-place kernel, if n has a plan (*ran = 1).
+// Launches the march of length n (which has a plan).
 template <bool BACKWARD>
-static int ms_mix_launch(const MsParams &q, cudaStream_t st, int *ran) {
+static int ms_launch(const MsParams &q, cudaStream_t st) {
+  int ran = 0;
+  const int rc = ms_reg_launch<BACKWARD>(q, st, &ran);
+  if (rc != TP_OK || ran) return rc;
   const MixPlan pl = make_mix_plan(q.n);
-  *ran = 1;
   auto go = [&](auto r0) -> int {
     constexpr int R0 = decltype(r0)::value;
     auto kern = ms_mix_kernel<R0, BACKWARD>;
@@ -603,21 +517,20 @@ static int ms_mix_launch(const MsParams &q, cudaStream_t st, int *ran) {
     return check_cuda(cudaGetLastError(), "multislice in-place kernel launch");
   };
   using std::integral_constant;
-  if (pl.stages >= 2) {
-    switch (pl.radix[0]) {
-      case 16: return go(integral_constant<int, 16>{});
-      case 15: return go(integral_constant<int, 15>{});
-      case 12: return go(integral_constant<int, 12>{});
-      case 10: return go(integral_constant<int, 10>{});
-      case 9: return go(integral_constant<int, 9>{});
-      case 8: return go(integral_constant<int, 8>{});
-      case 6: return go(integral_constant<int, 6>{});
-      case 5: return go(integral_constant<int, 5>{});
-      default: break;
-    }
+  switch (pl.radix[0]) {
+    case 16: return go(integral_constant<int, 16>{});
+    case 15: return go(integral_constant<int, 15>{});
+    case 12: return go(integral_constant<int, 12>{});
+    case 10: return go(integral_constant<int, 10>{});
+    case 9: return go(integral_constant<int, 9>{});
+    case 8: return go(integral_constant<int, 8>{});
+    case 6: return go(integral_constant<int, 6>{});
+    case 5: return go(integral_constant<int, 5>{});
+    case 4: return go(integral_constant<int, 4>{});
+    case 3: return go(integral_constant<int, 3>{});
+    case 2: return go(integral_constant<int, 2>{});
+    default: return set_error(TP_ERR_UNSUPPORTED, "multislice length %d has no plan", q.n);
   }
-  *ran = 0;
-  return TP_OK;
 }
 
 static size_t fft_smem(int n, int rows, int extra) { return (size_t)(extra * n + 2 * rows * n) * sizeof(float2); }
@@ -724,15 +637,6 @@ extern "C" int tp_ms2d_transmission(const tp_ms2d_op *op, const void *n_field, i
                                 reinterpret_cast<cudaStream_t>(stream));
 }
 
-// Probes per CTA of the single-radix lengths: at most kMsRows, and no more than needed
-// to give every SM a CTA.
-static int ms_rows(int num_probes) {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int fill = (num_probes + sms - 1) / sms;
-  return fill < kMsRows ? fill : kMsRows;
-}
-
 extern "C" int tp_ms2d_march(const tp_ms2d_op *op, const void *trans, const void *probes, int32_t num_probes,
                              void *u_store, void *exit_out, tp_stream_t stream) {
   MsParams q;
@@ -747,15 +651,7 @@ extern "C" int tp_ms2d_march(const tp_ms2d_op *op, const void *trans, const void
   q.probes = static_cast<const float2 *>(probes);
   q.u_store = static_cast<float2 *>(u_store);
   q.exit_out = static_cast<float2 *>(exit_out);
-  int ran = 0;
-  rc = ms_reg_launch<false>(q, reinterpret_cast<cudaStream_t>(stream), &ran);
-  if (rc != TP_OK || ran) return rc;
-  rc = ms_mix_launch<false>(q, reinterpret_cast<cudaStream_t>(stream), &ran);
-  if (rc != TP_OK || ran) return rc;
-  const int rows = ms_rows(num_probes);
-  const size_t smem = fft_smem(op->n, rows, 2);
-  ms_march_kernel<<<(num_probes + rows - 1) / rows, kFftThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(pl, q, rows);
-  return check_cuda(cudaGetLastError(), "ms_march_kernel launch");
+  return ms_launch<false>(q, reinterpret_cast<cudaStream_t>(stream));
 }
 
 extern "C" int tp_ms2d_backward(const tp_ms2d_op *op, const void *trans, const void *u_fwd, const void *src_exit,
@@ -772,13 +668,5 @@ extern "C" int tp_ms2d_backward(const tp_ms2d_op *op, const void *trans, const v
   q.u_fwd = static_cast<const float2 *>(u_fwd);
   q.src_exit = static_cast<const float2 *>(src_exit);
   q.grad_t = static_cast<float2 *>(grad_t);
-  int ran = 0;
-  rc = ms_reg_launch<true>(q, reinterpret_cast<cudaStream_t>(stream), &ran);
-  if (rc != TP_OK || ran) return rc;
-  rc = ms_mix_launch<true>(q, reinterpret_cast<cudaStream_t>(stream), &ran);
-  if (rc != TP_OK || ran) return rc;
-  const int rows = ms_rows(num_probes);
-  const size_t smem = fft_smem(op->n, rows, 2);
-  ms_backward_kernel<<<(num_probes + rows - 1) / rows, kFftThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(pl, q, rows);
-  return check_cuda(cudaGetLastError(), "ms_backward_kernel launch");
+  return ms_launch<true>(q, reinterpret_cast<cudaStream_t>(stream));
 }

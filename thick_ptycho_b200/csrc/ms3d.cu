@@ -38,7 +38,7 @@ int ms_transmission_launch(int n_total, int nz, double k, double dz, double nmr,
 struct Ms3Params {
   int n1, n2, N, nz, L, P;
   const float2 *trans;  // (L, N): T_z - 1
-  const float2 *hm1t;   // (H - 1) / N, (n2, n1), or (n1, n2) for the four-step column kernel
+  const float2 *hm1t;   // (H - 1) / N, (n1, n2)
   const float2 *tw1, *tw2;
   float2 *psi;          // (P, N): field (forward) or lambda (adjoint), in place
   float2 *W;            // (P, N): spectrum work buffer, in place
@@ -48,23 +48,21 @@ struct Ms3Params {
 
 enum Ms3Phase : int { kMs3FwdStart = 0, kMs3FwdStep = 1, kMs3BwdStart = 2, kMs3BwdStep = 3 };
 
-// Twiddle table W_n^t = exp(-2 pi i t / n) (fp64, rounded once) for the row
-// (n2) and column (n1) lengths.
-__global__ void ms3_twiddle_kernel(int n, float2 *tw) {
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n; t += gridDim.x * blockDim.x) {
-    double sv, cv;
-    sincospi(-2.0 * (double)t / (double)n, &sv, &cv);
-    tw[t] = make_float2((float)cv, (float)sv);
-  }
+// The stages' twiddles of an in-place plan.
+__global__ void ms3_twiddle_mix_kernel(const __grid_constant__ MixPlan pl, float2 *tw) {
+  mix_twiddles(pl, tw, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-// (H - 1) / N at hm1t[b * n1 + a] (by_row: at a * n2 + b); H - 1 = exp(i th) - 1 = -2 sin^2(th/2) + i sin th.
-__global__ void ms3_kernel_h_kernel(int n1, int n2, double k, double d1, double d2, double dz, int by_row,
-                                    float2 *hm1t) {
+// (H - 1) / N at a * n2 + b, the axes of an in-place plan (stages > 0) by place instead
+// of frequency; H - 1 = exp(i th) - 1 = -2 sin^2(th/2) + i sin th.
+__global__ void ms3_kernel_h_kernel(int n1, int n2, const __grid_constant__ MixPlan p1, const __grid_constant__ MixPlan p2,
+                                    double k, double d1, double d2, double dz, float2 *hm1t) {
   const int N = n1 * n2;
   const double inv = 1.0 / (double)N;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N; e += gridDim.x * blockDim.x) {
-    const int a = by_row ? e / n2 : e % n1, b = by_row ? e % n2 : e / n1;
+    int a = e / n2, b = e % n2;
+    if (p1.stages > 0) a = mix_frequency(p1, a);
+    if (p2.stages > 0) b = mix_frequency(p2, b);
     const int fa = (a < (n1 + 1) / 2) ? a : a - n1;
     const int fb = (b < (n2 + 1) / 2) ? b : b - n2;
     const double k1 = 2.0 * 3.14159265358979323846 * (double)fa / ((double)n1 * d1);
@@ -78,182 +76,192 @@ __global__ void ms3_kernel_h_kernel(int n1, int n2, double k, double d1, double 
   }
 }
 
-// Rows (columns) per CTA of the compile-time plans: at most 16 and 4096 elements.
-__host__ __device__ constexpr int ms3_fixed_per_cta(int n) { return 4096 / n > 16 ? 16 : 4096 / n; }
-
-// Row pass of slice z (phase selects start / step, forward / adjoint).
-// Grid (n1 / rpc, P): a CTA owns rpc rows of one probe.  The spectrum rows
-// (into a) and the step's third operand (T_{z+1} forward, u_z adjoint, into
-// the unpadded buffer c) are copied asynchronously at entry; with a
-// compile-time plan (N2 > 0, rpc = ms3_fixed_per_cta(N2)) every thread owns
-// EPT fixed elements whose field and T_z values are loaded into registers at
-// entry too, so all loads overlap the inverse FFT.
-template <int N2>
-__global__ void __launch_bounds__(kMs3Threads) ms3_rows_kernel(const FftPlan pl, const Ms3Params q, int phase, int z,
-                                                               int rpc_rt) {
+// ------------------------------------------------------ in-place transforms
+// The two passes at the other lengths (fft.cuh's in-place plans); the spectrum rows stay
+// in the order of the plan's last stage, and the H table with them.  psi holds X_z =
+// psi_z T_z in a step.
+//
+// Rows: a CTA owns rpc rows of one probe.  The inverse's last stage (the plan's first),
+// the slice's own arithmetic and the forward transform's first stage share registers.
+// 240 x 150, 32 probes: 58 -> 39 us per slice, adjoint 60 -> 39 (200 x 200, 50: 63 -> 57;
+// 48 x 60, 64: 17 -> 12; 90 x 75, 16: 19 -> 15.5; what remains is issue and latency)
+// against Stockham passes with radices up to 8 (a pass and a barrier per radix and
+// direction, four more rounds through shared memory, no CTA for a remainder of rows).
+template <int PHASE>
+__global__ void __launch_bounds__(kMs3Threads, 2) ms3_mix_rows_kernel(const Ms3Params q, const __grid_constant__ MixPlan pl,
+                                                                   int rpc, int z) {
   extern __shared__ __align__(16) float2 fsm[];
-  constexpr bool FIX = N2 > 0;
-  constexpr int RPC = FIX ? ms3_fixed_per_cta(N2 > 0 ? N2 : 1) : 1;
-  constexpr int EPT = FIX ? RPC * N2 / kMs3Threads : 1;
-  const int n = FIX ? N2 : q.n2, pr = blockIdx.y;
-  const int rpc = FIX ? RPC : rpc_rt;
-  float2 *tw = fsm, *a = tw + n, *b = a + rpc * fstride<N2>(n), *cbuf = b + rpc * fstride<N2>(n);
-  const size_t pbase = (size_t)pr * q.N;
-  const int g0 = blockIdx.x * rpc * n;  // first element of the CTA's rows within the slice
-  const int tot = rpc * n;
-  const int tid = threadIdx.x;
-  auto slot = [&](int e) { return fslot<N2>(e / n, e % n, n); };
-  load_twiddles(tw, q.tw2, n);
-  float2 *out = a;  // the buffer transformed forward into W at the end
-  bool fwd_fft = true;
-  if (phase == kMs3FwdStart) {
-    const float2 *T0 = q.trans;
-    for (int e = tid; e < tot; e += kMs3Threads) {
-      const int g = g0 + e;
-      const float2 v = q.probes[pbase + g];
-      q.psi[pbase + g] = v;
-      if (q.u_store) q.u_store[(size_t)pr * q.nz * q.N + g] = v;
-      a[slot(e)] = cfma(T0[g], v, v);
-    }
-  } else if (phase == kMs3BwdStart) {
-    for (int e = tid; e < tot; e += kMs3Threads) {
-      const int g = g0 + e;
-      const float2 v = q.src_exit[pbase + g];
-      q.psi[pbase + g] = v;
-      a[slot(e)] = v;
-    }
-  } else {
-    const float2 *Tz = q.trans + (size_t)z * q.N;
-    const bool last = (phase == kMs3FwdStep) && (z + 1 == q.L);
-    const float2 *third = phase == kMs3FwdStep ? (last ? nullptr : q.trans + (size_t)(z + 1) * q.N + g0)
-                                               : q.u_fwd + ((size_t)pr * q.nz + z) * q.N + g0;
-    for (int e = tid; e < tot; e += kMs3Threads) {
-      cp_async8(&a[slot(e)], &q.W[pbase + g0 + e]);
-      if (third) cp_async8(&cbuf[e], &third[e]);
-    }
-    float2 pz[EPT], tz[EPT];
-    if constexpr (FIX) {
-#pragma unroll
-      for (int j = 0; j < EPT; ++j) {
-        const int g = g0 + tid + j * kMs3Threads;
-        pz[j] = q.psi[pbase + g];
-        tz[j] = Tz[g];
-      }
-    }
-    cp_async_wait_all();
-    __syncthreads();
-    const float2 *R = fft_rows<N2>(a, b, pl, tw, true, rpc);
-    out = (R == a) ? b : a;
-    if (phase == kMs3FwdStep) {
-      // psi_{z+1} = X_z + IFFT2((H-1) FFT2 X_z), X_z = psi_z + (T_z - 1) psi_z
-      float2 *us = q.u_store ? q.u_store + ((size_t)pr * q.nz + z + 1) * q.N : nullptr;
-      auto one = [&](int e, float2 pv, float2 tm1) {
-        const int g = g0 + e;
-        const float2 v = cadd(cfma(tm1, pv, pv), R[slot(e)]);
-        q.psi[pbase + g] = v;
-        if (us) us[g] = v;
-        if (last) {
-          if (q.exit_out) q.exit_out[pbase + g] = v;
-        } else {
-          out[slot(e)] = cfma(cbuf[e], v, v);  // X_{z+1} = psi_{z+1} T_{z+1}
-        }
-      };
-      if constexpr (FIX) {
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) one(tid + j * kMs3Threads, pz[j], tz[j]);
-      } else {
-        for (int e = tid; e < tot; e += kMs3Threads) one(e, q.psi[pbase + g0 + e], Tz[g0 + e]);
-      }
-      fwd_fft = !last;
-    } else {
-      // g_z = lambda_{z+1} + IFFT2(conj(H-1) FFT2 lambda_{z+1});
-      // grad_t[z] += g_z conj(T_z u_z);  lambda_z = conj(T_z) g_z
-      float2 *gt = q.grad_t + (size_t)z * q.N;
-      auto one = [&](int e, float2 lam1, float2 tm1) {
-        const int g = g0 + e;
-        const float2 gv = cadd(lam1, R[slot(e)]);
-        const float2 u = cbuf[e];  // u_z
-        const float2 c = cmulc(gv, cfma(tm1, u, u));
-        asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(gt + g), "f"(c.x), "f"(c.y) : "memory");
-        const float2 lam = cadd(gv, cmulc(gv, tm1));
-        q.psi[pbase + g] = lam;
-        if (z > 0) out[slot(e)] = lam;
-      };
-      if constexpr (FIX) {
-#pragma unroll
-        for (int j = 0; j < EPT; ++j) one(tid + j * kMs3Threads, pz[j], tz[j]);
-      } else {
-        for (int e = tid; e < tot; e += kMs3Threads) one(e, q.psi[pbase + g0 + e], Tz[g0 + e]);
-      }
-      fwd_fft = z > 0;
-    }
-  }
-  if (!fwd_fft) return;
-  __syncthreads();
-  float2 *scratch = (out == a) ? b : a;
-  const float2 *F = fft_rows<N2>(out, scratch, pl, tw, false, rpc);
-  for (int e = tid; e < tot; e += kMs3Threads) q.W[pbase + g0 + e] = F[slot(e)];
-}
-
-// Column pass: FFT along a, times (H - 1)/N (conjugated for the adjoint),
-// inverse FFT along a, in place on W.  Grid (n2 / cpc, P).  The columns are
-// copied asynchronously and, with a compile-time plan, the CTA's (H - 1)/N
-// block is loaded into registers under the forward FFT.
-template <int N1>
-__global__ void __launch_bounds__(kMs3Threads) ms3_cols_kernel(const FftPlan pl, const Ms3Params q, int conj_h,
-                                                               int cpc_rt) {
-  extern __shared__ __align__(16) float2 fsm[];
-  constexpr bool FIX = N1 > 0;
-  constexpr int CPC = FIX ? ms3_fixed_per_cta(N1 > 0 ? N1 : 1) : 1;
-  constexpr int EPT = FIX ? CPC * N1 / kMs3Threads : 1;
-  const int n = FIX ? N1 : q.n1, pr = blockIdx.y;
-  const int cpc = FIX ? CPC : cpc_rt;
-  const int tid = threadIdx.x;
-  float2 *tw = fsm, *a = tw + n, *b = a + cpc * fstride<N1>(n);
-  const int b0 = blockIdx.x * cpc;
-  float2 *base = q.W + (size_t)pr * q.N;
-  const float2 *h = q.hm1t + (size_t)b0 * n;
-  load_twiddles(tw, q.tw1, n);
-  for (int e = tid; e < cpc * n; e += kMs3Threads) {
-    const int c = e % cpc, r = e / cpc;  // coalesced over c
-    cp_async8(&a[fslot<N1>(c, r, n)], &base[(size_t)r * q.n2 + b0 + c]);
-  }
-  float2 hv[EPT];
-  if constexpr (FIX) {
-#pragma unroll
-    for (int j = 0; j < EPT; ++j) hv[j] = h[tid + j * kMs3Threads];
+  const int n = pl.n, tid = threadIdx.x, row0 = blockIdx.x * rpc;
+  const int tot = min(rpc, q.n1 - row0) * n;
+  float2 *tw = fsm, *buf = tw + pl.tw_total;
+  const size_t pbase = (size_t)blockIdx.y * q.N;
+  const int g0 = row0 * n;  // first element of the CTA's rows within the slice
+  constexpr bool STEP = PHASE == kMs3FwdStep || PHASE == kMs3BwdStep;
+  const bool last = PHASE == kMs3FwdStep ? z + 1 == q.L : PHASE == kMs3BwdStep && z == 0;
+  pdl_trigger();
+  for (int e = tid; e < pl.tw_total; e += kMs3Threads) cp_async8(&tw[e], &q.tw2[e]);
+  pdl_wait();
+  if (STEP) {
+    for (int e = tid; e < tot; e += kMs3Threads) cp_async8(&buf[mix_pad(e)], &q.W[pbase + g0 + e]);
   }
   cp_async_wait_all();
   __syncthreads();
-  float2 *F = fft_rows<N1>(a, b, pl, tw, false, cpc);
-  float2 *o = (F == a) ? b : a;
-  auto mul = [&](int e, float2 hh) {
-    const int c = e / n, r = e - c * n;
-    const int sl = fslot<N1>(c, r, n);
-    F[sl] = conj_h ? cmulc(F[sl], hh) : cmul(F[sl], hh);
-  };
-  if constexpr (FIX) {
+  if (STEP) {
+    mix_run<16, 4>(pl, pl.stages - 1, tot, buf, tw, nullptr, tid, kMs3Threads);
+    __syncthreads();
+    for (int s = pl.stages - 2; s > 0; --s) {
+      mix_run<16, 1>(pl, s, tot, buf, tw, nullptr, tid, kMs3Threads);
+      __syncthreads();
+    }
+  }
+  const float2 *T = q.trans + (size_t)(PHASE == kMs3FwdStep ? (last ? z : z + 1) : z) * q.N + g0;
+  const float2 *uf = PHASE == kMs3BwdStep ? q.u_fwd + ((size_t)blockIdx.y * q.nz + z) * q.N + g0 : nullptr;
+  const float2 *in = (PHASE == kMs3FwdStart ? q.probes : q.src_exit) + pbase + g0;
+  float2 *psi = q.psi + pbase + g0, *ex = q.exit_out ? q.exit_out + pbase + g0 : nullptr;
+  float2 *us = q.u_store ? q.u_store + ((size_t)blockIdx.y * q.nz + (STEP ? z + 1 : 0)) * q.N + g0 : nullptr;
+  mix_radix<16>(pl.radix[0], [&](auto rc) {
+    constexpr int R = decltype(rc)::value;
+    const int str = pl.str[0];
+    for (int u = tid; u < tot / R; u += kMs3Threads) {
+      const int b = fast_div(u, pl.ms[0]), t = u - b * str, base = b * n + t;
+      const float2 *w = tw + t;
+      float2 v[16], pz[R], tz[R], uz[R];
 #pragma unroll
-    for (int j = 0; j < EPT; ++j) mul(tid + j * kMs3Threads, hv[j]);
-  } else {
-    for (int e = tid; e < cpc * n; e += kMs3Threads) mul(e, h[e]);
-  }
+      for (int r = 0; r < R; ++r) {
+        const int e = base + r * str;
+        if (STEP) pz[r] = psi[e];
+        else v[r] = in[e];
+        if (PHASE != kMs3BwdStart) tz[r] = T[e];
+        if (PHASE == kMs3BwdStep) uz[r] = __ldcs(&uf[e]);
+      }
+      if (STEP) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          v[r] = buf[mix_pad(base + r * str)];
+          if (r > 0) v[r] = cmulc(v[r], w[r * str]);
+        }
+        mix_dft<R>(v, 1.f);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int e = base + r * str;
+        if (PHASE == kMs3FwdStart || PHASE == kMs3FwdStep) {
+          // psi_{z+1} = X_z + IFFT2((H-1) FFT2 X_z), X_{z+1} = psi_{z+1} T_{z+1}
+          if (STEP) v[r] = cadd(pz[r], v[r]);
+          if (us) __stcs(&us[e], v[r]);
+          if (last) {
+            if (ex) ex[e] = v[r];
+          } else {
+            v[r] = cfma(tz[r], v[r], v[r]);
+          }
+        } else if (PHASE == kMs3BwdStep) {
+          // g_z = lambda_{z+1} + IFFT2(conj(H-1) FFT2 lambda_{z+1});
+          // grad_t[z] += g_z conj(T_z u_z);  lambda_z = conj(T_z) g_z
+          const float2 gv = cadd(pz[r], v[r]);
+          red_add_cx(q.grad_t + (size_t)z * q.N + g0 + e, cmulc(gv, cfma(tz[r], uz[r], uz[r])));
+          v[r] = cadd(gv, cmulc(gv, tz[r]));
+        }
+        if (!last) psi[e] = v[r];
+      }
+      if (last) continue;
+      mix_dft<R>(v, -1.f);
+#pragma unroll
+      for (int r = 0; r < R; ++r) buf[mix_pad(base + r * str)] = r ? cmul(v[r], w[r * str]) : v[0];
+    }
+  });
+  if (last) return;
   __syncthreads();
-  const float2 *R = fft_rows<N1>(F, o, pl, tw, true, cpc);
-  for (int e = tid; e < cpc * n; e += kMs3Threads) {
-    const int c = e % cpc, r = e / cpc;
-    base[(size_t)r * q.n2 + b0 + c] = R[fslot<N1>(c, r, n)];
+  for (int s = 1; s + 1 < pl.stages; ++s) {
+    mix_run<16, 0>(pl, s, tot, buf, tw, nullptr, tid, kMs3Threads);
+    __syncthreads();
   }
+  mix_run<16, 3>(pl, pl.stages - 1, tot, buf, tw, nullptr, tid, kMs3Threads);
+  __syncthreads();
+  for (int e = tid; e < tot; e += kMs3Threads) q.W[pbase + g0 + e] = buf[mix_pad(e)];
+}
+
+// Columns: a CTA owns 2^lc columns of one probe (the last one fewer), place i of column c
+// at i 2^lc + c in shared memory: every access runs along c.  The first stage reads and
+// the last one writes W directly.
+template <bool CONJ>
+__global__ void __launch_bounds__(kMs3Threads) ms3_mix_cols_kernel(const Ms3Params q, const __grid_constant__ MixPlan pl,
+                                                                   int lc) {
+  extern __shared__ __align__(16) float2 fsm[];
+  const int n = pl.n, w = q.n2, tid = threadIdx.x, C = 1 << lc, c = tid & (C - 1);  // kMs3Threads is a multiple of C
+  const int col = (blockIdx.x << lc) + c;
+  const bool ok = col < w;
+  float2 *tw = fsm, *buf = tw + pl.tw_total + c;
+  float2 *base = q.W + (size_t)blockIdx.y * q.N + col;
+  const float2 *h = q.hm1t + col;
+  pdl_trigger();
+  for (int e = tid; e < pl.tw_total; e += kMs3Threads) cp_async8(&tw[e], &q.tw1[e]);
+  cp_async_wait_all();
+  __syncthreads();
+  pdl_wait();
+  // stage s; KIND 0: forward, 1: inverse, 2: last forward, product and inverse; GLOBAL:
+  // the plan's first stage, W instead of shared memory on its outer side
+  auto run = [&](auto kind, auto global, int s) {
+    constexpr int KIND = decltype(kind)::value;
+    constexpr bool GLOBAL = decltype(global)::value;
+    mix_radix<16>(pl.radix[s], [&](auto rc) {
+      constexpr int R = decltype(rc)::value;
+      const int str = pl.str[s];
+      for (int u = tid >> lc; u < n / R; u += kMs3Threads >> lc) {
+        const int b = fast_div(u, pl.ms[s]), t = u - b * str, at = b * (R * str) + t;
+        const float2 *tws = tw + pl.tw[s] + t;
+        float2 v[16], hv[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int i = at + r * str;
+          if (GLOBAL && KIND == 0) v[r] = ok ? base[(size_t)i * w] : make_float2(0.f, 0.f);
+          else v[r] = buf[i << lc];
+          if (KIND == 1 && r > 0) v[r] = cmulc(v[r], tws[r * str]);
+          if (KIND == 2) hv[r] = ok ? h[(size_t)i * w] : make_float2(0.f, 0.f);
+        }
+        mix_dft<R>(v, KIND == 1 ? 1.f : -1.f);
+        if (KIND == 2) {
+#pragma unroll
+          for (int r = 0; r < R; ++r) v[r] = CONJ ? cmulc(v[r], hv[r]) : cmul(v[r], hv[r]);
+          mix_dft<R>(v, 1.f);
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int i = at + r * str;
+          if (KIND == 0 && r > 0) v[r] = cmul(v[r], tws[r * str]);
+          if (GLOBAL && KIND == 1) {
+            if (ok) base[(size_t)i * w] = v[r];
+          } else {
+            buf[i << lc] = v[r];
+          }
+        }
+      }
+    });
+  };
+  using std::integral_constant;
+  using std::bool_constant;
+  run(integral_constant<int, 0>{}, bool_constant<true>{}, 0);
+  __syncthreads();
+  for (int s = 1; s + 1 < pl.stages; ++s) {
+    run(integral_constant<int, 0>{}, bool_constant<false>{}, s);
+    __syncthreads();
+  }
+  run(integral_constant<int, 2>{}, bool_constant<false>{}, pl.stages - 1);
+  __syncthreads();
+  for (int s = pl.stages - 2; s > 0; --s) {
+    run(integral_constant<int, 1>{}, bool_constant<false>{}, s);
+    __syncthreads();
+  }
+  run(integral_constant<int, 1>{}, bool_constant<true>{}, 0);
 }
 
 // ------------------------------------------------ register four-step kernels
-// The same two passes for row and column lengths 64, 128, 192 and 256 (R1 R2) with
+// The two passes for row and column lengths 64, 128, 192 and 256 (R1 R2) with
 // the transforms in registers (fft.cuh): 256 threads, 256 / R1 rows or columns per
 // CTA.  The row kernel's inverse transform ends with the field's elements in the
 // registers where the next forward transform starts, so the multiplication by T and
 // everything else between the two happens there, and an element crosses shared memory
 // once per transform.  The psi buffer holds X_z = psi_z T_z here (psi_{z+1} = X_z +
-// update needs no T_z).  The shared-memory passes above were bound by shared memory
+// update needs no T_z).  Stockham passes in shared memory were bound by it
 // (73-83 % of its throughput); a slice of 64 probes of 256 x 256 took 95 us with them
 // (adjoint 99) and takes 42 us (51) with these.
 template <int R1, int R2, int PHASE>
@@ -437,47 +445,6 @@ static Ms3Cols4 pick_cols4(int n) {
   }
 }
 
-using Ms3Rows = void (*)(const FftPlan, const Ms3Params, int, int, int);
-using Ms3Cols = void (*)(const FftPlan, const Ms3Params, int, int);
-
-template <int N>
-static Ms3Rows ms3_rows_of() { return ms3_rows_kernel<N>; }
-template <int N>
-static Ms3Cols ms3_cols_of() { return ms3_cols_kernel<N>; }
-
-// Compile-time plans for the common lengths, per axis.
-static Ms3Rows pick_rows(int n) {
-  switch (n) {
-    case 32: return ms3_rows_of<32>();
-    case 64: return ms3_rows_of<64>();
-    case 128: return ms3_rows_of<128>();
-    case 192: return ms3_rows_of<192>();
-    case 256: return ms3_rows_of<256>();
-    case 512: return ms3_rows_of<512>();
-    default: return ms3_rows_of<0>();
-  }
-}
-static Ms3Cols pick_cols(int n) {
-  switch (n) {
-    case 32: return ms3_cols_of<32>();
-    case 64: return ms3_cols_of<64>();
-    case 128: return ms3_cols_of<128>();
-    case 192: return ms3_cols_of<192>();
-    case 256: return ms3_cols_of<256>();
-    case 512: return ms3_cols_of<512>();
-    default: return ms3_cols_of<0>();
-  }
-}
-
-// Transforms per CTA: at most 16 and 4096 elements, and a divisor of the count.
-static int ms3_per_cta(int n, int count) {
-  int r = 4096 / n;
-  if (r > 16) r = 16;
-  if (r < 1) r = 1;
-  while (count % r != 0) --r;
-  return r;
-}
-
 struct Ms3Work {
   float2 *psi, *W, *hm1t, *tw1, *tw2;
   size_t bytes;
@@ -497,9 +464,9 @@ static Ms3Work ms3_layout(char *base, int n1, int n2, int P) {
   w.psi = take((size_t)P * N * sizeof(float2));
   w.W = take((size_t)P * N * sizeof(float2));
   w.hm1t = take(N * sizeof(float2));
-  // room for the four-step kernels' padded tables as well
-  w.tw1 = take((size_t)(n1 + 16) * sizeof(float2));
-  w.tw2 = take((size_t)(n2 + 16) * sizeof(float2));
+  // room for either kernels' tables (in-place plans: at most 1.3 n)
+  w.tw1 = take((size_t)(n1 + n1 / 2 + 16) * sizeof(float2));
+  w.tw2 = take((size_t)(n2 + n2 / 2 + 16) * sizeof(float2));
   w.bytes = off;
   return w;
 }
@@ -533,44 +500,42 @@ static int ms3_run(const tp_ms3d_op *op, Ms3Params q, bool backward, void *works
   // splits into whole CTAs
   const bool four_r = four_step_size(n2) && n1 % (256 / four_r1(n2)) == 0;
   const bool four_c = four_step_size(n1) && n2 % (256 / four_r1(n1)) == 0;
+  const MixPlan p1 = four_c ? MixPlan{} : make_mix_plan(n1), p2 = four_r ? MixPlan{} : make_mix_plan(n2);
   if (four_c) ms3_twiddle4_kernel<<<1, 256, 0, st>>>(four_r1(n1), four_r2(n1), w.tw1);
-  else ms3_twiddle_kernel<<<(n1 + 255) / 256, 256, 0, st>>>(n1, w.tw1);
+  else ms3_twiddle_mix_kernel<<<(n1 + 255) / 256, 256, 0, st>>>(p1, w.tw1);
   if (four_r) ms3_twiddle4_kernel<<<1, 256, 0, st>>>(four_r1(n2), four_r2(n2), w.tw2);
-  else ms3_twiddle_kernel<<<(n2 + 255) / 256, 256, 0, st>>>(n2, w.tw2);
+  else ms3_twiddle_mix_kernel<<<(n2 + 255) / 256, 256, 0, st>>>(p2, w.tw2);
   ms3_kernel_h_kernel<<<(q.N + 255) / 256 < 1184 ? (q.N + 255) / 256 : 1184, 256, 0, st>>>(
-      n1, n2, op->k, op->d1, op->d2, op->dz, four_c ? 1 : 0, w.hm1t);
+      n1, n2, p1, p2, op->k, op->d1, op->d2, op->dz, w.hm1t);
   TP_CHECK_CUDA(cudaGetLastError());
-  const FftPlan p1 = make_fft_plan(n1), p2 = make_fft_plan(n2);
-  // compile-time plans (padded layout, fixed transforms per CTA) where the
-  // other axis splits into whole CTAs, else the runtime plan
-  const bool fix_r = fft_fixed_size(n2) && n1 % ms3_fixed_per_cta(n2) == 0;
-  const bool fix_c = fft_fixed_size(n1) && n2 % ms3_fixed_per_cta(n1) == 0;
-  const Ms3Rows rows = fix_r ? pick_rows(n2) : ms3_rows_of<0>();
-  const Ms3Cols cols = fix_c ? pick_cols(n1) : ms3_cols_of<0>();
-  const int srow = fix_r ? n2 + n2 / 8 + 1 : n2, scol = fix_c ? n1 + n1 / 8 + 1 : n1;
-  const int rpc = fix_r ? ms3_fixed_per_cta(n2) : ms3_per_cta(n2, n1);
-  const int cpc = fix_c ? ms3_fixed_per_cta(n1) : ms3_per_cta(n1, n2);
-  const size_t smem_r = (size_t)(n2 + 2 * rpc * srow + rpc * n2) * sizeof(float2);
-  const size_t smem_c = (size_t)(n1 + 2 * cpc * scol) * sizeof(float2);
-  TP_CHECK_CUDA(cudaFuncSetAttribute(rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r));
-  TP_CHECK_CUDA(cudaFuncSetAttribute(cols, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c));
-  const dim3 gr(n1 / rpc, q.P), gc(n2 / cpc, q.P);
+  // in-place kernels: rows and columns per CTA, about 4096 elements
+  int rpc = 4096 / n2 < 16 ? 4096 / n2 : 16, lc = 4;
+  if (rpc < 1) rpc = 1;
+  while (lc > 0 && (n1 << lc) > 4096) --lc;
+  const size_t smem_r = (size_t)(p2.tw_total + mix_pad(rpc * n2) + 1) * sizeof(float2);
+  const size_t smem_c = (size_t)(p1.tw_total + (n1 << lc)) * sizeof(float2);
+  const auto start_m = backward ? ms3_mix_rows_kernel<kMs3BwdStart> : ms3_mix_rows_kernel<kMs3FwdStart>;
+  const auto step_m = backward ? ms3_mix_rows_kernel<kMs3BwdStep> : ms3_mix_rows_kernel<kMs3FwdStep>;
+  const auto cols_m = backward ? ms3_mix_cols_kernel<true> : ms3_mix_cols_kernel<false>;
+  if (!four_r) {
+    TP_CHECK_CUDA(cudaFuncSetAttribute(start_m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r));
+    TP_CHECK_CUDA(cudaFuncSetAttribute(step_m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_r));
+  }
+  if (!four_c) TP_CHECK_CUDA(cudaFuncSetAttribute(cols_m, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_c));
+  const dim3 gr((n1 + rpc - 1) / rpc, q.P), gc((n2 + (1 << lc) - 1) >> lc, q.P);
   const dim3 gr4(four_r ? n1 / (256 / four_r1(n2)) : 1, q.P), gc4(four_c ? n2 / (256 / four_r1(n1)) : 1, q.P);
   const Ms3Rows4 start4 = backward ? pick_rows4<kMs3BwdStart>(n2) : pick_rows4<kMs3FwdStart>(n2);
   const Ms3Rows4 step4 = backward ? pick_rows4<kMs3BwdStep>(n2) : pick_rows4<kMs3FwdStep>(n2);
   const Ms3Cols4 cols4 = backward ? pick_cols4<true>(n1) : pick_cols4<false>(n1);
-  // the passes of a march with both four-step kernels start early (pdl_wait)
-  const bool early = four_r && four_c;
+  // every pass but the first starts early (pdl_wait)
   auto row_pass = [&](bool start, int z) -> cudaError_t {
-    if (four_r) return launch_dependent(start ? start4 : step4, gr4, dim3(256), 0, st, early && !start, q, w.tw2, z);
-    rows<<<gr, kMs3Threads, smem_r, st>>>(p2, q, backward ? (start ? kMs3BwdStart : kMs3BwdStep)
-                                                          : (start ? kMs3FwdStart : kMs3FwdStep), z, rpc);
-    return cudaSuccess;
+    if (four_r) return launch_dependent(start ? start4 : step4, gr4, dim3(256), 0, st, !start, q, w.tw2, z);
+    return launch_dependent(start ? start_m : step_m, gr, dim3(kMs3Threads), smem_r, st, !start, q, p2, rpc, z);
   };
   TP_CHECK_CUDA(row_pass(true, backward ? q.L : 0));
   for (int t = 0; t < q.L; ++t) {
-    if (four_c) TP_CHECK_CUDA(launch_dependent(cols4, gc4, dim3(256), 0, st, early, q, w.tw1));
-    else cols<<<gc, kMs3Threads, smem_c, st>>>(p1, q, backward ? 1 : 0, cpc);
+    if (four_c) TP_CHECK_CUDA(launch_dependent(cols4, gc4, dim3(256), 0, st, true, q, w.tw1));
+    else TP_CHECK_CUDA(launch_dependent(cols_m, gc, dim3(kMs3Threads), smem_c, st, true, q, p1, lc));
     TP_CHECK_CUDA(row_pass(false, backward ? q.L - 1 - t : t));
   }
   return check_cuda(cudaGetLastError(), "ms3d march launch");
