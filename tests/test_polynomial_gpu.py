@@ -46,6 +46,8 @@ def cplx(rng, *shape):
     (241, 7, 3, "impedance", 5e-3), (777, 9, 2, "impedance2", 5e-3), (1023, 6, 2, "impedance", 5e-3),
     (1201, 6, 5, "neumann", 5e-3), (2047, 5, 1, "impedance", 5e-3),
     (241, 7, 3, "impedance", 0.4),  # past the polynomial's bounds: the direct kernel
+    (200, 6, 2, "neumann", 2e-2),   # object phases beyond the free-space margin
+    (97, 4, 310, "impedance", 5e-3), (512, 6, 3, "impedance", 5e-3),  # large batch; team layout
 ])
 def test_2d_modes_sources_and_gradient(N, nz, P, bc, amp):
     rng = np.random.default_rng(N)
@@ -72,6 +74,10 @@ def test_2d_modes_sources_and_gradient(N, nz, P, bc, amp):
     eng.march(fs, P, probes=dev(probes), src_shared=dev(sh), t_begin=1, t_end=cut, state_out=state)
     eng.march(fs, P, src_shared=dev(sh), t_begin=cut + 1, t_end=L, state_in=state.clone(), exit_out=out)
     assert rel(out.cpu().numpy(), ref[:, :, -1]) < 1e-5
+    # and from a slice of the stored field
+    again = torch.empty_like(out)
+    eng.march(fs, P, src_shared=dev(sh), t_begin=cut + 1, t_end=L, state_from=(store, cut), exit_out=again)
+    assert torch.equal(again, out)
 
     plain = eng.new_store(P)
     eng.march(fs, P, probes=dev(probes), u_store=plain)

@@ -137,6 +137,7 @@ class CN2D:
         store_base: int = 0,
         ufwd_base: int = 0,
         store_sums: bool = False,
+        state_from: Optional[tuple] = None,
     ):
         """One batched march; every tensor is complex64 (complex128 in the
         check build), contiguous, on device.
@@ -151,6 +152,8 @@ class CN2D:
         exact-adjoint gradient contracts with the pair sum; the half sum is
         the Cayley step's solve result, stored at no extra cost) instead of
         ``u_t``, and an exact-adjoint march reads ``u_fwd`` as those.
+        ``state_from = (store, index)``: the initial state is slice ``index`` of
+        the chunked field ``store`` (P, S, Npad), read in place of ``state_in``.
         """
         P = int(num_probes)
         shapes = {
@@ -187,6 +190,14 @@ class CN2D:
         a.ufwd_slices = 0 if u_fwd is None else int(u_fwd.shape[1])
         a.ufwd_base = int(ufwd_base)
         a.store_sums = 1 if store_sums else 0
+        if state_from is not None:
+            store, index = state_from
+            if state_in is not None or store.dtype != self.cdtype or not store.is_contiguous() or not store.is_cuda or \
+                    store.dim() != 3 or store.shape[0] != P or store.shape[2] != self.npad or \
+                    not 0 <= index < store.shape[1]:
+                raise ValueError("state_from must be a chunked field (P, slices, Npad) and one of its slices")
+            a.state_in = ctypes.c_void_p(store.data_ptr() + index * self.npad * store.element_size())
+            a.store_sums |= store.shape[1] << 8
         o = self.op()
         rc = self.lib.tp_cn2d_march(ctypes.byref(o), _ptr(fs.buf), ctypes.byref(a), _stream(self.device))
         _native.check(rc, "tp_cn2d_march", self.lib)

@@ -153,6 +153,7 @@ __device__ __forceinline__ double2 p_sup(const FactorParams &f, int g) {  // P[g
 // runs.  Grid (Npad / 32, ceil(slices / 32)), block (32, 8).
 __global__ void __launch_bounds__(256) cn2d_diag_kernel(const FactorParams f, int count) {
   __shared__ double2 tile[32][33];
+  pdl_trigger();
   const int e0 = blockIdx.x * 32, i = e0 / f.C, c0 = e0 % f.C;
   const int s0 = blockIdx.y * 32;
   bool bad = false;
@@ -193,6 +194,8 @@ __global__ void __launch_bounds__(128) cn2d_factor_kernel(const FactorParams f) 
   cx *QD = base, *LF = base + M * C, *EP = base + 2 * M * C, *V = base + 3 * M * C, *W = base + 4 * M * C,
          *LR = base + 5 * M * C;
   const double2 *diag = reinterpret_cast<const double2 *>(V) + c;
+  pdl_trigger();
+  pdl_wait();
 
   double2 ipl[kMaxRowsPerLane], msl[kMaxRowsPerLane], fv[kMaxRowsPerLane];
   const int g0 = c * M;
@@ -417,6 +420,7 @@ __device__ __forceinline__ void add_natural(cx (&U)[M], const cx *__restrict__ s
 
 template <int M, bool ALIGNED, bool LAGGED>
 __global__ void __launch_bounds__(kMarchWarps * 32, 1) cn2d_march_kernel(const MarchParams p) {
+  pdl_wait();
   if (p.poly_bad != nullptr && *p.poly_bad == 0u) return;  // the polynomial kernel ran this march
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -448,7 +452,7 @@ __global__ void __launch_bounds__(kMarchWarps * 32, 1) cn2d_march_kernel(const M
 #pragma unroll
   for (int i = 0; i < M; ++i) U[i] = czero();
   if (active && p.state_in != nullptr) {
-    const cx *src = p.state_in + (size_t)probe * p.Npad;
+    const cx *src = p.state_in + (size_t)probe * p.state_stride;
 #pragma unroll
     for (int i = 0; i < M; ++i) U[i] = src[i * 32 + lane];
   } else if (active && p.probes != nullptr && p.t0 == 1) {
@@ -690,8 +694,7 @@ static int launch_march_t(const MarchParams &mp, cudaStream_t st) {
   const size_t smem = 2 * mp.slice_bytes + 2 * (size_t)M * 33 * sizeof(cx) + 2 * sizeof(uint64_t);
   TP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = (mp.P + kMarchWarps - 1) / kMarchWarps;
-  kern<<<grid, kMarchWarps * 32, smem, st>>>(mp);
-  return check_cuda(cudaGetLastError(), "cn2d_march_kernel launch");
+  return check_cuda(launch_dependent(kern, dim3(grid), dim3(kMarchWarps * 32), smem, st, true, mp), "cn2d_march_kernel launch");
 }
 
 template <int M>
@@ -810,7 +813,10 @@ static int factor_slices(const tp_cn2d_op *op, const void *n_field, int32_t n_dt
   const int count = s_end - s_begin + 1;
   cn2d_diag_kernel<<<dim3(pt.C * pt.M / 32, (count + 31) / 32), dim3(32, 8), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       f, count);
-  cn2d_factor_kernel<<<s_end - s_begin + 1, pt.C, smem, reinterpret_cast<cudaStream_t>(stream)>>>(f);
+  // this kernel and the march after it start early (pdl_wait): N = 256, 127 slices, 32
+  // probes 100 -> 93 us for the factorisation, march and far field
+  TP_CHECK_CUDA(launch_dependent(cn2d_factor_kernel, dim3(s_end - s_begin + 1), dim3(pt.C), smem,
+                                 reinterpret_cast<cudaStream_t>(stream), true, f));
   return check_cuda(cudaGetLastError(), "cn2d_factor_kernel launch");
 }
 
@@ -888,15 +894,17 @@ extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp
   if (mp.flip_out && (mp.t0 != 1 || mp.t1 != mp.L) && a->u_store != nullptr)
     return set_error(TP_ERR_INVALID, "the flipped ADJOINT store needs the full step range");
   mp.state_in = static_cast<const cx *>(a->state_in);
+  mp.state_stride = (size_t)(a->store_sums >> 8 > 0 ? a->store_sums >> 8 : 1) * mp.Npad;
   mp.state_out = static_cast<cx *>(a->state_out);
   mp.store_slices = a->store_slices > 0 ? a->store_slices : op->nz;
   mp.store_every = a->store_every;
   mp.store_base = a->store_base;
   mp.ufwd_slices = a->ufwd_slices > 0 ? a->ufwd_slices : op->nz;
   mp.ufwd_base = a->ufwd_base;
-  mp.store_sums = a->store_sums;
-  if (a->store_sums != 0) {
-    if (a->store_sums != 1) return set_error(TP_ERR_INVALID, "store_sums=%d (0 or 1)", a->store_sums);
+  if (a->store_sums < 0 || (a->store_sums & 0xfe) != 0 || (a->store_sums > 1 && a->state_in == nullptr))
+    return set_error(TP_ERR_INVALID, "store_sums=%d (0 or 1, and state_in's slices from bit 8)", a->store_sums);
+  mp.store_sums = a->store_sums & 1;
+  if (mp.store_sums) {
     if (a->mode != TP_MODE_FORWARD && a->mode != TP_MODE_ADJOINT_EXACT)
       return set_error(TP_ERR_INVALID, "store_sums needs mode FORWARD or ADJOINT_EXACT");
     if (a->mode == TP_MODE_FORWARD && a->store_every > 1)

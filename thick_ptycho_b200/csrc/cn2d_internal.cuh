@@ -100,7 +100,8 @@ struct MarchParams {
   const unsigned *poly_bad;     // direct kernel of the 32-chunk layout: 0 = the polynomial kernel runs instead
   int *err;
   int t0, t1;                   // step range
-  const cx *state_in;           // chunked (P, Npad) or null
+  const cx *state_in;           // chunked (P, Npad) or null, probes state_stride apart
+  size_t state_stride;
   cx *state_out;
   int store_slices, store_every, store_base;
   int ufwd_slices, ufwd_base;

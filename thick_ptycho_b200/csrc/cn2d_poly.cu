@@ -67,7 +67,6 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
   constexpr int HL = kHaloRows / R, USE = (32 - 2 * HL) * R;  // halo lanes, rows a warp owns
   constexpr int EX = HL * R;
   const MarchParams &p = q.p;
-  if (*q.bad != 0u) return;  // the direct kernel runs this march
   extern __shared__ __align__(16) float2 ex[];  // [2][nwarps][2][EX]
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const int g0 = w * USE + (lane - HL) * R;  // first row of this lane
@@ -91,6 +90,9 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
   }
   if (lane == 0) wl[0] = 0.f;  // beyond the halo
   if (lane == 31) wr[R - 1] = 0.f;
+  pdl_trigger();
+  pdl_wait();
+  if (*q.bad != 0u) return;  // the direct kernel runs this march
 
   auto slice_of = [&](int t) { return p.backward ? (p.L + 1 - t) : t; };
   auto diag = [&](int t, float2(&d)[R]) {
@@ -104,7 +106,7 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
   for (int i = 0; i < R; ++i) {
     u[i] = f1[i] = f0[i] = zero;
     if (!((in >> i) & 1u)) continue;
-    if (p.state_in != nullptr) u[i] = p.state_in[probe * p.Npad + off[i]];
+    if (p.state_in != nullptr) u[i] = p.state_in[probe * p.state_stride + off[i]];
     else if (p.probes != nullptr && p.t0 == 1) u[i] = p.probes[probe * p.N + g0 + i];
   }
   auto store = [&](float2 *dst, const float2(&v)[R]) {
@@ -259,8 +261,7 @@ int launch(const Poly2DParams &q, cudaStream_t st) {
   constexpr int HL = kHaloRows / R;
   const size_t smem = (size_t)4 * q.nwarps * HL * R * sizeof(float2);
   auto kern = q.m == 6 ? cn2d_poly_kernel<R, 6, LAGGED, MAXT, MINB> : cn2d_poly_kernel<R, 0, LAGGED, MAXT, MINB>;
-  kern<<<q.p.P, 32 * q.nwarps, smem, st>>>(q);
-  return check_cuda(cudaGetLastError(), "cn2d_poly_kernel launch");
+  return check_cuda(launch_dependent(kern, dim3(q.p.P), dim3(32 * q.nwarps), smem, st, true, q), "cn2d_poly_kernel launch");
 }
 
 std::complex<double> chebyshev(int m, std::complex<double> w) {

@@ -390,7 +390,6 @@ __global__ void __launch_bounds__(kTeamThreads *TM, 1) cn2d_team_kernel(const Ma
   const bool do_grad = LAGGED && (p.grad_c != nullptr);
   const size_t ssf = ss / sizeof(cx);
   const int p0 = (blockIdx.x * TM + team) * Q;
-  const bool pcr = p.coupling == nullptr || __uint_as_float(__ldg(p.coupling)) >= kPcrSkipBound;
 
   if (tid == 0) {
     mbar_init(&mbar[0], 1);
@@ -399,6 +398,12 @@ __global__ void __launch_bounds__(kTeamThreads *TM, 1) cn2d_team_kernel(const Ma
     for (int m = 0; m < TM; ++m) mbar_init(&gbar[m], 1);
     fence_mbar_init();
   }
+  // The marches of a checkpointed gradient follow one another in short launches: the
+  // next one's CTAs start as this one's leave (nothing above reads device memory).  1024 x
+  // 512, 256 probes, sqrt checkpoints, with the restart states read in place: 2213 -> 2045 us.
+  pdl_trigger();
+  pdl_wait();
+  const bool pcr = p.coupling == nullptr || __uint_as_float(__ldg(p.coupling)) >= kPcrSkipBound;
   __syncthreads();
   auto slice_of = [&](int t) { return p.backward ? (p.L + 1 - t) : t; };
   if (tid == 0)
@@ -411,7 +416,7 @@ __global__ void __launch_bounds__(kTeamThreads *TM, 1) cn2d_team_kernel(const Ma
     for (int i = 0; i < M; ++i) U[q][i] = czero();
     if (p0 + q >= p.P) continue;
     if (p.state_in != nullptr) {
-      const cx2 *src = reinterpret_cast<const cx2 *>(p.state_in + (size_t)(p0 + q) * p.Npad) + c;
+      const cx2 *src = reinterpret_cast<const cx2 *>(p.state_in + (size_t)(p0 + q) * p.state_stride) + c;
 #pragma unroll
       for (int j = 0; j < M / 2; ++j) {
         const cx2 v = src[j * C];
@@ -684,8 +689,8 @@ static int launch_team_t(const Partition &pt, MarchParams &mp, cudaStream_t st) 
   const size_t smem = team_smem_bytes(pt, mp.trunc, Q, TM, QD, STG);
   TP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = (mp.P + Q * TM - 1) / (Q * TM);
-  kern<<<grid, kTeamThreads * TM, smem, st>>>(mp);
-  return check_cuda(cudaGetLastError(), "cn2d_team_kernel launch");
+  return check_cuda(launch_dependent(kern, dim3(grid), dim3(kTeamThreads * TM), smem, st, true, mp),
+                    "cn2d_team_kernel launch");
 }
 
 template <int M, bool LAGGED, bool SUMS, int TS, bool STG>

@@ -210,14 +210,12 @@ class PWEGradient2D:
             ck = self._bufs["ckpt"]
             seg = self._buf("segment", P, S + 1)
             state = [self._buf("state0", P, 1)[:, 0], self._buf("state1", P, 1)[:, 0]]
-            start = self._buf("start", P, 1)[:, 0]
             nseg = -(-L // S)
             first = True
             for k in reversed(range(nseg)):
                 a, b = k * S, min(k * S + S, L)
-                start.copy_(ck[:, a // S])
                 # recompute u_a .. u_b of this segment (indices 0 .. b - a)
-                e.march(self._fs_fwd, P, t_begin=a + 1, t_end=b, state_in=start, u_store=seg, store_base=a,
+                e.march(self._fs_fwd, P, t_begin=a + 1, t_end=b, state_from=(ck, a // S), u_store=seg, store_base=a,
                         store_sums=self.sums)
                 # adjoint steps for slices b .. a+1 (step t = L + 1 - s)
                 e.march(fa, P, t_begin=L + 1 - b, t_end=L - a, src_exit=src if first else None,
