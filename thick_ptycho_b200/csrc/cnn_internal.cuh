@@ -22,17 +22,6 @@ constexpr int kConvTile = 128 * kConvBlocks;   // output pixels per CTA
 constexpr int kConvCout = 32;                  // output channels of every layer
 constexpr int kFilterTaps = 13;                // taps of the learned per-pixel filter
 
-// Offsets (row, column) of the filter taps: the centre, the 8 neighbours and
-// the 4 axial pixels at distance 2.
-__host__ __device__ inline int filter_tap_dy(int t) {
-  const int v[kFilterTaps] = {0, 0, 0, -1, 1, -1, -1, 1, 1, 0, 0, -2, 2};
-  return v[t];
-}
-__host__ __device__ inline int filter_tap_dx(int t) {
-  const int v[kFilterTaps] = {0, -1, 1, 0, 0, -1, 1, -1, 1, -2, 2, 0, 0};
-  return v[t];
-}
-
 struct ConvGeom {
   int H, W, Wp, batch;
   long long S;        // pixels of one padded image, (H + 2) * Wp
