@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kMs3Threads) ms3_mix_cols_kernel(const Ms3Para
 // once per transform.  The psi buffer holds X_z = psi_z T_z here (psi_{z+1} = X_z +
 // update needs no T_z).  Stockham passes in shared memory were bound by it
 // (73-83 % of its throughput); a slice of 64 probes of 256 x 256 took 95 us with them
-// (adjoint 99) and takes 42 us (51) with these.
+// (adjoint 99) and takes 43 us (48) with these.
 template <int R1, int R2, int PHASE>
 __global__ void __launch_bounds__(256, 2) ms3_rows4_kernel(const Ms3Params q, const float2 *__restrict__ twg, int z) {
   constexpr int N = R1 * R2, RPC = 256 / R1, S = R1 * (R2 + 1);
@@ -297,9 +297,14 @@ __global__ void __launch_bounds__(256, 2) ms3_rows4_kernel(const Ms3Params q, co
       }
     }
   } else {
-    if (inA) {  // what no kernel of the march writes, before the column pass is complete
-      const float2 *T = q.trans + (size_t)(PHASE == kMs3FwdStep ? (last ? z : z + 1) : z) * q.N;
-      const float2 *u = PHASE == kMs3BwdStep ? q.u_fwd + ((size_t)pr * q.nz + z) * q.N : nullptr;
+    // The adjoint's third and fourth operands at 192 and 256 wait until the field is in x:
+    // held from the start they spilled (64 probes, 256 x 256: 51.5 -> 47.4 us per slice, 192 x
+    // 192: 33.6 -> 31.2;
+    // 128 x 128 is faster with them early, 16.1 against 16.4).
+    constexpr bool LATE = PHASE == kMs3BwdStep && R2 > 8;
+    const float2 *T = q.trans + (size_t)(PHASE == kMs3FwdStep ? (last ? z : z + 1) : z) * q.N;
+    const float2 *u = PHASE == kMs3BwdStep ? q.u_fwd + ((size_t)pr * q.nz + z) * q.N : nullptr;
+    if (inA && !LATE) {  // what no kernel of the march writes, before the column pass is complete
 #pragma unroll
       for (int j = 0; j < R1; ++j) {
         tz[j] = T[ga + R2 * j];
@@ -309,26 +314,37 @@ __global__ void __launch_bounds__(256, 2) ms3_rows4_kernel(const Ms3Params q, co
     pdl_wait();
 #pragma unroll
     for (int k2 = 0; k2 < R2; ++k2) x[k2] = wrow[R1 * k2];
-    if (inA) {
+    auto load_psi = [&]() {
 #pragma unroll
       for (int j = 0; j < R1; ++j) pz[j] = q.psi[pbase + ga + R2 * j];
-    }
+    };
+    if (inA && !LATE) load_psi();
     dft_reg<R2>(x, 1.f);
     __syncthreads();  // the twiddles are in place
 #pragma unroll
     for (int m = 0; m < R2; ++m)
       buf[rc * S + k1 * (R2 + 1) + m] = m ? cmulc(x[m], tw[k1 * (R2 + 1) + m]) : x[0];
+    if (inA && LATE) load_psi();
     __syncthreads();
     if (inA) {
 #pragma unroll
       for (int k = 0; k < R1; ++k) x[k] = buf[ra * S + k * (R2 + 1) + n2];
       dft_reg<R1>(x, 1.f);
+#pragma unroll
+      for (int j = 0; j < R1; ++j) x[j] = cadd(pz[j], x[j]);
+      if (LATE) {
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+          tz[j] = T[ga + R2 * j];
+          uz[j] = __ldcs(&u[ga + R2 * j]);
+        }
+      }
       if (PHASE == kMs3FwdStep) {
         // psi_{z+1} = X_z + IFFT2((H-1) FFT2 X_z), X_{z+1} = psi_{z+1} T_{z+1}
         float2 *us = q.u_store ? q.u_store + ((size_t)pr * q.nz + z + 1) * q.N + ga : nullptr;
 #pragma unroll
         for (int j = 0; j < R1; ++j) {
-          const float2 v = cadd(pz[j], x[j]);
+          const float2 v = x[j];
           if (us) __stcs(&us[R2 * j], v);
           if (last) {
             if (q.exit_out) q.exit_out[pbase + ga + R2 * j] = v;
@@ -343,7 +359,7 @@ __global__ void __launch_bounds__(256, 2) ms3_rows4_kernel(const Ms3Params q, co
         float2 *gt = q.grad_t + (size_t)z * q.N + ga;
 #pragma unroll
         for (int j = 0; j < R1; ++j) {
-          const float2 gv = cadd(pz[j], x[j]);
+          const float2 gv = x[j];
           red_add_cx(gt + R2 * j, cmulc(gv, cfma(tz[j], uz[j], uz[j])));
           x[j] = cadd(gv, cmulc(gv, tz[j]));
           if (z > 0) q.psi[pbase + ga + R2 * j] = x[j];
