@@ -555,14 +555,15 @@ __global__ void __launch_bounds__(kMarchWarps * 32, 1) cn2d_march_kernel(const M
 // Layout and gradient helpers
 // --------------------------------------------------------------------------
 // Chunked (P, nz, Npad) -> natural (P, N, nz): both sides are read and written in
-// runs along their own fast index through a tile of 32 offsets x 32 slices (element
-// by element, one side is a gather: 1201 x 600 x 100: 384 -> 317 us).
-// Grid (Npad / 32, ceil(nz / 32), P), block (32, 8).
+// runs along their own fast index through a tile of 32 offsets x 64 slices (1201 x 600
+// x 100: 384 us element by element, one side a gather; 311 with 32 slices, 265 with 64,
+// eight loads in flight per thread and 512-byte runs, 309 with 128 and fewer CTAs per
+// SM; the bytes alone take 179).  Grid (Npad / 32, ceil(nz / 64), P), block (32, 8).
 __global__ void __launch_bounds__(256) cn2d_unchunk_kernel(const cx *__restrict__ st, cx *__restrict__ out, int N, int nz,
                                                            int M, int C, int pair) {
-  __shared__ cx tile[32][33];
+  __shared__ cx tile[64][33];
   const int Npad = C * M;
-  const int e0 = blockIdx.x * 32, t0 = blockIdx.y * 32;
+  const int e0 = blockIdx.x * 32, t0 = blockIdx.y * 64;
   const size_t pr = blockIdx.z;
   const auto row_of = [&](int e) {  // offset e holds row k M + i
     if (pair) return ((e >> 1) % C) * M + 2 * ((e >> 1) / C) + (e & 1);
@@ -570,14 +571,17 @@ __global__ void __launch_bounds__(256) cn2d_unchunk_kernel(const cx *__restrict_
   };
   const int gx = row_of(e0 + threadIdx.x);
 #pragma unroll
-  for (int r = threadIdx.y; r < 32; r += 8)
+  for (int r = threadIdx.y; r < 64; r += 8)
     if (t0 + r < nz && gx < N) tile[r][threadIdx.x] = st[(pr * nz + t0 + r) * Npad + e0 + threadIdx.x];
   __syncthreads();
-  const int t = t0 + threadIdx.x;
-  if (t >= nz) return;
+#pragma unroll
   for (int r = threadIdx.y; r < 32; r += 8) {
     const int g = row_of(e0 + r);
-    if (g < N) out[(pr * N + g) * nz + t] = tile[threadIdx.x][r];
+    if (g >= N) continue;
+    cx *dst = out + (pr * N + g) * nz + t0;
+#pragma unroll
+    for (int t = threadIdx.x; t < 64; t += 32)
+      if (t0 + t < nz) dst[t] = tile[t][r];
   }
 }
 
@@ -958,7 +962,7 @@ extern "C" int tp_cn2d_unchunk(const tp_cn2d_op *op, int32_t num_probes, const v
   cx *dst = static_cast<cx *>(u_out);
   for (int p0 = 0; p0 < num_probes; p0 += 65535) {
     const int count = num_probes - p0 < 65535 ? num_probes - p0 : 65535;
-    cn2d_unchunk_kernel<<<dim3(pt.C * pt.M / 32, (op->nz + 31) / 32, count), dim3(32, 8), 0,
+    cn2d_unchunk_kernel<<<dim3(pt.C * pt.M / 32, (op->nz + 63) / 64, count), dim3(32, 8), 0,
                           reinterpret_cast<cudaStream_t>(stream)>>>(
         src + (size_t)p0 * op->nz * pt.C * pt.M, dst + (size_t)p0 * op->nz * op->n, op->n, op->nz, pt.M, pt.C, pt.team);
   }
