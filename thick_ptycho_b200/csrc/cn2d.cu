@@ -40,6 +40,8 @@
 #include <cuda_runtime.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #include "cn2d_internal.cuh"
 #include "tp_common.cuh"
 #include "tp_errors.h"
@@ -942,6 +944,19 @@ extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp
   const Poly2DPlan plan = direct ? Poly2DPlan{} : poly2d_plan(op);
   if (plan.m > 0) {
     mp.poly_bad = mp.coupling + 1;
+    if (mp.grad_c != nullptr && (mp.t0 != 1 || mp.t1 != mp.L)) {
+      // A partial march may run while later ranges are factorised on another stream and
+      // raise the verdict between the two kernels; the one that adds to a gradient must
+      // run once, so both read a copy.  (Everything else they write is the same from
+      // either, and a march of all slices follows the whole factorisation.)  The copies
+      // take turns in the rest of the tail.
+      static std::atomic<unsigned> turn{0};
+      constexpr unsigned kWords = kFactorTailBytes / sizeof(unsigned) - 2;
+      unsigned *copy = const_cast<unsigned *>(mp.coupling) + 2 + turn.fetch_add(1, std::memory_order_relaxed) % kWords;
+      TP_CHECK_CUDA(cudaMemcpyAsync(copy, mp.poly_bad, sizeof(unsigned), cudaMemcpyDeviceToDevice,
+                                    reinterpret_cast<cudaStream_t>(stream)));
+      mp.poly_bad = copy;
+    }
     rc = launch_poly_march(pt, mp, plan, mp.poly_bad, lagged, reinterpret_cast<cudaStream_t>(stream));
     if (rc) return rc;
   }

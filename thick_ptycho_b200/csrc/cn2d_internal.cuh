@@ -34,7 +34,8 @@ __host__ __device__ inline int rec_rde(int levels) { return 2 + 2 * levels; }
 // each) then the records ([nrec][C]), padded to 256 bytes.  The workspace of a
 // factorisation holds L slices and then kFactorTailBytes: the largest PCR
 // coefficient of all slices (float bits), which the team march reads, and a word
-// that is non-zero when a row is outside the polynomial march's bounds.
+// that is non-zero when a row is outside the polynomial march's bounds; the rest holds
+// the copies of that word that partial gradient marches decide by.
 __host__ __device__ inline size_t slice_bytes(const Partition &pt) {
   size_t b = (size_t)(5 * pt.M + pt.nrec) * pt.C * sizeof(cx);
   return (b + 255) & ~size_t(255);
