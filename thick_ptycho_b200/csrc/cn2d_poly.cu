@@ -109,6 +109,10 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
     if (p.state_in != nullptr) u[i] = p.state_in[probe * p.state_stride + off[i]];
     else if (p.probes != nullptr && p.t0 == 1) u[i] = p.probes[probe * p.N + g0 + i];
   }
+  // The halo rows belong to neighbouring warps, whose outputs may replace the inputs
+  // (state_out or exit_out on state_in, probes or a source): every warp has read before
+  // one writes.  A march of several steps has the halos' barriers in between.
+  __syncthreads();
   auto store = [&](float2 *dst, const float2(&v)[R]) {
 #pragma unroll
     for (int i = 0; i < R; ++i)
@@ -195,6 +199,10 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
 #pragma unroll 1
       for (int k = q.m - 2; k >= 0; k -= 2) pair(k);
     }
+    // the last step's outputs, the same for its sources
+    auto sources_read = [&]() {
+      if (sources && t == p.t1) __syncthreads();
+    };
     float2 *dst = nullptr;
     if (p.u_store != nullptr && store_index(p, t) >= 0)
       dst = p.u_store + (probe * p.store_slices + store_index(p, t)) * p.Npad;
@@ -202,6 +210,7 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
       float2 lam[R];
 #pragma unroll
       for (int i = 0; i < R; ++i) lam[i] = cadd(u[i], e[i]);
+      sources_read();
       if (dst) store(dst, lam);
       if (t == p.L && p.exit_out != nullptr) {
 #pragma unroll
@@ -221,6 +230,7 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
     for (int i = 0; i < R; ++i) u[i] = caxpy(2.f, e[i], u[i]);
     if constexpr (!LAGGED) {
       if (sources) add_sources(t, 0.5f, u);
+      sources_read();
       if (dst) store(dst, u);
       if (t == p.L && p.exit_out != nullptr) {
 #pragma unroll
