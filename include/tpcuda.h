@@ -111,7 +111,11 @@ typedef struct tp_cn2d_march_args {
                                 chunked layout of tp_cn2d_layout; the caller
                                 zeroes it; row s-1 holds slice s               */
   /* Partial marches (checkpointed gradients).  All zero = one march over all
-   * L steps storing every slice at its own index. */
+   * L steps storing every slice at its own index.  A march reads the factor set
+   * and does not write it: several streams may march one set, and slices that a
+   * march does not read may be factorised meanwhile.  state_out may be state_in,
+   * and exit_out the probes or a source of the last step (each probe's inputs are
+   * read before its outputs replace them). */
   int32_t t_begin, t_end;    /* step range [t_begin, t_end], 1-based; 0 = 1 / L */
   const void *state_in;      /* float2 (P, Npad) chunked state before t_begin
                                 (overrides probes), or NULL                   */

@@ -72,3 +72,83 @@ def test_2d_one_slice_exit_on_its_input(N, P):
                     eng.march(fs, P, exit_out=got[name].view(P, N), **got)
                     assert torch.equal(got[name].view(P, N), ref), (mode, sorted(kw), name)
     eng.device_status()
+
+
+# ------------------------------------------- which kernel a partial march runs
+def slice_size(eng):
+    return (eng.factor_bytes - 256) // eng.L
+
+
+def verdicts(eng, fs):
+    """The slices' verdict words (the first entry of the forward multipliers)."""
+    rows = fs.buf[: slice_size(eng) * eng.L].view(eng.L, -1)
+    return rows[:, eng.npad * 8:eng.npad * 8 + 4].contiguous().view(torch.float32)[:, 0]
+
+
+def set_verdict(eng, fs, s, value):
+    at = (s - 1) * slice_size(eng) + eng.npad * 8
+    fs.buf[at:at + 4] = torch.tensor([value], dtype=torch.float32).view(torch.uint8).cuda()
+
+
+@pytest.mark.parametrize("N", [97, 777])
+@pytest.mark.parametrize("mode", ["forward", "adjoint", "adjoint_exact"])
+def test_2d_partial_march_decides_by_its_own_slices(N, mode):
+    """A slice outside the polynomial's bounds (here by its verdict, set from the host)
+    sends the marches that read it, and only those, to the direct kernel, in place as well,
+    and no march writes the factor set."""
+    rng = np.random.default_rng(N + 2)
+    nz, P = 13, 4
+    L = nz - 1
+    eng = CN2D(N, nz, K, 1.0, 1.0, "impedance")
+    fs = eng.factor(index(rng, N, nz), mode)
+    assert verdicts(eng, fs).tolist() == [0.0] * L
+    start = torch.zeros((P, eng.npad), dtype=torch.complex64, device="cuda")
+    eng.march(fs, P, probes=None if mode == "adjoint_exact" else cplx(rng, P, N),
+              src_exit=cplx(rng, P, N) if mode == "adjoint_exact" else None, t_begin=1, t_end=4, state_out=start)
+    grad = mode == "adjoint_exact"
+    fwd = eng.new_store(P).copy_(cplx(rng, P, nz, eng.npad)) if grad else None
+
+    def part():
+        """Steps 5..8 in place; the state and the gradient of four probes."""
+        before = fs.buf.clone()
+        state = start.clone()
+        gc = eng.new_grad_buffer() if grad else None
+        eng.march(fs, P, t_begin=5, t_end=8, state_in=state, state_out=state, u_fwd=fwd, grad_c=gc)
+        assert torch.equal(fs.buf, before)
+        return [state] + ([torch.view_as_real(gc)] if grad else [])
+
+    slices = range(5, 9) if mode == "forward" else range(L + 1 - 8, L + 1 - 4)
+    poly = part()
+    for s in range(1, L + 1):
+        set_verdict(eng, fs, s, 1.0)
+    direct = part()
+    assert not torch.equal(poly[0], direct[0])
+    scale = max(float(direct[0].abs().max()), 1.0)
+    assert float((poly[0] - direct[0]).abs().max()) < 1e-5 * scale
+    for s in range(1, L + 1):
+        set_verdict(eng, fs, s, 0.0)
+    for s in range(1, L + 1):
+        set_verdict(eng, fs, s, 1.0)
+        got, want = part(), (direct if s in slices else poly)
+        assert torch.equal(got[0], want[0]), s
+        if grad:  # sums over probes in any order
+            assert float((got[1] - want[1]).abs().max()) < 1e-5 * float(want[1].abs().max())
+        set_verdict(eng, fs, s, 0.0)
+    eng.device_status()
+
+
+def test_2d_verdicts_follow_the_factorised_slices():
+    rng = np.random.default_rng(7)
+    N, nz = 241, 40
+    eng = CN2D(N, nz, K, 1.0, 1.0, "impedance")
+    weak = index(rng, N, nz)
+    strong = weak.clone()
+    strong[100, 20] += 1.5  # nodes 20: slices 20 and 21
+    fs = eng.factor(strong, "forward")
+    assert [s + 1 for s, v in enumerate(verdicts(eng, fs).tolist()) if v] == [20, 21]
+    eng.factor_range(weak, "forward", 10, 30, out=fs.buf)
+    assert not verdicts(eng, fs).any()
+    for bad in (float("nan"), float("inf")):
+        strong[100, 20] = bad
+        eng.factor_range(strong, "forward", 15, 25, out=fs.buf)
+        assert [s + 1 for s, v in enumerate(verdicts(eng, fs).tolist()) if v] == [20, 21]

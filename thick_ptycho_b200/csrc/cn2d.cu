@@ -28,7 +28,8 @@
 // right-hand-side work.  Data layout of one slice of the factor set (cx
 // [rows][32 lanes], row i of lane k is matrix row k*M + i):
 //   QD  [M][32]  diagonal of P_s
-//   LF  [M][32]  interior forward multipliers (row 0 unused)
+//   LF  [M][32]  interior forward multipliers (none in row 0, whose first entry is
+//                the slice's verdict, cn2d_internal.cuh)
 //   EP  [M][32]  interior inverse pivots minus one
 //   V   [M][32]  spike: response of the interior to the left separator
 //   W   [M][32]  spike: response of the interior to the own separator
@@ -39,8 +40,6 @@
 
 #include <cuda_runtime.h>
 #include <stdio.h>
-
-#include <atomic>
 
 #include "cn2d_internal.cuh"
 #include "tp_common.cuh"
@@ -158,21 +157,10 @@ __global__ void __launch_bounds__(256) cn2d_diag_kernel(const FactorParams f, in
   pdl_trigger();
   const int e0 = blockIdx.x * 32, i = e0 / f.C, c0 = e0 % f.C;
   const int s0 = blockIdx.y * 32;
-  bool bad = false;
   for (int r = threadIdx.y; r < 32; r += 8) {
     const int s = s0 + threadIdx.x, g = (c0 + r) * f.M + i;
-    if (s >= count) continue;
-    const double2 pd = p_diag(f, g, f.sl0 + s);
-    tile[r][threadIdx.x] = pd;
-    if (f.poly_bad != nullptr && g < f.N) {  // the polynomial march's bounds on this row
-      // (K's own row also for the transposed modes: the spectra are conjugate)
-      const float sum = (float)((g > 0 ? fabs(k_sub(f, g).y) : 0.0) + (g < f.N - 1 ? fabs(k_sup(f, g).y) : 0.0));
-      const float dr = (float)(1.0 - pd.x), di = (float)-pd.y, d2 = dr * dr + di * di;
-      if (!(d2 > 1e-4f && d2 < 1e8f)) bad = true;
-      if (sum > 0.f && !(sum * sum <= f.tau_max * f.tau_max * d2 && fabsf(atan2f(di, dr)) <= f.arg_max)) bad = true;
-    }
+    if (s < count) tile[r][threadIdx.x] = p_diag(f, g, f.sl0 + s);
   }
-  if (bad) atomicOr(f.poly_bad, 1u);
   __syncthreads();
   for (int r = threadIdx.y; r < 32; r += 8) {
     const int s = s0 + r;
@@ -181,6 +169,16 @@ __global__ void __launch_bounds__(256) cn2d_diag_kernel(const FactorParams f, in
                                                (size_t)3 * f.M * f.C * sizeof(cx));
     dst[e0 + threadIdx.x] = tile[threadIdx.x][r];
   }
+}
+
+// Whether row g, with D's entry md, is within the polynomial march's bounds (K's own row
+// also for the transposed modes: the spectra are conjugate); |arg md| <= its bound, below
+// pi / 2, by the tangent.
+__device__ __forceinline__ bool poly_row(const FactorParams &f, int g, double2 md) {
+  const float sum = (float)((g > 0 ? fabs(k_sub(f, g).y) : 0.0) + (g < f.N - 1 ? fabs(k_sup(f, g).y) : 0.0));
+  const float dr = (float)md.x, di = (float)md.y, d2 = dr * dr + di * di;
+  if (!(d2 > 1e-4f && d2 < 1e8f)) return false;
+  return !(sum > 0.f) || (sum * sum <= f.tau_max * f.tau_max * d2 && fabsf(di) <= f.tan_max * dr);
 }
 
 // One block of C threads per slice, one thread per chunk; the slice's diagonal
@@ -203,6 +201,7 @@ __global__ void __launch_bounds__(128) cn2d_factor_kernel(const FactorParams f) 
   const int g0 = c * M;
   double2 ip_prev = z2(1, 0), msup_prev = z2(0, 0), fvv = z2(0, 0);
   double2 me_a = z2(0, 0), me_d = z2(1, 0), me_c = z2(0, 0);
+  bool outside = !(f.tau_max > 0.f);
   constexpr int AHEAD = 4;
   double2 next[AHEAD];
 #pragma unroll
@@ -222,6 +221,7 @@ __global__ void __launch_bounds__(128) cn2d_factor_kernel(const FactorParams f) 
       const double2 pd = cur[j];
       QD[i * C + c] = to_cx(pd);
       const double2 md = z2(1.0 - pd.x, -pd.y);
+      if (f.tau_max > 0.f && g < f.N && !poly_row(f, g, md)) outside = true;
       const double2 msub = zneg(p_sub(f, g));
       const double2 msup = zneg(p_sup(f, g));
       if (i < M - 1) {
@@ -252,7 +252,10 @@ __global__ void __launch_bounds__(128) cn2d_factor_kernel(const FactorParams f) 
       }
     }
   }
-  __syncthreads();  // every chunk's diagonal has been read: V and W may be written
+  outside = __syncthreads_or(outside) != 0;  // every chunk's diagonal has been read: V and W may be written
+#ifndef TP_C128_CHECK
+  if (C == 32 && c == 0) LF[0] = mkcx(outside ? 1.f : 0.f, 0.f);
+#endif
   V[(M - 1) * C + c] = czero();
   W[(M - 1) * C + c] = czero();
   double2 v_last, w_last, v_first, w_first;
@@ -423,7 +426,7 @@ __device__ __forceinline__ void add_natural(cx (&U)[M], const cx *__restrict__ s
 template <int M, bool ALIGNED, bool LAGGED>
 __global__ void __launch_bounds__(kMarchWarps * 32, 1) cn2d_march_kernel(const MarchParams p) {
   pdl_wait();
-  if (p.poly_bad != nullptr && *p.poly_bad == 0u) return;  // the polynomial kernel ran this march
+  if (p.poly && !poly_excluded(p)) return;  // the polynomial kernel ran this march
   extern __shared__ __align__(128) unsigned char smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int probe = blockIdx.x * kMarchWarps + warp;
@@ -801,9 +804,8 @@ static int factor_slices(const tp_cn2d_op *op, const void *n_field, int32_t n_dt
   if (!pt.team) {
     const Poly2DPlan plan = poly2d_plan(op);
     if (plan.m > 0) {
-      f.poly_bad = f.coupling + 1;
       f.tau_max = plan.tau_max;
-      f.arg_max = plan.arg_max;
+      f.tan_max = tanf(plan.arg_max);
     }
   }
 #endif
@@ -811,10 +813,10 @@ static int factor_slices(const tp_cn2d_op *op, const void *n_field, int32_t n_dt
   if (s_begin < 1 || s_end > f.L || s_begin > s_end)
     return set_error(TP_ERR_INVALID, "slice range [%d, %d] outside [1, %d]", s_begin, s_end, f.L);
   f.sl0 = s_begin - 1;
-  // the PCR coupling bound (and the word after it) is a running maximum over the slices factorised
+  // the PCR coupling bound is a running maximum over the slices factorised
   // since the last reset, which the range starting at slice 1 performs
   if (s_begin == 1)
-    TP_CHECK_CUDA(cudaMemsetAsync(f.coupling, 0, 2 * sizeof(unsigned), reinterpret_cast<cudaStream_t>(stream)));
+    TP_CHECK_CUDA(cudaMemsetAsync(f.coupling, 0, sizeof(unsigned), reinterpret_cast<cudaStream_t>(stream)));
   const size_t smem = 5 * (size_t)pt.C * sizeof(double2);
   const int count = s_end - s_begin + 1;
   cn2d_diag_kernel<<<dim3(pt.C * pt.M / 32, (count + 31) / 32), dim3(32, 8), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
@@ -943,21 +945,8 @@ extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp
   const bool direct = mp.P > 2 * sms && mp.grad_c == nullptr && (pt.M <= 32 || lagged);
   const Poly2DPlan plan = direct ? Poly2DPlan{} : poly2d_plan(op);
   if (plan.m > 0) {
-    mp.poly_bad = mp.coupling + 1;
-    if (mp.grad_c != nullptr && (mp.t0 != 1 || mp.t1 != mp.L)) {
-      // A partial march may run while later ranges are factorised on another stream and
-      // raise the verdict between the two kernels; the one that adds to a gradient must
-      // run once, so both read a copy.  (Everything else they write is the same from
-      // either, and a march of all slices follows the whole factorisation.)  The copies
-      // take turns in the rest of the tail.
-      static std::atomic<unsigned> turn{0};
-      constexpr unsigned kWords = kFactorTailBytes / sizeof(unsigned) - 2;
-      unsigned *copy = const_cast<unsigned *>(mp.coupling) + 2 + turn.fetch_add(1, std::memory_order_relaxed) % kWords;
-      TP_CHECK_CUDA(cudaMemcpyAsync(copy, mp.poly_bad, sizeof(unsigned), cudaMemcpyDeviceToDevice,
-                                    reinterpret_cast<cudaStream_t>(stream)));
-      mp.poly_bad = copy;
-    }
-    rc = launch_poly_march(pt, mp, plan, mp.poly_bad, lagged, reinterpret_cast<cudaStream_t>(stream));
+    mp.poly = 1;
+    rc = launch_poly_march(pt, mp, plan, lagged, reinterpret_cast<cudaStream_t>(stream));
     if (rc) return rc;
   }
 #endif

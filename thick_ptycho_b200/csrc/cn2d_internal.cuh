@@ -33,9 +33,9 @@ __host__ __device__ inline int rec_rde(int levels) { return 2 + 2 * levels; }
 // Global factor set of one slice: QD, LF, EP, V, W ([M][C] complex values
 // each) then the records ([nrec][C]), padded to 256 bytes.  The workspace of a
 // factorisation holds L slices and then kFactorTailBytes: the largest PCR
-// coefficient of all slices (float bits), which the team march reads, and a word
-// that is non-zero when a row is outside the polynomial march's bounds; the rest holds
-// the copies of that word that partial gradient marches decide by.
+// coefficient of all slices (float bits), which the team march reads.  In the 32-chunk
+// layout LF's first entry (its row 0 is not a multiplier) is the slice's verdict: non-zero
+// when one of its rows is outside the polynomial march's bounds.
 __host__ __device__ inline size_t slice_bytes(const Partition &pt) {
   size_t b = (size_t)(5 * pt.M + pt.nrec) * pt.C * sizeof(cx);
   return (b + 255) & ~size_t(255);
@@ -73,8 +73,7 @@ struct FactorParams {
   char *factors;
   size_t slice_bytes;
   unsigned *coupling;  // max |alpha|, |gamma| of the PCR records (float bits), atomically maxed
-  unsigned *poly_bad;  // set where a row exceeds the bounds below (the word after `coupling`)
-  float tau_max, arg_max;
+  float tau_max, tan_max;  // the polynomial march's bounds on a row (0: no polynomial, every slice is outside)
   int *err;
 };
 
@@ -98,7 +97,7 @@ struct MarchParams {
   const cx *u_fwd;
   cx *grad_c;
   const unsigned *coupling;     // the factor set's PCR coupling bound (float bits), or NULL
-  const unsigned *poly_bad;     // direct kernel of the 32-chunk layout: 0 = the polynomial kernel runs instead
+  int poly;                     // direct kernel of the 32-chunk layout: the polynomial kernel runs instead where it may
   int *err;
   int t0, t1;                   // step range
   const cx *state_in;           // chunked (P, Npad) or null, probes state_stride apart
@@ -138,8 +137,20 @@ struct Poly2DPlan {
   float tau_max, arg_max;
 };
 Poly2DPlan poly2d_plan(const tp_cn2d_op *op);
-int launch_poly_march(const Partition &pt, const MarchParams &mp, const Poly2DPlan &plan, const unsigned *bad,
-                      bool lagged, cudaStream_t st);
+int launch_poly_march(const Partition &pt, const MarchParams &mp, const Poly2DPlan &plan, bool lagged, cudaStream_t st);
+
+// Whether a slice of this march is outside the polynomial march's bounds (the same for
+// every thread; a barrier of the CTA).  Both kernels of a march decide by the verdicts of
+// the slices it reads, which are factorised before it and stay: whatever is factorised
+// beside it, one of the two runs, and every CTA of it.
+__device__ __forceinline__ bool poly_excluded(const MarchParams &p) {
+  const int lo = p.backward ? p.L + 1 - p.t1 : p.t0, hi = p.backward ? p.L + 1 - p.t0 : p.t1;
+  const char *lf = p.factors + (size_t)p.Npad * sizeof(cx);
+  int bad = 0;
+  for (int s = lo + (int)threadIdx.x; s <= hi; s += (int)blockDim.x)
+    bad |= reinterpret_cast<const cx *>(lf + (size_t)(s - 1) * p.slice_bytes)->x != TP_R(0.0);
+  return __syncthreads_or(bad) != 0;
+}
 
 // Team-path launcher (cn2d_team.cu).
 int launch_team_march(const Partition &pt, MarchParams &mp, bool lagged, cudaStream_t st);

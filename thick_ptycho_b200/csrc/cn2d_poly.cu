@@ -23,9 +23,9 @@
 // against 4.18; exact adjoint with the gradient 2.4 against 31.4, whose sums went
 // through shared-memory float atomics).
 //
-// The factorisation checks every row and slice against the bounds the degree was
-// chosen for and leaves the verdict in the factor set's tail; this kernel and the
-// direct one (cn2d.cu) read it, and one of the two returns at once.
+// The factorisation checks every row of a slice against the bounds the degree was
+// chosen for and leaves the verdict in the slice; this kernel and the direct one
+// (cn2d.cu) read those of the march's slices, and one of the two returns at once.
 #include <math.h>
 
 #include <complex>
@@ -44,7 +44,6 @@ struct Poly2DParams {
   MarchParams p;
   int M, nwarps, m;  // rows per chunk, warps per probe, degree
   float a[kPoly2DMaxDeg];
-  const unsigned *bad;
 };
 
 // i/(1 - qd), qd the diagonal of P.
@@ -92,7 +91,6 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
   if (lane == 31) wr[R - 1] = 0.f;
   pdl_trigger();
   pdl_wait();
-  if (*q.bad != 0u) return;  // the direct kernel runs this march
 
   auto slice_of = [&](int t) { return p.backward ? (p.L + 1 - t) : t; };
   auto diag = [&](int t, float2(&d)[R]) {
@@ -109,10 +107,12 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
     if (p.state_in != nullptr) u[i] = p.state_in[probe * p.state_stride + off[i]];
     else if (p.probes != nullptr && p.t0 == 1) u[i] = p.probes[probe * p.N + g0 + i];
   }
+  diag(p.t0, qn);  // (on their way while the verdicts are read)
   // The halo rows belong to neighbouring warps, whose outputs may replace the inputs
   // (state_out or exit_out on state_in, probes or a source): every warp has read before
-  // one writes.  A march of several steps has the halos' barriers in between.
-  __syncthreads();
+  // one writes, by the barrier in here.  A march of several steps has the halos' barriers
+  // in between.
+  if (poly_excluded(p)) return;  // the direct kernel runs this march
   auto store = [&](float2 *dst, const float2(&v)[R]) {
 #pragma unroll
     for (int i = 0; i < R; ++i)
@@ -127,7 +127,6 @@ __global__ void __launch_bounds__(MAXT, MINB) cn2d_poly_kernel(const __grid_cons
       if (own && ((in >> i) & 1u)) f[i] = src[off[i]];
   };
   if (do_grad) forward_slice(slice_of(p.t0), f1);
-  diag(p.t0, qn);
   const bool sources = p.src_shared != nullptr || p.src_probe != nullptr || p.src_exit != nullptr;
   auto add_sources = [&](int t, float sw, float2(&v)[R]) {
     const float2 *s0 = p.src_shared ? p.src_shared + (size_t)(t - 1) * p.N + g0 : nullptr;
@@ -297,6 +296,7 @@ Poly2DPlan poly2d_plan(const tp_cn2d_op *op) {
   // margins over the free-space slice for the object and the boundary rows
   const double tau = 1.15 * 2.0 * mu / d + 0.002;
   double arg = fabs(atan2(di, dr)) + 0.1;
+  if (!(arg < 1.5)) return pl;  // the factorisation compares tangents
   const std::complex<double> it(0.0, tau);
   for (int m = 4; m <= kPoly2DMaxDeg; m += 2) {
     const std::complex<double> scale = chebyshev(m, 1.0 / it);
@@ -325,13 +325,11 @@ Poly2DPlan poly2d_plan(const tp_cn2d_op *op) {
   return pl;
 }
 
-int launch_poly_march(const Partition &pt, const MarchParams &mp, const Poly2DPlan &plan, const unsigned *bad,
-                      bool lagged, cudaStream_t st) {
+int launch_poly_march(const Partition &pt, const MarchParams &mp, const Poly2DPlan &plan, bool lagged, cudaStream_t st) {
   Poly2DParams q{};
   q.p = mp;
   q.M = pt.M;
   q.m = plan.m;
-  q.bad = bad;
   for (int k = 0; k < plan.m; ++k) q.a[k] = plan.a[k];
   auto warps = [&](int R) {
     const int use = 32 * R - 2 * kHaloRows;
