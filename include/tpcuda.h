@@ -128,15 +128,15 @@ typedef struct tp_cn2d_march_args {
   int32_t store_base;
   int32_t ufwd_slices;       /* slices per probe in u_fwd (0 = nz)             */
   int32_t ufwd_base;         /* u_fwd index of forward slice s is s - ufwd_base */
-  int32_t store_sums;        /* bit 0 (N in {512, 1024, 2048} only): FORWARD
+  int32_t store_sums;        /* 0, or 1 (N in {512, 1024, 2048} only): FORWARD
                                 stores the half pair sums (u_t + u_{t-1})/2 the
                                 gradient contracts with instead of u_t (the
                                 initial state is not stored; needs
                                 store_every <= 1); ADJOINT_EXACT reads u_fwd as
-                                such sums (one slice per step instead of two).
-                                Bits 8 and up: slices per probe of the stored
-                                field that state_in is a slice of (probes are
-                                that many Npad apart; 0 = state_in alone)     */
+                                such sums (one slice per step instead of two) */
+  int32_t state_slices;      /* slices per probe of the stored field that state_in
+                                is a slice of: probe p's state is p state_slices
+                                Npad after it (0 or 1: state_in is (P, Npad))  */
 } tp_cn2d_march_args;
 
 /* Partition of N rows into `chunks` chunks of `rows_per_chunk` rows (padded

@@ -4,6 +4,8 @@ A march in place is the march out of place (every input is read before the outpu
 replaces it is written): to the bit where both run the same kernel.
 """
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -13,6 +15,7 @@ torch = pytest.importorskip("torch")
 if not torch.cuda.is_available():  # pragma: no cover
     pytest.skip("needs a CUDA device", allow_module_level=True)
 
+from thick_ptycho_b200 import _native  # noqa: E402
 from thick_ptycho_b200.cn2d import CN2D  # noqa: E402
 
 K = 4 * np.pi
@@ -152,3 +155,23 @@ def test_2d_verdicts_follow_the_factorised_slices():
         strong[100, 20] = bad
         eng.factor_range(strong, "forward", 15, 25, out=fs.buf)
         assert [s + 1 for s, v in enumerate(verdicts(eng, fs).tolist()) if v] == [20, 21]
+
+
+@pytest.mark.parametrize("N", [97, 1024])
+def test_2d_march_arguments_refused(N):
+    """store_sums is 0 or 1; the stride of state_in is a field of its own."""
+    rng = np.random.default_rng(N)
+    eng = CN2D(N, 5, K, 1.0, 1.0, "impedance")
+    fs = eng.factor(index(rng, N, 5), "forward")
+    state = torch.zeros((2, 3, eng.npad), dtype=torch.complex64, device="cuda")
+    for sums, slices, with_state, ok in [(0, 0, True, True), (0, 3, True, True), (0, 3, False, False), (0, -1, True, False),
+                                         (2, 0, True, False), (-1, 0, True, False), (256, 0, True, False),
+                                         (768, 0, True, False), (1, 0, True, N == 1024)]:
+        a = _native.TpCn2dMarchArgs()
+        a.num_probes, a.mode, a.t_begin, a.t_end = 2, _native.MODE_FORWARD, 2, 3
+        a.store_sums, a.state_slices = sums, slices
+        if with_state:
+            a.state_in = ctypes.c_void_p(state.data_ptr())
+        rc = eng.lib.tp_cn2d_march(ctypes.byref(eng.op()), ctypes.c_void_p(fs.buf.data_ptr()), ctypes.byref(a), None)
+        assert (rc == 0) == ok, (sums, slices, with_state, rc)
+    torch.cuda.synchronize()

@@ -76,6 +76,7 @@ class TpCn2dMarchArgs(ctypes.Structure):
         ("ufwd_slices", ctypes.c_int32),
         ("ufwd_base", ctypes.c_int32),
         ("store_sums", ctypes.c_int32),
+        ("state_slices", ctypes.c_int32),
     ]
 
 

@@ -197,7 +197,7 @@ class CN2D:
                     not 0 <= index < store.shape[1]:
                 raise ValueError("state_from must be a chunked field (P, slices, Npad) and one of its slices")
             a.state_in = ctypes.c_void_p(store.data_ptr() + index * self.npad * store.element_size())
-            a.store_sums |= store.shape[1] << 8
+            a.state_slices = store.shape[1]
         o = self.op()
         rc = self.lib.tp_cn2d_march(ctypes.byref(o), _ptr(fs.buf), ctypes.byref(a), _stream(self.device))
         _native.check(rc, "tp_cn2d_march", self.lib)

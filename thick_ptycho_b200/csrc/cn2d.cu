@@ -902,17 +902,18 @@ extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp
   if (mp.flip_out && (mp.t0 != 1 || mp.t1 != mp.L) && a->u_store != nullptr)
     return set_error(TP_ERR_INVALID, "the flipped ADJOINT store needs the full step range");
   mp.state_in = static_cast<const cx *>(a->state_in);
-  mp.state_stride = (size_t)(a->store_sums >> 8 > 0 ? a->store_sums >> 8 : 1) * mp.Npad;
+  if (a->state_slices < 0 || (a->state_slices > 0 && a->state_in == nullptr))
+    return set_error(TP_ERR_INVALID, "state_slices=%d needs state_in", a->state_slices);
+  mp.state_stride = (size_t)(a->state_slices > 0 ? a->state_slices : 1) * mp.Npad;
   mp.state_out = static_cast<cx *>(a->state_out);
   mp.store_slices = a->store_slices > 0 ? a->store_slices : op->nz;
   mp.store_every = a->store_every;
   mp.store_base = a->store_base;
   mp.ufwd_slices = a->ufwd_slices > 0 ? a->ufwd_slices : op->nz;
   mp.ufwd_base = a->ufwd_base;
-  if (a->store_sums < 0 || (a->store_sums & 0xfe) != 0 || (a->store_sums > 1 && a->state_in == nullptr))
-    return set_error(TP_ERR_INVALID, "store_sums=%d (0 or 1, and state_in's slices from bit 8)", a->store_sums);
-  mp.store_sums = a->store_sums & 1;
-  if (mp.store_sums) {
+  mp.store_sums = a->store_sums;
+  if (a->store_sums != 0) {
+    if (a->store_sums != 1) return set_error(TP_ERR_INVALID, "store_sums=%d (0 or 1)", a->store_sums);
     if (a->mode != TP_MODE_FORWARD && a->mode != TP_MODE_ADJOINT_EXACT)
       return set_error(TP_ERR_INVALID, "store_sums needs mode FORWARD or ADJOINT_EXACT");
     if (a->mode == TP_MODE_FORWARD && a->store_every > 1)
