@@ -1,7 +1,8 @@
 """Marches whose outputs replace their inputs, and partial marches of one factor set.
 
 A march in place is the march out of place (every input is read before the output that
-replaces it is written): to the bit where both run the same kernel.
+replaces it is written): to the bit where both run the same kernel; in 3D, where a march
+whose outputs lie on its sources runs the Krylov solves, to 1.2e-5 (test_polynomial_gpu.py).
 """
 
 import ctypes
@@ -17,6 +18,7 @@ if not torch.cuda.is_available():  # pragma: no cover
 
 from thick_ptycho_b200 import _native  # noqa: E402
 from thick_ptycho_b200.cn2d import CN2D  # noqa: E402
+from thick_ptycho_b200.cn3d import CN3D  # noqa: E402
 
 K = 4 * np.pi
 
@@ -175,3 +177,41 @@ def test_2d_march_arguments_refused(N):
         rc = eng.lib.tp_cn2d_march(ctypes.byref(eng.op()), ctypes.c_void_p(fs.buf.data_ptr()), ctypes.byref(a), None)
         assert (rc == 0) == ok, (sums, slices, with_state, rc)
     torch.cuda.synchronize()
+
+
+# ------------------------------------------------------------------ 3D
+@pytest.mark.parametrize("case", ["exit on src_exit", "exit on src_exit, exact", "exit on src_shared", "store on src_exit",
+                                  "exit on src_exit, later", "exit on probes"])
+def test_3d_outputs_on_sources(case):
+    rng = np.random.default_rng(3)
+    nf, nb, P = 130, 66, 1 if "shared" in case or "store" in case else 5
+    nz = 4 if "shared" in case or "later" in case else 2
+    N, L = nf * nb, nz - 1
+    field = index(rng, N, nz)
+    mode = "adjoint_exact" if "exact" in case else "adjoint" if case.startswith("exit on src_exit") else "forward"
+    src = cplx(rng, P, N)
+    kw = {}
+    if "src_exit" in case:
+        kw["src_exit"] = src
+    if "shared" in case:
+        kw["src_shared"] = cplx(rng, L, N)
+    if mode == "forward":
+        kw["probes"] = cplx(rng, P, N)
+    eng = CN3D(nf, nb, nz, K, 1.0, 1.0, 1.0, "impedance")
+    ref, store = torch.empty((P, N), dtype=torch.complex64, device="cuda"), eng.new_store(P)
+    eng.march(field, P, mode, exit_out=ref, u_store=store, **kw)
+    assert (eng.stats.cpu().tolist()[4] == 2) == (nz > 2)
+    if "store" in case:
+        again = eng.new_store(P)
+        again[:, 1] = src
+        eng.march(field, P, mode, u_store=again, **{**kw, "src_exit": again[0, 1:2]})
+        got, want = again, store
+    else:
+        kw = {k: v.clone() for k, v in kw.items()}
+        got = kw["src_shared"][L - 1:L] if "shared" in case else kw["probes" if "probes" in case else "src_exit"]
+        eng.march(field, P, mode, exit_out=got, **kw)
+        want = ref
+    # a march of several steps has used src_exit before it writes the exit
+    assert (eng.stats.cpu().tolist()[4] == 2) == ("later" in case)
+    assert float(torch.linalg.vector_norm(got - want)) < 1.2e-5 * float(torch.linalg.vector_norm(want))
+    eng.device_status()

@@ -2088,6 +2088,24 @@ extern "C" size_t tp_cn3d_workspace_bytes(int32_t n_total, int32_t num_probes) {
   return c3_layout(nullptr, n_total, num_probes).bytes;
 }
 
+#ifndef TP_C128_CHECK
+// Whether an output of a step may lie where the step's source does.  The polynomial step
+// reads a source with its halo while other CTAs write the step's outputs; the Krylov
+// march has read it into its right-hand side before.  (exit_out on src_exit is no such
+// case: they meet at nz = 2 only, where the polynomial march does not run.)
+static bool outputs_replace_sources(const tp_cn3d_march_args *a, size_t image, int nz) {
+  const size_t L = (size_t)nz - 1, P = (size_t)a->num_probes;
+  auto meet = [](const void *x, size_t nx, const void *y, size_t ny) {
+    const char *p = static_cast<const char *>(x), *q = static_cast<const char *>(y);
+    return p != nullptr && q != nullptr && p < q + ny && q < p + nx;
+  };
+  const char *shared = static_cast<const char *>(a->src_shared);
+  const void *last = shared ? shared + (L - 1) * image : nullptr;  // the source of the step that writes exit_out
+  return meet(a->exit_out, P * image, last, image) || meet(a->u_store, P * nz * image, shared, L * image) ||
+         meet(a->u_store, P * nz * image, a->src_exit, P * image);
+}
+#endif
+
 extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t n_dtype, const tp_cn3d_march_args *a,
                              void *workspace, size_t workspace_bytes, tp_stream_t stream) {
   if (op == nullptr || a == nullptr || n_field == nullptr || workspace == nullptr)
@@ -2143,7 +2161,8 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
   cudaStreamCaptureStatus poly_cap = cudaStreamCaptureStatusNone;
   TP_CHECK_CUDA(cudaStreamIsCapturing(st, &poly_cap));
   if (a->precond == 1 && (a->kernels & 0xff) == 0 && a->launch == 0 && a->host_check != 0 && a->train_every <= 0 &&
-      a->mode != TP_MODE_REVERSE && poly_cap == cudaStreamCaptureStatusNone && q.mu_x.x == 0.0 && q.mu_y.x == 0.0) {
+      a->mode != TP_MODE_REVERSE && poly_cap == cudaStreamCaptureStatusNone && q.mu_x.x == 0.0 && q.mu_y.x == 0.0 &&
+      !outputs_replace_sources(a, (size_t)N * sizeof(cx), nz)) {
     c3_diag_kernel<<<296, 256, 0, st>>>(N, nf, q.sigma, q.conj_t, static_cast<const cx *>(op->kc),
                                         static_cast<const cx *>(op->kw), static_cast<const cx *>(op->ke),
                                         static_cast<const cx *>(op->ks), static_cast<const cx *>(op->kn), w.dc, w.dw,
