@@ -486,7 +486,7 @@ def bench_learned_3d(dev, reps=2, train_steps=1500, pairs="mixed"):
         exits[name] = ex.clone()
         out[name] = {"value": P * L / (t / 1e3), "ms_per_step": t,
                      "iterations_per_solve": st["iterations"] / max(st["solves"], 1),
-                     "failed_solves": st["failed"], "graph": st["graph"],
+                     "failed_solves": st["failed"], "graph": st["graph"], "polynomial": st["polynomial"],
                      "exit_rel_error_vs_fp64_fixture": fixture_exit_error("config2", ex)}
     diff = float(torch.linalg.vector_norm(exits["learned"] - exits["plain"]) / torch.linalg.vector_norm(exits["plain"]))
     return {

@@ -215,3 +215,13 @@ def test_3d_outputs_on_sources(case):
     assert (eng.stats.cpu().tolist()[4] == 2) == ("later" in case)
     assert float(torch.linalg.vector_norm(got - want)) < 1.2e-5 * float(torch.linalg.vector_norm(want))
     eng.device_status()
+
+
+@pytest.mark.parametrize("kernels,launch,how", [(0, 0, "polynomial"), (8, 0, "graph"), (8, 1, None)])
+def test_3d_stats_name_the_march(kernels, launch, how):
+    rng = np.random.default_rng(4)
+    eng = CN3D(32, 32, 4, K, 1.0, 1.0, 1.0, "impedance")
+    eng.kernels, eng.launch = kernels, launch
+    eng.march(index(rng, 1024, 4), 2, "forward", probes=cplx(rng, 2, 1024), u_store=eng.new_store(2))
+    st = eng.read_stats()
+    assert [st["graph"], st["polynomial"]] == [how == "graph", how == "polynomial"]

@@ -189,11 +189,14 @@ class CN3D:
 
     def read_stats(self, reset=True):
         """(total iterations, solves, failed solves, max iterations per solve,
-        whether the last march ran as one CUDA graph)."""
+        and how the last march ran: "graph" = as one CUDA graph of Krylov solves,
+        "polynomial" = by a fixed polynomial per slice, whose degree counts as a
+        solve's iterations; neither = Krylov solves launched step by step)."""
         s = self.stats.cpu().tolist()
         if reset:
             self.stats.zero_()
-        return {"iterations": s[0], "solves": s[1], "failed": s[2], "max_iterations": s[3], "graph": bool(s[4])}
+        return {"iterations": s[0], "solves": s[1], "failed": s[2], "max_iterations": s[3], "graph": s[4] == 1,
+                "polynomial": s[4] == 2}
 
     def grad_to_n(self, grad_c: torch.Tensor, field=None, is_delta=False) -> torch.Tensor:
         """Σ_p λ conj(u_s + u_{s−1}) (L, N) → torch-convention ∂/∂n (N, nz)."""
