@@ -98,3 +98,30 @@ def test_weight_gradient_sizes(cin, nf, nb, batch):
     got = dw.view(3, 3, cin, 32).permute(3, 2, 0, 1).cpu().numpy()
     assert rel(got, co.conv3x3_wgrad(bf(x), bf(dy))) < 1e-4
     assert np.allclose(db.cpu().numpy(), bf(dy).sum(axis=(0, 2, 3)), rtol=1e-4, atol=1e-3)
+
+
+def test_training_step_operands():
+    """Lazily conjugated, real and broadcast operands give what their values give; operands
+    of another device are refused."""
+    from thick_ptycho_b200.learned import LearnedPreconditioner
+
+    rng = np.random.default_rng(5)
+    nf, nb, nimg, per = 24, 10, 2, 3
+    N, V = nf * nb, nimg * per
+    m = LearnedPreconditioner(nf, nb, kappa=20.0)
+    d, z, t = c64(0.01 * cplx(rng, nimg, N)), c64(cplx(rng, V, N)), c64(cplx(rng, V, N))
+    sc = torch.rand(V, device="cuda")
+    same = [((t, sc), (t.conj().resolve_conj().conj(), sc.double())),
+            ((t.real.to(torch.complex64), torch.ones_like(sc)), (t.real, torch.ones(1, device="cuda"))),
+            ((torch.zeros_like(t), sc), (0.0, sc)), ((torch.zeros_like(t), sc), (torch.tensor(0.0), sc))]
+    for a, b in same:
+        la, wa, ba = m.loss_and_grads(d, z, *a, per)
+        lb, wb, bb = m.loss_and_grads(d, z, *b, per)
+        assert abs(float(la) - float(lb)) <= 1e-6 * float(la)
+        for x, y in zip(wa + ba, wb + bb):  # sums in any order
+            assert float((x - y).abs().max()) <= 1e-4 * float(x.abs().max())
+    for bad in ((t.cpu(), sc), (t, sc.cpu())):
+        with pytest.raises(RuntimeError):
+            m.loss_and_grads(d, z, *bad, per)
+    with pytest.raises(RuntimeError):
+        m.loss_and_grads(d, z.cpu(), t, sc, per)

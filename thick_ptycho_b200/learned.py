@@ -223,6 +223,27 @@ class LearnedPreconditioner:
         return y
 
     # ----------------------------------------------------------- backward
+    @staticmethod
+    def _residual_operands(z, target, scale, device):
+        """z, target and scale as the residual kernel reads them: contiguous, on ``device``,
+        complex64 / float32, no lazy conjugation.  ``target`` may be anything that
+        ``y - target`` takes (a number, a real tensor, one that broadcasts to z)."""
+        if not torch.is_tensor(target):
+            target = torch.as_tensor(target, device=device)
+        if target.dim() == 0:
+            target = target.to(device)
+        for name, t in (("z", z), ("target", target), ("scale", scale)):
+            if t.device != device:
+                raise RuntimeError(f"{name} is on {t.device}, expected {device}")
+        if z.dtype != torch.complex64 or scale.is_complex() or scale.dim() != 1:
+            raise TypeError("z must be complex64, scale a real vector")
+
+        def plain(t, shape, dtype):
+            return torch.broadcast_to(t, shape).to(dtype).resolve_conj().resolve_neg().contiguous()
+
+        return (plain(z, z.shape, torch.complex64), plain(target, z.shape, torch.complex64),
+                plain(scale, z.shape[:1], torch.float32))
+
     def loss_and_grads(self, diag, z, target, scale, per_image):
         """L = Σ_v scale_v |y_v − target_v|² and d L / d (weights, biases), all on the GPU.
 
@@ -234,11 +255,7 @@ class LearnedPreconditioner:
         L = self.lib
         st = _stream(self.device)
         F = self.filter(diag)
-        z = z.contiguous()
-        target = torch.broadcast_to(target, z.shape).contiguous()
-        scale = torch.broadcast_to(scale, (V,)).contiguous()
-        if z.dtype != torch.complex64 or target.dtype != torch.complex64 or scale.dtype != torch.float32:
-            raise TypeError("z and target must be complex64, scale float32")
+        z, target, scale = self._residual_operands(z, target, scale, F.device)
         e = torch.empty_like(z)
         # the sums that the kernels add to, in one cleared buffer: the loss (fp64),
         # then the weight gradients (9, cin, 32) and the bias gradients of the layers
