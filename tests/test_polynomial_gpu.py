@@ -154,3 +154,25 @@ def test_preconditioner_on_tiles_is_the_transform(nf, nb, P, mu, mode):
         assert eng.read_stats()["max_iterations"] == 1
         got.append(store.cpu().numpy())
     assert rel(got[0], got[1]) < 4e-6, rel(got[0], got[1])
+
+
+def test_3d_norms_are_fp64_sums():
+    """The right-hand side's norms that solves are judged by: one pixel in 16 of size 1 among
+    pixels of 1e-4, whose squares a sum in fp32 drops beside it (2e-7 of the norm).  The
+    first exact-adjoint step's right-hand side is its source, and the march leaves the
+    norms (fp64 pairs, by step and probe) behind its two state vectors."""
+    nf, nb, nz, P = 128, 96, 4, 3
+    N = nf * nb
+    rng = np.random.default_rng(11)
+    src = np.full((P, nb, nf), 1e-4, np.complex64)
+    src[:, ::8, ::2] = 1
+    src *= np.exp(2j * np.pi * rng.integers(0, 4, src.shape) / 4).round().astype(np.complex64)
+    eng = CN3D(nf, nb, nz, K, 1.0, 1.0, 1.0, "impedance")
+    field = dev(1 + 5e-3 * rng.standard_normal((N, nz)), np.complex128)
+    eng.march(field, P, "adjoint_exact", src_exit=dev(src.reshape(P, N)), exit_out=torch.empty((P, N), dtype=torch.complex64, device="cuda"))
+    assert eng.stats.cpu().tolist()[4] == 2
+    at = 2 * (-(-P * N * 8 // 256) * 256)
+    norms = eng.workspace(P)[at:at + 16 * P].cpu().numpy().view(np.float64).reshape(P, 2)
+    exact = np.sum(np.abs(src.astype(complex)) ** 2, axis=(1, 2))
+    assert np.all(np.abs(norms[:, 0] - exact) < 1e-12 * exact), norms[:, 0] / exact - 1
+    assert np.all(norms[:, 1] < 1e-12 * norms[:, 0])
