@@ -417,7 +417,8 @@ typedef struct tp_cn3d_march_args {
   void *grad_c;              /* ADJOINT_EXACT: float2 (L, N) accumulator of
                                 sum_p lambda_s conj(u_s + u_{s-1}); caller zeroes */
   int32_t *stats;            /* device int32[5]: total iterations, solves, solves
-                                whose true residual exceeded 10 tol, largest
+                                whose true residual exceeded 10 tol (polynomial
+                                steps: evaluated tile by tile), largest
                                 iteration count (accumulated), and [4] = 1 when
                                 the march ran as one graph (0 step by step, 2 as
                                 polynomial steps);

@@ -14,8 +14,8 @@
 // One CTA per probe.  A thread keeps R consecutive rows of the state for the whole
 // march; a half-sweep's neighbours are its own rows and one warp shuffle.  Warps do
 // not wait for one another inside a step: each computes H extra rows on both sides
-// (what lies h rows outside changes a row by mu^h; H = 8 rows leave 1e-13 at
-// mu = 0.02) and the halos are renewed through shared memory once per step, behind
+// (what lies h rows outside changes a row by (tau / 2)^h, tau / 2 the largest entry of J;
+// H = 8 rows leave 1e-13 at mu = 0.02 and 3e-10 at the largest mu taken, 0.056) and the halos are renewed through shared memory once per step, behind
 // the step's only barrier.  The slices' diagonals (the QD rows of the factor set, in
 // the layout of the stored field) are read one step ahead.  The partitioned
 // solve it replaces runs one warp per probe through a chain of ceil(N / 32) dependent
@@ -289,12 +289,13 @@ Poly2DPlan poly2d_plan(const tp_cn2d_op *op) {
   Poly2DPlan pl{};
   if (op->k_off[0] != 0.0 || op->k_01[0] != 0.0 || op->k_nm[0] != 0.0) return pl;
   const double mu = fabs(op->k_off[1]);
-  // halo rows leave 1e-10 of what lies beyond them
-  if (!(pow(mu, (double)kHaloRows) <= 1e-10)) return pl;
   const double dr = 1.0 - op->k_diag[0], di = op->k_diag[1], d = hypot(dr, di);
   if (!(d > 0.5)) return pl;
   // margins over the free-space slice for the object and the boundary rows
   const double tau = 1.15 * 2.0 * mu / d + 0.002;
+  // halo rows leave 3e-10 of what lies beyond them (rows within tau couple by at most
+  // tau / 2 to either side, but for the doubled couplings of the edges)
+  if (!(pow(0.5 * tau, (double)kHaloRows) <= 3.3e-10)) return pl;
   double arg = fabs(atan2(di, dr)) + 0.1;
   if (!(arg < 1.5)) return pl;  // the factorisation compares tangents
   const std::complex<double> it(0.0, tau);

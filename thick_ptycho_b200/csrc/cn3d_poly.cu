@@ -27,11 +27,12 @@
 // column, the rows above and below), one warp shuffle (left or right) and, at
 // the warp's first and last row, shared memory.  A tile computes a core smaller
 // than itself: the value of a pixel at the core's edge depends on what is h rows
-// outside it only through mu^h, so a halo of h = 1 + log(1e-8) / log(mu) pixels
-// (6 at mu = 0.02) gives the core to below complex64 round-off, whatever m.  The
-// tiles of u arrive by tiled tensor copies (zero outside the image),
+// outside it only through |J|^h, so a halo of h = 1 + log(1e-8) / log(max |J_ij|) pixels
+// (6 at mu = 0.02 and |D| ~ 1) gives the core to below complex64 round-off, whatever m.
+// The tiles of u arrive by tiled tensor copies (zero outside the image),
 // double-buffered over the group's probes.  Each solve is judged by its true
-// residual, as in the Krylov march.
+// residual, as in the Krylov march, but tile by tile with the tile's own d in its halo:
+// what the halo leaves out does not show in it.
 //
 // 256 x 256, 64 probes, m = 6: a forward step to the exit 42.7 us, keeping the field
 // 44.7; forward and exact adjoint with the gradient over 255 slices 191 -> 30 ms against
@@ -59,8 +60,9 @@ namespace tp {
 namespace {
 
 struct PolyCheck {
-  // bits of the largest row and column sums of |J| and the largest |arg D| (non-negative floats)
-  unsigned tau, tau_col, arg;
+  // bits of the largest row and column sums of |J|, the largest |arg D| and the largest
+  // 1 / |D| (non-negative floats)
+  unsigned tau, tau_col, arg, inv;
   int bad;
 };
 
@@ -113,7 +115,7 @@ __global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q,
                                                              int s_hi, float2 *cd, PolyCheck *chk) {
   __shared__ float2 tile[32][33];
   const int i0 = blockIdx.x * 32, s0 = s_first + blockIdx.y * 32;
-  float tau = 0.f, tcol = 0.f, arg = 0.f;
+  float tau = 0.f, tcol = 0.f, arg = 0.f, inv = 0.f;
   int bad = 0;
   for (int r = threadIdx.y; r < 32; r += 8) {
     const int i = i0 + r, s = s0 + threadIdx.x;
@@ -131,13 +133,14 @@ __global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q,
       const float sum = (fabsf(cw.x) + fabsf(cw.y)) * rw.z + fabsf(rw.x) + fabsf(rw.y);
       if (sum > 0.f) {
         const float dr = 1.f - d.x, di = -d.y;
-        const float t = sum / sqrtf(dr * dr + di * di);
+        const float n = sqrtf(dr * dr + di * di), t = sum / n;
         if (!(t < 1e6f)) bad = 1;
         tau = fmaxf(tau, t);
+        inv = fmaxf(inv, 1.f / n);
         // what row i's element reaches: its neighbours' couplings back to it
         const float col = ((f + 1 < q.nf ? fabsf(q.colw[f + 1].x) : 0.f) + (f > 0 ? fabsf(q.colw[f - 1].y) : 0.f)) * rw.z +
                           (b + 1 < q.nb ? fabsf(q.roww[b + 1].x) : 0.f) + (b > 0 ? fabsf(q.roww[b - 1].y) : 0.f);
-        tcol = fmaxf(tcol, col / sqrtf(dr * dr + di * di));
+        tcol = fmaxf(tcol, col / n);
         arg = fmaxf(arg, fabsf(atan2f(di, dr)));
       } else {
         const float dr = 1.f - d.x, n2 = dr * dr + d.y * d.y;
@@ -162,6 +165,7 @@ __global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q,
     tau = fmaxf(tau, __shfl_down_sync(0xffffffffu, tau, o));
     tcol = fmaxf(tcol, __shfl_down_sync(0xffffffffu, tcol, o));
     arg = fmaxf(arg, __shfl_down_sync(0xffffffffu, arg, o));
+    inv = fmaxf(inv, __shfl_down_sync(0xffffffffu, inv, o));
     bad |= __shfl_down_sync(0xffffffffu, bad, o);
   }
   if (threadIdx.x == 0) {
@@ -170,6 +174,7 @@ __global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q,
     if (__float_as_uint(tau) > c->tau) atomicMax(&chk->tau, __float_as_uint(tau));
     if (__float_as_uint(tcol) > c->tau_col) atomicMax(&chk->tau_col, __float_as_uint(tcol));
     if (__float_as_uint(arg) > c->arg) atomicMax(&chk->arg, __float_as_uint(arg));
+    if (__float_as_uint(inv) > c->inv) atomicMax(&chk->inv, __float_as_uint(inv));
     if (bad) atomicOr(&chk->bad, 1);
   }
 }
@@ -700,19 +705,21 @@ int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
   if (host.bad) return TP_OK;
   // either norm bounds the spectral radius (a transposed operator's rows are the
   // original's columns: the doubled Neumann couplings add up in one of the two)
-  float tau, tcol, theta;
+  float tau, tcol, theta, inv;
   memcpy(&tau, &host.tau, 4);
   memcpy(&tcol, &host.tau_col, 4);
   if (tcol < tau) tau = tcol;
   memcpy(&theta, &host.arg, 4);
+  memcpy(&inv, &host.inv, 4);
 
   PolyStep q{};
   const double target = 0.1 * (job.tol < 1e-6 ? job.tol : 1e-6);
   q.m = poly_degree(tau, theta, target, kPolyMaxDeg < job.max_iter ? kPolyMaxDeg : job.max_iter, q.a);
   if (q.m == 0) return TP_OK;
-  // halo: one pixel for the right-hand side and the reach of 1e-8 (no more than the polynomial's)
-  const double mu = fmax(1e-6, fmax(fabs(job.mu_x), fabs(job.mu_y)));
-  int h = 1 + (mu < 1.0 ? (int)ceil(log(1e-8) / log(mu)) : kPolyMaxHalo);
+  // halo: one pixel for the right-hand side and the reach of 1e-8 of J's largest entry
+  // between interior pixels (no more than the polynomial's)
+  const double ent = fmax(1e-6, fmax(fabs(job.mu_x), fabs(job.mu_y)) * (double)inv);
+  int h = 1 + (ent < 1.0 ? (int)ceil(log(1e-8) / log(ent)) : kPolyMaxHalo);
   if (h > q.m + 1) h = q.m + 1;
   if (h > kPolyMaxHalo) return TP_OK;
 

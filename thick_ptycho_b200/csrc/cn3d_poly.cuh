@@ -25,7 +25,7 @@ struct C3PolyJob {
   size_t scratch_bytes;
   float2 *colw;  // (nf)
   float4 *roww;  // (nb)
-  int *check;    // 4 words
+  int *check;    // 5 words
   const float2 *probes, *src_exit, *src_shared, *u_fwd;
   float2 *u_store, *exit_out, *grad_c;
   int *stats;
