@@ -6,6 +6,9 @@ Tolerances: a multislice slice adds FFT round-off (4e-7 relative, two transforms
 an update |H - 1| |psi| <= 2 |psi| and two roundings of psi, so L slices stay below
 L * 1e-6 of the field; the adjoint's transmission gradient, a product of the two
 fields, below 2 L * 1e-6.  The space-time solve stops at a 1e-6 residual: 1e-5.
+Long marches of white noise: a transform pair's roundings (1e-7 relative, 1.4e-7 on two
+axes) add up like their square root over the slices; what the constants and twiddles are
+off, the same in every slice, may add 3e-9 per slice and axis.
 """
 
 import numpy as np
@@ -109,3 +112,42 @@ def test_pit_block_and_z_lengths(N, nz, P):
     for p in range(P):
         ref = po.full_system_solve(A, B, C, po.pit_rhs(B, probes[p], nz - 1)).reshape(nz - 1, N).T
         assert rel(u[p][:, 1:], ref) < 1e-5, (p, rel(u[p][:, 1:], ref))
+
+
+def march_error(eng, H, T, x, u, axes):
+    """Relative errors of the exit and of the last gradient slice, white noise through all slices."""
+    Ln, P = T.shape[0], x.shape[0]
+    N = int(np.prod(x.shape[1:]))
+    psi = lam = x.astype(complex)
+    for z in range(Ln):
+        psi = np.fft.ifftn(H * np.fft.fftn(psi * T[z], axes=axes), axes=axes)
+    for z in reversed(range(Ln)):
+        g = np.fft.ifftn(H.conj() * np.fft.fftn(lam, axes=axes), axes=axes)
+        lam = np.conj(T[z]) * g
+    grad = np.sum(g * np.conj(T[0] * u[:, 0]), 0)
+    t1 = dev((T - 1).reshape(Ln, N))
+    ex = torch.empty((P, N), dtype=torch.complex64, device="cuda")
+    eng.march(t1, dev(x), exit_out=ex)
+    gt = torch.zeros((Ln, N), dtype=torch.complex64, device="cuda")
+    eng.backward(t1, dev(u.reshape(P, Ln + 1, N)), dev(x), gt)
+    return rel(ex.cpu().numpy(), psi.reshape(P, N)), rel(gt[0].cpu().numpy(), grad.reshape(N))
+
+
+@pytest.mark.parametrize("n", [512, 2048, 243, 270, 625, 960, 1000, 1500])
+def test_ms2d_errors_do_not_add_up_over_slices(n):
+    rng = np.random.default_rng(n)
+    Ln, P = 255, 3
+    T = 1 + (np.exp(0.02j * rng.standard_normal((Ln, n))) - 1).astype(np.complex64).astype(complex)
+    x, u = cplx(rng, P, n).astype(np.complex64), cplx(rng, P, Ln + 1, n).astype(np.complex64)
+    err = march_error(MS2D(n, Ln + 1, K, 1.0, 1.0), po.ms_kernel(n, 1.0, K, 1.0), T, x, u, (-1,))
+    assert max(err) < np.sqrt(Ln) * 1e-7 + Ln * 3e-9, err
+
+
+@pytest.mark.parametrize("n1,n2", [(64, 64), (128, 192), (256, 256), (48, 60), (75, 90)])
+def test_ms3d_errors_do_not_add_up_over_slices(n1, n2):
+    rng = np.random.default_rng(n1)
+    Ln, P = 48, 2
+    T = 1 + (np.exp(0.02j * rng.standard_normal((Ln, n1, n2))) - 1).astype(np.complex64).astype(complex)
+    x, u = cplx(rng, P, n1, n2).astype(np.complex64), cplx(rng, P, Ln + 1, n1, n2).astype(np.complex64)
+    err = march_error(MS3D(n1, n2, Ln + 1, K, 1.0, 1.0, 1.0), po.ms_kernel_3d(n1, n2, 1.0, 1.0, K, 1.0), T, x, u, (-2, -1))
+    assert max(err) < np.sqrt(Ln) * 1.4e-7 + Ln * 6e-9, err

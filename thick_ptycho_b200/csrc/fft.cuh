@@ -526,6 +526,50 @@ struct UnitRoots {
   }
 };
 
+// 3- and 5-point DFTs with their constants to twice the precision, c + (the rest of c):
+// rounded, they are the same error in every slice of a march (255 slices of white noise
+// at n = 1500: 2.1e-6 -> 1.9e-6; 64 probes 3.1 -> 3.3 us per slice).
+template <int R>
+__device__ __forceinline__ void dft_odd(cx (&v)[8], rx sign) {
+#ifdef TP_C128_CHECK
+  dft_small<R>(v, sign);
+#else
+  constexpr auto rest = [](double c) constexpr { return (float)(c - (double)(float)c); };
+  if constexpr (R == 3) {
+    constexpr double s = 0.86602540378443864676;  // sin(2 pi / 3)
+    const cx t = padd(v[1], v[2]), b = psub(v[1], v[2]);
+    const cx d = mul_si(mkcx(fmaf((float)s, b.x, rest(s) * b.x), fmaf((float)s, b.y, rest(s) * b.y)), sign);
+    const cx m = mkcx(fmaf(-0.5f, t.x, v[0].x), fmaf(-0.5f, t.y, v[0].y));
+    v[0] = padd(v[0], t);
+    v[1] = cadd(m, d);
+    v[2] = csub(m, d);
+  } else {
+    constexpr double c1 = 0.30901699437494742410, c2 = -0.80901699437494742410;  // cos(2 pi / 5), cos(4 pi / 5)
+    constexpr double s1 = 0.95105651629515357212, s2 = 0.58778525229247312917;
+    auto pair = [](double p, double q, float a, float b, float c) {  // c + p a + q b
+      return fmaf((float)p, a, fmaf((float)q, b, fmaf(rest(p), a, fmaf(rest(q), b, c))));
+    };
+    const cx a1 = padd(v[1], v[4]), b1 = psub(v[1], v[4]);
+    const cx a2 = padd(v[2], v[3]), b2 = psub(v[2], v[3]);
+    const cx x0 = v[0];
+    const cx m1 = mkcx(pair(c1, c2, a1.x, a2.x, x0.x), pair(c1, c2, a1.y, a2.y, x0.y));
+    const cx m2 = mkcx(pair(c2, c1, a1.x, a2.x, x0.x), pair(c2, c1, a1.y, a2.y, x0.y));
+    const cx n1 = mul_si(mkcx(pair(s1, s2, b1.x, b2.x, 0.f), pair(s1, s2, b1.y, b2.y, 0.f)), sign);
+    const cx n2 = mul_si(mkcx(pair(s2, -s1, b1.x, b2.x, 0.f), pair(s2, -s1, b1.y, b2.y, 0.f)), sign);
+    v[0] = padd(x0, padd(a1, a2));
+    v[1] = cadd(m1, n1);
+    v[4] = csub(m1, n1);
+    v[2] = cadd(m2, n2);
+    v[3] = csub(m2, n2);
+  }
+#endif
+}
+template <int R>
+__device__ __forceinline__ void dft_part(cx (&v)[8], rx sign) {
+  if constexpr (R == 3 || R == 5) dft_odd<R>(v, sign);
+  else dft_small<R>(v, sign);
+}
+
 // R = A B points: n = B n1 + n2, k = k1 + A k2; A-point DFTs over n1, the roots
 // exp(sign 2 pi i n2 k1 / R), B-point DFTs over n2.
 template <int A, int B>
@@ -537,7 +581,7 @@ __device__ __forceinline__ void dft_two(cx (&v)[16], rx sign) {
     cx t[8];
 #pragma unroll
     for (int n1 = 0; n1 < A; ++n1) t[n1] = v[B * n1 + n2];
-    dft_small<A>(t, sign);
+    dft_part<A>(t, sign);
 #pragma unroll
     for (int k1 = 0; k1 < A; ++k1)
       o[B * k1 + n2] = n2 * k1 ? cmul(t[k1], mkcx(w.c[n2 * k1], sign * w.s[n2 * k1])) : t[k1];
@@ -547,7 +591,7 @@ __device__ __forceinline__ void dft_two(cx (&v)[16], rx sign) {
     cx t[8];
 #pragma unroll
     for (int n2 = 0; n2 < B; ++n2) t[n2] = o[B * k1 + n2];
-    dft_small<B>(t, sign);
+    dft_part<B>(t, sign);
 #pragma unroll
     for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = t[k2];
   }
@@ -566,7 +610,7 @@ __device__ __forceinline__ void mix_dft(cx (&v)[16], rx sign) {
     cx w[8];
 #pragma unroll
     for (int j = 0; j < R; ++j) w[j] = v[j];
-    dft_small<R>(w, sign);
+    dft_part<R>(w, sign);
 #pragma unroll
     for (int j = 0; j < R; ++j) v[j] = w[j];
   }
@@ -631,11 +675,76 @@ __device__ __forceinline__ void mix_run(const MixPlan &pl, int s, int count, cx 
   });
 }
 
+// ------------------------------------------- gain of a transform and its inverse
+// A forward transform followed by the inverse that undoes its stages returns its input
+// times n (1 + g): an element meets the same fp32 constants and twiddles in both
+// directions, whose moduli are not quite one.  A march that multiplies a spectrum and
+// goes back in every slice adds g (-8e-8 .. 9e-8) up; it folds 1 / (1 + g) into the
+// spectrum's factor instead, which rounds once from fp64.  255 slices of white noise,
+// error against complex128: n = 2048 3.7e-6 without it, 1.8e-6 with it; n = 1500 3.5e-6,
+// 2.1e-6 (1.9e-6 with dft_odd's constants); 48 slices of 256 x 256: 1.8e-6, 8.8e-7.
+//
+// To first order g is a sum over the stages; this is the share of an R-point DFT's own
+// constants (R of mix_dft and dft_reg).
+template <int A, int B>
+constexpr double root_gain() {
+  const UnitRoots<A * B> w{};
+  double g = 0.0;
+  for (int a = 0; a < A; ++a)
+    for (int b = 0; b < B; ++b) g += (double)w.c[a * b] * w.c[a * b] + (double)w.s[a * b] * w.s[a * b] - 1.0;
+  return g / (A * B);
+}
+constexpr double dft_gain(int R) {
+  constexpr double s3 = TP_R(0.86602540378443864676);  // rounded in dft12 only
+  return R == 16 ? root_gain<4, 4>()
+       : R == 15 ? root_gain<3, 5>()
+       : R == 12 ? root_gain<4, 3>() + 4.0 * (s3 * s3 - 0.75) / 9.0
+       : R == 10 ? root_gain<2, 5>()
+       : R == 9  ? root_gain<3, 3>()
+       : R == 8  ? root_gain<2, 4>()
+       : R == 6  ? root_gain<2, 3>()
+                 : 0.0;
+}
+inline double mix_dft_gain(const MixPlan &pl) {
+  double g = 0.0;
+  for (int s = 0; s < pl.stages; ++s) g += dft_gain(pl.radix[s]);
+  return g;
+}
+__device__ __forceinline__ double modulus_less_1(cx w) { return (double)w.x * w.x + (double)w.y * w.y - 1.0; }
+// This thread's part of the share of an in-place plan's twiddles (the table at tw).
+__device__ __forceinline__ double mix_twiddle_gain(const MixPlan &pl, const cx *tw, int tid, int nth) {
+  double g = 0.0;
+  for (int s = 0; s + 1 < pl.stages; ++s) {
+    double v = 0.0;
+    for (int e = tid; e < pl.len[s]; e += nth) v += modulus_less_1(tw[pl.tw[s] + e]);
+    g += v / pl.len[s];
+  }
+  return g;
+}
+// The sum of v over the CTA (whole warps, at most 32), for every thread; red: 32 values.
+__device__ __forceinline__ double cta_sum(double v, double *red) {
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double s = 0.0;
+  for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
+  __syncthreads();
+  return s;
+}
+
 // Factors of the lengths with a four-step plan (R1 >= R2, both <= 16).
 __host__ __device__ constexpr int four_r1(int n) { return n == 64 ? 8 : 16; }
 __host__ __device__ constexpr int four_r2(int n) { return n / four_r1(n); }
 __host__ __device__ constexpr bool four_step_size(int n) { return n == 64 || n == 128 || n == 192 || n == 256; }
 // Entries of the padded twiddle table.
 __host__ __device__ constexpr int four_tw_len(int n) { return four_r1(n) * (four_r2(n) + 1); }
+// The gain's shares as above.
+inline double four_dft_gain(int n) { return dft_gain(four_r1(n)) + dft_gain(four_r2(n)); }
+__device__ __forceinline__ double four_twiddle_gain(int n, const cx *tw, int tid, int nth) {
+  const int r2 = four_r2(n);
+  double v = 0.0;
+  for (int e = tid; e < n; e += nth) v += modulus_less_1(tw[e / r2 * (r2 + 1) + e % r2]);
+  return v / n;
+}
 
 }  // namespace tp

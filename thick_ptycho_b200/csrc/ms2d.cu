@@ -142,10 +142,10 @@ __global__ void ms_transmission_kernel(const MsParams q, float2 *__restrict__ tr
   }
 }
 
-// H[j] - 1 with H[j] = exp(i (kz - k) dz), kz = sqrt(max(k^2 - kx^2, 0)),
+// (H[j] - 1) scale with H[j] = exp(i (kz - k) dz), kz = sqrt(max(k^2 - kx^2, 0)),
 // kx = 2 pi fftfreq(n, dx) (ms_solver.py:49-72); fp64, kept as the deviation
 // from one like the transmission.
-__device__ __forceinline__ float2 ms_h_minus_1(const MsParams &q, int j) {
+__device__ __forceinline__ float2 ms_h_minus_1(const MsParams &q, int j, double scale) {
   const int f = (j < (q.n + 1) / 2) ? j : j - q.n;
   const double kx = 2.0 * 3.14159265358979323846 * (double)f / ((double)q.n * q.dx);
   const double kz = sqrt(fmax(q.k * q.k - kx * kx, 0.0));
@@ -153,7 +153,7 @@ __device__ __forceinline__ float2 ms_h_minus_1(const MsParams &q, int j) {
   double s, c, sh, ch;
   sincos(th, &s, &c);
   sincos(0.5 * th, &sh, &ch);
-  return make_float2((float)(-2.0 * sh * sh), (float)s);
+  return make_float2((float)(-2.0 * sh * sh * scale), (float)(s * scale));
 }
 // Each slice is evaluated in delta form,
 //   X = psi + (T_z - 1) psi,   psi' = X + IFFT((H - 1) . FFT(X)),
@@ -202,14 +202,23 @@ struct RegFft {
 #pragma unroll
       for (int k = 1; k < R2; ++k) tw2[m][k - 1] = root(a * k, T);
     }
-    // (H - 1) / n of this thread's frequencies
+    __shared__ double red[32];
+    double g = 0.0;
+#pragma unroll
+    for (int k = 0; k < 15; ++k) g += modulus_less_1(tw1[k]);
+#pragma unroll
+    for (int m = 0; m < M2; ++m)
+#pragma unroll
+      for (int k = 0; k < R2 - 1; ++k) g += modulus_less_1(tw2[m][k]);
+    g = cta_sum(g, red) / N + (dft_gain(16) + dft_gain(R2) + dft_gain(R3));
+    const double scale = 1.0 / (N * (1.0 + g));
+    // (H - 1) / n of this thread's frequencies, less the transforms' gain
 #pragma unroll
     for (int m = 0; m < M3; ++m) {
       const int p = v + T * m, k1 = p / R2, k2 = p % R2;
 #pragma unroll
       for (int k3 = 0; k3 < R3; ++k3) {
-        const float2 w = ms_h_minus_1(q, k1 + 16 * k2 + 16 * R2 * k3);
-        h[m * R3 + k3] = make_float2(w.x * (1.f / N), w.y * (1.f / N));
+        h[m * R3 + k3] = ms_h_minus_1(q, k1 + 16 * k2 + 16 * R2 * k3, scale);
       }
     }
   }
@@ -404,7 +413,8 @@ static int ms_reg_launch(const MsParams &q, cudaStream_t st, int *ran) {
 template <int R0>
 constexpr int kMixThreads = R0 == 5 ? 640 : 512;  // n / R0 at most (625 = 3125 / 5)
 template <int R0, bool BACKWARD>
-__global__ void __launch_bounds__(kMixThreads<R0>) ms_mix_kernel(const MsParams q, const __grid_constant__ MixPlan pl) {
+__global__ void __launch_bounds__(kMixThreads<R0>) ms_mix_kernel(const MsParams q, const __grid_constant__ MixPlan pl,
+                                                                double gain) {
   extern __shared__ __align__(16) float2 fsm[];
   const int n = q.n, tid = threadIdx.x, nth = blockDim.x, str = pl.str[0];
   float2 *ts = fsm, *us = ts + n, *H = us + (BACKWARD ? n : 0), *tw = H + n, *buf = tw + pl.tw_total;
@@ -423,10 +433,13 @@ __global__ void __launch_bounds__(kMixThreads<R0>) ms_mix_kernel(const MsParams 
   };
   stage(BACKWARD ? q.L - 1 : 0);
   mix_twiddles(pl, tw, tid, nth);
-  const float s = 1.f / (float)n;
+  __syncthreads();
+  __shared__ double red[32];
+  gain += cta_sum(mix_twiddle_gain(pl, tw, tid, nth), red);
+  const double scale = 1.0 / (n * (1.0 + gain));
   for (int e = tid; e < n; e += nth) {
-    const float2 w = ms_h_minus_1(q, mix_frequency(pl, e));
-    H[e] = make_float2(s * w.x, BACKWARD ? -s * w.y : s * w.y);
+    const float2 w = ms_h_minus_1(q, mix_frequency(pl, e), scale);
+    H[e] = make_float2(w.x, BACKWARD ? -w.y : w.y);
   }
   float2 X[16], y[16];
   float2 *store = !BACKWARD && q.u_store ? q.u_store + p * q.nz * n + tid : nullptr;
@@ -513,7 +526,7 @@ static int ms_launch(const MsParams &q, cudaStream_t st) {
     const int threads = pl.threads < kMixThreads<R0> ? pl.threads : kMixThreads<R0>;
     const size_t smem = (size_t)((BACKWARD ? 3 : 2) * q.n + pl.tw_total + mix_pad(q.n) + 1) * sizeof(float2);
     TP_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    kern<<<q.P, threads, smem, st>>>(q, pl);
+    kern<<<q.P, threads, smem, st>>>(q, pl, mix_dft_gain(pl));
     return check_cuda(cudaGetLastError(), "multislice in-place kernel launch");
   };
   using std::integral_constant;

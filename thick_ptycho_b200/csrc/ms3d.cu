@@ -54,11 +54,16 @@ __global__ void ms3_twiddle_mix_kernel(const __grid_constant__ MixPlan pl, float
 }
 
 // (H - 1) / N at a * n2 + b, the axes of an in-place plan (stages > 0) by place instead
-// of frequency; H - 1 = exp(i th) - 1 = -2 sin^2(th/2) + i sin th.
+// of frequency; H - 1 = exp(i th) - 1 = -2 sin^2(th/2) + i sin th.  Less the transforms'
+// gain (fft.cuh): `gain` is the share of their constants, those of the twiddles are summed here.
 __global__ void ms3_kernel_h_kernel(int n1, int n2, const __grid_constant__ MixPlan p1, const __grid_constant__ MixPlan p2,
-                                    double k, double d1, double d2, double dz, float2 *hm1t) {
-  const int N = n1 * n2;
-  const double inv = 1.0 / (double)N;
+                                    const float2 *tw1, const float2 *tw2, double gain, double k, double d1, double d2,
+                                    double dz, float2 *hm1t) {
+  __shared__ double red[32];
+  const int N = n1 * n2, tid = threadIdx.x, nth = blockDim.x;
+  gain += cta_sum((p1.stages > 0 ? mix_twiddle_gain(p1, tw1, tid, nth) : four_twiddle_gain(n1, tw1, tid, nth)) +
+                        (p2.stages > 0 ? mix_twiddle_gain(p2, tw2, tid, nth) : four_twiddle_gain(n2, tw2, tid, nth)), red);
+  const double inv = 1.0 / ((double)N * (1.0 + gain));
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < N; e += gridDim.x * blockDim.x) {
     int a = e / n2, b = e % n2;
     if (p1.stages > 0) a = mix_frequency(p1, a);
@@ -522,7 +527,8 @@ static int ms3_run(const tp_ms3d_op *op, Ms3Params q, bool backward, void *works
   if (four_r) ms3_twiddle4_kernel<<<1, 256, 0, st>>>(four_r1(n2), four_r2(n2), w.tw2);
   else ms3_twiddle_mix_kernel<<<(n2 + 255) / 256, 256, 0, st>>>(p2, w.tw2);
   ms3_kernel_h_kernel<<<(q.N + 255) / 256 < 1184 ? (q.N + 255) / 256 : 1184, 256, 0, st>>>(
-      n1, n2, p1, p2, op->k, op->d1, op->d2, op->dz, w.hm1t);
+      n1, n2, p1, p2, w.tw1, w.tw2, (four_c ? four_dft_gain(n1) : mix_dft_gain(p1)) + (four_r ? four_dft_gain(n2) : mix_dft_gain(p2)),
+      op->k, op->d1, op->d2, op->dz, w.hm1t);
   TP_CHECK_CUDA(cudaGetLastError());
   // in-place kernels: rows and columns per CTA, about 4096 elements
   int rpc = 4096 / n2 < 16 ? 4096 / n2 : 16, lc = 4;
