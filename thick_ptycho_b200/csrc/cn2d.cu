@@ -51,6 +51,7 @@ namespace tp {
 // Warp path: 32 chunks (one per lane), 5 PCR levels, 13 records per chunk.
 constexpr int kRecMA = 0, kRecMC = 1, kRecAlpha = 2, kRecGamma = 7, kRecRDE = 12;
 constexpr int kMarchWarps = 4;
+constexpr int kMaxGridY = 65535;  // of a grid's y and z extents
 
 // Rows-per-lane values of the warp path with compiled kernels.
 static const int kRowSet[] = {1, 2, 3, 4, 6, 8, 12, 16, 24, 32, 48, 64};
@@ -563,12 +564,13 @@ __global__ void __launch_bounds__(kMarchWarps * 32, 1) cn2d_march_kernel(const M
 // runs along their own fast index through a tile of 32 offsets x 64 slices (1201 x 600
 // x 100: 384 us element by element, one side a gather; 311 with 32 slices, 265 with 64,
 // eight loads in flight per thread and 512-byte runs, 309 with 128 and fewer CTAs per
-// SM; the bytes alone take 179).  Grid (Npad / 32, ceil(nz / 64), P), block (32, 8).
+// SM; the bytes alone take 179).  Slices from `first` on; grid (Npad / 32, ceil(slices /
+// 64), P), block (32, 8).
 __global__ void __launch_bounds__(256) cn2d_unchunk_kernel(const cx *__restrict__ st, cx *__restrict__ out, int N, int nz,
-                                                           int M, int C, int pair) {
+                                                           int M, int C, int pair, int first) {
   __shared__ cx tile[64][33];
   const int Npad = C * M;
-  const int e0 = blockIdx.x * 32, t0 = blockIdx.y * 64;
+  const int e0 = blockIdx.x * 32, t0 = first + blockIdx.y * 64;
   const size_t pr = blockIdx.z;
   const auto row_of = [&](int e) {  // offset e holds row k M + i
     if (pair) return ((e >> 1) % C) * M + 2 * ((e >> 1) / C) + (e & 1);
@@ -819,8 +821,13 @@ static int factor_slices(const tp_cn2d_op *op, const void *n_field, int32_t n_dt
     TP_CHECK_CUDA(cudaMemsetAsync(f.coupling, 0, sizeof(unsigned), reinterpret_cast<cudaStream_t>(stream)));
   const size_t smem = 5 * (size_t)pt.C * sizeof(double2);
   const int count = s_end - s_begin + 1;
-  cn2d_diag_kernel<<<dim3(pt.C * pt.M / 32, (count + 31) / 32), dim3(32, 8), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      f, count);
+  FactorParams part = f;
+  for (int s0 = 0; s0 < count; s0 += 32 * kMaxGridY) {  // (one launch but for millions of slices)
+    const int n = count - s0 < 32 * kMaxGridY ? count - s0 : 32 * kMaxGridY;
+    part.sl0 = f.sl0 + s0;
+    cn2d_diag_kernel<<<dim3(pt.C * pt.M / 32, (n + 31) / 32), dim3(32, 8), 0, reinterpret_cast<cudaStream_t>(stream)>>>(
+        part, n);
+  }
   // this kernel and the march after it start early (pdl_wait): N = 256, 127 slices, 32
   // probes 100 -> 93 us for the factorisation, march and far field
   TP_CHECK_CUDA(launch_dependent(cn2d_factor_kernel, dim3(s_end - s_begin + 1), dim3(pt.C), smem,
@@ -962,14 +969,18 @@ extern "C" int tp_cn2d_unchunk(const tp_cn2d_op *op, int32_t num_probes, const v
   Partition pt;
   rc = partition_for(op->n, &pt);
   if (rc) return rc;
-  // the grid's z extent bounds the probes of one launch
+  // the grid's y and z extents bound the slices and probes of one launch
   const cx *src = static_cast<const cx *>(u_store);
   cx *dst = static_cast<cx *>(u_out);
-  for (int p0 = 0; p0 < num_probes; p0 += 65535) {
-    const int count = num_probes - p0 < 65535 ? num_probes - p0 : 65535;
-    cn2d_unchunk_kernel<<<dim3(pt.C * pt.M / 32, (op->nz + 63) / 64, count), dim3(32, 8), 0,
-                          reinterpret_cast<cudaStream_t>(stream)>>>(
-        src + (size_t)p0 * op->nz * pt.C * pt.M, dst + (size_t)p0 * op->nz * op->n, op->n, op->nz, pt.M, pt.C, pt.team);
+  for (int p0 = 0; p0 < num_probes; p0 += kMaxGridY) {
+    const int count = num_probes - p0 < kMaxGridY ? num_probes - p0 : kMaxGridY;
+    for (int first = 0; first < op->nz; first += 64 * kMaxGridY) {
+      const int n = op->nz - first < 64 * kMaxGridY ? op->nz - first : 64 * kMaxGridY;
+      cn2d_unchunk_kernel<<<dim3(pt.C * pt.M / 32, (n + 63) / 64, count), dim3(32, 8), 0,
+                            reinterpret_cast<cudaStream_t>(stream)>>>(src + (size_t)p0 * op->nz * pt.C * pt.M,
+                                                                      dst + (size_t)p0 * op->nz * op->n, op->n, op->nz,
+                                                                      pt.M, pt.C, pt.team, first);
+    }
   }
   return check_cuda(cudaGetLastError(), "cn2d_unchunk_kernel launch");
 }

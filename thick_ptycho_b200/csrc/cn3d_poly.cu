@@ -655,7 +655,8 @@ int poly_degree(double tau, double theta, double target, int max_m, float *a) {
 int c3_poly_march(const C3PolyJob &job, cudaStream_t st, int *ran) {
   *ran = 0;
   const int nf = job.nf, nb = job.nb, N = nf * nb, nz = job.nz, L = nz - 1, P = job.P;
-  if (nf > kPolyMaxSide || nb > kPolyMaxSide || job.tol < 4e-7) return TP_OK;
+  constexpr int kMaxSlices = 32 * 65535;  // of one launch over all slices
+  if (nf > kPolyMaxSide || nb > kPolyMaxSide || job.tol < 4e-7 || L > kMaxSlices) return TP_OK;
   const bool adj_exact = job.mode == TP_MODE_ADJOINT_EXACT;
   const size_t norms_bytes = ((size_t)L * P * sizeof(double2) + 255) & ~size_t(255);
   if (job.scratch_bytes < norms_bytes) return TP_OK;

@@ -26,6 +26,7 @@
 // Every wait is bounded and records kDevMbarTimeout instead of hanging.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
+#include <limits.h>
 #include <stdint.h>
 
 #include "cnn_internal.cuh"
@@ -530,16 +531,24 @@ struct FilterArgs {
   double *loss;
 };
 
-// y_v = z_v + sum_t F_t z_v(x + o_t).  Grid (tiles of columns, of rows, images * nsplit).
+// The CTA's tile of columns and of rows, and what is left of its index (the image and its part).
+__device__ __forceinline__ int filter_tile(int H, int W, int &c0, int &r0) {
+  const int gx = (W + kFtW - 1) / kFtW, gy = (H + kFtH - 1) / kFtH, row = blockIdx.x / gx;
+  c0 = (int)(blockIdx.x % gx) * kFtW;
+  r0 = row % gy * kFtH;
+  return row / gy;
+}
+
+// y_v = z_v + sum_t F_t z_v(x + o_t).  Grid (tiles of columns x of rows x images x nsplit).
 template <bool RESIDUAL>
 __global__ void __launch_bounds__(kFtThreads, 2) cnn_filter_kernel(const FilterArgs a) {
   __shared__ __align__(16) float2 sm[kFtStages][kFtSW * kFtSH];
   __shared__ double red[kFtThreads / 32];
-  const int img = blockIdx.z / a.nsplit, part = blockIdx.z % a.nsplit;
+  int c0, r0;
+  const int work = filter_tile(a.H, a.W, c0, r0), img = work / a.nsplit, part = work % a.nsplit;
   const int chunk = (a.per + a.nsplit - 1) / a.nsplit;
   const int v0 = img * a.per + part * chunk;
   const int v1 = min(min(v0 + chunk, (img + 1) * a.per), a.nvec);
-  const int c0 = blockIdx.x * kFtW, r0 = blockIdx.y * kFtH;
   const int c = c0 + threadIdx.x % kFtW, r = r0 + 2 * (threadIdx.x / kFtW);
   const bool ina = c < a.W && r < a.H, inb = c < a.W && r + 1 < a.H;
   const size_t hw = (size_t)a.H * a.W, at = (size_t)r * a.W + c;
@@ -611,13 +620,14 @@ __global__ void __launch_bounds__(kFtThreads, 2) cnn_filter_kernel(const FilterA
 // e_v = scale_v (y_v - target_v):  dF_t(x) = 2 sum_v conj(z_v(x + o_t)) e_v(x)
 // (d/dRe + i d/dIm), times out_scale (F = out_scale * last layer), written as
 // the 32-channel bf16 gradient of the last layer (channels 2t, 2t+1;
-// channels 26..31 zero).  Grid (tiles of columns, of rows, images).
+// channels 26..31 zero).  Grid (tiles of columns x of rows x images).
 __global__ void __launch_bounds__(kFtThreads, 2) cnn_filter_grad_kernel(const ConvGeom g, int per_image,
                                                                         const float2 *__restrict__ z,
                                                                         const float2 *__restrict__ e, float out_scale,
                                                                         bf16 *dy) {
   __shared__ __align__(16) float2 sm[kFtStages][kFtSW * kFtSH];
-  const int img = blockIdx.z, c0 = blockIdx.x * kFtW, r0 = blockIdx.y * kFtH;
+  int c0, r0;
+  const int img = filter_tile(g.H, g.W, c0, r0);
   const int c = c0 + threadIdx.x % kFtW, r = r0 + 2 * (threadIdx.x / kFtW);
   const bool ina = c < g.W && r < g.H, inb = c < g.W && r + 1 < g.H;
   const size_t hw = (size_t)g.H * g.W, at = (size_t)r * g.W + c;
@@ -675,6 +685,10 @@ static int max_smem_optin() {
   return v;
 }
 
+static long long filter_tiles(int nf, int nb) {
+  return (long long)((nf + kFtW - 1) / kFtW) * ((nb + kFtH - 1) / kFtH);
+}
+
 // Vectors of an image are split over CTAs until the grid holds about two waves.
 template <bool RESIDUAL>
 static int launch_filter(FilterArgs a, int nf, int nb, int nvec, int per_image, cudaStream_t st) {
@@ -684,12 +698,12 @@ static int launch_filter(FilterArgs a, int nf, int nb, int nvec, int per_image, 
   a.nvec = nvec;
   a.per = per_image > 0 ? per_image : nvec;
   a.np_img = (size_t)nf * nb * nimg;
-  const int gx = (nf + kFtW - 1) / kFtW, gy = (nb + kFtH - 1) / kFtH;
-  int split = 888 / (gx * gy * nimg);
+  const long long tiles = filter_tiles(nf, nb) * nimg;
+  long long split = 888 / tiles;
   if (split > (a.per + 3) / 4) split = (a.per + 3) / 4;
-  a.nsplit = split < 1 ? 1 : split;
-  if ((long long)nimg * a.nsplit > 65535 || gy > 65535) return set_error(TP_ERR_UNSUPPORTED, "filter: grid too large");
-  cnn_filter_kernel<RESIDUAL><<<dim3(gx, gy, nimg * a.nsplit), kFtThreads, 0, st>>>(a);
+  a.nsplit = split < 1 ? 1 : (int)split;
+  if (tiles * a.nsplit > INT_MAX) return set_error(TP_ERR_UNSUPPORTED, "filter: grid too large");
+  cnn_filter_kernel<RESIDUAL><<<(unsigned)(tiles * a.nsplit), kFtThreads, 0, st>>>(a);
   return check_cuda(cudaGetLastError(), "cnn_filter_kernel launch");
 }
 
@@ -851,9 +865,9 @@ extern "C" int tp_cnn_filter_grad(int32_t nf, int32_t nb, int32_t nimg, int32_t 
   const ConvGeom g = conv_geom(nb, nf, nimg);
   int rc = check_geom(g);
   if (rc != TP_OK) return rc;
-  if (nimg > 65535 || (nb + kFtH - 1) / kFtH > 65535) return set_error(TP_ERR_UNSUPPORTED, "tp_cnn_filter_grad: grid too large");
-  cnn_filter_grad_kernel<<<dim3((nf + kFtW - 1) / kFtW, (nb + kFtH - 1) / kFtH, nimg), kFtThreads, 0,
-                           reinterpret_cast<cudaStream_t>(stream)>>>(
+  const long long tiles = filter_tiles(nf, nb) * nimg;
+  if (tiles > INT_MAX) return set_error(TP_ERR_UNSUPPORTED, "tp_cnn_filter_grad: grid too large");
+  cnn_filter_grad_kernel<<<(unsigned)tiles, kFtThreads, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
       g, per_image, static_cast<const float2 *>(z), static_cast<const float2 *>(e), out_scale, static_cast<bf16 *>(dy));
   return check_cuda(cudaGetLastError(), "cnn_filter_grad_kernel launch");
 }
