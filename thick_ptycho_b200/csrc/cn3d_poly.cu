@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(256) c3_poly_slices_kernel(const PolySlices q,
       if (sum > 0.f) {
         const float dr = 1.f - d.x, di = -d.y;
         const float n = sqrtf(dr * dr + di * di), t = sum / n;
-        if (!(t < 1e6f)) bad = 1;
+        if (!(t < 1e6f && n < 1e12f)) bad = 1;  // (an infinite D would pass as t = 0)
         tau = fmaxf(tau, t);
         inv = fmaxf(inv, 1.f / n);
         // what row i's element reaches: its neighbours' couplings back to it
