@@ -134,9 +134,6 @@ typedef struct tp_cn2d_march_args {
                                 initial state is not stored; needs
                                 store_every <= 1); ADJOINT_EXACT reads u_fwd as
                                 such sums (one slice per step instead of two) */
-  int32_t state_slices;      /* slices per probe of the stored field that state_in
-                                is a slice of: probe p's state is p state_slices
-                                Npad after it (0 or 1: state_in is (P, Npad))  */
 } tp_cn2d_march_args;
 
 /* Partition of N rows into `chunks` chunks of `rows_per_chunk` rows (padded
@@ -184,6 +181,11 @@ TP_API int tp_copy_columns(void *dst, const void *src, int64_t rows, int64_t row
  */
 TP_API int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp_cn2d_march_args *args,
                   tp_stream_t stream);
+/* The same from a slice of a stored field: args->state_in is that slice of the
+ * first probe's field, `state_slices` (at least 1) the slices per probe: probe
+ * p's state is p state_slices Npad entries after it. */
+TP_API int tp_cn2d_march_from(const tp_cn2d_op *op, const void *factors, const tp_cn2d_march_args *args,
+                              int32_t state_slices, tp_stream_t stream);
 
 /*
  * Map the per-step gradient sum_p lambda_s conj(u_s + u_{s-1}) (L, Npad,

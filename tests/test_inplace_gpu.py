@@ -161,20 +161,26 @@ def test_2d_verdicts_follow_the_factorised_slices():
 
 @pytest.mark.parametrize("N", [97, 1024])
 def test_2d_march_arguments_refused(N):
-    """store_sums is 0 or 1; the stride of state_in is a field of its own."""
+    """store_sums is 0 or 1; the stride of state_in is an argument of its own entry."""
     rng = np.random.default_rng(N)
     eng = CN2D(N, 5, K, 1.0, 1.0, "impedance")
     fs = eng.factor(index(rng, N, 5), "forward")
     state = torch.zeros((2, 3, eng.npad), dtype=torch.complex64, device="cuda")
-    for sums, slices, with_state, ok in [(0, 0, True, True), (0, 3, True, True), (0, 3, False, False), (0, -1, True, False),
-                                         (2, 0, True, False), (-1, 0, True, False), (256, 0, True, False),
-                                         (768, 0, True, False), (1, 0, True, N == 1024)]:
+    for sums, slices, with_state, ok in [(0, None, True, True), (0, None, False, True), (0, 3, True, True),
+                                         (0, 1, True, True), (0, 3, False, False), (0, 0, True, False),
+                                         (0, -1, True, False), (2, None, True, False), (-1, None, True, False),
+                                         (256, None, True, False), (768, None, True, False), (768, 3, True, False),
+                                         (1, None, True, N == 1024), (1, 3, True, N == 1024)]:
         a = _native.TpCn2dMarchArgs()
         a.num_probes, a.mode, a.t_begin, a.t_end = 2, _native.MODE_FORWARD, 2, 3
-        a.store_sums, a.state_slices = sums, slices
+        a.store_sums = sums
         if with_state:
             a.state_in = ctypes.c_void_p(state.data_ptr())
-        rc = eng.lib.tp_cn2d_march(ctypes.byref(eng.op()), ctypes.c_void_p(fs.buf.data_ptr()), ctypes.byref(a), None)
+        op, buf = eng.op(), ctypes.c_void_p(fs.buf.data_ptr())
+        if slices is None:
+            rc = eng.lib.tp_cn2d_march(ctypes.byref(op), buf, ctypes.byref(a), None)
+        else:
+            rc = eng.lib.tp_cn2d_march_from(ctypes.byref(op), buf, ctypes.byref(a), slices, None)
         assert (rc == 0) == ok, (sums, slices, with_state, rc)
     torch.cuda.synchronize()
 

@@ -76,7 +76,6 @@ class TpCn2dMarchArgs(ctypes.Structure):
         ("ufwd_slices", ctypes.c_int32),
         ("ufwd_base", ctypes.c_int32),
         ("store_sums", ctypes.c_int32),
-        ("state_slices", ctypes.c_int32),
     ]
 
 
@@ -175,6 +174,8 @@ SIGNATURES = [
                                        ctypes.c_int64, ctypes.c_int64, ctypes.c_void_p]),
     ("tp_cn2d_march", ctypes.c_int, [ctypes.POINTER(TpCn2dOp), ctypes.c_void_p, ctypes.POINTER(TpCn2dMarchArgs),
                                      ctypes.c_void_p]),
+    ("tp_cn2d_march_from", ctypes.c_int, [ctypes.POINTER(TpCn2dOp), ctypes.c_void_p, ctypes.POINTER(TpCn2dMarchArgs),
+                                          ctypes.c_int32, ctypes.c_void_p]),
     ("tp_cn2d_grad_to_n", ctypes.c_int, [ctypes.POINTER(TpCn2dOp), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int32,
                                          ctypes.c_void_p, ctypes.c_void_p]),
     ("tp_cn2d_grad_to_n_range", ctypes.c_int, [ctypes.POINTER(TpCn2dOp), ctypes.c_void_p, ctypes.c_void_p,

@@ -197,9 +197,12 @@ class CN2D:
                     not 0 <= index < store.shape[1]:
                 raise ValueError("state_from must be a chunked field (P, slices, Npad) and one of its slices")
             a.state_in = ctypes.c_void_p(store.data_ptr() + index * self.npad * store.element_size())
-            a.state_slices = store.shape[1]
         o = self.op()
-        rc = self.lib.tp_cn2d_march(ctypes.byref(o), _ptr(fs.buf), ctypes.byref(a), _stream(self.device))
+        if state_from is not None:
+            rc = self.lib.tp_cn2d_march_from(ctypes.byref(o), _ptr(fs.buf), ctypes.byref(a), store.shape[1],
+                                             _stream(self.device))
+        else:
+            rc = self.lib.tp_cn2d_march(ctypes.byref(o), _ptr(fs.buf), ctypes.byref(a), _stream(self.device))
         _native.check(rc, "tp_cn2d_march", self.lib)
 
     # ------------------------------------------------------------ helpers

@@ -860,8 +860,8 @@ extern "C" int tp_copy_columns(void *dst, const void *src, int64_t rows, int64_t
                     "tp_copy_columns");
 }
 
-extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp_cn2d_march_args *a,
-                             tp_stream_t stream) {
+static int march_from(const tp_cn2d_op *op, const void *factors, const tp_cn2d_march_args *a, int state_slices,
+                      tp_stream_t stream) {
   int rc = validate_op(op);
   if (rc) return rc;
   if (a == nullptr || factors == nullptr) return set_error(TP_ERR_INVALID, "args/factors is NULL");
@@ -909,9 +909,7 @@ extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp
   if (mp.flip_out && (mp.t0 != 1 || mp.t1 != mp.L) && a->u_store != nullptr)
     return set_error(TP_ERR_INVALID, "the flipped ADJOINT store needs the full step range");
   mp.state_in = static_cast<const cx *>(a->state_in);
-  if (a->state_slices < 0 || (a->state_slices > 0 && a->state_in == nullptr))
-    return set_error(TP_ERR_INVALID, "state_slices=%d needs state_in", a->state_slices);
-  mp.state_stride = (size_t)(a->state_slices > 0 ? a->state_slices : 1) * mp.Npad;
+  mp.state_stride = (size_t)state_slices * mp.Npad;
   mp.state_out = static_cast<cx *>(a->state_out);
   mp.store_slices = a->store_slices > 0 ? a->store_slices : op->nz;
   mp.store_every = a->store_every;
@@ -959,6 +957,18 @@ extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp
   }
 #endif
   return launch_march(pt.M, mp, op->n == pt.C * pt.M, lagged, reinterpret_cast<cudaStream_t>(stream));
+}
+
+extern "C" int tp_cn2d_march(const tp_cn2d_op *op, const void *factors, const tp_cn2d_march_args *a,
+                             tp_stream_t stream) {
+  return march_from(op, factors, a, 1, stream);
+}
+
+extern "C" int tp_cn2d_march_from(const tp_cn2d_op *op, const void *factors, const tp_cn2d_march_args *a,
+                                  int32_t state_slices, tp_stream_t stream) {
+  if (a == nullptr || a->state_in == nullptr || state_slices < 1)
+    return set_error(TP_ERR_INVALID, "tp_cn2d_march_from: needs state_in and state_slices >= 1 (%d)", state_slices);
+  return march_from(op, factors, a, state_slices, stream);
 }
 
 extern "C" int tp_cn2d_unchunk(const tp_cn2d_op *op, int32_t num_probes, const void *u_store, void *u_out,
