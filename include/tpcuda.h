@@ -446,8 +446,11 @@ typedef struct tp_cn3d_march_args {
                                 (from the previous march with it, e.g. the
                                 forward before the adjoint): the network is not
                                 run again                                       */
-  int32_t kernels;           /* kernel choice, the same arithmetic either way
-                                (0 = automatic).  Bit 0: the preconditioner
+  int32_t kernels;           /* kernel choice (0 = automatic).  Bits 1 and 2 keep
+                                the arithmetic; bits 0 and 3 choose the method,
+                                whose results differ by round-off (bit 0) or
+                                within the tolerance, with other iteration
+                                counts (bit 3).  Bit 0: the preconditioner
                                 always by the shared-memory Stockham transforms
                                 (automatic: on tiles by a polynomial that equals
                                 it to 1e-7 where nf is even and the couplings

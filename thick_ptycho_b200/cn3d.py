@@ -60,11 +60,12 @@ class CN3D:
         # 0: each march runs as one CUDA graph with device-side step and
         # iteration loops; 1: step by step (host loop)
         self.launch = 0
-        # kernel choice (tp_cn3d_march_args.kernels; the same arithmetic):
-        # 0 = automatic; bit 0 = the preconditioner by Stockham transforms always, bit 1 = the
-        # stencil kernels with per-thread loads instead of tensor-memory copies,
-        # bit 2 = the learned filter by register shuffles instead of bulk-staged rows,
-        # bit 3 = the Krylov march also where a fixed polynomial solves each slice
+        # kernel choice (tp_cn3d_march_args.kernels): 0 = automatic.  The same arithmetic:
+        # bit 1 = the stencil kernels with per-thread loads instead of tensor-memory copies,
+        # bit 2 = the learned filter by register shuffles instead of bulk-staged rows.
+        # Another method: bit 0 = the preconditioner by Stockham transforms always (not by a
+        # polynomial on tiles, equal to 1e-7), bit 3 = the Krylov march also where a fixed
+        # polynomial solves each slice
         self.kernels = 0
 
     def op(self, is_delta=False) -> _native.TpCn3dOp:

@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(kPThreads, 3) c3_prec_tile_kernel(const __grid
 // four: the transform has register four-step kernels.  Those are the faster ones
 // once the halo grows past 6 pixels (mu > 0.046): a preconditioned march of 256 x
 // 256, 64 probes takes 453 us per step on tiles and 510 by transforms at mu = 0.02
-// (m = 6, halo 5), 477 and 522 at 0.044 (m = 8, halo 6), 562 and 541 at 0.061 (m = 8,
+// (m = 6, halo 5), 477 and 522 at 0.044 (m = 8, halo 6), 562 and 541 at 0.061 (m = 10,
 // halo 7).  The shared-memory transforms are slower at every mu in reach (150 x 150:
 // 225 and 385 us at 0.02, 255 and 393 at 0.051).
 static PrecTile prec_tile_plan(const C3Params &q, bool four) {
@@ -2153,9 +2153,9 @@ extern "C" int tp_cn3d_march(const tp_cn3d_op *op, const void *n_field, int32_t 
 #ifndef TP_C128_CHECK
   // Plain marches whose operator is a small perturbation of the identity (the
   // paraxial sampling) solve each slice by a fixed polynomial, one kernel per
-  // step (cn3d_poly.cu): 256 x 256, 64 probes 43 us per step against 453 of the Krylov
-  // march at mu = 0.02 (m = 6), 74 against 548 at 0.051 (m = 8), 90 x 76, 9 probes 10
-  // against 117; where degree 10 no longer reaches the tolerance (mu > 0.08), training
+  // step (cn3d_poly.cu): 256 x 256, 64 probes 45 us per step against 453 of the Krylov
+  // march at mu = 0.02 (m = 6), 73 against 548 at 0.051 (m = 10), 90 x 76, 9 probes 8
+  // against 115; where degree 10 no longer reaches the tolerance (mu > 0.063), training
   // pairs, step-by-step launches, a capturing stream, REVERSE, other kernel choices and
   // tolerances under complex64 round-off keep the Krylov march below.
   cudaStreamCaptureStatus poly_cap = cudaStreamCaptureStatusNone;

@@ -34,13 +34,15 @@
 // residual, as in the Krylov march, but tile by tile with the tile's own d in its halo:
 // what the halo leaves out does not show in it.
 //
-// 256 x 256, 64 probes, m = 6: a forward step to the exit 42.7 us, keeping the field
-// 44.7; forward and exact adjoint with the gradient over 255 slices 191 -> 30 ms against
-// the Krylov march with transforms (90 x 75 x 48, 9 probes, forward: 6.5 -> 0.35 ms).
-// About 12 us of a step is issue and 5 us the stored field's bytes; the rest is the
-// latency of the half-sweeps' exchanges with 16 warps per SM.  Four rows per warp and 12,
-// 14 or 16 warps per CTA (80, 72, 64 registers) take 55.8, 57.4 and 53.8 us: twice the
-// exchanges, and taller halos where the tile shrinks.
+// 256 x 256, 64 probes, m = 6: a forward step to the exit 45.4 us, keeping the field
+// 47.6, an exact adjoint step with the gradient 58.6; both marches over 255 slices 191 ->
+// 27.4 ms against the Krylov march with transforms (90 x 75 x 48, 9 probes, forward: 6.5 ->
+// 0.37 ms).  The schedulers issue in 52 % of a step's cycles and DRAM is 11 % busy; a warp
+// waits for the fixed latency of its own arithmetic, for shared memory and shuffles and at
+// the exchanges' barriers, about one issue's time each, with 16 warps per SM to cover it.
+// Four rows per warp and 12, 14 or 16 warps per CTA (80, 72, 64 registers) were slower
+// (55.8, 57.4 and 53.8 us against 42.7 with fp32 norms): twice the exchanges, and taller
+// halos where the tile shrinks.
 #include <cuda.h>
 #include <math.h>
 #include <string.h>

@@ -232,10 +232,10 @@ __device__ __forceinline__ void fft_pass(const cx *a, cx *b, int n, int Ns, uint
 }
 
 // ------------------------------------------------------ fixed-size plans
-// The same passes with the length and the radix sequence known at compile
-// time, so that every index division and modulo is by a constant.  Used by
-// the 3D preconditioner for the common transverse sizes.
-// Padded shared-memory layout of the fixed-size transforms: element i of a
+// The passes with the length and the radix sequence known at compile time, so that
+// every index division and modulo is by a constant: the Stockham form of the 3D
+// preconditioner at the common transverse sizes, in a padded shared-memory layout.
+// Element i of a
 // transform sits at i + i/8 (one spare slot per 8 elements) and transform bi
 // starts at bi * S, S = N + N/8 + 1.  The Stockham writes of the early passes
 // (stride R elements) and column transposes (stride S) then spread over the

@@ -1,6 +1,6 @@
-// Batched 1D FFTs, far-field / amplitude-loss heads and the 2D multislice
-// (angular-spectrum) march with its adjoint, all on the shared-memory FFT of
-// fft.cuh.
+// Batched 1D FFTs and far-field / amplitude-loss heads on the shared-memory FFT of
+// fft.cuh, and the 2D multislice (angular-spectrum) march with its adjoint on register
+// and in-place transforms.
 //
 // Replaces: numpy.fft in the far field (forward_model/base/base_solver.py:
 // 234-242) and the phase-retrieval projection (reconstruction/
@@ -408,8 +408,8 @@ static int ms_reg_launch(const MsParams &q, cudaStream_t st, int *ran) {
 // own arithmetic and the next forward transform's first stage need no exchange between
 // them; the last forward stage, the product with H - 1 and the first inverse one are a
 // single pass.  A slice is 2 (stages - 1) barriers, against two per pass and four more of
-// Stockham passes in shared memory: 64 probes, n = 1500 (10 10 15): 9.1 -> 3.1 us per slice
-// with the field kept, the adjoint 9.7 -> 3.4 (1000: 6.0 -> 2.4; 243, 32 probes: 4.1 -> 1.9).
+// Stockham passes in shared memory: 64 probes, n = 1500 (10 10 15): 9.1 -> 3.3 us per slice
+// with the field kept, the adjoint 9.7 -> 3.8 (1000: 6.0 -> 2.6; 243, 32 probes: 4.1 -> 1.9).
 template <int R0>
 constexpr int kMixThreads = R0 == 5 ? 640 : 512;  // n / R0 at most (625 = 3125 / 5)
 template <int R0, bool BACKWARD>
