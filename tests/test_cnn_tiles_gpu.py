@@ -125,3 +125,29 @@ def test_training_step_operands():
             m.loss_and_grads(d, z, *bad, per)
     with pytest.raises(RuntimeError):
         m.loss_and_grads(d, z.cpu(), t, sc, per)
+
+
+@pytest.mark.parametrize("nf,nb", [(1, 1), (2, 3), (5, 2), (65, 9)])
+def test_filter_taps_that_leave_the_image(nf, nb):
+    """They have no part in the sum, whatever the filter holds there."""
+    rng = np.random.default_rng(nf)
+    dy = [0, 0, 0, -1, 1, -1, -1, 1, 1, 0, 0, -2, 2]
+    dx = [0, -1, 1, 0, 0, -1, 1, -1, 1, -2, 2, 0, 0]
+    y, x = np.mgrid[:nb, :nf]
+    F = cplx(rng, 13, nb, nf).astype(np.complex64)
+    for t in range(13):
+        out = (y + dy[t] < 0) | (y + dy[t] >= nb) | (x + dx[t] < 0) | (x + dx[t] >= nf)
+        F[t][out] = 0
+    hole = F.copy()
+    hole[F == 0] = np.nan
+    z, t = c64(cplx(rng, 2, nb * nf)), c64(cplx(rng, 2, nb * nf))
+    res = []
+    for f in (F, hole):
+        f, a, e = c64(f.reshape(13, -1)), torch.empty_like(z), torch.empty_like(z)
+        loss, sc = torch.zeros(1, dtype=torch.float64, device="cuda"), torch.ones(2, device="cuda")
+        assert LIB.tp_cnn_filter_apply(nf, nb, 2, 0, 0, ptr(f), ptr(z), ptr(a), stream()) == 0
+        assert LIB.tp_cnn_filter_residual(nf, nb, 2, 0, ptr(f), ptr(z), ptr(t), ptr(sc), ptr(e), ptr(loss), stream()) == 0
+        res.append((a, e, loss))
+    assert torch.isfinite(torch.view_as_real(res[1][0])).all()
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+    assert abs(float(res[0][2]) - float(res[1][2])) <= 1e-12 * float(res[0][2])

@@ -562,6 +562,17 @@ __global__ void __launch_bounds__(kFtThreads, 2) cnn_filter_kernel(const FilterA
     wa[t] = make_float2(fa.x, cs * fa.y);
     wb[t] = make_float2(fb.x, cs * fb.y);
   }
+  if (c0 < 2 || r0 < 2 || c0 + kFtW + 2 > a.W || r0 + kFtH + 2 > a.H) {
+    // a tap that leaves the image has no part in the sum, whatever its filter holds
+    constexpr int dy[kFilterTaps] = {0, 0, 0, -1, 1, -1, -1, 1, 1, 0, 0, -2, 2};
+    constexpr int dx[kFilterTaps] = {0, -1, 1, 0, 0, -1, 1, -1, 1, -2, 2, 0, 0};
+#pragma unroll
+    for (int t = 0; t < kFilterTaps; ++t) {
+      const int y = r + dy[t], x = c + dx[t];
+      if (x < 0 || x >= a.W || y < 0 || y >= a.H) wa[t] = make_float2(0.f, 0.f);
+      if (x < 0 || x >= a.W || y + 1 < 0 || y + 1 >= a.H) wb[t] = make_float2(0.f, 0.f);
+    }
+  }
   double loss = 0.0;
   const float2 zero = make_float2(0.f, 0.f);
   float2 ta = zero, tb = zero;
