@@ -57,7 +57,7 @@ def test_2d_slice_by_slice_in_place(N, P, mode):
     eng.device_status()
 
 
-@pytest.mark.parametrize("N,P", [(97, 40), (777, 20), (2047, 9)])
+@pytest.mark.parametrize("N,P", [(97, 40), (777, 20), (2047, 9), (97, 310), (1024, 5)])
 def test_2d_one_slice_exit_on_its_input(N, P):
     rng = np.random.default_rng(N + 1)
     eng = CN2D(N, 2, K, 1.0, 1.0, "impedance")
